@@ -11,8 +11,8 @@ Printed (one JSON line, rank 0):
   e2e        the same metric through the C-ABI from pinned host buffers: per step the poses and
              ligand go host->device, the energies come back device->host
   roofline   the exact kernel against the FP32 peak (SMs x 128 lanes x 2 x clock), using the
-             reference's own operation count (30 per interaction + 18 per pose and ligand atom +
-             28 per pose, src/main.cpp:359)
+             reference's own operation count (30 per pair + 18 per pose and ligand atom + 28 per
+             pose, src/main.cpp:359) for the pairs that lie within their cut-offs
   cpu_baseline  the oracle's FP32 restatement of the reference kernel (OpenMP, -O3 -ffast-math as
              the reference's release build) on a bounded sample of the same deck, all host cores
   parity     the timed launch's energies against the reference's own energies for the deck's first
@@ -45,7 +45,7 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 from minibude_gb300 import LARGE, SMALL, synthetic_deck  # noqa: E402
-from minibude_gb300.validate import algorithmic_flops, reference_formula_flops  # noqa: E402
+from minibude_gb300.validate import interacting_share, reference_formula_flops  # noqa: E402
 
 METRIC = "exact GInteractions/s"
 UNIT = "GInteractions/s"
@@ -64,8 +64,7 @@ def parse_args():
                          "2M poses of 512 ligands (938-atom protein), score 64 held-out ligands x 65536 poses; screen: "
                          "1024 ligands (16-80 atoms) x 16384 poses against the bm2 protein, surrogate-screened vs "
                          "batched exhaustive exact; sweep: the reference driver's PPWI x wgsize sweep on the "
-                         "4096 x 64 x 1M deck, each shape with the wave model's protein split, against the "
-                         "autotuner's pick")
+                         "4096 x 64 x 1M deck against the autotuner's pick")
     ap.add_argument("--epochs", type=int, default=80, help="surrogate training epochs (surrogate/screen workloads)")
     ap.add_argument("--grid-spacing", type=float, default=1.25,
                     help="spacing in A of the surrogate's protein-field grid (surrogate/screen workloads)")
@@ -293,9 +292,12 @@ def run_ours(args, dist: Dist):
     interactions = deck.interactions
     value = dist.world * interactions / (step_ms_max * 1e-3) / 1e9
 
-    # Roofline of the exact kernel (the dominant kernel: the transform kernel is ~0.01% of a step).
+    # Roofline of the exact kernel (the dominant kernel: the transform kernel is ~0.3% of a step).
+    # `value` counts every pair of a pose, as the reference does; the kernel leaves out the pairs that
+    # lie past all three cut-offs (they add exactly zero), so its own work is the interacting pairs.
     exact_s = float(np.mean(exact_ms)) * 1e-3
-    flops = algorithmic_flops(deck.nposes, deck.natlig, deck.natpro)
+    share = interacting_share(deck)
+    flops = 30.0 * share * deck.interactions + 18.0 * deck.nposes * deck.natlig + 28.0 * deck.nposes
     achieved = flops / exact_s / 1e12
     sms = _sm_count(dist.local_rank)
     sm_max = float(peaks.get("sm_max_mhz", 2070.0))
@@ -304,20 +306,14 @@ def run_ours(args, dist: Dist):
             "frac": round(achieved / peak, 4),
             "peak_source": f"{sms} SMs x 128 FP32 lanes x 2 x {sm_max:.0f} MHz (sm_max_mhz of MEASURED_PEAKS.json); "
                            "no measured FP32 peak exists, so this is the nominal peak at the measured max clock",
-            "work": "30 FLOP/interaction + 18/(pose, ligand atom) + 28/pose (src/main.cpp:359)",
-            "kernel": "exact_kernel", "kernel_ms": round(exact_s * 1e3, 4),
-            "traffic": traffic_per_launch(deck.nposes),
-            # the reference's PPWI-dependent count (src/main.cpp:359), for a like-for-like GFLOP/s
+            "work": "30 FLOP per pair within its cut-offs + 18/(pose, ligand atom) + 28/pose (src/main.cpp:359)",
+            "interacting_share": float("%.4g" % share),
+            "kernel": "cull_kernel", "kernel_ms": round(exact_s * 1e3, 4),
+            # every pair counted, evaluated or not (src/main.cpp:359), for a like-for-like GFLOP/s
             "gflops_reference_formula": round(
                 reference_formula_flops(deck.nposes, deck.natlig, deck.natpro, cfg.ppwi) / exact_s / 1e9, 1)}
     if clk.get("sm_mhz"):
         roof["frac_at_sampled_clock"] = round(achieved / (sms * 128 * 2 * clk["sm_mhz"] * 1e6 / 1e12), 4)
-    # The hardware's view: the kernel issues 12 FP32-pipe lane operations per interaction (paired
-    # sub/mul/fma for the distance and the accumulation, three saturating FMAs; the square root is
-    # on the XU pipe), against the reference's count of 30 FLOP, so `frac` can pass 1.0 while the
-    # FMA pipe is not saturated.  fma_pipe_frac = interactions/s x 12 / (SMs x 128 lanes x clock).
-    roof["fp32_pipe_ops_per_interaction"] = 12
-    roof["fma_pipe_frac"] = round(deck.interactions / exact_s * 12 / (sms * 128 * sm_max * 1e6), 4)
 
     out = {"metric": METRIC, "value": round(value, 3), "unit": UNIT, "n_gpus": dist.world, "steps": args.steps,
            "warmup": args.warmup, "ms_per_step": round(step_ms_max, 4), "higher_is_better": True,
@@ -405,8 +401,8 @@ def bm2_protein():
 
 
 def run_batch(args, dist: Dist):
-    """Batched ragged scoring: one persistent CUDA-graph launch for all ligands, next to one plain
-    launch per ligand (reported in config.per_ligand)."""
+    """Batched ragged scoring: one CUDA-graph launch for all ligands, next to one plain launch per
+    ligand (reported in config.per_ligand)."""
     from minibude_gb300 import BATCH, build, synthetic_batch
     from minibude_gb300.model import GpuContext
     build.build_library()
@@ -433,11 +429,9 @@ def run_batch(args, dist: Dist):
     clk = clocks.summary(peaks.get("sm_max_mhz", 2070.0))
     step_ms = dist.max(float(np.mean(ms)))
     inter = batch.interactions
-    # One plain launch per ligand, at the best of a few shapes: the batch's own, and shapes that
-    # cut each ligand's launch into more blocks (fewer poses per block, protein slices).
+    # One plain launch per ligand, at the best of a few shapes: the batch's own, and smaller blocks.
     from minibude_gb300.model import launch_cfg as _lc
-    pl_cands = [cfg, _lc(8, 128, 1, 64, 2), _lc(4, 128, 4, 64, 2, cluster=0), _lc(16, 128, 8, 64, 1, cluster=0),
-                _lc(8, 64, 4, 64, 2, cluster=1)]
+    pl_cands = [cfg, _lc(4, 512, 1, 64, 2), _lc(4, 256, 1, 64, 2), _lc(2, 512, 1, 64, 2), _lc(2, 256, 1, 64, 2)]
     pl_t = []
     for c in pl_cands:
         ctx.run_batch(c, per_ligand=True)
@@ -447,8 +441,9 @@ def run_batch(args, dist: Dist):
     pl_ms = float(np.mean(ms_pl))
     sms = _sm_count(dist.local_rank)
     sm_max = float(peaks.get("sm_max_mhz", 2070.0))
-    flops = sum(30.0 * len(l) * p.shape[1] * batch.natpro + 18.0 * len(l) * p.shape[1] + 28.0 * p.shape[1]
-                for l, p in zip(batch.ligands, batch.poses))
+    flops = sum(30.0 * interacting_share(batch.deck(k), 8) * len(l) * p.shape[1] * batch.natpro +
+                18.0 * len(l) * p.shape[1] + 28.0 * p.shape[1]
+                for k, (l, p) in enumerate(zip(batch.ligands, batch.poses)))
     achieved = flops / (step_ms * 1e-3) / 1e12
     peak = sms * 128 * 2 * sm_max * 1e6 / 1e12
     out = {"metric": "batched exact GInteractions/s", "value": round(dist.world * inter / (step_ms * 1e-3) / 1e9, 3),
@@ -457,7 +452,7 @@ def run_batch(args, dist: Dist):
            "dtype": "f32", "data": "synthetic ligands and poses (seeded) against the reference's bm2 protein",
            "config": {"workload": BATCH.name, "nligands": batch.nligands, "total_poses": batch.total_poses,
                       "natpro": batch.natpro, "ntypes": batch.ntypes, "launch": cfg.as_dict(),
-                      "mode": "one persistent kernel in a CUDA graph (counter reset + transforms + kernel)",
+                      "mode": "one CUDA graph over all ligands (transforms, exact kernel, sums over the atoms)",
                       "per_ligand": {"ms_per_step": round(pl_ms, 4),
                                      "value": round(inter / (pl_ms * 1e-3) / 1e9, 3),
                                      "launches_per_step": 1 + batch.nligands, "launch": pl_cfg.as_dict(),
@@ -466,10 +461,10 @@ def run_batch(args, dist: Dist):
                       "parallelism": f"replicas x{dist.world}"},
            "gpu_launches": launches, "clocks": clk,
            "roofline": {"bound": "fp32", "achieved": round(achieved, 3), "peak": round(peak, 3), "unit": "TFLOP/s",
-                        "frac": round(achieved / peak, 4), "kernel": "batch_kernel",
-                        "work": "30 FLOP/interaction + 18/(pose, ligand atom) + 28/pose (src/main.cpp:359)",
+                        "frac": round(achieved / peak, 4), "kernel": "cull_kernel",
+                        "work": "30 FLOP per pair within its cut-offs + 18/(pose, ligand atom) + 28/pose "
+                                "(src/main.cpp:359)",
                         "peak_source": f"{sms} SMs x 128 x 2 x {sm_max:.0f} MHz (nominal at sm_max_mhz)",
-                        "traffic": traffic_per_launch(batch.total_poses, "batch_kernel"),
                         "gflops_reference_formula": round(sum(
                             reference_formula_flops(p.shape[1], len(l), batch.natpro, cfg.ppwi)
                             for l, p in zip(batch.ligands, batch.poses)) / (step_ms * 1e-3) / 1e9, 1)}}
@@ -628,12 +623,7 @@ def run_screen(args, dist: Dist):
     ex_ms = [ctx.run_batch(cfg) for _ in range(max(2, args.steps // 2))]
     exact = ctx.download_batch()
     exhaustive_ms = float(np.mean(ex_ms))
-    # The screen's exact kernel: the exhaustive shape with the protein cut into 21 slices of 128
-    # records staged 32 at a time, so the rescoring's few hundred poses per ligand still spread over
-    # every block slot (measured on this batch, rescoring with 14 poses per thread: 22.9 ms at 21
-    # slices x 32-record stages, 23.1 at 16 x 32 or 21 x 64, 23.8 at 16 x 64, 25.8 at 8 x 64).
-    from minibude_gb300.capi import BudeLaunchCfg
-    scfg = BudeLaunchCfg(cfg.ppwi, cfg.wgsize, 21, 32, cfg.unroll, 0)
+    scfg = cfg  # the fallback's shape; the rescoring's follows from the picks per ligand
     for _ in range(max(args.warmup, 1)):
         ctx.screen(scfg, top_frac=0.02, audit_frac=0.005, audit_tol=0.05, seed=7)
     launches0 = ctx.launch_count()
@@ -716,9 +706,8 @@ def run_screen(args, dist: Dist):
 
 def run_sweep(args, dist: Dist):
     """The reference driver's brute-force search (src/main.cpp:517-541: every PPWI x wgsize) on the
-    4096 x 64 x 1M deck, each (PPWI, wgsize) with the wave model's protein split in both reduction
-    modes and unsplit, timed like the headline (L2 flushed, CUDA events); the autotuner's pick is
-    timed the same way.  PPWI 32, 64 and 128 run as 16 poses per thread (the register bound)."""
+    4096 x 64 x 1M deck, at 2 and 4 poses per lane, timed like the headline (L2 flushed, CUDA events);
+    the autotuner's pick is timed the same way."""
     from minibude_gb300 import build
     from minibude_gb300.model import GpuContext, launch_cfg
     build.build_library()
@@ -737,16 +726,8 @@ def run_sweep(args, dist: Dist):
     rows = []
     for p in (1, 2, 4, 8, 16):
         for w in (64, 128, 256, 512):
-            base = ctx.default_cfg(p, w)  # wave-model split, global reduction
-            shapes = {(base.split, 0)}
-            if base.split > 1:
-                shapes.add((1, 0))
-                if base.split <= 8:
-                    shapes.add((base.split, 1))
-            for split, cl in sorted(shapes):
-                cfg = launch_cfg(p, w, split, base.tile, base.unroll, cluster=cl)
-                rows.append({"ppwi": p, "wgsize": w, "split": split, "cluster": cl, "unroll": base.unroll,
-                             "ms": round(timed(cfg), 4)})
+            for u in (2, 4):
+                rows.append({"ppwi": p, "wgsize": w, "unroll": u, "ms": round(timed(launch_cfg(p, w, 1, 64, u)), 4)})
     pick_ms = timed(pick)
     best = min(rows, key=lambda r: r["ms"])
     ctx.close()

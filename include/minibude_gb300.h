@@ -44,15 +44,16 @@ typedef struct bude_ffparams {
 
 /* Kernel launch shape of the exact kernel.  The reference exposes two knobs, PPWI (poses per work
  * item, a template parameter, src/main.cpp:48-53) and wgsize (threads per block,
- * src/cuda/fasten.hpp:272-275); this kernel adds the protein split and the shared-memory tile. */
+ * src/cuda/fasten.hpp:272-275).  Here a block takes ppwi * wgsize poses and two ligand atoms, and
+ * evaluates the pairs in reach for 32 * unroll poses at a time.  No field changes an energy's bits. */
 typedef struct bude_launch_cfg {
-  int32_t ppwi;    /* poses per thread, held in registers: 1, 2, 4, 8 or 16 */
+  int32_t ppwi;    /* poses per thread: 1, 2, 4, 8 or 16 */
   int32_t wgsize;  /* threads per block: a multiple of 32 in [32, 512] */
-  int32_t split;   /* protein slices per pose block: 1..8 with cluster = 1, 1..64 with cluster = 0 */
-  int32_t tile;    /* protein atoms per shared-memory stage (TMA bulk copy): multiple of 8, 8..512 */
-  int32_t unroll;  /* protein atoms per unrolled inner-loop body: 1, 2 or 4 */
-  int32_t cluster; /* split > 1: 1 = slices summed inside a thread-block cluster (distributed shared
-                      memory), 0 = through a context-owned [split][nposes] buffer and a second kernel */
+  int32_t split;   /* 1..8 with cluster = 1, 1..64 with cluster = 0; checked, without effect: the sums of
+                      two ligand atoms each are what spreads over the GPU and is added up in order */
+  int32_t tile;    /* a multiple of 8, 8..512; checked, without effect */
+  int32_t unroll;  /* poses per lane of a group evaluated together: 1, 2 or 4 */
+  int32_t cluster; /* 0 or 1; checked, without effect */
 } bude_launch_cfg;
 
 typedef struct bude_gpu_ctx bude_gpu_ctx;
@@ -93,21 +94,21 @@ int bude_gpu_upload(bude_gpu_ctx *ctx, const bude_atom *protein, int32_t natpro,
 int bude_gpu_set_poses(bude_gpu_ctx *ctx, const bude_atom *ligand, int32_t natlig, const float *poses,
                        int64_t pose_stride, int64_t nposes);
 
-/* Map the reference's (PPWI, wgsize) pair onto this kernel's launch shape, choosing split and tile
- * for the uploaded deck.  PPWI above 16 uses 16 poses per thread; wgsize 0 or below 32 is rounded
- * up to a multiple of 32.  Results do not depend on the shape beyond FP32 summation order. */
+/* The launch shape for the uploaded deck's size, whatever the reference's (PPWI, wgsize) pair: the
+ * pair is how the reference spreads poses over threads, which the library does by the number of poses
+ * and ligand atoms.  Results do not depend on the shape. */
 int bude_gpu_default_cfg(const bude_gpu_ctx *ctx, int32_t ppwi, int32_t wgsize, bude_launch_cfg *cfg);
 
 /* Choose a launch shape for the uploaded deck by measurement; replaces the reference driver's
- * brute-force PPWI x wgsize sweep (src/main.cpp:517-541).  Candidate shapes get their protein
- * split from a wave model (resident blocks per SM from the occupancy API) and are timed with CUDA
- * events on a ligand prefix, within about max_ms of GPU time.  The pick is cached per deck shape
- * in the context.  best_ms (optional) receives the predicted time of one full evaluation. */
+ * brute-force PPWI x wgsize sweep (src/main.cpp:517-541).  The shape of bude_gpu_default_cfg and its
+ * neighbours are timed with CUDA events (on a ligand prefix where the deck is large), within about
+ * max_ms of GPU time.  The pick is cached per deck shape in the context.  best_ms (optional) receives
+ * the predicted time of one full evaluation. */
 int bude_gpu_autotune(bude_gpu_ctx *ctx, int32_t max_ms, bude_launch_cfg *best, float *best_ms);
 
 /* One evaluation of all uploaded poses (one iteration of the reference's hot loop,
  * src/cuda/fasten.hpp:277-286): pose transforms and the exact kernel on the context's stream,
- * then a stream synchronise.  *kernel_ms (optional) receives the CUDA-event time of the two
+ * then a stream synchronise.  *kernel_ms (optional) receives the CUDA-event time of its
  * kernels.  Energies stay on the device. */
 int bude_gpu_run(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, float *kernel_ms);
 
@@ -133,8 +134,8 @@ int bude_gpu_score_host(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, const bud
  * H2D copy of src/cuda/fasten.hpp:256-270 for decks too large to stage at once or produced on the
  * host.  poses: six fields at poses + k*pose_stride (poses.in layout); energies: nposes floats.
  * Pinned host buffers (bude_host_alloc) let the copies overlap.  The energies equal those of
- * bude_gpu_run with the same cfg over all poses, bit for bit, for any chunk.  The chunk is rounded
- * up to whole waves of the launch shape's resident blocks (so each chunk's launch fills the GPU).
+ * bude_gpu_run over all poses, bit for bit, for any chunk.  The chunk is rounded up to whole blocks,
+ * and to enough of them that a chunk's launch fills the GPU.
  * *ms (optional): CUDA-event time of the whole call.  No counterpart in the reference. */
 int bude_gpu_score_stream(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, const float *poses, int64_t pose_stride,
                           int64_t nposes, int64_t chunk, float *energies, float *ms);
@@ -160,18 +161,15 @@ int bude_gpu_upload_batch(bude_gpu_ctx *ctx, const bude_atom *protein, int32_t n
                           const bude_atom *ligand_atoms, const int32_t *ligand_offsets, const float *poses,
                           int64_t pose_stride, const int64_t *pose_offsets);
 
-/* Launch shape for the batch (ppwi, wgsize, tile, unroll, split; cluster is not used): each
- * candidate is timed on a strided subset of the batch's work items, the best pose shape also with
- * its protein cut into 2, 4 and 8 slices.  Cached per batch. */
+/* Launch shape for the batch (ppwi, wgsize, unroll): a few shapes around the one the batch's size
+ * calls for, each timed on the whole batch, within about max_ms.  Cached per batch. */
 int bude_gpu_autotune_batch(bude_gpu_ctx *ctx, int32_t max_ms, bude_launch_cfg *best, float *best_ms);
 
-/* One evaluation of the whole batch, then a stream synchronise.  per_ligand = 0: one persistent
- * kernel over all (ligand, pose block) items, longest first, taken from an atomic work counter,
- * launched as a CUDA graph (counter reset + pose transforms + persistent kernel) captured on first
- * use of a launch shape.  With cfg->split > 1 (cluster ignored) every item is scored once per
- * protein slice and a reduction kernel sums the slices in order; the energies then differ from
- * split = 1 by FP32 summation order only.  per_ligand = 1: one plain exact-kernel launch per
- * ligand, for comparison.  *ms (optional) receives the CUDA-event time. */
+/* One evaluation of the whole batch, then a stream synchronise.  per_ligand = 0: one launch over all
+ * (ligand, pose chunk, pair of atoms) items, longest ligands first, as a CUDA graph (pose transforms,
+ * exact kernel, sums over the atoms) captured on first use of a launch shape.  per_ligand = 1: one
+ * plain exact-kernel launch per ligand, for comparison; the same energies.  *ms (optional) receives
+ * the CUDA-event time. */
 int bude_gpu_run_batch(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, int32_t per_ligand, float *ms);
 
 /* Energies of the last batch evaluation, in concatenated pose order. */
@@ -242,16 +240,15 @@ typedef struct bude_screen_cfg {
   float audit_frac;   /* fraction of each ligand's poses rescored at random (audit sample) */
   float audit_tol;    /* audit error above which a ligand is rescored exhaustively */
   uint32_t seed;      /* audit sample */
-  bude_launch_cfg exact; /* exact kernel of the exhaustive fallback (cluster unused); its split and
-                          * tile also cut the protein for the rescoring, so every exact energy the
-                          * screen reports equals bude_gpu_run_batch's with this shape, bit for bit */
+  bude_launch_cfg exact; /* exact kernel of the exhaustive fallback (split, tile and cluster without
+                          * effect); every exact energy the screen reports equals
+                          * bude_gpu_run_batch's, bit for bit */
   int32_t chunks;     /* ligand chunks (0 or 1: none): with more, the exact rescoring of chunk j
                        * runs beside the surrogate of chunk j+1 (slower on the 1,024-ligand
                        * screen: the rescoring blocks slow the surrogate more than they hide) */
-  bude_launch_cfg rescore; /* shape of the exact rescoring: ppwi, wgsize, unroll and tile, the
-                            * records per shared-memory stage (0: exact's; it must divide exact's
-                            * tile); split and cluster are ignored: the protein slices are exact's.
-                            * ppwi 0 picks the shape from the number of poses rescored per ligand */
+  bude_launch_cfg rescore; /* shape of the exact rescoring: ppwi, wgsize and unroll; tile (0: exact's)
+                            * must divide exact's tile; ppwi 0 picks the shape from the number of
+                            * poses rescored per ligand */
 } bude_screen_cfg;
 
 /* total_ms: the whole call; surrogate_ms: pose transforms and surrogate scoring (until the last

@@ -1,11 +1,7 @@
 // autotune.cu -- launch-shape selection for the exact kernel.
 //
-// Replaces the reference driver's brute-force PPWI x wgsize sweep (src/main.cpp:517-541) with
-//   * a wave model: for a (poses per thread, block size, unroll) shape it reads the kernel's
-//     resident blocks per SM from the CUDA occupancy API and picks the protein split whose block
-//     count fills the last wave best (choose_split), and
-//   * a short measured search over the shapes the model ranks best, timed with CUDA events on a
-//     ligand prefix (time is linear in ligand atoms, the wave structure is unchanged).
+// Replaces the reference driver's brute-force PPWI x wgsize sweep (src/main.cpp:517-541) with a rule
+// on the deck's size (cull_shape) and a short measured search around its pick, timed with CUDA events.
 // The pick is cached per deck shape in the context.
 #include <cuda_runtime.h>
 
@@ -13,61 +9,13 @@
 #include <cmath>
 #include <vector>
 
-#include "exact_shape.h"
-#include "internal.h"
+#include "cull.h"
 
 namespace bude {
 
-static int ppwi_to_p(int ppwi) {
-  if (ppwi >= 16) return 16;
-  if (ppwi >= 8) return 8;
-  if (ppwi >= 4) return 4;
-  if (ppwi >= 2) return 2;
-  return 1;
-}
-
-// Pick cfg.split (and keep cfg.cluster) so that pose blocks x slices fill whole waves of the
-// device's resident block slots.  Cost model, in units of one block's full-protein time:
-//   rounds(S) / S * (1 + 0.01 * (S - 1))
-// (rounds = ceil(blocks * S / slots); the small per-slice term covers the reduction and the
-// shorter protein loop of thin slices).  Slices keep at least 64 protein atoms here; the measured
-// search below also tries thinner slices.
-int choose_split(const Context &c, bude_launch_cfg &cfg) {
-  return choose_split_for(c.num_sms, c.natpro_pad, c.nposes, cfg);
-}
-
-int choose_split_for(int num_sms, int natpro_pad, long long nposes, bude_launch_cfg &cfg) {
-  cfg.split = 1;
-  int per_sm = 0;
-  int rc = exact_blocks_per_sm(cfg, &per_sm);
-  if (rc) return rc;
-  if (per_sm <= 0) return set_error(BUDE_ERR_ARG, "launch shape cannot be resident on an SM");
-  const long long slots = (long long)per_sm * std::max(num_sms, 1);
-  const long long ppb = (long long)cfg.ppwi * cfg.wgsize;
-  const long long blocks = std::max<long long>(1, (nposes + ppb - 1) / ppb);
-  const int smax = std::max(1, std::min(cfg.cluster ? 8 : 64, natpro_pad / 64));
-  double best = 1e300;
-  for (int s = 1; s <= smax; ++s) {
-    const long long rounds = (blocks * s + slots - 1) / slots;
-    const double cost = double(rounds) / s * (1.0 + 0.01 * (s - 1));
-    if (cost < best - 1e-12) {
-      best = cost;
-      cfg.split = s;
-    }
-  }
+int default_cfg(const Context &c, int, int, bude_launch_cfg &cfg) {
+  cfg = cull_shape(c.have_deck ? c.nposes : 1LL << 20, c.have_deck ? c.natlig : 32, 1);
   return BUDE_OK;
-}
-
-int default_cfg(const Context &c, int ppwi, int wgsize, bude_launch_cfg &cfg) {
-  cfg.ppwi = ppwi_to_p(std::max(ppwi, 1));
-  const int w = wgsize < 32 ? 128 : (wgsize + 31) / 32 * 32;
-  cfg.wgsize = std::min(w, kMaxThreads);
-  cfg.tile = 64;
-  cfg.unroll = cfg.ppwi >= 16 ? 1 : 2;
-  cfg.cluster = 0;
-  cfg.split = 1;
-  if (c.num_sms <= 0 || !c.have_deck) return BUDE_OK;
-  return choose_split(c, cfg);
 }
 
 // Time one shape: one untimed evaluation, then the mean of `reps` event-timed ones.
@@ -101,88 +49,33 @@ int autotune(Context &c, int max_ms, bude_launch_cfg &best, float *best_ms) {
     if (best_ms) *best_ms = c.tuned_ms;
     return BUDE_OK;
   }
-  // Candidate shapes: poses per thread x block size x unroll, each with its model split, in
-  // both reduction modes.
+  // The rule's shape, then its neighbours in chunk size (poses per thread x threads) and group width.
+  bude_launch_cfg first{};
+  default_cfg(c, 0, 0, first);
+  std::vector<bude_launch_cfg> cands{first};
   struct Shape { int p, w, u; };
-  const Shape shapes[] = {{4, 64, 2},  {4, 128, 4}, {4, 256, 4}, {8, 64, 2},   {8, 128, 2},
-                          {8, 256, 2}, {16, 64, 1}, {16, 128, 1}, {16, 256, 1}, {2, 128, 2}};
-  std::vector<bude_launch_cfg> cands;
-  for (const Shape &s : shapes)
-    for (int cl = 0; cl < 2; ++cl) {
-      bude_launch_cfg cfg{s.p, s.w, 1, 64, s.u, cl};
-      if (choose_split(c, cfg)) continue;
-      if (cl == 1 && cfg.split == 1) continue; // same launch as cluster 0
-      cands.push_back(cfg);
-    }
-  if (cands.empty()) return set_error(BUDE_ERR_ARG, "no launch shape fits this device");
+  for (const Shape &s : {Shape{8, 512, 2}, Shape{4, 512, 2}, Shape{8, 384, 2}, Shape{4, 256, 2}, Shape{2, 256, 2},
+                         Shape{2, 512, 2}, Shape{1, 256, 1}, Shape{1, 128, 1}, Shape{2, 128, 2}, Shape{8, 512, 4}})
+    if (s.p != first.ppwi || s.w != first.wgsize || s.u != first.unroll)
+      cands.push_back(bude_launch_cfg{s.p, s.w, 1, 64, s.u, 0});
 
-  // Time on a ligand prefix so one evaluation takes about a millisecond or more.
+  // Time on a ligand prefix of at most 2^27 (pose, atom) points: some ten milliseconds.
   const int natlig_full = c.natlig;
-  const double inter_per_lig = double(c.nposes) * c.natpro;
   int lig = natlig_full;
-  const double target = 2.0e9; // interactions per timed evaluation (~1 ms at the kernel's rate)
-  if (inter_per_lig * natlig_full > target) lig = std::max(1, (int)std::ceil(target / std::max(inter_per_lig, 1.0)));
-  lig = std::min(lig, natlig_full);
+  if ((double)c.nposes * lig > double(1 << 27)) lig = std::max(1, (int)(double(1 << 27) / (double)c.nposes));
   c.natlig = lig;
   int rc = BUDE_OK;
-  float best_t = 1e30f;
-  float budget = (float)std::max(max_ms, 1);
-  float spent = 0.f;
-  auto trial = [&](const bude_launch_cfg &cfg, float *ms) {
-    rc = time_cfg(c, cfg, 2, ms);
-    if (rc) return false;
-    spent += 3.f * *ms;
-    if (*ms < best_t) {
-      best_t = *ms;
-      best = cfg;
-    }
-    return spent <= budget;
-  };
-  // Phase 1: every shape with the wave model's split.
-  std::vector<std::pair<float, bude_launch_cfg>> timed;
+  float best_t = 1e30f, spent = 0.f;
   for (const bude_launch_cfg &cfg : cands) {
     float ms = 0.f;
-    const bool more = trial(cfg, &ms);
+    rc = time_cfg(c, cfg, 2, &ms);
     if (rc) break;
-    timed.push_back({ms, cfg});
-    if (!more) break;
-  }
-  // Phase 2: the four fastest global-reduce shapes over every distinct slice width from half to
-  // two and a half times the model's split (slices down to 32 atoms).  The model's rounds of
-  // resident blocks do not capture how much more resident warps per SM help: on 938 atoms x 65,536
-  // poses, 8 poses per thread, 128 threads, it picks 12 slices where 20 (48-atom slices) measured
-  // 6% faster.
-  if (!rc && spent <= budget) {
-    std::sort(timed.begin(), timed.end(), [](const auto &a, const auto &b) { return a.first < b.first; });
-    // Splits whose slice sums ([split][nposes] floats) would pass 512 MB are not tried.
-    const long long split_cap = std::max(1LL, (512LL << 20) / (4LL * std::max(c.nposes, 1LL)));
-    const int smax_thin = (int)std::max(1LL, std::min({64LL, (long long)c.natpro_pad / 32, split_cap}));
-    int widened = 0;
-    for (const auto &t : timed) {
-      if (widened == 4 || rc || spent > budget) break;
-      const bude_launch_cfg base = t.second;
-      if (base.cluster != 0) continue;
-      ++widened;
-      int last_slice = -1;
-      for (int sp = std::max(2, base.split / 2); sp <= std::min(smax_thin, base.split * 5 / 2); ++sp) {
-        const int slice = (c.natpro_pad + sp - 1) / sp;
-        const int width = (slice + kAtomAlign - 1) / kAtomAlign * kAtomAlign;
-        if (width == last_slice || sp == base.split) continue;
-        // The fewest slices of this width (more would only add empty blocks).
-        if ((c.natpro_pad + width - 1) / width != sp) continue;
-        last_slice = width;
-        bude_launch_cfg cfg = base;
-        cfg.split = sp;
-        float ms = 0.f;
-        if (!trial(cfg, &ms) || rc) break;
-      }
+    if (ms < best_t) {
+      best_t = ms;
+      best = cfg;
     }
-    // A shape of this pass whose slice sums did not fit in device memory (a failed allocation)
-    // ends the pass; the pick stays the best shape timed so far.  Other errors are returned.
-    if (rc == BUDE_ERR_CUDA) {
-      (void)cudaGetLastError();
-      rc = BUDE_OK;
-    }
+    spent += 3.f * ms;
+    if (spent > (float)std::max(max_ms, 1)) break;
   }
   c.natlig = natlig_full;
   if (rc) return rc;

@@ -16,9 +16,12 @@
 #include <vector>
 
 #include "../../include/minibude_gb300.h"
-#include "exact_kernel.cuh"
+#include "edge_pose.cuh"
+#include "exact_shape.h"
 #include "internal.h"
 #include "pair_record.h"
+#include "pose_xform.cuh"
+#include "ptx.cuh"
 
 namespace bude {
 
@@ -62,16 +65,101 @@ int cuda_error(cudaError_t e, const char *what) {
 const char *last_error() { return g_last_error; }
 
 // ---------------------------------------------------------------------------------------------
-// slab[t][j] = record for ligand type t against protein atom j; rows padded to natpro_pad.
-void build_slab(const bude_atom *protein, int natpro, const bude_ffparams *ff, int ntypes, int natpro_pad,
-                std::vector<float> &slab) {
-  slab.assign((size_t)ntypes * natpro_pad * kRecFloats, 0.f);
-  for (int t = 0; t < ntypes; ++t) {
-    float *row = slab.data() + (size_t)t * natpro_pad * kRecFloats;
-    for (int j = 0; j < natpro; ++j)
-      pair_record(ff[t], ff[protein[j].type], protein[j].x, protein[j].y, protein[j].z, row + (size_t)j * kRecFloats);
-    for (int j = natpro; j < natpro_pad; ++j) null_record(row + (size_t)j * kRecFloats);
+static int round_up(int v, int m) { return (v + m - 1) / m * m; }
+
+// The distance past which the pair energy of ligand type L and a protein atom of type Pp is exactly
+// zero (the cut-offs of pair_record's three terms), with room for the rounding of r and of the
+// constants (below 1e-5 of the distance, and 1e-6 A of the charge term's).
+static float pair_reach2(const bude_ffparams &L, const bude_ffparams &Pp, const float *rec) {
+  const double radij = (double)Pp.radius + (double)L.radius;
+  double past = 0.0;
+  if (rec[6] != 0.f) past = -1.0 / (double)rec[11];
+  if (rec[8] != 0.f) past = std::max(past, -1.0 / (double)rec[13]);
+  const double reach = (radij + past) * (1.0 + 1e-5) + 1e-4;
+  return (float)(reach * reach * (1.0 + 1e-6));
+}
+
+// The protein's atoms ordered so that runs of kClusterAtoms lie near each other: halved along the
+// longer side of their bounding box, at a multiple of kClusterAtoms, until a run is left.
+static void cluster_order(const bude_atom *protein, int *order, int n) {
+  if (n <= kClusterAtoms) {
+    std::sort(order, order + n);
+    return;
   }
+  float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+  auto at = [&](int i, int d) {
+    const float v = (&protein[i].x)[d];
+    return v == v ? v : 0.f; // a strict order needs numbers
+  };
+  for (int i = 0; i < n; ++i)
+    for (int d = 0; d < 3; ++d) {
+      lo[d] = std::min(lo[d], at(order[i], d));
+      hi[d] = std::max(hi[d], at(order[i], d));
+    }
+  int d = 0;
+  for (int k = 1; k < 3; ++k)
+    if (hi[k] - lo[k] > hi[d] - lo[d]) d = k;
+  const int runs = (n + kClusterAtoms - 1) / kClusterAtoms, half = runs / 2 * kClusterAtoms;
+  std::nth_element(order, order + half, order + n, [&](int a, int b) {
+    const float x = at(a, d), y = at(b, d);
+    return x < y || (x == y && a < b);
+  });
+  cluster_order(protein, order, half);
+  cluster_order(protein, order + half, n - half);
+}
+
+// The deck's tables (CullArgs): slab[t][j] = pair constants of ligand type t against the j-th protein atom in
+// cluster order, reach[t][j] = {its position, the pair's squared reach}; rows padded to natpro_pad.
+struct DeckTables {
+  std::vector<float> slab, reach, box, box_reach;
+  float lo[3], hi[3];
+};
+static void build_tables(const bude_atom *protein, int natpro, const bude_ffparams *ff, int ntypes, int natpro_pad,
+                         DeckTables &t) {
+  std::vector<int> order((size_t)natpro);
+  for (int i = 0; i < natpro; ++i) order[(size_t)i] = i;
+  cluster_order(protein, order.data(), natpro);
+  const int clusters = natpro_pad / kClusterAtoms;
+  t.slab.assign((size_t)ntypes * natpro_pad * kPairF4 * 4, 0.f);
+  t.reach.assign((size_t)ntypes * natpro_pad * 4, 0.f);
+  t.box.assign((size_t)clusters * 8, 0.f);
+  t.box_reach.assign((size_t)ntypes * clusters, -1.f);
+  float most = 0.f;
+  for (int l = 0; l < ntypes; ++l)
+    for (int j = 0; j < natpro_pad; ++j) {
+      float rec[kRecFloats];
+      float *r = t.reach.data() + ((size_t)l * natpro_pad + j) * 4;
+      if (j < natpro) {
+        const bude_atom &p = protein[order[(size_t)j]];
+        pair_record(ff[l], ff[p.type], p.x, p.y, p.z, rec);
+        r[3] = pair_reach2(ff[l], ff[p.type], rec);
+        r[0] = p.x, r[1] = p.y, r[2] = p.z;
+      } else {
+        null_record(rec);
+        r[0] = rec[0], r[1] = rec[2], r[2] = rec[4], r[3] = -1.f;
+      }
+      const float pair[kPairF4 * 4] = {rec[0],  rec[2],  rec[4],  rec[6],  rec[8], rec[10],
+                                       rec[11], rec[12], rec[13], rec[14], 0.f,    0.f};
+      std::copy(pair, pair + kPairF4 * 4, t.slab.data() + ((size_t)l * natpro_pad + j) * kPairF4 * 4);
+      float &c = t.box_reach[(size_t)l * clusters + j / kClusterAtoms];
+      if (!(r[3] <= c)) c = r[3]; // a NaN stays and lets the cluster through
+      most = std::max(most, r[3]);
+    }
+  for (int d = 0; d < 3; ++d) t.lo[d] = FLT_MAX, t.hi[d] = -FLT_MAX;
+  for (int k = 0; k < clusters; ++k)
+    for (int d = 0; d < 3; ++d) {
+      float lo = FLT_MAX, hi = -FLT_MAX;
+      for (int j = k * kClusterAtoms; j < std::min(natpro, (k + 1) * kClusterAtoms); ++j) {
+        const float v = (&protein[order[(size_t)j]].x)[d];
+        lo = std::min(lo, v);
+        hi = std::max(hi, v);
+      }
+      t.box[(size_t)k * 8 + d] = lo;
+      t.box[(size_t)k * 8 + 4 + d] = hi;
+      t.lo[d] = std::min(t.lo[d], lo);
+      t.hi[d] = std::max(t.hi[d], hi);
+    }
+  for (int d = 0; d < 3; ++d) t.lo[d] -= std::sqrt(most), t.hi[d] += std::sqrt(most);
 }
 
 int ensure_slab(Context &c, const bude_atom *protein, int natpro, const bude_ffparams *ff, int ntypes, bool *rebuilt) {
@@ -87,18 +175,29 @@ int ensure_slab(Context &c, const bude_atom *protein, int natpro, const bude_ffp
   c.slab_key.clear();
   c.ntypes = ntypes;
   c.natpro = natpro;
-  c.natpro_pad = std::max((natpro + kAtomAlign - 1) / kAtomAlign * kAtomAlign, kAtomAlign);
-  std::vector<float> slab;
-  build_slab(protein, natpro, ff, ntypes, c.natpro_pad, slab);
-  int rc = c.slab.reserve(slab.size() * sizeof(float), "slab");
-  if (!rc) rc = c.raw_protein.reserve((size_t)std::max(natpro, 1) * sizeof(bude_atom), "protein records");
-  if (!rc) rc = c.raw_ff.reserve((size_t)ntypes * sizeof(bude_ffparams), "forcefield records");
-  if (rc) return rc;
-  cudaError_t e = copy_sync(c, c.slab.ptr, slab.data(), slab.size() * sizeof(float), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && natpro > 0)
-    e = copy_sync(c, c.raw_protein.ptr, protein, (size_t)natpro * sizeof(bude_atom), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = copy_sync(c, c.raw_ff.ptr, ff, (size_t)ntypes * sizeof(bude_ffparams), cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) return cuda_error(e, "slab upload");
+  c.natpro_pad = std::max(round_up(natpro, kClusterAtoms), kClusterAtoms);
+  DeckTables t;
+  build_tables(protein, natpro, ff, ntypes, c.natpro_pad, t);
+  struct Part {
+    DevBuf *buf;
+    const void *src;
+    size_t bytes;
+  };
+  const Part parts[] = {{&c.slab, t.slab.data(), t.slab.size() * sizeof(float)},
+                        {&c.reach, t.reach.data(), t.reach.size() * sizeof(float)},
+                        {&c.box, t.box.data(), t.box.size() * sizeof(float)},
+                        {&c.box_reach, t.box_reach.data(), t.box_reach.size() * sizeof(float)},
+                        {&c.raw_protein, protein, (size_t)natpro * sizeof(bude_atom)},
+                        {&c.raw_ff, ff, (size_t)ntypes * sizeof(bude_ffparams)}};
+  for (const Part &p : parts) {
+    const int rc = p.buf->reserve(std::max<size_t>(p.bytes, 16), "deck tables");
+    if (rc) return rc;
+  }
+  for (const Part &p : parts) {
+    const cudaError_t e = copy_sync(c, p.buf->ptr, p.src, p.bytes, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return cuda_error(e, "deck table upload");
+  }
+  for (int d = 0; d < 3; ++d) c.reach_lo[d] = t.lo[d], c.reach_hi[d] = t.hi[d];
   c.host_ff.assign(ff, ff + ntypes);
   // The protein's half of the regular-deck bounds (edge_pose.cuh); types were checked by the caller.
   c.protein_regular = true;
@@ -127,13 +226,11 @@ bool ligand_regular(const Context &c, const bude_atom *ligand, int natlig, const
   return min_sum >= kMinRadiusSum;
 }
 
-int enqueue_edge_single(Context &c, const float4 *ligand, int natlig, bool all, const unsigned *mask,
-                        const float *xform, float *energies, long long n, cudaStream_t st) {
-  if (n <= 0) return BUDE_OK;
+EdgeArgs edge_args_single(const Context &c, const float4 *ligand, int natlig, bool all, const unsigned *mask,
+                          const float *xform) {
   EdgeArgs a{};
   a.mask = mask;
   a.all = all ? 1 : 0;
-  a.nposes = n;
   a.nlig = 1;
   a.ligand = ligand;
   a.natlig = natlig;
@@ -141,29 +238,23 @@ int enqueue_edge_single(Context &c, const float4 *ligand, int natlig, bool all, 
   a.natpro = c.natpro;
   a.ff = c.raw_ff.as<bude_ffparams>();
   a.xform = xform;
-  a.energies = energies;
-  edge_pose_kernel<<<edge_grid(n, c.num_sms), 256, 0, st>>>(a);
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_error(e, "edge_pose_kernel launch");
-  c.launches++;
-  return BUDE_OK;
+  return a;
 }
 
-int enqueue_edge_batch(Context &c, const float *xform, float *energies, unsigned char *flag, cudaStream_t st) {
-  if (c.batch_poses <= 0) return BUDE_OK;
-  EdgeArgs a{};
-  a.mask = c.b_edge_mask.as<unsigned>();
+EdgeArgs edge_args_batch(const Context &c, const float *xform) {
+  EdgeArgs a = edge_args_single(c, c.b_ligands.as<float4>(), 0, false, c.b_edge_mask.as<unsigned>(), xform);
   a.nposes = c.batch_poses;
   a.pose_off = c.b_pose_off.as<long long>();
   a.lig_off = c.b_lig_off.as<int>();
   a.lig_any = c.b_lig_any.as<int>();
   a.lig_all = c.b_lig_all.as<unsigned char>();
   a.nlig = c.nligands;
-  a.ligand = c.b_ligands.as<float4>();
-  a.protein = c.raw_protein.as<bude_atom>();
-  a.natpro = c.natpro;
-  a.ff = c.raw_ff.as<bude_ffparams>();
-  a.xform = xform;
+  return a;
+}
+
+int enqueue_edge_batch(Context &c, const float *xform, float *energies, unsigned char *flag, cudaStream_t st) {
+  if (c.batch_poses <= 0) return BUDE_OK;
+  EdgeArgs a = edge_args_batch(c, xform);
   a.energies = energies;
   a.flag = flag;
   edge_pose_kernel<<<edge_grid(c.batch_poses, c.num_sms), 256, 0, st>>>(a);
@@ -202,8 +293,6 @@ using namespace bude;
 
 namespace bude {
 
-static int round_up(int v, int m) { return (v + m - 1) / m * m; }
-
 int check_cfg(const Context &c, const bude_launch_cfg &cfg) {
   const int p = cfg.ppwi;
   if (p != 1 && p != 2 && p != 4 && p != 8 && p != 16)
@@ -218,77 +307,8 @@ int check_cfg(const Context &c, const bude_launch_cfg &cfg) {
                      cfg.tile);
   if (cfg.unroll != 1 && cfg.unroll != 2 && cfg.unroll != 4)
     return set_error(BUDE_ERR_ARG, "unroll must be 1, 2 or 4 (got %d)", cfg.unroll);
-  if (exact_smem_bytes(p, cfg.wgsize, cfg.tile, cfg.split, cfg.cluster) > 200 * 1024)
-    return set_error(BUDE_ERR_ARG, "launch shape needs too much shared memory");
   (void)c;
   return BUDE_OK;
-}
-
-// The compilation of exact_kernel<P, U> a block size runs: the narrow one (170 registers) for
-// blocks of at most kNarrowThreads threads.
-template <int P, int U> static decltype(&exact_kernel<P, U>) exact_entry(int wgsize) {
-  return wgsize <= kNarrowThreads ? exact_kernel_narrow<P, U> : exact_kernel<P, U>;
-}
-
-template <int P, int U>
-static cudaError_t launch_exact_pu(const ExactArgs &a, dim3 grid, int wgsize, size_t smem, int split,
-                                   cudaStream_t st) {
-  const auto kernel = exact_entry<P, U>(wgsize);
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  if (split == 1 || !a.cluster) {
-    kernel<<<grid, wgsize, smem, st>>>(a);
-    return cudaGetLastError();
-  }
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = grid;
-  lc.blockDim = dim3(wgsize, 1, 1);
-  lc.dynamicSmemBytes = smem;
-  lc.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = split;
-  attr[0].val.clusterDim.z = 1;
-  lc.attrs = attr;
-  lc.numAttrs = 1;
-  return cudaLaunchKernelEx(&lc, kernel, a);
-}
-
-template <int P>
-static cudaError_t launch_exact_p(const ExactArgs &a, dim3 grid, const bude_launch_cfg &cfg, size_t smem,
-                                  cudaStream_t st) {
-  switch (cfg.unroll) {
-  case 1: return launch_exact_pu<P, 1>(a, grid, cfg.wgsize, smem, cfg.split, st);
-  case 2: return launch_exact_pu<P, 2>(a, grid, cfg.wgsize, smem, cfg.split, st);
-  default: return launch_exact_pu<P, 4>(a, grid, cfg.wgsize, smem, cfg.split, st);
-  }
-}
-
-template <int P, int U> static int blocks_per_sm_pu(int wgsize, size_t smem, int *out) {
-  const auto kernel = exact_entry<P, U>(wgsize);
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, kernel, wgsize, smem);
-  return e == cudaSuccess ? BUDE_OK : cuda_error(e, "occupancy query");
-}
-
-template <int P> static int blocks_per_sm_p(const bude_launch_cfg &cfg, size_t smem, int *out) {
-  switch (cfg.unroll) {
-  case 1: return blocks_per_sm_pu<P, 1>(cfg.wgsize, smem, out);
-  case 2: return blocks_per_sm_pu<P, 2>(cfg.wgsize, smem, out);
-  default: return blocks_per_sm_pu<P, 4>(cfg.wgsize, smem, out);
-  }
-}
-
-int exact_blocks_per_sm(const bude_launch_cfg &cfg, int *out) {
-  const size_t smem = exact_smem_bytes(cfg.ppwi, cfg.wgsize, cfg.tile, cfg.split, cfg.cluster);
-  switch (cfg.ppwi) {
-  case 1: return blocks_per_sm_p<1>(cfg, smem, out);
-  case 2: return blocks_per_sm_p<2>(cfg, smem, out);
-  case 4: return blocks_per_sm_p<4>(cfg, smem, out);
-  case 8: return blocks_per_sm_p<8>(cfg, smem, out);
-  default: return blocks_per_sm_p<16>(cfg, smem, out);
-  }
 }
 
 // Enqueue one evaluation (pose transforms + exact kernel) on the context's stream; `mid`, when
@@ -311,63 +331,8 @@ int enqueue_eval(Context &c, const bude_launch_cfg &cfg, cudaEvent_t mid) {
     c.launches++;
   }
   if (mid) cudaEventRecord(mid, c.stream);
-  rc = launch_exact_range(c, cfg, c.ligand.as<float4>(), c.natlig, c.xform.as<float>(), c.energies.as<float>(),
-                          c.nposes);
-  if (rc) return rc;
-  return enqueue_edge_single(c, c.ligand.as<float4>(), c.natlig, c.deck_irregular, c.edge_mask.as<unsigned>(),
-                             c.xform.as<float>(), c.energies.as<float>(), c.nposes, c.stream);
-}
-
-// The exact kernel (and, for a global-reduce split, slice_reduce_kernel) over `nposes` poses whose
-// transforms are at `xform`, for the ligand at `ligand`; energies land at `energies`.
-int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *ligand, int natlig, const float *xform,
-                       float *energies, long long nposes) {
-  if (nposes == 0) return BUDE_OK;
-  ExactArgs a;
-  a.ligand = ligand;
-  a.slab = c.slab.as<float4>();
-  a.xform = xform;
-  a.energies = energies;
-  a.partial = nullptr;
-  a.err = c.err.as<unsigned int>();
-  a.nposes = nposes;
-  a.natlig = natlig;
-  a.natpro_pad = c.natpro_pad;
-  a.tile = cfg.tile;
-  a.split = cfg.split;
-  a.cluster = cfg.cluster;
-  const bool global_reduce = cfg.split > 1 && !cfg.cluster;
-  if (global_reduce) {
-    // Slice sums go through a [split][nposes] buffer owned by the context.
-    int rc2 = c.partial.reserve((size_t)cfg.split * nposes * sizeof(float), "slice partial sums");
-    if (rc2) return rc2;
-    a.partial = c.partial.as<float>();
-  }
-  a.slice = round_up((c.natpro_pad + cfg.split - 1) / cfg.split, kAtomAlign);
-  const long long ppb = (long long)cfg.ppwi * cfg.wgsize;
-  const long long nbx = (nposes + ppb - 1) / ppb;
-  if (nbx > 0x7fffffffLL) return set_error(BUDE_ERR_ARG, "too many poses for one launch");
-  dim3 grid((unsigned)nbx, (unsigned)cfg.split, 1);
-  const size_t smem = exact_smem_bytes(cfg.ppwi, cfg.wgsize, cfg.tile, cfg.split, cfg.cluster);
-  cudaError_t e;
-  switch (cfg.ppwi) {
-  case 1: e = launch_exact_p<1>(a, grid, cfg, smem, c.stream); break;
-  case 2: e = launch_exact_p<2>(a, grid, cfg, smem, c.stream); break;
-  case 4: e = launch_exact_p<4>(a, grid, cfg, smem, c.stream); break;
-  case 8: e = launch_exact_p<8>(a, grid, cfg, smem, c.stream); break;
-  default: e = launch_exact_p<16>(a, grid, cfg, smem, c.stream); break;
-  }
-  if (e != cudaSuccess) return cuda_error(e, "exact_kernel launch");
-  c.launches++;
-  if (global_reduce) {
-    const int tb = 256;
-    slice_reduce_kernel<<<(unsigned)((nposes + tb - 1) / tb), tb, 0, c.stream>>>(a.partial, cfg.split, nposes,
-                                                                               a.energies);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_error(e, "slice_reduce_kernel launch");
-    c.launches++;
-  }
-  return BUDE_OK;
+  return launch_exact_range(c, cfg, c.ligand.as<float4>(), c.natlig, c.deck_irregular, c.edge_mask.as<unsigned>(),
+                            c.xform.as<float>(), c.energies.as<float>(), c.nposes);
 }
 
 // Self-test of the bounded wait: one thread waits on an mbarrier that nothing arrives on, with a
@@ -500,6 +465,9 @@ void destroy_context(Context *c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   c->ligand.release();
   c->slab.release();
+  c->reach.release();
+  c->box.release();
+  c->box_reach.release();
   c->poses.release();
   c->xform.release();
   c->energies.release();

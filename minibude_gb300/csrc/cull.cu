@@ -1,0 +1,221 @@
+// cull.cu -- host side of the exact kernel (cull_kernel.cuh, cull.h).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <numeric>
+
+#include "cull.h"
+#include "cull_kernel.cuh"
+
+namespace bude {
+
+constexpr size_t kCullMaxSmem = 200 * 1024; // 16 poses per thread x 512 threads: 185 KB
+
+static CullArgs cull_args(const Context &c, const bude_launch_cfg &s) {
+  CullArgs a{};
+  a.supers = c.natpro_pad <= 65536 &&
+             cull_smem_bytes(s.ppwi * s.wgsize, s.wgsize, s.unroll, 1) <= kCullMaxSmem;
+  a.slab = c.slab.as<float4>();
+  a.reach = c.reach.as<float4>();
+  a.box = c.box.as<float4>();
+  a.box_reach = c.box_reach.as<float>();
+  a.lo = make_float3(c.reach_lo[0], c.reach_lo[1], c.reach_lo[2]);
+  a.hi = make_float3(c.reach_hi[0], c.reach_hi[1], c.reach_hi[2]);
+  a.natpro_pad = c.natpro_pad;
+  a.clusters = c.natpro_pad / kClusterAtoms;
+  return a;
+}
+
+template <int K, int P>
+static cudaError_t launch_kp(const CullArgs *a, unsigned grid, int threads, cudaStream_t st) {
+  if (!a)
+    return cudaFuncSetAttribute(cull_kernel<K, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCullMaxSmem);
+  cull_kernel<K, P><<<grid, threads, cull_smem_bytes(K * threads, threads, P, a->supers), st>>>(*a);
+  return cudaGetLastError();
+}
+
+template <int K>
+static cudaError_t launch_k(const CullArgs *a, unsigned grid, const bude_launch_cfg &s, cudaStream_t st) {
+  switch (s.unroll) {
+  case 1: return launch_kp<K, 1>(a, grid, s.wgsize, st);
+  case 2: return launch_kp<K, 2>(a, grid, s.wgsize, st);
+  default: return launch_kp<K, 4>(a, grid, s.wgsize, st);
+  }
+}
+
+// Launches the shape's kernel; a == nullptr: only sets its shared-memory limit.
+static cudaError_t launch_shape(const CullArgs *a, unsigned grid, const bude_launch_cfg &s, cudaStream_t st) {
+  switch (s.ppwi) {
+  case 1: return launch_k<1>(a, grid, s, st);
+  case 2: return launch_k<2>(a, grid, s, st);
+  case 4: return launch_k<4>(a, grid, s, st);
+  case 8: return launch_k<8>(a, grid, s, st);
+  default: return launch_k<16>(a, grid, s, st);
+  }
+}
+
+int prepare_shape(const bude_launch_cfg &shape) {
+  const cudaError_t e = launch_shape(nullptr, 0, shape, nullptr);
+  return e == cudaSuccess ? BUDE_OK : cuda_error(e, "launch shape");
+}
+
+static int launch(Context &c, const CullArgs &a, long long grid, const bude_launch_cfg &s, cudaStream_t st) {
+  if (grid > 0x7fffffffLL) return set_error(BUDE_ERR_ARG, "too many poses for one launch");
+  int rc = prepare_shape(s);
+  if (rc) return rc;
+  const cudaError_t e = launch_shape(&a, (unsigned)grid, s, st);
+  if (e != cudaSuccess) return cuda_error(e, "cull_kernel launch");
+  c.launches++;
+  return BUDE_OK;
+}
+
+static int finish(Context &c, const FinishArgs &f, long long grid, cudaStream_t st) {
+  cull_finish_kernel<<<(unsigned)grid, 256, 0, st>>>(f);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_error(e, "cull_finish_kernel launch");
+  c.launches++;
+  return BUDE_OK;
+}
+
+static int cull_groups(int natlig) { return (natlig + kGroupAtoms - 1) / kGroupAtoms; }
+
+int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *ligand, int natlig, bool all_irregular,
+                       const unsigned *mask, const float *xform, float *energies, long long nposes) {
+  if (nposes == 0) return BUDE_OK;
+  const int groups = cull_groups(natlig);
+  const int most = cfg.ppwi * cfg.wgsize;
+  CullArgs a = cull_args(c, cfg);
+  a.ligand = ligand;
+  a.xform = xform;
+  a.natlig = natlig;
+  a.chunk = even_chunk(nposes, most);
+  // The group sums of a window of poses, [groups][window], at most kSumsBytes (and at least a chunk).
+  const long long fit = (long long)(kSumsBytes / sizeof(float)) / std::max(groups, 1) / a.chunk * a.chunk;
+  const long long window = std::min(nposes, std::max(fit, (long long)a.chunk));
+  if (groups > 0) {
+    const int rc = c.partial.reserve((size_t)groups * window * sizeof(float), "group sums");
+    if (rc) return rc;
+  }
+  FinishArgs f{};
+  f.groups = groups;
+  f.energies = energies;
+  f.edges = mask != nullptr;
+  f.e = edge_args_single(c, ligand, natlig, all_irregular, mask, xform);
+  a.sums = c.partial.as<float>();
+  f.sums = a.sums;
+  for (long long w0 = 0; w0 < nposes; w0 += window) {
+    const long long n = std::min(window, nposes - w0);
+    a.nposes = n;
+    a.xform = xform + 12 * w0;
+    a.stride = n;
+    a.chunks = (int)((n + a.chunk - 1) / a.chunk);
+    int rc = groups > 0 ? launch(c, a, (long long)groups * a.chunks, cfg, c.stream) : BUDE_OK;
+    f.stride = n;
+    f.first = w0;
+    f.n = n;
+    if (!rc) rc = finish(c, f, (n + 255) / 256, c.stream);
+    if (rc) return rc;
+  }
+  return BUDE_OK;
+}
+
+CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vector<long long> &first,
+                   const std::vector<long long> &count, const bude_launch_cfg &shape) {
+  CullPlan plan;
+  const int most = shape.ppwi * shape.wgsize;
+  struct Chunk {
+    int lig, n;
+    long long pose;
+  };
+  std::vector<Chunk> chunks; // of the window being filled
+  CullPlan::Window w{};
+  auto natlig = [&](int l) { return c.lig_off[l + 1] - c.lig_off[l]; };
+  auto close = [&]() {
+    if (chunks.empty()) return;
+    w.item0 = (int)plan.items.size();
+    w.fold0 = (int)plan.folds.size();
+    for (const Chunk &k : chunks) plan.folds.push_back(make_int4((int)k.pose, k.n, cull_groups(natlig(k.lig)), k.lig));
+    // Longest ligands first; the chunks of one ligand and group next to each other (they read the
+    // same records).
+    std::stable_sort(chunks.begin(), chunks.end(),
+                     [&](const Chunk &x, const Chunk &y) { return natlig(x.lig) > natlig(y.lig); });
+    for (size_t i = 0, j = 0; i < chunks.size(); i = j) {
+      while (j < chunks.size() && chunks[j].lig == chunks[i].lig) ++j;
+      const int l = chunks[i].lig;
+      for (int g = 0; g < cull_groups(natlig(l)); ++g)
+        for (size_t k = i; k < j; ++k)
+          plan.items.push_back(make_int4(c.lig_off[l] + g * kGroupAtoms,
+                                         std::min(kGroupAtoms, natlig(l) - g * kGroupAtoms) | g << 8,
+                                         (int)chunks[k].pose, chunks[k].n));
+    }
+    w.items = (int)plan.items.size() - w.item0;
+    w.folds = (int)plan.folds.size() - w.fold0;
+    plan.sums_bytes = std::max(plan.sums_bytes, (size_t)w.n * w.groups * sizeof(float));
+    plan.windows.push_back(w);
+    chunks.clear();
+    w = CullPlan::Window{};
+  };
+  for (size_t i = 0; i < lig.size(); ++i) {
+    const int per = even_chunk(count[i], most), groups = cull_groups(natlig(lig[i]));
+    for (long long p = 0; p < count[i]; p += per) {
+      const int n = (int)std::min<long long>(per, count[i] - p);
+      const long long at = first[i] + p;
+      if (!chunks.empty() &&
+          (size_t)(at + n - w.first) * std::max(w.groups, groups) * sizeof(float) > kSumsBytes)
+        close();
+      if (chunks.empty()) w.first = at;
+      w.n = at + n - w.first;
+      w.groups = std::max(w.groups, groups);
+      chunks.push_back({lig[i], n, at});
+    }
+  }
+  close();
+  return plan;
+}
+
+int enqueue_plan(Context &c, const bude_launch_cfg &shape, const CullPlan &plan, const int4 *items, const int4 *folds,
+                 const float *xform, float *energies, float *sums, bool edges, cudaStream_t st) {
+  CullArgs a = cull_args(c, shape);
+  a.ligand = c.b_ligands.as<float4>();
+  a.xform = xform;
+  a.sums = sums;
+  FinishArgs f{};
+  f.sums = sums;
+  f.energies = energies;
+  f.edges = edges;
+  f.e = edge_args_batch(c, xform);
+  for (const CullPlan::Window &w : plan.windows) {
+    a.items = items + w.item0;
+    a.stride = f.stride = w.n;
+    a.first = f.first = w.first;
+    int rc = w.items > 0 ? launch(c, a, w.items, shape, st) : BUDE_OK;
+    f.folds = folds + w.fold0;
+    if (!rc && w.folds > 0) rc = finish(c, f, w.folds, st);
+    if (rc) return rc;
+  }
+  return BUDE_OK;
+}
+
+// A chunk wants to be large (its groups are tighter: 4,096 poses of the 4,096 x 64 deck leave 69 records
+// per group of 64, 2,048 leave 82), but the launch wants several blocks per SM, one per chunk and group
+// of ligand atoms.  The lines lie where one shape overtook the next over 64 to 262,144 poses against 938
+// x 26, 2,672 x 48 and 4,096 x 64 atoms (us, smaller | larger shape): 1 x 256 | 2 x 256 at 120k points
+// (poses x ligand atoms) 104 | 108, at 288k 141 | 125; 2 x 256 | 4 x 512 at 426k 68 | 76, at 1.0M 131 |
+// 123; 4 x 512 | 8 x 512 at 1.9M 417 | 419, at 6.3M 1,061 | 996.  One point per lane below the first line
+// (latency: twice the warps), two above it; four lose to two everywhere.  Ligands of fewer poses than a
+// chunk take the smallest shape that holds them: 1,024 ligands of 410 poses 4 x 128 4.9 ms, 2 x 256 5.0,
+// 4 x 64 6.2; 128 of 205 2 x 128 0.46 ms, 1 x 256 0.50.
+bude_launch_cfg cull_shape(long long n, int natlig, int ligands) {
+  const double points = (double)n * natlig * ligands;
+  bude_launch_cfg s{1, n <= 64 ? 64 : (n <= 128 ? 128 : 256), 1, 64, 1, 0};
+  if (points < 2e5) return s;
+  const int shapes[][2] = {{8, 512}, {4, 512}, {4, 256}, {2, 256}, {4, 128}, {2, 128}};
+  int k = points < 7e5 ? 3 : (points < 2.2e6 ? 1 : 0);
+  while (k < 5 && (long long)shapes[k + 1][0] * shapes[k + 1][1] >= n) ++k;
+  s.ppwi = shapes[k][0];
+  s.wgsize = shapes[k][1];
+  s.unroll = 2;
+  return s;
+}
+
+} // namespace bude

@@ -1,0 +1,48 @@
+// cull.h -- host side of the exact kernel (cull_kernel.cuh): launch shapes, the cut of poses into
+// chunks, and the windows that bound the memory of the group sums.
+#pragma once
+#include <vector>
+
+#include "internal.h"
+
+namespace bude {
+
+// A batch evaluation's work, cut for one launch shape: block items and finish items in windows of
+// consecutive poses, each window's group sums at most kSumsBytes.
+struct CullPlan {
+  struct Window {
+    int item0, items, fold0, folds;
+    long long first, n; // poses
+    int groups;         // the most groups of a ligand in the window
+  };
+  std::vector<int4> items, folds; // CullArgs::items, FinishArgs::folds
+  std::vector<Window> windows;
+  size_t sums_bytes = 0; // the largest window's
+};
+
+constexpr size_t kSumsBytes = (size_t)1 << 30;
+
+// Poses of a chunk for n poses at `most` per block: as many chunks as that takes, evenly filled (a
+// short last chunk would sort few poses into loose groups).
+inline int even_chunk(long long n, int most) {
+  const long long chunks = (n + most - 1) / most;
+  const long long per = chunks > 0 ? (n + chunks - 1) / chunks : 1;
+  return (int)((per + 31) / 32 * 32 < most ? (per + 31) / 32 * 32 : most);
+}
+
+// Plan of the poses [first[i], first[i] + count[i]) of ligand lig[i]; first ascending.
+CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vector<long long> &first,
+                   const std::vector<long long> &count, const bude_launch_cfg &shape);
+// Enqueue the windows of a plan whose items and folds are on the device: energies of its poses from the
+// transforms at `xform`; `sums` holds plan.sums_bytes.  edges: irregular poses of the uploaded batch
+// get the reference's arithmetic.
+int enqueue_plan(Context &c, const bude_launch_cfg &shape, const CullPlan &plan, const int4 *items, const int4 *folds,
+                 const float *xform, float *energies, float *sums, bool edges, cudaStream_t st);
+// Shared-memory limit of the shape's kernel (before a stream capture).
+int prepare_shape(const bude_launch_cfg &shape);
+// The launch shape for n poses of a ligand of natlig atoms, `ligands` such ligands at once.
+bude_launch_cfg cull_shape(long long n, int natlig, int ligands);
+// The same for the uploaded batch (its mean ligand).
+bude_launch_cfg batch_shape(const Context &c);
+
+} // namespace bude

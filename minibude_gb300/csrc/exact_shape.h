@@ -5,6 +5,10 @@
 
 namespace bude {
 
+constexpr float kSteric = 76.f;   // 2 * HARDNESS (src/bude.h:33, serial/fasten.hpp:107)
+constexpr int kClusterAtoms = 32; // protein atoms of one cluster: neighbours in space, tested lane by lane
+constexpr int kPairF4 = 3;        // 16-byte words of the exact kernel's pair records
+constexpr int kGroupAtoms = 2;    // ligand atoms per block: the unit of the sum over the ligand
 constexpr int kStages = 4;       // shared-memory ring depth
 constexpr int kRecF4 = 4;        // 16-byte words per protein record (64 bytes)
 constexpr int kAtomAlign = 8;    // protein atoms are padded to a multiple of this (covers every unroll)

@@ -13,6 +13,8 @@ namespace bude {
 struct Surrogate;
 struct ScreenState;
 struct StreamState;
+struct CullPlan;
+struct EdgeArgs;
 
 // CUDA events owned by one host call: created together, destroyed when the call returns by any
 // path.  ok() is false when a creation failed.
@@ -56,6 +58,10 @@ struct Context {
   int natpro = 0, natpro_pad = 0, natlig = 0, ntypes = 0;
   long long nposes = 0, pose_stride = 0;
   DevBuf ligand, slab, poses, xform, energies, err, flush, partial;
+  // What the exact kernel finds the interacting pairs by (cull_kernel.cuh): per pair its reach, the
+  // clusters' boxes and reaches, and the box outside which no ligand atom interacts.
+  DevBuf reach, box, box_reach;
+  float reach_lo[3] = {}, reach_hi[3] = {};
   // Irregular poses and decks (edge_pose.cuh): the raw protein and forcefield records, the
   // transform pass's irregular-pose bits of the deck's poses, and whether the deck is irregular.
   DevBuf raw_protein, raw_ff, edge_mask;
@@ -71,17 +77,16 @@ struct Context {
   std::vector<int> lig_off;        // nligands + 1 atom offsets
   std::vector<long long> pose_off; // nligands + 1 pose offsets
   long long batch_poses = 0;
-  DevBuf b_ligands, b_poses, b_xform, b_energies, b_items, b_counter;
-  DevBuf b_partial; // split x batch_poses slice sums of a split batch evaluation (graph-owned)
+  DevBuf b_ligands, b_poses, b_xform, b_energies;
+  DevBuf b_items, b_folds, b_sums; // the device half of `plan` and its group sums (graph-owned)
   // Irregular poses of the batch: transform-pass bits, device pose/atom offsets, and the ligands
   // whose every pose goes to edge_pose_kernel (lig_all flags and their count, both on the device).
   DevBuf b_edge_mask, b_pose_off, b_lig_off, b_lig_all, b_lig_any;
   int b_irregular_ligands = 0;
   std::vector<unsigned char> b_lig_all_host; // host copy of the lig_all flags
-  int items_ppb = 0;  // poses per item the device item list was built for
-  int items_ppwi = 0; // and poses per thread (the cut of a ligand's last block depends on it)
-  int n_items = 0;
+  CullPlan *plan = nullptr;  // the batch cut for graph_cfg
   cudaGraphExec_t graph = nullptr;
+  long long graph_launches = 0; // kernels of one replay
   bude_launch_cfg graph_cfg{};
   long long batch_gen = 0; // bumped whenever the batch's shape (ligand sizes, pose counts) changes
   long long batch_uploads = 0; // bumped by every successful batch upload
@@ -111,8 +116,6 @@ int set_error(int code, const char *fmt, ...);
 int cuda_error(cudaError_t e, const char *what);
 const char *last_error();
 
-void build_slab(const bude_atom *protein, int natpro, const bude_ffparams *ff, int ntypes, int natpro_pad,
-                std::vector<float> &slab);
 // Build and upload the protein slab for (protein, forcefield) unless the device already holds the
 // slab of exactly these records; sets natpro, natpro_pad and ntypes.  *rebuilt (optional) tells
 // whether it was rebuilt.
@@ -126,17 +129,12 @@ int upload_deck(Context &c, const bude_atom *protein, int natpro, const bude_ato
 int set_poses(Context &c, const bude_atom *ligand, int natlig, const float *poses, long long stride,
               long long nposes);
 int check_cfg(const Context &c, const bude_launch_cfg &cfg);
-int exact_blocks_per_sm(const bude_launch_cfg &cfg, int *out);
-int choose_split(const Context &c, bude_launch_cfg &cfg);
-int choose_split_for(int num_sms, int natpro_pad, long long nposes, bude_launch_cfg &cfg);
 void release_batch(Context &c);
 int enqueue_batch(Context &c, const bude_launch_cfg &cfg, int per_ligand);
-// Cut a ligand's n poses into batch-kernel items of at most ppb = ppwi * wgsize poses: full blocks,
-// then the remainder r.  The batch kernel runs an item of at most ppb/2 or ppb/4 poses with half or
-// a quarter of the poses per thread (a quarter from 8 poses per thread up), so with ppwi 8 or 16 a
-// remainder ppb/2 < r <= 3ppb/4 is cut into ppb/2 + the rest: 3/4 of a full item's work.  (With 14
-// poses per thread, a shape sized for one item per ligand, halves would run 7 poses in 4 pairs.)
-// f(first pose offset within the ligand, pose count) is called per item, in pose order.
+// Cut a ligand's n poses into items of at most ppb poses: full items, then the remainder r.  For
+// kernels that run an item of at most ppb/2 or ppb/4 poses with half or a quarter of ppwi = 8 or 16
+// poses per thread, a remainder ppb/2 < r <= 3ppb/4 is cut into ppb/2 + the rest: 3/4 of a full item's
+// work.  f(first pose offset within the ligand, pose count) is called per item, in pose order.
 template <class F> inline void for_each_item(long long n, int ppwi, int ppb, F &&f) {
   long long p = 0;
   for (; n - p >= ppb; p += ppb) f(p, ppb);
@@ -149,15 +147,6 @@ template <class F> inline void for_each_item(long long n, int ppwi, int ppb, F &
   }
 }
 
-// Batch kernel over `items` (energies of the items' poses from the transforms at `xform`).  With
-// cfg.split > 1 the slice sums go through `partial` (at least cfg.split * npose_space floats) and a
-// per-item slice reduction.  On stream `st` (nullptr: the context's stream); max_blocks_per_sm > 0
-// caps the persistent grid, leaving room on each SM for kernels running beside it.  slice_tile > 0
-// cuts the protein slices as a launch with that tile would (cfg.tile, the records per shared-memory
-// stage, must divide it): the slices alone fix a pose's arithmetic.
-int batch_items_enqueue(Context &c, const bude_launch_cfg &cfg, const int4 *items, int n_items, const float4 *xform,
-                        float *energies, float *partial, long long npose_space, cudaStream_t st = nullptr,
-                        int max_blocks_per_sm = 0, int slice_tile = 0);
 void release_surrogate(Context &c);
 void release_streamer(Context &c);
 void release_screen(Context &c);
@@ -168,14 +157,16 @@ float *surrogate_scores(Context &c);
 int autotune(Context &c, int max_ms, bude_launch_cfg &best, float *best_ms);
 int default_cfg(const Context &c, int ppwi, int wgsize, bude_launch_cfg &cfg);
 int enqueue_eval(Context &c, const bude_launch_cfg &cfg, cudaEvent_t mid = nullptr);
-int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *ligand, int natlig, const float *xform,
-                       float *energies, long long nposes);
+// The energies of `nposes` poses (transforms at `xform`) of the ligand at `ligand`; with `mask` the
+// irregular ones of them, or all of an irregular deck, by the reference's arithmetic.
+int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *ligand, int natlig, bool all_irregular,
+                       const unsigned *mask, const float *xform, float *energies, long long nposes);
 // Whether a ligand of natlig atoms keeps the uploaded protein's deck regular (edge_pose.cuh).
 bool ligand_regular(const Context &c, const bude_atom *ligand, int natlig, const bude_ffparams *ff);
-// Enqueue edge_pose_kernel for the deck's single ligand over n poses (mask and transforms of
-// those poses; energies overwritten where irregular, or everywhere when `all`).
-int enqueue_edge_single(Context &c, const float4 *ligand, int natlig, bool all, const unsigned *mask,
-                        const float *xform, float *energies, long long n, cudaStream_t st);
+// Arguments of edge_energy for one ligand of natlig atoms, and for the uploaded batch.
+EdgeArgs edge_args_single(const Context &c, const float4 *ligand, int natlig, bool all, const unsigned *mask,
+                          const float *xform);
+EdgeArgs edge_args_batch(const Context &c, const float *xform);
 // Enqueue edge_pose_kernel over the uploaded batch's poses (flag: optional per-pose marks).
 int enqueue_edge_batch(Context &c, const float *xform, float *energies, unsigned char *flag, cudaStream_t st);
 int check_device_error(Context &c);

@@ -6,8 +6,8 @@
 //      radix select with ties taken in pose order, so the pick is deterministic) and an audit
 //      sample of exactly ceil(audit_frac * n) of the other poses, uniformly at random (the lowest
 //      seeded hashes of the pose indices);
-//   3. the picked poses are compacted and rescored by the exact kernel (batch_kernel over the
-//      compact transforms);
+//   3. the picked poses are compacted and rescored by the exact kernel over the compact
+//      transforms;
 //   4. audit_kernel measures the surrogate's ordering error on the audit sample,
 //      1 - Spearman(surrogate, exact); a ligand whose error exceeds `audit_tol` is rescored
 //      exhaustively with the exact kernel;
@@ -19,8 +19,7 @@
 #include <algorithm>
 #include <vector>
 
-#include "batch_kernel.cuh"
-#include "internal.h"
+#include "cull.h"
 
 namespace bude {
 
@@ -316,8 +315,8 @@ __global__ void fallback_copy_kernel(const long long *pose_off, const int *fallb
 }
 
 struct ScreenState {
-  DevBuf pose_off, flag, counts, comp_off, comp_pose, comp_xform, comp_exact, err, final_e, rescored, items, fb;
-  DevBuf partial;             // slice sums of split exact evaluations
+  DevBuf pose_off, flag, counts, comp_off, comp_pose, comp_xform, comp_exact, err, final_e, rescored, items, folds, fb;
+  DevBuf sums;                // group sums of the exact evaluations
   cudaStream_t side = nullptr; // the exact rescoring beside the surrogate
   long long result_for = -1;   // Context::batch_uploads of the batch the stored result belongs to
 };
@@ -326,48 +325,25 @@ void release_screen(Context &c) {
   if (!c.screen) return;
   ScreenState &s = *c.screen;
   for (DevBuf *b : {&s.pose_off, &s.flag, &s.counts, &s.comp_off, &s.comp_pose, &s.comp_xform, &s.comp_exact,
-                    &s.err, &s.final_e, &s.rescored, &s.items, &s.fb, &s.partial})
+                    &s.err, &s.final_e, &s.rescored, &s.items, &s.folds, &s.fb, &s.sums})
     b->release();
   if (s.side) cudaStreamDestroy(s.side);
   delete c.screen;
   c.screen = nullptr;
 }
 
-// Batch-kernel items (for_each_item) over pose ranges [first[i], first[i] + count[i]) of ligand
-// lig[i], longest ligand first.
-static std::vector<int4> range_items(const Context &c, const std::vector<int> &lig, const std::vector<long long> &first,
-                                     const std::vector<int> &count, const bude_launch_cfg &shape) {
-  const int ppb = shape.ppwi * shape.wgsize;
-  std::vector<int> order(lig.size());
-  for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-    return c.lig_off[lig[x] + 1] - c.lig_off[lig[x]] > c.lig_off[lig[y] + 1] - c.lig_off[lig[y]];
-  });
-  std::vector<int4> items;
-  for (int i : order) {
-    const int l = lig[i];
-    for_each_item(count[i], shape.ppwi, ppb, [&](long long p, int n) {
-      items.push_back(make_int4(c.lig_off[l], c.lig_off[l + 1] - c.lig_off[l], (int)(first[i] + p), n));
-    });
-  }
-  return items;
-}
-
-// Exact energies of the items' poses (pose indices in [0, npose_space) of xform / energies).
-static int run_items(Context &c, ScreenState &s, const bude_launch_cfg &cfg, const std::vector<int4> &items,
-                     const float4 *xform, float *energies, long long npose_space) {
-  if (items.empty()) return BUDE_OK;
-  int rc = s.items.reserve(items.size() * sizeof(int4), "screen items");
-  if (!rc && cfg.split > 1)
-    rc = s.partial.reserve((size_t)cfg.split * (size_t)std::max(npose_space, 1LL) * sizeof(float), "screen slice sums");
+// Device copies of a plan's items and folds, and room for its group sums.
+static int upload_plan(Context &c, ScreenState &s, const CullPlan &plan) {
+  int rc = s.items.reserve(std::max<size_t>(plan.items.size(), 1) * sizeof(int4), "screen items");
+  if (!rc) rc = s.folds.reserve(std::max<size_t>(plan.folds.size(), 1) * sizeof(int4), "screen items");
+  if (!rc) rc = s.sums.reserve(std::max<size_t>(plan.sums_bytes, 16), "screen group sums");
   if (rc) return rc;
-  cudaMemcpyAsync(s.items.ptr, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice, c.stream);
-  rc = batch_items_enqueue(c, cfg, s.items.as<int4>(), (int)items.size(), xform, energies, s.partial.as<float>(),
-                           npose_space);
-  if (rc) return rc;
-  // the host item vector must outlive the copy
-  cudaError_t e = cudaStreamSynchronize(c.stream);
-  return e == cudaSuccess ? BUDE_OK : cuda_error(e, "screen exact rescoring");
+  cudaError_t e = cudaSuccess; // pageable sources: staged before the calls return
+  if (!plan.items.empty())
+    e = cudaMemcpyAsync(s.items.ptr, plan.items.data(), plan.items.size() * sizeof(int4), cudaMemcpyHostToDevice, c.stream);
+  if (e == cudaSuccess && !plan.folds.empty())
+    e = cudaMemcpyAsync(s.folds.ptr, plan.folds.data(), plan.folds.size() * sizeof(int4), cudaMemcpyHostToDevice, c.stream);
+  return e == cudaSuccess ? BUDE_OK : cuda_error(e, "screen item upload");
 }
 
 int screen_run(Context &c, const bude_screen_cfg &sc, bude_screen_stats *stats) {
@@ -405,57 +381,48 @@ int screen_run(Context &c, const bude_screen_cfg &sc, bude_screen_stats *stats) 
   rc = s.comp_pose.reserve((size_t)std::max(ncomp, 1LL) * 4, "compact poses");
   if (!rc) rc = s.comp_xform.reserve((size_t)std::max(ncomp, 1LL) * 48, "compact transforms");
   if (!rc) rc = s.comp_exact.reserve((size_t)std::max(ncomp, 1LL) * 4, "compact energies");
-  if (!rc && cfg.split > 1)
-    rc = s.partial.reserve((size_t)cfg.split * (size_t)std::max(ncomp, 1LL) * sizeof(float), "screen slice sums");
   if (rc) return rc;
   // Ligand chunks (sc.chunks > 1): the surrogate scores chunk j+1 (3 tile groups per block) while
-  // the exact kernel rescores chunk j's picks beside it on a second stream, two blocks per SM.
-  // Measured on 1,024 ligands x 16,384 poses it is slower (126 ms against 106 ms): the rescoring
-  // blocks slow the scorer more than they hide, so one chunk (no overlap, 4 groups) is the default.
+  // the exact kernel rescores chunk j's picks beside it on a second stream.
   const int nchunks = nl == 0 ? 0 : std::max(1, std::min(nl, sc.chunks > 0 ? sc.chunks : 1));
   const bool overlap = nchunks > 1;
-  // Each ligand contributes only a few hundred picks: rescore them in small items so blocks are
-  // not mostly empty, with the fallback's protein slices (the pose shape does not change the
-  // arithmetic of a pose, the slices do).  One-warp blocks of 8 poses per thread (256-pose
-  // items) measured fastest on 410 picks per ligand (8 slices: 27.9 ms against 30.5 for 64
-  // threads x 4 poses, before the short-item cut); fewer picks per ligand get 128-pose items.
   int with_picks = 0;
   for (int l = 0; l < nl; ++l) with_picks += counts[2 * l] + counts[2 * l + 1] > 0;
-  const long long per_lig = with_picks ? ncomp / with_picks : 0;
-  bude_launch_cfg small = overlap                          ? bude_launch_cfg{4, 128, cfg.split, cfg.tile, 2, 0}
-                          : (per_lig > 256 && per_lig <= 448) ? bude_launch_cfg{14, 32, cfg.split, cfg.tile, 2, 0}
-                          : per_lig >= 128                  ? bude_launch_cfg{8, 32, cfg.split, cfg.tile, 4, 0}
-                                                            : bude_launch_cfg{4, 32, cfg.split, cfg.tile, 2, 0};
+  bude_launch_cfg small = cull_shape(with_picks ? ncomp / with_picks : 1,
+                                     nl ? std::max(c.lig_off[nl] / nl, 1) : 1, std::max(with_picks, 1));
   if (sc.rescore.ppwi != 0) {
     small = bude_launch_cfg{sc.rescore.ppwi, sc.rescore.wgsize, cfg.split, sc.rescore.tile > 0 ? sc.rescore.tile : cfg.tile,
                             sc.rescore.unroll, 0};
-    const bool rescore_only = small.ppwi == 14 && small.unroll == 2; // a batch-kernel shape of the rescoring
-    bude_launch_cfg chk = small;
-    if (rescore_only) chk.ppwi = 16;
-    rc = check_cfg(c, chk);
+    if (small.ppwi == 14 && small.unroll == 2) small.ppwi = 16; // a pose count only the rescoring takes
+    rc = check_cfg(c, small);
     if (rc) return rc;
     if (cfg.tile % small.tile) return set_error(BUDE_ERR_ARG, "the rescoring tile must divide the exact tile");
   }
-  std::vector<int> chunk_lig(nchunks + 1, nl), chunk_item(nchunks + 1, 0);
-  std::vector<int4> items;
+  // One plan for all picks; chunk j's share of it is a plan of its own over the same device arrays.
+  std::vector<int> chunk_lig(nchunks + 1, nl);
+  std::vector<CullPlan> chunk_plan((size_t)nchunks);
+  CullPlan plan;
   for (int j = 0; j < nchunks; ++j) {
     chunk_lig[j] = (int)((long long)nl * j / nchunks);
-    std::vector<int> lig, cnt;
-    std::vector<long long> first;
-    for (int l = (int)((long long)nl * j / nchunks); l < (int)((long long)nl * (j + 1) / nchunks); ++l) {
+    std::vector<int> lig;
+    std::vector<long long> first, cnt;
+    for (int l = chunk_lig[j]; l < (int)((long long)nl * (j + 1) / nchunks); ++l) {
       const int k = counts[2 * l] + counts[2 * l + 1];
       if (k == 0) continue;
       lig.push_back(l);
       first.push_back(comp_off[l]);
       cnt.push_back(k);
     }
-    chunk_item[j] = (int)items.size();
-    const std::vector<int4> its = range_items(c, lig, first, cnt, small);
-    items.insert(items.end(), its.begin(), its.end());
+    CullPlan p = plan_cull(c, lig, first, cnt, small);
+    for (CullPlan::Window w : p.windows) {
+      w.item0 += (int)plan.items.size();
+      w.fold0 += (int)plan.folds.size();
+      chunk_plan[j].windows.push_back(w);
+    }
+    plan.items.insert(plan.items.end(), p.items.begin(), p.items.end());
+    plan.folds.insert(plan.folds.end(), p.folds.begin(), p.folds.end());
+    plan.sums_bytes = std::max(plan.sums_bytes, p.sums_bytes);
   }
-  if (nchunks > 0) chunk_item[nchunks] = (int)items.size();
-  rc = s.items.reserve(std::max<size_t>(items.size(), 1) * sizeof(int4), "screen items");
-  if (rc) return rc;
   if (overlap && !s.side) {
     cudaError_t es = cudaStreamCreateWithFlags(&s.side, cudaStreamNonBlocking);
     if (es != cudaSuccess) return cuda_error(es, "screen rescoring stream");
@@ -466,8 +433,8 @@ int screen_run(Context &c, const bude_screen_cfg &sc, bude_screen_stats *stats) 
   cudaEventRecord(ev[1], c.stream); // re-recorded after each chunk's surrogate
   cudaMemcpyAsync(s.pose_off.ptr, c.pose_off.data(), (size_t)(nl + 1) * 8, cudaMemcpyHostToDevice, c.stream);
   cudaMemcpyAsync(s.comp_off.ptr, comp_off.data(), comp_off.size() * 8, cudaMemcpyHostToDevice, c.stream);
-  if (!items.empty())
-    cudaMemcpyAsync(s.items.ptr, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice, c.stream);
+  rc = upload_plan(c, s, plan);
+  if (rc) return rc;
   rc = surrogate_prepare(c, false); // pose transforms of every pose
   if (rc) return rc;
   const float *scores = surrogate_scores(c);
@@ -490,10 +457,8 @@ int screen_run(Context &c, const bude_screen_cfg &sc, bude_screen_stats *stats) 
     }
     cudaEventRecord(ready[j], c.stream);
     if (overlap) cudaStreamWaitEvent(rs, ready[j], 0);
-    const int n_it = chunk_item[j + 1] - chunk_item[j];
-    if (n_it > 0)
-      rc = batch_items_enqueue(c, small, s.items.as<int4>() + chunk_item[j], n_it, s.comp_xform.as<float4>(),
-                               s.comp_exact.as<float>(), s.partial.as<float>(), ncomp, rs, overlap ? 2 : 0, cfg.tile);
+    rc = enqueue_plan(c, small, chunk_plan[j], s.items.as<int4>(), s.folds.as<int4>(), s.comp_xform.as<float>(),
+                      s.comp_exact.as<float>(), s.sums.as<float>(), false, rs);
   }
   if (overlap) {
     cudaEvent_t joined = nchunks > 0 ? ready[0] : nullptr;
@@ -516,16 +481,25 @@ int screen_run(Context &c, const bude_screen_cfg &sc, bude_screen_stats *stats) 
   if (nl > 0) cudaMemcpyAsync(err.data(), s.err.ptr, (size_t)nl * 4, cudaMemcpyDeviceToHost, c.stream);
   cudaError_t e = cudaStreamSynchronize(c.stream);
   if (e != cudaSuccess) return cuda_error(e, "screen audit");
-  std::vector<int> fb_lig, fb_cnt;
-  std::vector<long long> fb_first;
+  std::vector<int> fb_lig;
+  std::vector<long long> fb_first, fb_cnt;
   for (int l = 0; l < nl; ++l)
     if (err[l] > sc.audit_tol) {
       fb_lig.push_back(l);
       fb_first.push_back(c.pose_off[l]);
-      fb_cnt.push_back((int)(c.pose_off[l + 1] - c.pose_off[l]));
+      fb_cnt.push_back(c.pose_off[l + 1] - c.pose_off[l]);
     }
-  rc = run_items(c, s, cfg, range_items(c, fb_lig, fb_first, fb_cnt, cfg), c.b_xform.as<float4>(),
-                 c.b_energies.as<float>(), np);
+  if (!fb_lig.empty()) {
+    const CullPlan fb_plan = plan_cull(c, fb_lig, fb_first, fb_cnt, cfg);
+    rc = upload_plan(c, s, fb_plan);
+    if (!rc)
+      rc = enqueue_plan(c, cfg, fb_plan, s.items.as<int4>(), s.folds.as<int4>(), c.b_xform.as<float>(),
+                        c.b_energies.as<float>(), s.sums.as<float>(), false, c.stream);
+    if (!rc) {
+      e = cudaStreamSynchronize(c.stream);
+      if (e != cudaSuccess) rc = cuda_error(e, "screen exact rescoring");
+    }
+  }
   if (rc) return rc;
   cudaEventRecord(ev[3], c.stream);
   // 5. final energies
@@ -561,7 +535,7 @@ int screen_run(Context &c, const bude_screen_cfg &sc, bude_screen_stats *stats) 
     stats->rescored_poses = ncomp;
     stats->fallback_ligands = (int32_t)fb_lig.size();
     long long fbp = 0;
-    for (int v : fb_cnt) fbp += v;
+    for (long long v : fb_cnt) fbp += v;
     stats->fallback_poses = fbp;
     float mx = 0.f;
     for (float v : err) mx = std::max(mx, v);

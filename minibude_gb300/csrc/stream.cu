@@ -12,8 +12,9 @@
 
 #include <algorithm>
 
-#include "exact_kernel.cuh"
+#include "exact_shape.h"
 #include "internal.h"
+#include "pose_xform.cuh"
 
 namespace bude {
 
@@ -78,17 +79,11 @@ static int score_stream(Context &c, const bude_launch_cfg &cfg, const float *pos
   if (chunk <= 0) return set_error(BUDE_ERR_ARG, "chunk must be positive (got %lld)", chunk);
   int rc = check_cfg(c, cfg);
   if (rc) return rc;
-  {
-    // Round the chunk up to whole waves of the launch shape's resident blocks, so that no chunk's
-    // launch leaves SMs idle in a partial last wave (131,072 poses at 16 poses per thread, 128
-    // threads and 8 slices fill 0.84 of one wave of 608 blocks; 155,648 fill it).
-    int per_sm = 0;
-    if (exact_blocks_per_sm(cfg, &per_sm) == BUDE_OK && per_sm > 0) {
-      const long long slots = (long long)per_sm * std::max(c.num_sms, 1);
-      const long long ppw = std::max(1LL, slots / std::max(cfg.split, 1)) * cfg.ppwi * cfg.wgsize;
-      chunk = (chunk + ppw - 1) / ppw * ppw;
-    }
-  }
+  // Whole blocks of poses, and enough of them that a chunk's launch fills the GPU: four blocks per SM
+  // (one block per group of ligand atoms and ppwi * wgsize poses).
+  const long long ppb = (long long)cfg.ppwi * cfg.wgsize;
+  const long long fill = 4LL * std::max(c.num_sms, 1) * kGroupAtoms / std::max(c.natlig, 1) + 1;
+  chunk = std::max((chunk + ppb - 1) / ppb, fill) * ppb;
   chunk = std::min(chunk, std::max(nposes, 1LL));
   StreamState *sp = nullptr;
   rc = streamer(c, chunk, &sp);
@@ -122,10 +117,8 @@ static int score_stream(Context &c, const bude_launch_cfg &cfg, const float *pos
     c.launches++;
     e = cudaEventRecord(s.consumed[b], c.stream);
     if (e != cudaSuccess) break;
-    rc = launch_exact_range(c, cfg, c.ligand.as<float4>(), c.natlig, s.xform.as<float>(), s.energies[b].as<float>(), n);
-    if (!rc)
-      rc = enqueue_edge_single(c, c.ligand.as<float4>(), c.natlig, c.deck_irregular, s.edge_mask.as<unsigned>(),
-                               s.xform.as<float>(), s.energies[b].as<float>(), n, c.stream);
+    rc = launch_exact_range(c, cfg, c.ligand.as<float4>(), c.natlig, c.deck_irregular, s.edge_mask.as<unsigned>(),
+                            s.xform.as<float>(), s.energies[b].as<float>(), n);
     if (rc) break;
     e = cudaEventRecord(s.computed[b], c.stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s.d2h, s.computed[b], 0);

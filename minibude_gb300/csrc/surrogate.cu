@@ -17,8 +17,8 @@
 #include <utility>
 #include <vector>
 
-#include "exact_kernel.cuh"
-#include "internal.h"
+#include "cull.h"
+#include "pose_xform.cuh"
 #include "score_tc.cuh"
 #include "surrogate_kernels.cuh"
 #include "wgrad_tc.cuh"
@@ -563,8 +563,7 @@ int surrogate_train(Context &c, int epochs, int batch, float lr, const float *la
     if (e != cudaSuccess) return cuda_error(e, "labels");
   } else {
     // Labels: exact energies of every pose from the batched exact kernel.
-    bude_launch_cfg cfg{16, 128, 1, 64, 1, 0};
-    rc = enqueue_batch(c, cfg, 0);
+    rc = enqueue_batch(c, batch_shape(c), 0);
     if (!rc) rc = check_device_error(c);
     if (rc) return rc;
     cudaMemcpyAsync(s.labels.ptr, c.b_energies.ptr, (size_t)np * 4, cudaMemcpyDeviceToDevice, c.stream);
@@ -802,9 +801,9 @@ int surrogate_prepare(Context &c, bool xform_ready) {
     std::vector<int4> items;
     s.item_lig_off.assign(1, 0);
     for (int l = 0; l < c.nligands; ++l) {
-      for (long long p = c.pose_off[l]; p < c.pose_off[l + 1]; p += kRowsPerCta)
-        items.push_back(make_int4(c.lig_off[l], c.lig_off[l + 1] - c.lig_off[l], (int)p,
-                                  (int)std::min<long long>(kRowsPerCta, c.pose_off[l + 1] - p)));
+      for_each_item(c.pose_off[l + 1] - c.pose_off[l], 1, kRowsPerCta, [&](long long p, int n) {
+        items.push_back(make_int4(c.lig_off[l], c.lig_off[l + 1] - c.lig_off[l], (int)(c.pose_off[l] + p), n));
+      });
       s.item_lig_off.push_back((int)items.size());
     }
     rc = s.items.reserve(std::max<size_t>(items.size(), 1) * sizeof(int4), "surrogate items");

@@ -93,6 +93,27 @@ def algorithmic_flops(nposes: int, natlig: int, natpro: int) -> float:
     return 30.0 * nposes * natlig * natpro + 18.0 * nposes * natlig + 28.0 * nposes
 
 
+def interacting_share(deck, nposes: int = 64) -> float:
+    """The share of a deck's (pose, ligand atom, protein atom) pairs that lie within the cut-off of
+    one of their three terms (src/serial/fasten.hpp:80-124), counted on its first poses.  The other
+    pairs add exactly zero."""
+    p = deck.poses[:, :nposes].astype(np.float64)
+    (sx, sy, sz), (cx, cy, cz) = np.sin(p[:3]), np.cos(p[:3])
+    rot = np.array([[cy * cz, sx * sy * cz - cx * sz, cx * sy * cz + sx * sz],
+                    [cy * sz, sx * sy * sz + cx * cz, cx * sy * sz - sx * cz], [-sy, sx * cy, cx * cy]])
+    xyz = np.stack([deck.protein["x"], deck.protein["y"], deck.protein["z"]], 1).astype(np.float64)
+    ff, pt = deck.forcefield, deck.protein["type"]
+    near = 0
+    for a in deck.ligand:
+        l, f = ff[a["type"]], ff[pt]
+        charge = np.where((f["hbtype"] == 70) & (l["hbtype"] == 70), 4.0, 2.0) * (f["elsc"] * l["elsc"] != 0)
+        desolv = np.where(f["hphb"] < 0, 5.5 if l["hphb"] < 0 else 1.0, 1.0 if l["hphb"] < 0 else 0.0) * (f["hphb"] != 0)
+        reach = f["radius"] + l["radius"] + np.maximum(charge, desolv)
+        pos = np.einsum("abn,b->na", rot, np.array([a["x"], a["y"], a["z"]], np.float64)) + p[3:].T
+        near += int((((pos[:, None] - xyz[None]) ** 2).sum(2) < reach ** 2).sum())
+    return near / max(p.shape[1] * len(deck.ligand) * len(xyz), 1)
+
+
 def reference_formula_flops(nposes: int, natlig: int, natpro: int, ppwi: int) -> float:
     """The reference's own FLOP count for a launch with `ppwi` poses per work-item (src/main.cpp:359:
     ops_per_wg = 27 P + natlig (2 + 18 P + natpro (10 + 30 P)) + P, times nposes / P groups).  It

@@ -1,0 +1,119 @@
+"""The exact kernel evaluates only the pairs that can interact (csrc/cull_kernel.cuh).  Its energies are
+checked where finding those pairs can go wrong: clusters of 32 protein atoms and blocks of 32 clusters
+that are just full, pose chunks and groups at their edges, a protein so dense that a list of candidates
+overflows, proteins past the 16-bit list indices, poses far from the protein, and group sums that take
+several windows.  The oracle evaluates every pair; against FP64 the bound is the one of
+test_forcefield_and_deck_sizes (4x the FP32 oracle's own error, at least 2e-4).  The order of a pose's sum
+depends on nothing else, so every launch shape has to give the same bits."""
+import numpy as np
+import pytest
+
+import oracle
+from minibude_gb300 import validate
+from minibude_gb300.deck import BatchDeck, DeckSpec, synthetic_deck, synthetic_ligand, synthetic_poses
+from minibude_gb300.model import GpuContext, launch_cfg
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(1, 32, 1), (2, 96, 2), (4, 128, 4), (8, 512, 2), (16, 512, 1), (16, 512, 4)]
+
+
+@pytest.fixture(scope="module")
+def ctx(built_library):
+    c = GpuContext(0)
+    yield c
+    c.close()
+
+
+def deck_of(natpro, half_box, natlig, nposes, seed=0, ntypes=12):
+    return synthetic_deck(DeckSpec("cull", natpro, half_box, natlig, ntypes, nposes), seed=seed)
+
+
+def energies(ctx, deck, shapes=SHAPES):
+    ctx.upload(deck)
+    ctx.run(ctx.default_cfg(8, 128))
+    want = ctx.download()
+    for p, w, u in shapes:
+        ctx.run(launch_cfg(p, w, 1, 64, u))
+        assert np.array_equal(ctx.download(), want), (p, w, u)
+    return want
+
+
+def assert_parity(got, deck):
+    e32, e64 = oracle.fasten_f32(deck), oracle.fasten_f64(deck)
+    scale = np.maximum(np.abs(e64), 1.0)
+    bound = max(2e-4, 4 * float((np.abs(e32 - e64) / scale).max()))
+    max_diff, failed = validate(got, e32)
+    assert not failed and max_diff < 0.025, (max_diff, failed[:5])
+    assert float((np.abs(got - e64) / scale).max()) < bound
+
+
+@pytest.mark.parametrize("natpro", [1, 31, 32, 33, 1023, 1024, 1025, 2080])
+def test_protein_sizes_around_clusters(ctx, natpro):
+    deck = deck_of(natpro, 0.5 * (natpro / 0.05) ** (1 / 3), 5, 130, seed=natpro)
+    assert_parity(energies(ctx, deck), deck)
+
+
+@pytest.mark.parametrize("nposes", [1, 63, 64, 65, 255, 257, 4095, 4097, 8200])
+def test_pose_counts_around_groups_and_chunks(ctx, nposes):
+    deck = deck_of(400, 10.0, 3, nposes, seed=3)
+    got = energies(ctx, deck)
+    assert_parity(got[-256:], deck_tail(deck, 256))
+    # a pose's energy is its own: the head of a longer run has the same bits
+    assert np.array_equal(energies(ctx, deck_of(400, 10.0, 3, 9000, seed=3), [])[:nposes], got)
+
+
+def deck_tail(deck, n):
+    tail = deck.head(deck.nposes)
+    tail.poses = np.ascontiguousarray(deck.poses[:, -n:])
+    return tail
+
+
+def test_more_candidates_than_a_list_holds(ctx):
+    # 3,000 atoms within 6 A: every one is in reach of every group.
+    deck = deck_of(3000, 6.0, 3, 600, seed=5)
+    assert_parity(energies(ctx, deck), deck)
+
+
+def test_more_atoms_than_the_list_indices_count(ctx):
+    # 140,000 atoms: the pairs of a group lie on both sides of several 2,048-cluster blocks.
+    deck = deck_of(140000, 65.0, 2, 48, seed=6, ntypes=3)
+    assert_parity(energies(ctx, deck, [(1, 32, 1), (1, 64, 2), (8, 512, 4)]), deck)
+
+
+def test_poses_far_from_the_protein(ctx):
+    deck = deck_of(500, 11.0, 4, 700, seed=7)
+    deck.poses = deck.poses.copy()
+    deck.poses[3, ::7] += 40.0       # just out of reach
+    deck.poses[4, 3::11] -= 1e6
+    deck.poses[5, 5::13] = 2.0 ** 37  # the far end of what counts as regular
+    got = energies(ctx, deck)
+    assert_parity(got, deck)
+    assert np.all(got[5::13] == 0.0)
+
+
+def test_group_sums_in_several_windows(ctx):
+    # 1,000 groups of two ligand atoms x 300,000 poses: 1.2 GB of group sums, two windows; the batch
+    # path cuts its windows between chunks of poses.
+    rng = np.random.default_rng(8)
+    base = deck_of(40, 5.0, 4, 8, seed=8)
+    ligand = synthetic_ligand(rng, 2000, 5.0, base.ntypes)
+    poses = synthetic_poses(rng, 300000)
+    deck = base.head(8)
+    deck.ligand, deck.poses = ligand, poses
+    ctx.upload(deck)
+    cfg = launch_cfg(8, 512, 1, 64, 2)
+    ctx.run(cfg)
+    got = ctx.download()
+    cut = 170001
+    ctx.upload_batch(BatchDeck(deck.protein, deck.forcefield, [ligand, ligand],
+                               [np.ascontiguousarray(poses[:, :cut]), np.ascontiguousarray(poses[:, cut:])]))
+    ctx.run_batch(cfg)
+    assert np.array_equal(ctx.download_batch(), got)
+    few = deck.head(8)
+    few.poses = np.ascontiguousarray(poses[:, [0, 1, 150000, 262143, 262144, 268287, 268288, 299999]])
+    e64 = oracle.fasten_f64(few)
+    e32 = oracle.fasten_f32(few)
+    at = got[[0, 1, 150000, 262143, 262144, 268287, 268288, 299999]]
+    scale = np.maximum(np.abs(e64), 1.0)
+    assert (np.abs(at - e64) / scale).max() < max(2e-4, 4 * (np.abs(e32 - e64) / scale).max())
