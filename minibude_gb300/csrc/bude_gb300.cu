@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "../../include/minibude_gb300.h"
+#include "deck_tables.cuh"
 #include "edge_pose.cuh"
 #include "exact_shape.h"
 #include "internal.h"
@@ -67,18 +68,6 @@ const char *last_error() { return g_last_error; }
 // ---------------------------------------------------------------------------------------------
 static int round_up(int v, int m) { return (v + m - 1) / m * m; }
 
-// The distance past which the pair energy of ligand type L and a protein atom of type Pp is exactly
-// zero (the cut-offs of pair_record's three terms), with room for the rounding of r and of the
-// constants (below 1e-5 of the distance, and 1e-6 A of the charge term's).
-static float pair_reach2(const bude_ffparams &L, const bude_ffparams &Pp, const float *rec) {
-  const double radij = (double)Pp.radius + (double)L.radius;
-  double past = 0.0;
-  if (rec[6] != 0.f) past = -1.0 / (double)rec[11];
-  if (rec[8] != 0.f) past = std::max(past, -1.0 / (double)rec[13]);
-  const double reach = (radij + past) * (1.0 + 1e-5) + 1e-4;
-  return (float)(reach * reach * (1.0 + 1e-6));
-}
-
 // The protein's atoms ordered so that runs of kClusterAtoms lie near each other: halved along the
 // longer side of their bounding box, at a multiple of kClusterAtoms, until a run is left.
 static void cluster_order(const bude_atom *protein, int *order, int n) {
@@ -108,60 +97,6 @@ static void cluster_order(const bude_atom *protein, int *order, int n) {
   cluster_order(protein, order + half, n - half);
 }
 
-// The deck's tables (CullArgs): slab[t][j] = pair constants of ligand type t against the j-th protein atom in
-// cluster order, reach[t][j] = {its position, the pair's squared reach}; rows padded to natpro_pad.
-struct DeckTables {
-  std::vector<float> slab, reach, box, box_reach;
-  float lo[3], hi[3];
-};
-static void build_tables(const bude_atom *protein, int natpro, const bude_ffparams *ff, int ntypes, int natpro_pad,
-                         DeckTables &t) {
-  std::vector<int> order((size_t)natpro);
-  for (int i = 0; i < natpro; ++i) order[(size_t)i] = i;
-  cluster_order(protein, order.data(), natpro);
-  const int clusters = natpro_pad / kClusterAtoms;
-  t.slab.assign((size_t)ntypes * natpro_pad * kPairF4 * 4, 0.f);
-  t.reach.assign((size_t)ntypes * natpro_pad * 4, 0.f);
-  t.box.assign((size_t)clusters * 8, 0.f);
-  t.box_reach.assign((size_t)ntypes * clusters, -1.f);
-  float most = 0.f;
-  for (int l = 0; l < ntypes; ++l)
-    for (int j = 0; j < natpro_pad; ++j) {
-      float rec[kRecFloats];
-      float *r = t.reach.data() + ((size_t)l * natpro_pad + j) * 4;
-      if (j < natpro) {
-        const bude_atom &p = protein[order[(size_t)j]];
-        pair_record(ff[l], ff[p.type], p.x, p.y, p.z, rec);
-        r[3] = pair_reach2(ff[l], ff[p.type], rec);
-        r[0] = p.x, r[1] = p.y, r[2] = p.z;
-      } else {
-        null_record(rec);
-        r[0] = rec[0], r[1] = rec[2], r[2] = rec[4], r[3] = -1.f;
-      }
-      const float pair[kPairF4 * 4] = {rec[0],  rec[2],  rec[4],  rec[6],  rec[8], rec[10],
-                                       rec[11], rec[12], rec[13], rec[14], 0.f,    0.f};
-      std::copy(pair, pair + kPairF4 * 4, t.slab.data() + ((size_t)l * natpro_pad + j) * kPairF4 * 4);
-      float &c = t.box_reach[(size_t)l * clusters + j / kClusterAtoms];
-      if (!(r[3] <= c)) c = r[3]; // a NaN stays and lets the cluster through
-      most = std::max(most, r[3]);
-    }
-  for (int d = 0; d < 3; ++d) t.lo[d] = FLT_MAX, t.hi[d] = -FLT_MAX;
-  for (int k = 0; k < clusters; ++k)
-    for (int d = 0; d < 3; ++d) {
-      float lo = FLT_MAX, hi = -FLT_MAX;
-      for (int j = k * kClusterAtoms; j < std::min(natpro, (k + 1) * kClusterAtoms); ++j) {
-        const float v = (&protein[order[(size_t)j]].x)[d];
-        lo = std::min(lo, v);
-        hi = std::max(hi, v);
-      }
-      t.box[(size_t)k * 8 + d] = lo;
-      t.box[(size_t)k * 8 + 4 + d] = hi;
-      t.lo[d] = std::min(t.lo[d], lo);
-      t.hi[d] = std::max(t.hi[d], hi);
-    }
-  for (int d = 0; d < 3; ++d) t.lo[d] -= std::sqrt(most), t.hi[d] += std::sqrt(most);
-}
-
 int ensure_slab(Context &c, const bude_atom *protein, int natpro, const bude_ffparams *ff, int ntypes, bool *rebuilt) {
   std::vector<unsigned char> key(2 * sizeof(int) + (size_t)natpro * sizeof(bude_atom) +
                                  (size_t)ntypes * sizeof(bude_ffparams));
@@ -176,28 +111,46 @@ int ensure_slab(Context &c, const bude_atom *protein, int natpro, const bude_ffp
   c.ntypes = ntypes;
   c.natpro = natpro;
   c.natpro_pad = std::max(round_up(natpro, kClusterAtoms), kClusterAtoms);
-  DeckTables t;
-  build_tables(protein, natpro, ff, ntypes, c.natpro_pad, t);
-  struct Part {
-    DevBuf *buf;
-    const void *src;
-    size_t bytes;
-  };
-  const Part parts[] = {{&c.slab, t.slab.data(), t.slab.size() * sizeof(float)},
-                        {&c.reach, t.reach.data(), t.reach.size() * sizeof(float)},
-                        {&c.box, t.box.data(), t.box.size() * sizeof(float)},
-                        {&c.box_reach, t.box_reach.data(), t.box_reach.size() * sizeof(float)},
-                        {&c.raw_protein, protein, (size_t)natpro * sizeof(bude_atom)},
-                        {&c.raw_ff, ff, (size_t)ntypes * sizeof(bude_ffparams)}};
-  for (const Part &p : parts) {
-    const int rc = p.buf->reserve(std::max<size_t>(p.bytes, 16), "deck tables");
-    if (rc) return rc;
+  const int clusters = c.natpro_pad / kClusterAtoms;
+  const size_t records = (size_t)ntypes * c.natpro_pad;
+  const size_t nb = (size_t)natpro * sizeof(bude_atom), nf = (size_t)ntypes * sizeof(bude_ffparams);
+  int rc = c.slab.reserve(records * kPairF4 * sizeof(float4), "deck tables");
+  if (!rc) rc = c.reach.reserve(records * sizeof(float4), "deck tables");
+  if (!rc) rc = c.box.reserve((size_t)clusters * 2 * sizeof(float4), "deck tables");
+  if (!rc) rc = c.box_reach.reserve((size_t)ntypes * clusters * sizeof(float), "deck tables");
+  if (!rc) rc = c.raw.reserve(2 * nb + nf, "deck records");
+  if (rc) return rc;
+  // One copy: the protein in cluster order, the protein as given, the forcefield.
+  std::vector<int> order((size_t)natpro);
+  for (int i = 0; i < natpro; ++i) order[(size_t)i] = i;
+  cluster_order(protein, order.data(), natpro);
+  std::vector<unsigned char> raw(2 * nb + nf);
+  auto *sorted = reinterpret_cast<bude_atom *>(raw.data());
+  for (int i = 0; i < natpro; ++i) sorted[i] = protein[order[(size_t)i]];
+  if (nb) std::memcpy(raw.data() + nb, protein, nb);
+  std::memcpy(raw.data() + 2 * nb, ff, nf);
+  cudaError_t e = copy_sync(c, c.raw.ptr, raw.data(), raw.size(), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) return cuda_error(e, "deck upload");
+  c.raw_protein = c.raw.as<bude_atom>() + natpro;
+  c.raw_ff = reinterpret_cast<const bude_ffparams *>(c.raw.as<bude_atom>() + 2 * (size_t)natpro);
+  deck_table_kernel<<<deck_table_grid(ntypes, clusters), 256, 0, c.stream>>>(
+      c.raw.as<bude_atom>(), natpro, c.raw_ff, ntypes, c.natpro_pad, clusters, c.slab.as<float4>(), c.reach.as<float4>(),
+      c.box.as<float4>(), c.box_reach.as<float>(), nullptr, 0u);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_error(e, "deck_table_kernel launch");
+  // Where ligand atoms can interact at all (only how well the positions are binned depends on it): the
+  // protein's box and twice the largest radius plus the longest cut-off.
+  float wide = 0.f;
+  for (int t = 0; t < ntypes; ++t) wide = std::max(wide, 2.f * std::fabs(ff[t].radius) + kNpNpDist);
+  for (int d = 0; d < 3; ++d) {
+    c.reach_lo[d] = FLT_MAX, c.reach_hi[d] = -FLT_MAX;
+    for (int i = 0; i < natpro; ++i) {
+      c.reach_lo[d] = std::min(c.reach_lo[d], (&protein[i].x)[d]);
+      c.reach_hi[d] = std::max(c.reach_hi[d], (&protein[i].x)[d]);
+    }
+    c.reach_lo[d] -= wide;
+    c.reach_hi[d] += wide;
   }
-  for (const Part &p : parts) {
-    const cudaError_t e = copy_sync(c, p.buf->ptr, p.src, p.bytes, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return cuda_error(e, "deck table upload");
-  }
-  for (int d = 0; d < 3; ++d) c.reach_lo[d] = t.lo[d], c.reach_hi[d] = t.hi[d];
   c.host_ff.assign(ff, ff + ntypes);
   // The protein's half of the regular-deck bounds (edge_pose.cuh); types were checked by the caller.
   c.protein_regular = true;
@@ -234,9 +187,9 @@ EdgeArgs edge_args_single(const Context &c, const float4 *ligand, int natlig, bo
   a.nlig = 1;
   a.ligand = ligand;
   a.natlig = natlig;
-  a.protein = c.raw_protein.as<bude_atom>();
+  a.protein = c.raw_protein;
   a.natpro = c.natpro;
-  a.ff = c.raw_ff.as<bude_ffparams>();
+  a.ff = c.raw_ff;
   a.xform = xform;
   return a;
 }
@@ -474,8 +427,7 @@ void destroy_context(Context *c) {
   c->err.release();
   c->flush.release();
   c->partial.release();
-  c->raw_protein.release();
-  c->raw_ff.release();
+  c->raw.release();
   c->edge_mask.release();
   release_batch(*c);
   release_surrogate(*c);

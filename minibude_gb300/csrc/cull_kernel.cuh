@@ -41,6 +41,7 @@
 #include "edge_pose.cuh"
 #include "exact_shape.h"
 #include "ptx.cuh"
+#include "warp.cuh"
 
 namespace bude {
 
@@ -97,18 +98,6 @@ struct HilbertTable {
   }
 };
 static __device__ constexpr HilbertTable kHilbert{};
-
-// Smallest and largest value of a warp (a NaN gives way to a number).
-__device__ __forceinline__ float warp_min(float v) {
-  float r;
-  asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-  return r;
-}
-__device__ __forceinline__ float warp_max(float v) {
-  float r;
-  asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-  return r;
-}
 
 // Squared distance of the box [lo, hi] to the box [plo, phi].
 __device__ __forceinline__ float box_d2(float3 lo, float3 hi, float4 plo, float4 phi) {

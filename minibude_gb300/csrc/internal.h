@@ -64,7 +64,9 @@ struct Context {
   float reach_lo[3] = {}, reach_hi[3] = {};
   // Irregular poses and decks (edge_pose.cuh): the raw protein and forcefield records, the
   // transform pass's irregular-pose bits of the deck's poses, and whether the deck is irregular.
-  DevBuf raw_protein, raw_ff, edge_mask;
+  DevBuf raw, edge_mask; // raw: the protein in cluster order, as given, the forcefield
+  const bude_atom *raw_protein = nullptr; // as given
+  const bude_ffparams *raw_ff = nullptr;
   std::vector<bude_ffparams> host_ff; // the forcefield the slab was built from
   bool protein_regular = true;      // every protein atom and its forcefield record within bounds
   float protein_min_radius = 0.f;   // smallest radius of the protein's atom types

@@ -39,7 +39,7 @@ BUDE_HD inline void pair_record(const bude_ffparams &L, const bude_ffparams &Pp,
   const float l_hphb = L.hphb * ((p_gtz && l_ltz) ? -1.f : 1.f);
   const float distdslv = p_ltz ? (l_ltz ? kNpNpDist : kNpPDist) : (l_ltz ? kNpPDist : -FLT_MAX);
   const bool dslv_on = p_nz && distdslv > 0.f; // -FLT_MAX distance: the term can never fire
-  const double r_distdslv = dslv_on ? 1.0 / (double)distdslv : 1.0;
+  const double r_distdslv = dslv_on && distdslv == kNpNpDist ? 1.0 / (double)kNpNpDist : 1.0; // kNpPDist = 1
   const float chrg_init = L.elsc * Pp.elsc;
   const float dslv_init = p_hphb + l_hphb;
   const float k_chrg = kCnstnt * (type_e ? -fabsf(chrg_init) : chrg_init);
