@@ -295,8 +295,8 @@ int bude_gpu_selftest_wait(bude_gpu_ctx *ctx, int32_t limit_us, float *elapsed_m
  * poses + k*pose_stride, and the output energies[nposes]; host memory and other GPUs' memory give
  * BUDE_ERR_ARG.  `stream` is a cudaStream_t (NULL: the default stream); the call reads a status
  * word back and returns after `stream` has drained, with the energies written.  The working
- * memory (per-deck protein slab, pose transforms, irregular-pose bits, status words) is one fixed
- * device array inside the library of about 11 MiB, held by every GPU that loads it until the
+ * memory (the deck's tables, pose transforms, irregular-pose bits, sums, status words) is one fixed
+ * device array inside the library of about 12 MiB, held by every GPU that loads it until the
  * process exits: sizes above BUDE_NOALLOC_MAX_POSES poses or BUDE_NOALLOC_MAX_SLAB_RECORDS slab
  * records (forcefield types x protein atoms rounded up to 8) are rejected with BUDE_ERR_ARG.
  * Calls share that array: calls whose work overlaps on one GPU race and must be serialised by the

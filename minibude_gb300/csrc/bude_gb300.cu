@@ -2,7 +2,7 @@
 //
 // It owns what the reference's CudaBude owns (src/cuda/fasten.hpp:174-305): device selection,
 // device buffers for the deck, kernel launches, per-iteration timing and the copy back -- plus
-// the per-deck slab of protein records the exact kernel streams (see exact_kernel.cuh).
+// the per-deck tables the exact kernel reads (see deck_tables.cuh, cull_kernel.cuh).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -135,7 +135,7 @@ int ensure_slab(Context &c, const bude_atom *protein, int natpro, const bude_ffp
   c.raw_ff = reinterpret_cast<const bude_ffparams *>(c.raw.as<bude_atom>() + 2 * (size_t)natpro);
   deck_table_kernel<<<deck_table_grid(ntypes, clusters), 256, 0, c.stream>>>(
       c.raw.as<bude_atom>(), natpro, c.raw_ff, ntypes, c.natpro_pad, clusters, c.slab.as<float4>(), c.reach.as<float4>(),
-      c.box.as<float4>(), c.box_reach.as<float>(), nullptr, 0u);
+      c.box.as<float4>(), c.box_reach.as<float>());
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_error(e, "deck_table_kernel launch");
   // Where ligand atoms can interact at all (only how well the positions are binned depends on it): the

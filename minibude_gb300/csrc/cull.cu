@@ -11,10 +11,13 @@ namespace bude {
 
 constexpr size_t kCullMaxSmem = 200 * 1024; // 16 poses per thread x 512 threads: 185 KB
 
+int cull_supers(int natpro_pad, const bude_launch_cfg &s) {
+  return natpro_pad <= 65536 && cull_smem_bytes(s.ppwi * s.wgsize, s.wgsize, s.unroll, 1) <= kCullMaxSmem;
+}
+
 static CullArgs cull_args(const Context &c, const bude_launch_cfg &s) {
   CullArgs a{};
-  a.supers = c.natpro_pad <= 65536 &&
-             cull_smem_bytes(s.ppwi * s.wgsize, s.wgsize, s.unroll, 1) <= kCullMaxSmem;
+  a.supers = cull_supers(c.natpro_pad, s);
   a.slab = c.slab.as<float4>();
   a.reach = c.reach.as<float4>();
   a.box = c.box.as<float4>();
@@ -59,64 +62,79 @@ int prepare_shape(const bude_launch_cfg &shape) {
   return e == cudaSuccess ? BUDE_OK : cuda_error(e, "launch shape");
 }
 
-static int launch(Context &c, const CullArgs &a, long long grid, const bude_launch_cfg &s, cudaStream_t st) {
+static int launch(const CullArgs &a, long long grid, const bude_launch_cfg &s, cudaStream_t st, long long &launches) {
   if (grid > 0x7fffffffLL) return set_error(BUDE_ERR_ARG, "too many poses for one launch");
   int rc = prepare_shape(s);
   if (rc) return rc;
   const cudaError_t e = launch_shape(&a, (unsigned)grid, s, st);
   if (e != cudaSuccess) return cuda_error(e, "cull_kernel launch");
-  c.launches++;
+  launches++;
   return BUDE_OK;
 }
 
-static int finish(Context &c, const FinishArgs &f, long long grid, cudaStream_t st) {
+static int finish(const FinishArgs &f, long long grid, cudaStream_t st, long long &launches) {
   cull_finish_kernel<<<(unsigned)grid, 256, 0, st>>>(f);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_error(e, "cull_finish_kernel launch");
-  c.launches++;
+  launches++;
   return BUDE_OK;
 }
 
 static int cull_groups(int natlig) { return (natlig + kGroupAtoms - 1) / kGroupAtoms; }
 
+SumsWindow sums_window(int natlig, long long nposes, const bude_launch_cfg &cfg, size_t most) {
+  SumsWindow w;
+  w.chunk = even_chunk(nposes, cfg.ppwi * cfg.wgsize);
+  const long long floats = std::max((long long)(most / sizeof(float)), (long long)w.chunk);
+  w.groups = (int)std::min<long long>(cull_groups(natlig), floats / w.chunk);
+  w.poses = std::min(nposes, floats / std::max(w.groups, 1) / w.chunk * w.chunk);
+  return w;
+}
+
+int cull_range(CullArgs a, FinishArgs f, const bude_launch_cfg &cfg, const SumsWindow &w, int natlig, long long nposes,
+               cudaStream_t st, long long &launches) {
+  const int groups = cull_groups(natlig);
+  const float *xform = a.xform;
+  a.natlig = natlig;
+  a.chunk = w.chunk;
+  f.sums = a.sums;
+  for (long long w0 = 0; w0 < nposes; w0 += w.poses) {
+    const long long n = std::min(w.poses, nposes - w0);
+    a.nposes = f.n = n;
+    a.xform = xform + 12 * w0;
+    a.stride = f.stride = n;
+    a.chunks = (int)((n + a.chunk - 1) / a.chunk);
+    f.first = w0;
+    int g = 0;
+    do {
+      a.group0 = g;
+      f.groups = std::min(w.groups, groups - g);
+      f.more = g > 0;
+      g += f.groups;
+      f.last = g >= groups;
+      int rc = f.groups > 0 ? launch(a, (long long)f.groups * a.chunks, cfg, st, launches) : BUDE_OK;
+      if (!rc) rc = finish(f, (n + 255) / 256, st, launches);
+      if (rc) return rc;
+    } while (g < groups);
+  }
+  return BUDE_OK;
+}
+
 int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *ligand, int natlig, bool all_irregular,
                        const unsigned *mask, const float *xform, float *energies, long long nposes) {
   if (nposes == 0) return BUDE_OK;
-  const int groups = cull_groups(natlig);
-  const int most = cfg.ppwi * cfg.wgsize;
+  const SumsWindow w = sums_window(natlig, nposes, cfg, kSumsBytes);
+  const int rc = c.partial.reserve((size_t)w.groups * w.poses * sizeof(float), "group sums");
+  if (rc) return rc;
   CullArgs a = cull_args(c, cfg);
   a.ligand = ligand;
   a.xform = xform;
-  a.natlig = natlig;
-  a.chunk = even_chunk(nposes, most);
-  // The group sums of a window of poses, [groups][window], at most kSumsBytes (and at least a chunk).
-  const long long fit = (long long)(kSumsBytes / sizeof(float)) / std::max(groups, 1) / a.chunk * a.chunk;
-  const long long window = std::min(nposes, std::max(fit, (long long)a.chunk));
-  if (groups > 0) {
-    const int rc = c.partial.reserve((size_t)groups * window * sizeof(float), "group sums");
-    if (rc) return rc;
-  }
+  a.sums = c.partial.as<float>();
   FinishArgs f{};
-  f.groups = groups;
   f.energies = energies;
   f.edges = mask != nullptr;
   f.e = edge_args_single(c, ligand, natlig, all_irregular, mask, xform);
-  a.sums = c.partial.as<float>();
-  f.sums = a.sums;
-  for (long long w0 = 0; w0 < nposes; w0 += window) {
-    const long long n = std::min(window, nposes - w0);
-    a.nposes = n;
-    a.xform = xform + 12 * w0;
-    a.stride = n;
-    a.chunks = (int)((n + a.chunk - 1) / a.chunk);
-    int rc = groups > 0 ? launch(c, a, (long long)groups * a.chunks, cfg, c.stream) : BUDE_OK;
-    f.stride = n;
-    f.first = w0;
-    f.n = n;
-    if (!rc) rc = finish(c, f, (n + 255) / 256, c.stream);
-    if (rc) return rc;
-  }
-  return BUDE_OK;
+  return cull_range(a, f, cfg, w, natlig, nposes, c.stream, c.launches);
 }
 
 CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vector<long long> &first,
@@ -183,14 +201,15 @@ int enqueue_plan(Context &c, const bude_launch_cfg &shape, const CullPlan &plan,
   f.sums = sums;
   f.energies = energies;
   f.edges = edges;
+  f.last = 1;
   f.e = edge_args_batch(c, xform);
   for (const CullPlan::Window &w : plan.windows) {
     a.items = items + w.item0;
     a.stride = f.stride = w.n;
     a.first = f.first = w.first;
-    int rc = w.items > 0 ? launch(c, a, w.items, shape, st) : BUDE_OK;
+    int rc = w.items > 0 ? launch(a, w.items, shape, st, c.launches) : BUDE_OK;
     f.folds = folds + w.fold0;
-    if (!rc && w.folds > 0) rc = finish(c, f, w.folds, st);
+    if (!rc && w.folds > 0) rc = finish(f, w.folds, st, c.launches);
     if (rc) return rc;
   }
   return BUDE_OK;

@@ -7,6 +7,9 @@
 
 namespace bude {
 
+struct CullArgs;
+struct FinishArgs;
+
 // A batch evaluation's work, cut for one launch shape: block items and finish items in windows of
 // consecutive poses, each window's group sums at most kSumsBytes.
 struct CullPlan {
@@ -29,6 +32,18 @@ inline int even_chunk(long long n, int most) {
   const long long per = chunks > 0 ? (n + chunks - 1) / chunks : 1;
   return (int)((per + 31) / 32 * 32 < most ? (per + 31) / 32 * 32 : most);
 }
+
+// One ligand's poses, evaluated in windows whose group sums, [groups][poses], take at most `most` bytes
+// (and room for one group of a chunk).
+struct SumsWindow {
+  int chunk, groups;
+  long long poses;
+};
+SumsWindow sums_window(int natlig, long long nposes, const bude_launch_cfg &cfg, size_t most);
+int cull_range(CullArgs a, FinishArgs f, const bude_launch_cfg &cfg, const SumsWindow &w, int natlig, long long nposes,
+               cudaStream_t st, long long &launches);
+// Whether the groups of a launch share candidate lists (CullArgs::supers).
+int cull_supers(int natpro_pad, const bude_launch_cfg &shape);
 
 // Plan of the poses [first[i], first[i] + count[i]) of ligand lig[i]; first ascending.
 CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vector<long long> &first,

@@ -2,9 +2,21 @@
 // can interact are evaluated.
 //
 // Computes, for every pose, the energy of reference `fasten_main` (src/cuda/fasten.hpp:20-161,
-// src/serial/fasten.hpp:18-132).  The pair energy is the restated form of exact_kernel.cuh: three
-// saturating FMAs of the distance, each exactly zero past its own cut-off.  A pair past all three
-// adds +0, so leaving it out changes no bit of a sum.  Of the 4,096 x 64 pairs of a pose of the
+// src/serial/fasten.hpp:18-132).
+//
+// Restatement of the pair energy.  For a ligand atom of type L and a protein atom of type P at
+// distance r (radij = radius_L + radius_P), the reference's three terms are piecewise linear in r
+// and each one is zero past its cut-off:
+//   steric   76 * (1 - r/radij)                          for r < radij
+//   charge   45*c * clamp(1 - (r - radij)/elcdst, 0, 1)  (c = elsc_L*elsc_P, sign forced negative
+//                                                        when either type is 'E'; elcdst 4 or 2)
+//   desolv   d * clamp(1 - (r - radij)/distdslv, 0, 1)   (d = signed hphb sum; zero unless the
+//                                                        protein hphb is non-zero and distdslv > 0)
+// The steric factor lies in [0, 1] as well (r >= 0), so all three are one `fma.rn.sat` each with
+// per-type-pair constants (pair_record.h).  One interaction is 3 FADD + FMUL + 2 FFMA (distance^2),
+// one MUFU square root, 3 FFMA.SAT and 3 FFMA: 12 FP32 operations against the reference's ~30.
+//
+// A pair past all three cut-offs adds +0, so leaving it out changes no bit of a sum.  Of the 4,096 x 64 pairs of a pose of the
 // scaled-up workload 0.8% interact, of a 2,672-atom protein at real density 1.8%.
 //
 // What makes the pairs cheap to find: a rotated ligand atom of many poses fills a ball of a few
@@ -60,10 +72,12 @@ struct CullArgs {
   long long stride, first;
   long long nposes;      // without items: poses of the ligand
   float3 lo, hi;         // protein atoms' bounding box, widened by the longest reach
+  const unsigned *words; // optional: a deck checked on the device (edge_pose.cuh); nothing runs on a bad one
   int natlig;            // without items: the ligand's atoms
+  int group0;            // without items: the first group (row 0 of sums)
   int chunk, chunks;     // without items: poses of a chunk (at most K * blockDim.x) and chunks of the ligand
-  int natpro_pad;        // multiple of kClusterAtoms
-  int clusters;          // natpro_pad / kClusterAtoms
+  int natpro_pad;        // records per type
+  int clusters;          // of kClusterAtoms; the last may be short
   int supers;            // groups share lists of candidates (protein indices below 65,536)
 };
 
@@ -232,11 +246,11 @@ __device__ __forceinline__ unsigned near_clusters(float3 lo, float3 hi, int c0, 
 // The next four clusters of `todo` (bits from cluster c0 on): this lane's atom of each, as an index from
 // cluster `base` on, and its entry of `reach`; a reach of -1 where there is none.
 __device__ __forceinline__ void next_clusters(unsigned &todo, int c0, int base, const float4 *reach, int (&at)[4],
-                                              float4 (&t)[4]) {
+                                              int atoms, float4 (&t)[4]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int atom = (c0 + __ffs(todo) - 1) * kClusterAtoms + (threadIdx.x & 31);
-    t[i] = todo ? __ldg(&reach[atom]) : make_float4(0.f, 0.f, 0.f, -1.f);
+    t[i] = todo && atom < atoms ? __ldg(&reach[atom]) : make_float4(0.f, 0.f, 0.f, -1.f);
     at[i] = atom - base * kClusterAtoms;
     todo &= todo - 1u;
   }
@@ -284,7 +298,7 @@ __device__ __forceinline__ void cull_eval(Points<P> &pt, float3 lo, float3 hi, i
         }
         more = todo || pos < a.clusters;
         if (!todo) break;
-        next_clusters(todo, c0, base, reach, at, t);
+        next_clusters(todo, c0, base, reach, at, a.natpro_pad, t);
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i) push_hits(l.at, count, lo, hi, t[i], at[i]);
@@ -338,12 +352,13 @@ template <int K, int P> __global__ void __launch_bounds__(kMaxThreads, 2) cull_k
     const int4 it = __ldg(&a.items[blockIdx.x]);
     atom0 = it.x, natoms = it.y & 255, group = it.y >> 8, pose0 = it.z, n = it.w;
   } else {
-    group = (int)(blockIdx.x / (unsigned)a.chunks);
+    group = (int)(blockIdx.x / (unsigned)a.chunks) + a.group0;
     pose0 = (long long)(blockIdx.x % (unsigned)a.chunks) * a.chunk;
     atom0 = group * kGroupAtoms;
     natoms = min(kGroupAtoms, a.natlig - atom0);
     n = (int)min((long long)a.chunk, a.nposes - pose0);
   }
+  if (a.words && deck_bad_type(a.words)) return;
   const float4 *xf = reinterpret_cast<const float4 *>(a.xform) + pose0 * 3;
 
   // Range of the chunk's translations (regular poses, edge_pose.cuh).
@@ -450,7 +465,7 @@ template <int K, int P> __global__ void __launch_bounds__(kMaxThreads, 2) cull_k
           while (todo && count <= kCandidates) {
             int at[4];
             float4 t[4];
-            next_clusters(todo, c0, 0, reach, at, t);
+            next_clusters(todo, c0, 0, reach, at, a.natpro_pad, t);
 #pragma unroll
             for (int i = 0; i < 4; ++i) push_hits(cand[sg].at, count, lo, hi, t[i], at[i]);
           }
@@ -481,7 +496,7 @@ template <int K, int P> __global__ void __launch_bounds__(kMaxThreads, 2) cull_k
     }
     __syncthreads();
     // 6. the atom's energies in pose order, added to the group's
-    float *out = a.sums + (long long)group * a.stride + (pose0 - a.first);
+    float *out = a.sums + (long long)(group - a.group0) * a.stride + (pose0 - a.first);
     float *flat = reinterpret_cast<float *>(pts);
     float e[K];
     int at[K];
@@ -509,8 +524,10 @@ struct FinishArgs {
   const float *sums; // [group][stride], from pose `first` on
   long long stride, first, n;
   int groups;
+  int more, last; // the sums add to what energies hold; these are the last groups
   const int4 *folds;
   float *energies;
+  const unsigned *words; // as CullArgs::words; its deck decides whether every pose is irregular
   int edges;
   EdgeArgs e;
 };
@@ -519,6 +536,10 @@ static __global__ void __launch_bounds__(256) cull_finish_kernel(const FinishArg
   long long p0 = a.first + (long long)blockIdx.x * blockDim.x, p1 = min(p0 + blockDim.x, a.first + a.n);
   int groups = a.groups;
   bool all = a.e.all != 0;
+  if (a.words) {
+    if (deck_bad_type(a.words)) return;
+    all = deck_irregular(a.words, a.e.natpro, a.e.natlig);
+  }
   if (a.folds) {
     const int4 f = __ldg(&a.folds[blockIdx.x]);
     p0 = f.x, p1 = (long long)f.x + f.y, groups = f.z;
@@ -529,7 +550,7 @@ static __global__ void __launch_bounds__(256) cull_finish_kernel(const FinishArg
     bool irregular = false;
     if (p < p1) {
       const float *s = a.sums + (p - a.first);
-      float acc = 0.f;
+      float acc = a.more ? a.energies[p] : 0.f;
       int g = 0;
       for (; g + 8 <= groups; g += 8) {
         float v[8];
@@ -539,8 +560,8 @@ static __global__ void __launch_bounds__(256) cull_finish_kernel(const FinishArg
         for (int j = 0; j < 8; ++j) acc = __fadd_rn(acc, v[j]);
       }
       for (; g < groups; ++g) acc = __fadd_rn(acc, s[(long long)g * a.stride]);
-      a.energies[p] = 0.5f * acc;
-      irregular = a.edges && (all || ((a.e.mask[p >> 5] >> (p & 31)) & 1u));
+      a.energies[p] = a.last ? 0.5f * acc : acc;
+      irregular = a.edges && a.last && (all || ((a.e.mask[p >> 5] >> (p & 31)) & 1u));
     }
     unsigned bits = __ballot_sync(0xffffffffu, irregular);
     while (bits) {

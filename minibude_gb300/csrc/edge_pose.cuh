@@ -1,7 +1,7 @@
-// edge_pose.cuh -- poses and decks outside the range where exact_kernel's restated pair energy is
+// edge_pose.cuh -- poses and decks outside the range where cull_kernel's restated pair energy is
 // the reference's, and the kernel that scores them with the reference's own arithmetic.
 //
-// exact_kernel.cuh evaluates each pair term as one saturating FMA (fma.rn.sat.f32), which turns a
+// cull_kernel.cuh evaluates each pair term as one saturating FMA (fma.rn.sat.f32), which turns a
 // NaN into +0 and relies on radij > 0.  The reference (src/serial/fasten.hpp:98-124) instead
 // propagates non-finite values: a NaN or infinite pose, a translation large enough that
 // x*x + y*y + z*z overflows (|d| > ~1.8e19 A), or a radius sum of zero gives a NaN energy, and a
@@ -40,7 +40,7 @@ constexpr float kLigandReach = 0x1p36f;   // |x|+|y|+|z| bound of a ligand atom 
 constexpr float kParamReach = 0x1p20f;    // |radius|, |hphb|, |elsc| bound in a regular deck
 constexpr float kMinRadiusSum = 0x1p-20f; // smallest FP32 radius sum of a regular deck
 
-// A pose whose transform rows {r00, r01, r02, tx}, ... keep exact_kernel exact (NaN fails every
+// A pose whose transform rows {r00, r01, r02, tx}, ... keep cull_kernel exact (NaN fails every
 // comparison, so a non-finite transform is irregular).
 __host__ __device__ __forceinline__ bool pose_regular(float4 r0, float4 r1, float4 r2) {
   const float rs = fabsf(r0.x) + fabsf(r0.y) + fabsf(r0.z) + fabsf(r1.x) + fabsf(r1.y) + fabsf(r1.z) + fabsf(r2.x) +
@@ -90,6 +90,28 @@ __device__ __forceinline__ float ref_pair_energy(const bude_ffparams &l, float l
   float dslv_e = dslv_init * ((distbb < distdslv && p_nz) ? 1.f : 0.f);
   dslv_e *= zone1 ? 1.f : coeff;
   return e + dslv_e;
+}
+
+// Floats as unsigned keys of the same order, so that atomicMin finds the smallest radius.
+__device__ __forceinline__ unsigned order_key(float f) {
+  const unsigned u = __float_as_uint(f);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float key_float(unsigned k) {
+  return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
+}
+
+// A deck checked on the device: word 0 has kDeckBadType where an atom's type lies outside the forcefield
+// and kDeckIrregular where an atom or forcefield record in use is out of bounds; words 1 and 2 are the
+// order keys of the smallest forcefield radius of the protein's and of the ligand's atoms.
+constexpr unsigned kDeckBadProtein = 2u, kDeckBadLigand = 4u, kDeckIrregular = 8u;
+__device__ __forceinline__ bool deck_bad_type(const unsigned *words) {
+  return (words[0] & (kDeckBadProtein | kDeckBadLigand)) != 0;
+}
+// FP32 addition is monotone, so the smallest radii bound every pair's sum; without a pair every energy is 0.
+__device__ __forceinline__ bool deck_irregular(const unsigned *words, int natpro, int natlig) {
+  return natpro > 0 && natlig > 0 &&
+         ((words[0] & kDeckIrregular) || !(key_float(words[1]) + key_float(words[2]) >= kMinRadiusSum));
 }
 
 struct EdgeArgs {

@@ -5,24 +5,23 @@
 // hosts that hand a plugin its buffers and forbid it to allocate, and latency-bound loops where
 // cudaMalloc/cudaFree (which can synchronise the device) are not allowed.  They pass device
 // buffers for the inputs and the output; the working memory the evaluation needs beyond those --
-// the per-deck protein slab, the pose transforms and an error word -- comes from one fixed
-// file-scope array in device memory, `g_noalloc_scratch`, instead of the cudaMalloc'd buffers of
-// a bude_gpu_ctx.
+// the deck's tables, the pose transforms, sums and check words -- comes from one fixed file-scope
+// array in device memory, `g_noalloc_scratch`, instead of the cudaMalloc'd buffers of a bude_gpu_ctx.
 //
 // Rules of the array:
 //   * its size is fixed at build time (BUDE_NOALLOC_MAX_POSES transforms and
-//     BUDE_NOALLOC_MAX_SLAB_RECORDS slab records, about 11 MiB), and every GPU that loads this
+//     BUDE_NOALLOC_MAX_SLAB_RECORDS slab records, about 12 MiB), and every GPU that loads this
 //     module holds it until the process exits;
-//   * every call on a device shares it and it keeps the last call's contents: the error and check
-//     words are reset at the start of each call, the slab, transforms and irregular-pose bits are
-//     rewritten in full;
+//   * every call on a device shares it and it keeps the last call's contents: each call rewrites
+//     what it reads;
 //   * calls whose work overlaps on one GPU (two host threads, or two streams) race on it and
 //     must be serialised by the caller;
 //   * in host code the array's name is only a stand-in: its device address is looked up once per
 //     device with cudaGetSymbolAddress, with that device current, by the first call made on the
 //     device, and kept for the life of the process.  A cudaDeviceReset would leave that address
 //     stale, so the entry point must not be used on a device after it has been reset.
-// Each call reads its error word back and synchronises the stream before it returns.
+// Each call reads its check word back and synchronises the stream before it returns; until then the
+// kernels themselves leave a deck with a bad type alone.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -30,28 +29,34 @@
 #include <cstring>
 #include <mutex>
 
-#include "exact_kernel.cuh"
+#include "cull.h"
+#include "cull_kernel.cuh"
+#include "deck_tables.cuh"
+#include "pose_xform.cuh"
 #include "internal.h"
 #include "pair_record.h"
 
 namespace bude {
 namespace {
 
-constexpr size_t kNaErrBytes = 256;
+constexpr size_t kNaWordBytes = 256; // words [0..2]: the deck's checks (edge_pose.cuh)
 constexpr size_t kNaXformBytes = (size_t)BUDE_NOALLOC_MAX_POSES * 3 * sizeof(float4);
-constexpr size_t kNaSlabBytes = (size_t)BUDE_NOALLOC_MAX_SLAB_RECORDS * kRecF4 * sizeof(float4);
 constexpr size_t kNaMaskBytes = (size_t)BUDE_NOALLOC_MAX_POSES / 32 * sizeof(unsigned);
-constexpr size_t kNaScratchBytes = kNaErrBytes + kNaXformBytes + kNaSlabBytes + kNaMaskBytes;
+// Clusters of the largest protein (one type), and (type, cluster) pairs: a row of 8 records has one.
+constexpr size_t kNaBoxBytes = (size_t)BUDE_NOALLOC_MAX_SLAB_RECORDS / kClusterAtoms * 2 * sizeof(float4);
+constexpr size_t kNaBoxReachBytes = (size_t)BUDE_NOALLOC_MAX_SLAB_RECORDS / kAtomAlign * sizeof(float);
+// Per record its pair constants and its reach; then the protein in cluster order, until the tables are
+// built, and the group sums, which also take what the records leave.
+constexpr size_t kNaRecordBytes = (kPairF4 + 1) * sizeof(float4);
+constexpr size_t kNaTableBytes = (size_t)BUDE_NOALLOC_MAX_SLAB_RECORDS * kNaRecordBytes;
+constexpr int kNaSortMax = 16384; // atoms one block sorts; a larger protein keeps its order
+constexpr size_t kNaSumsBytes = 512 * 1024;
+static_assert(kNaSumsBytes >= kNaSortMax * sizeof(bude_atom), "the protein in cluster order fits the sums");
+constexpr size_t kNaScratchBytes =
+    kNaWordBytes + kNaXformBytes + kNaMaskBytes + kNaBoxBytes + kNaBoxReachBytes + kNaTableBytes + kNaSumsBytes;
 
-// Words of the scratch's first 256 bytes: [0] error bits, [1] and [2] the smallest forcefield
-// radius of the protein's and of the ligand's atoms as order-preserving keys (atomicMin).
-// Error bits (bit 0 is the exact kernel's bounded-wait timeout):
-constexpr unsigned kNaErrProteinType = 2u;
-constexpr unsigned kNaErrLigandType = 4u;
-constexpr unsigned kNaIrregular = 8u; // an atom or forcefield record outside the regular-deck bounds
-
-// The working memory of bude_gpu_fasten_noalloc:
-// [error and check words | pose transforms | protein slab | irregular-pose bits].
+// The working memory of bude_gpu_fasten_noalloc: [check words | pose transforms | irregular-pose bits |
+// cluster boxes | cluster reaches | tables | sums].
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNaScratchBytes];
 
 constexpr int kNaMaxDevices = 64;
@@ -74,66 +79,82 @@ int na_scratch(int device, unsigned char **out) {
   return BUDE_OK;
 }
 
-// The per-ligand-type protein slab, built on the device from device-resident protein and
-// forcefield (the same records as the host build: pair_record is shared).  Atom types outside
-// the forcefield set an error bit and get a padding record instead of being read.
-__global__ void __launch_bounds__(256) na_slab_kernel(const bude_atom *__restrict__ protein, int natpro,
-                                                      const bude_ffparams *__restrict__ ff, int ntypes, int natpro_pad,
-                                                      float4 *__restrict__ slab, unsigned *err) {
-  const long long n = (long long)ntypes * natpro_pad;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const int t = (int)(idx / natpro_pad);
-    const int j = (int)(idx - (long long)t * natpro_pad);
-    float rec[kRecFloats];
-    if (j < natpro) {
-      const bude_atom a = protein[j];
-      if (a.type >= 0 && a.type < ntypes) {
-        pair_record(ff[t], ff[a.type], a.x, a.y, a.z, rec);
-      } else {
-        null_record(rec);
-        atomicOr(err, kNaErrProteinType);
-      }
-    } else {
-      null_record(rec);
-    }
-    float4 *dst = slab + idx * kRecF4;
-#pragma unroll
-    for (int k = 0; k < kRecF4; ++k) dst[k] = make_float4(rec[4 * k], rec[4 * k + 1], rec[4 * k + 2], rec[4 * k + 3]);
-  }
-}
-
-__device__ __forceinline__ unsigned radius_key(float f) {
-  const unsigned u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u); // ascending float order as unsigned order
-}
-
-// Per atom: ligand atom types must index the slab (the exact kernel reads them unchecked), and
-// the atoms and their forcefield records are checked against the regular-deck bounds
-// (edge_pose.cuh); the smallest radii of both sides go to words [1] and [2].  Atoms with a type
-// outside the forcefield are only flagged.
-__global__ void na_deck_check_kernel(const bude_atom *__restrict__ protein, int natpro,
-                                     const bude_atom *__restrict__ ligand, int natlig,
-                                     const bude_ffparams *__restrict__ ff, int ntypes, unsigned *words) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < natpro + natlig; i += gridDim.x * blockDim.x) {
+// One block checks the deck (words, edge_pose.cuh) and writes the protein in cluster order: sorted by the
+// cell of a 16 x 16 x 16 grid over its box (the 8 x 8 x 8 Hilbert cell, then the octant in it) and by
+// index, a bitonic sort of 32-bit keys in shared memory.  Latency-bound, one block: 1,237 atoms take
+// 19 us of a call.
+__global__ void __launch_bounds__(1024) na_deck_kernel(const bude_atom *__restrict__ protein, int natpro,
+                                                       const bude_atom *__restrict__ ligand, int natlig,
+                                                       const bude_ffparams *__restrict__ ff, int ntypes, int sort,
+                                                       unsigned *words, bude_atom *__restrict__ sorted) {
+  extern __shared__ unsigned keys[];
+  __shared__ unsigned flags, min_key[2];
+  __shared__ float red[6][32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) flags = 0, min_key[0] = min_key[1] = 0xffffffffu;
+  __syncthreads();
+  float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+  unsigned bad = 0, least[2] = {0xffffffffu, 0xffffffffu};
+  for (long long i = tid; i < (long long)natpro + natlig; i += blockDim.x) {
     const bool is_lig = i >= natpro;
     const bude_atom a = is_lig ? ligand[i - natpro] : protein[i];
+    if (!is_lig) {
+      lo[0] = fminf(lo[0], a.x), lo[1] = fminf(lo[1], a.y), lo[2] = fminf(lo[2], a.z);
+      hi[0] = fmaxf(hi[0], a.x), hi[1] = fmaxf(hi[1], a.y), hi[2] = fmaxf(hi[2], a.z);
+    }
     if (a.type < 0 || a.type >= ntypes) {
-      if (is_lig) atomicOr(&words[0], kNaErrLigandType); // protein types: na_slab_kernel
+      bad |= is_lig ? kDeckBadLigand : kDeckBadProtein;
       continue;
     }
     const bude_ffparams f = ff[a.type];
-    const bool ok = param_regular(f) && (is_lig ? ligand_atom_regular(a.x, a.y, a.z) : protein_atom_regular(a));
-    if (!ok) atomicOr(&words[0], kNaIrregular);
-    atomicMin(&words[is_lig ? 2 : 1], radius_key(f.radius));
+    if (!param_regular(f) || !(is_lig ? ligand_atom_regular(a.x, a.y, a.z) : protein_atom_regular(a)))
+      bad |= kDeckIrregular;
+    unsigned &l = least[is_lig];
+    l = min(l, order_key(f.radius));
   }
-}
-
-float key_radius(unsigned k) {
-  const unsigned u = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
-  float f;
-  std::memcpy(&f, &u, sizeof f);
-  return f;
+  if (bad) atomicOr(&flags, bad);
+  for (int k = 0; k < 2; ++k) {
+    const unsigned m = __reduce_min_sync(0xffffffffu, least[k]);
+    if (lane == 0) atomicMin(&min_key[k], m);
+  }
+  for (int d = 0; d < 3; ++d) {
+    const float l = warp_min(lo[d]), h = warp_max(hi[d]);
+    if (lane == 0) red[d][warp] = l, red[3 + d][warp] = h;
+  }
+  __syncthreads();
+  if (tid == 0) words[0] = flags, words[1] = min_key[0], words[2] = min_key[1];
+  if (!sort) return;
+  int n2 = 32;
+  while (n2 < natpro) n2 <<= 1;
+  float inv[3];
+  for (int d = 0; d < 3; ++d) {
+    lo[d] = warp_min(red[d][lane]);
+    const float w = warp_max(red[3 + d][lane]) - lo[d];
+    inv[d] = w > 0.f ? 16.f / w : 0.f;
+  }
+  for (int i = tid; i < n2; i += blockDim.x) {
+    unsigned k = 0xffffffffu;
+    if (i < natpro) {
+      const bude_atom a = protein[i];
+      const int x = min(max((int)((a.x - lo[0]) * inv[0]), 0), 15), y = min(max((int)((a.y - lo[1]) * inv[1]), 0), 15),
+                z = min(max((int)((a.z - lo[2]) * inv[2]), 0), 15);
+      const unsigned cell = (unsigned)kHilbert.at[(z >> 1) * 64 + (y >> 1) * 8 + (x >> 1)] * 8u +
+                            (unsigned)((z & 1) * 4 + (y & 1) * 2 + (x & 1));
+      k = cell << 14 | (unsigned)i;
+    }
+    keys[i] = k;
+  }
+  for (int size = 2; size <= n2; size <<= 1)
+    for (int step = size >> 1; step > 0; step >>= 1) {
+      __syncthreads();
+      for (int t = tid; t < n2 / 2; t += blockDim.x) {
+        const int i = 2 * t - (t & (step - 1)), j = i + step;
+        const unsigned u = keys[i], v = keys[j];
+        if ((u > v) == ((i & size) == 0)) keys[i] = v, keys[j] = u;
+      }
+    }
+  __syncthreads();
+  for (int i = tid; i < natpro; i += blockDim.x) sorted[i] = protein[keys[i] & 0x3fffu];
 }
 
 // Read n words from the device into a caller-provided host array (no allocation) and wait.
@@ -193,96 +214,78 @@ extern "C" int bude_gpu_fasten_noalloc(const bude_atom *protein, int32_t natpro,
   unsigned char *scratch = nullptr;
   int rc = na_scratch(device, &scratch);
   if (rc) return rc;
-  unsigned *err = reinterpret_cast<unsigned *>(scratch);
-  float4 *xform = reinterpret_cast<float4 *>(scratch + kNaErrBytes);
-  float4 *slab = reinterpret_cast<float4 *>(scratch + kNaErrBytes + kNaXformBytes);
-  unsigned *mask = reinterpret_cast<unsigned *>(scratch + kNaErrBytes + kNaXformBytes + kNaSlabBytes);
+  unsigned char *at = scratch;
+  auto take = [&at](size_t bytes) {
+    unsigned char *p = at;
+    at += bytes;
+    return p;
+  };
+  unsigned *words = reinterpret_cast<unsigned *>(take(kNaWordBytes));
+  float4 *xform = reinterpret_cast<float4 *>(take(kNaXformBytes));
+  unsigned *mask = reinterpret_cast<unsigned *>(take(kNaMaskBytes));
+  float4 *box = reinterpret_cast<float4 *>(take(kNaBoxBytes));
+  float *box_reach = reinterpret_cast<float *>(take(kNaBoxReachBytes));
+  const size_t records = (size_t)ntypes * natpro_pad;
+  float4 *slab = reinterpret_cast<float4 *>(take(records * kPairF4 * sizeof(float4)));
+  float4 *reach = reinterpret_cast<float4 *>(take(records * sizeof(float4)));
+  unsigned char *rest = at; // the sums, and before them the protein in cluster order
+  const size_t rest_bytes = (size_t)(scratch + kNaScratchBytes - rest);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int sms = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
 
-  // 1. reset the error word and the two radius minima; slab and deck checks.
-  e = cudaMemsetAsync(err, 0, sizeof(unsigned), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(err + 1, 0xff, 2 * sizeof(unsigned), st);
-  if (e != cudaSuccess) return cuda_error(e, "no-alloc error word clear");
-  {
-    const long long n = (long long)ntypes * natpro_pad;
-    const int blocks = (int)std::min<long long>((n + 255) / 256, 8LL * std::max(sms, 1));
-    na_slab_kernel<<<blocks, 256, 0, st>>>(protein, natpro, forcefield, ntypes, natpro_pad, slab, err);
-    if (natpro + natlig > 0)
-      na_deck_check_kernel<<<(unsigned)std::min((natpro + natlig + 255) / 256, 4 * std::max(sms, 1)), 256, 0, st>>>(
-          protein, natpro, ligand, natlig, forcefield, ntypes, err);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_error(e, "no-alloc slab launch");
-  }
-  unsigned h[3] = {0, 0, 0};
-  rc = na_read_words(err, 3, st, h);
-  if (rc) return rc;
-  if (h[0] & (kNaErrProteinType | kNaErrLigandType))
-    return set_error(BUDE_ERR_TYPE, "%s atom type outside the forcefield (%d types)",
-                     (h[0] & kNaErrLigandType) ? "a ligand" : "a protein", ntypes);
-  // The deck is irregular when an atom or record is out of bounds or the smallest FP32 radius sum
-  // is below the bound (FP32 addition is monotone); with no ligand-protein pair every energy is 0.
-  const float min_sum = key_radius(h[1]) + key_radius(h[2]);
-  const bool irregular = natpro > 0 && natlig > 0 && ((h[0] & kNaIrregular) || !(min_sum >= kMinRadiusSum));
-
-  // 2. pose transforms and the exact kernel; protein slices (if any) are summed in a cluster, so
-  //    no slice buffer is needed.
+  // 1. the deck: checks, cluster order and tables.  Nothing after them runs on a deck with a bad type.
+  const int clusters = (natpro_pad + kClusterAtoms - 1) / kClusterAtoms;
+  const bool sort = natpro > kClusterAtoms && natpro <= kNaSortMax;
+  size_t keys = 0;
+  if (sort)
+    for (keys = 32 * sizeof(unsigned); keys < natpro * sizeof(unsigned);) keys *= 2;
+  e = cudaFuncSetAttribute(na_deck_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)(kNaSortMax * sizeof(unsigned)));
+  if (e != cudaSuccess) return cuda_error(e, "no-alloc deck kernel");
+  auto *sorted = reinterpret_cast<bude_atom *>(rest);
+  na_deck_kernel<<<1, 1024, keys, st>>>(protein, natpro, ligand, natlig, forcefield, ntypes, sort, words, sorted);
+  deck_table_kernel<<<deck_table_grid(ntypes, clusters), 256, 0, st>>>(sort ? sorted : protein, natpro, forcefield,
+                                                                       ntypes, natpro_pad, clusters, slab, reach, box,
+                                                                       box_reach);
+  // 2. pose transforms and the exact kernel; irregular poses (or every pose of an irregular deck) by the
+  //    reference's arithmetic.
   pose_xform_kernel<<<(unsigned)((nposes + 255) / 256), 256, 0, st>>>(poses, pose_stride, nposes, xform, mask);
-  constexpr int P = 8, U = 2, W = 128, T = 64;
-  const long long blocks = (nposes + (long long)P * W - 1) / ((long long)P * W);
-  int split = 1;
-  while (split < 8 && blocks * split < 4LL * std::max(sms, 1) && natpro_pad / (split * 2) >= 64) split *= 2;
-  ExactArgs a;
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_error(e, "no-alloc deck launch");
+  const bude_launch_cfg cfg = cull_shape(nposes, natlig, 1);
+  CullArgs a{};
   a.ligand = reinterpret_cast<const float4 *>(ligand);
   a.slab = slab;
+  a.reach = reach;
+  a.box = box;
+  a.box_reach = box_reach;
   a.xform = reinterpret_cast<const float *>(xform);
-  a.energies = energies;
-  a.partial = nullptr;
-  a.err = err;
-  a.nposes = nposes;
-  a.natlig = natlig;
+  a.sums = reinterpret_cast<float *>(rest);
+  a.lo = make_float3(-INFINITY, -INFINITY, -INFINITY); // the poses' own range bins them
+  a.hi = make_float3(INFINITY, INFINITY, INFINITY);
+  a.words = words;
   a.natpro_pad = natpro_pad;
-  a.tile = T;
-  a.split = split;
-  a.cluster = 1;
-  a.slice = ((natpro_pad + split - 1) / split + kAtomAlign - 1) / kAtomAlign * kAtomAlign;
-  const size_t smem = exact_smem_bytes(P, W, T, split, 1);
-  e = cudaFuncSetAttribute(exact_kernel<P, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) {
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3((unsigned)blocks, (unsigned)split, 1);
-    lc.blockDim = dim3(W, 1, 1);
-    lc.dynamicSmemBytes = smem;
-    lc.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = split;
-    attr[0].val.clusterDim.z = 1;
-    lc.attrs = attr;
-    lc.numAttrs = 1;
-    e = cudaLaunchKernelEx(&lc, exact_kernel<P, U>, a);
-  }
-  if (e != cudaSuccess) return cuda_error(e, "no-alloc exact_kernel launch");
-  // 3. irregular poses (or every pose of an irregular deck) by the reference's arithmetic.
-  EdgeArgs ea{};
-  ea.mask = mask;
-  ea.all = irregular ? 1 : 0;
-  ea.nposes = nposes;
-  ea.nlig = 1;
-  ea.ligand = reinterpret_cast<const float4 *>(ligand);
-  ea.natlig = natlig;
-  ea.protein = protein;
-  ea.natpro = natpro;
-  ea.ff = forcefield;
-  ea.xform = reinterpret_cast<const float *>(xform);
-  ea.energies = energies;
-  edge_pose_kernel<<<edge_grid(nposes, sms), 256, 0, st>>>(ea);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_error(e, "no-alloc edge_pose_kernel launch");
-  rc = na_read_words(err, 1, st, h);
+  a.clusters = clusters;
+  a.supers = cull_supers(natpro_pad, cfg);
+  FinishArgs f{};
+  f.energies = energies;
+  f.words = words;
+  f.edges = 1;
+  f.e.mask = mask;
+  f.e.nlig = 1;
+  f.e.ligand = a.ligand;
+  f.e.natlig = natlig;
+  f.e.protein = protein;
+  f.e.natpro = natpro;
+  f.e.ff = forcefield;
+  f.e.xform = a.xform;
+  long long launches = 0;
+  rc = cull_range(a, f, cfg, sums_window(natlig, nposes, cfg, rest_bytes), natlig, nposes, st, launches);
   if (rc) return rc;
-  if (h[0] & 1u) return set_error(BUDE_ERR_TIMEOUT, "a bounded device wait ran out; energies are invalid");
+  unsigned h = 0;
+  rc = na_read_words(words, 1, st, &h);
+  if (rc) return rc;
+  if (h & (kDeckBadProtein | kDeckBadLigand))
+    return set_error(BUDE_ERR_TYPE, "%s atom type outside the forcefield (%d types)",
+                     (h & kDeckBadLigand) ? "a ligand" : "a protein", ntypes);
   return BUDE_OK;
 }

@@ -1,7 +1,7 @@
 // pair_record.h -- the per-(ligand type, protein atom) record the exact kernel streams.
 //
 // Restates the reference's pair set-up (src/serial/fasten.hpp:80-96, constants src/bude.h:22-35)
-// as the constants of the three saturating FMAs of exact_kernel.cuh.  Usable from host and device
+// as the constants of the three saturating FMAs of cull_kernel.cuh.  Usable from host and device
 // code; the derived constants are evaluated in double with explicit fma and rounded to float once,
 // so host and device builds of a record are bit-identical.
 #pragma once

@@ -20,13 +20,9 @@
 #include <vector>
 
 #include "cull.h"
+#include "edge_pose.cuh"
 
 namespace bude {
-
-__device__ __forceinline__ uint32_t order_key(float f) {
-  const uint32_t u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u); // ascending float order as unsigned order
-}
 
 __device__ __forceinline__ uint32_t mix_hash(uint32_t seed, uint32_t i) {
   uint32_t h = seed ^ (i * 0x9E3779B9u);
