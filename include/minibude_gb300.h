@@ -44,13 +44,13 @@ typedef struct bude_ffparams {
 
 /* Kernel launch shape of the exact kernel.  The reference exposes two knobs, PPWI (poses per work
  * item, a template parameter, src/main.cpp:48-53) and wgsize (threads per block,
- * src/cuda/fasten.hpp:272-275).  Here a block takes ppwi * wgsize poses and two ligand atoms, and
+ * src/cuda/fasten.hpp:272-275).  Here a block takes ppwi * wgsize poses and one ligand atom, and
  * evaluates the pairs in reach for 32 * unroll poses at a time.  No field changes an energy's bits. */
 typedef struct bude_launch_cfg {
   int32_t ppwi;    /* poses per thread: 1, 2, 4, 8 or 16 */
   int32_t wgsize;  /* threads per block: a multiple of 32 in [32, 512] */
-  int32_t split;   /* 1..8 with cluster = 1, 1..64 with cluster = 0; checked, without effect: the sums of
-                      two ligand atoms each are what spreads over the GPU and is added up in order */
+  int32_t split;   /* 1..8 with cluster = 1, 1..64 with cluster = 0; checked, without effect: the ligand's
+                      atoms are what spreads over the GPU, and their sums are added up in order */
   int32_t tile;    /* a multiple of 8, 8..512; checked, without effect */
   int32_t unroll;  /* poses per lane of a group evaluated together: 1, 2 or 4 */
   int32_t cluster; /* 0 or 1; checked, without effect */
@@ -166,7 +166,7 @@ int bude_gpu_upload_batch(bude_gpu_ctx *ctx, const bude_atom *protein, int32_t n
 int bude_gpu_autotune_batch(bude_gpu_ctx *ctx, int32_t max_ms, bude_launch_cfg *best, float *best_ms);
 
 /* One evaluation of the whole batch, then a stream synchronise.  per_ligand = 0: one launch over all
- * (ligand, pose chunk, pair of atoms) items, longest ligands first, as a CUDA graph (pose transforms,
+ * (ligand, pose chunk, atom) items, longest ligands first, as a CUDA graph (pose transforms,
  * exact kernel, sums over the atoms) captured on first use of a launch shape.  per_ligand = 1: one
  * plain exact-kernel launch per ligand, for comparison; the same energies.  *ms (optional) receives
  * the CUDA-event time. */

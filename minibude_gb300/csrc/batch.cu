@@ -142,7 +142,7 @@ static int build_plan(Context &c, const bude_launch_cfg &cfg, CullPlan *out) {
   *out = plan_cull(c, lig, c.pose_off, count, cfg);
   int rc = c.b_items.reserve(std::max<size_t>(out->items.size(), 1) * sizeof(int4), "batch items");
   if (!rc) rc = c.b_folds.reserve(std::max<size_t>(out->folds.size(), 1) * sizeof(int4), "batch items");
-  if (!rc) rc = c.b_sums.reserve(std::max<size_t>(out->sums_bytes, 16), "batch group sums");
+  if (!rc) rc = c.b_sums.reserve(std::max<size_t>(out->sums_bytes, 16), "batch atom sums");
   if (rc) return rc;
   cudaError_t e = copy_sync(c, c.b_items.ptr, out->items.data(), out->items.size() * sizeof(int4), cudaMemcpyHostToDevice);
   if (e == cudaSuccess)

@@ -80,22 +80,18 @@ static int finish(const FinishArgs &f, long long grid, cudaStream_t st, long lon
   return BUDE_OK;
 }
 
-static int cull_groups(int natlig) { return (natlig + kGroupAtoms - 1) / kGroupAtoms; }
-
 SumsWindow sums_window(int natlig, long long nposes, const bude_launch_cfg &cfg, size_t most) {
   SumsWindow w;
   w.chunk = even_chunk(nposes, cfg.ppwi * cfg.wgsize);
   const long long floats = std::max((long long)(most / sizeof(float)), (long long)w.chunk);
-  w.groups = (int)std::min<long long>(cull_groups(natlig), floats / w.chunk);
-  w.poses = std::min(nposes, floats / std::max(w.groups, 1) / w.chunk * w.chunk);
+  w.atoms = (int)std::min<long long>(natlig, floats / w.chunk);
+  w.poses = std::min(nposes, floats / std::max(w.atoms, 1) / w.chunk * w.chunk);
   return w;
 }
 
 int cull_range(CullArgs a, FinishArgs f, const bude_launch_cfg &cfg, const SumsWindow &w, int natlig, long long nposes,
                cudaStream_t st, long long &launches) {
-  const int groups = cull_groups(natlig);
   const float *xform = a.xform;
-  a.natlig = natlig;
   a.chunk = w.chunk;
   f.sums = a.sums;
   for (long long w0 = 0; w0 < nposes; w0 += w.poses) {
@@ -105,17 +101,17 @@ int cull_range(CullArgs a, FinishArgs f, const bude_launch_cfg &cfg, const SumsW
     a.stride = f.stride = n;
     a.chunks = (int)((n + a.chunk - 1) / a.chunk);
     f.first = w0;
-    int g = 0;
+    int l = 0;
     do {
-      a.group0 = g;
-      f.groups = std::min(w.groups, groups - g);
-      f.more = g > 0;
-      g += f.groups;
-      f.last = g >= groups;
-      int rc = f.groups > 0 ? launch(a, (long long)f.groups * a.chunks, cfg, st, launches) : BUDE_OK;
+      a.atom0 = l;
+      f.rows = std::min(w.atoms, natlig - l);
+      f.more = l > 0;
+      l += f.rows;
+      f.last = l >= natlig;
+      int rc = f.rows > 0 ? launch(a, (long long)f.rows * a.chunks, cfg, st, launches) : BUDE_OK;
       if (!rc) rc = finish(f, (n + 255) / 256, st, launches);
       if (rc) return rc;
-    } while (g < groups);
+    } while (l < natlig);
   }
   return BUDE_OK;
 }
@@ -124,7 +120,7 @@ int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *lig
                        const unsigned *mask, const float *xform, float *energies, long long nposes) {
   if (nposes == 0) return BUDE_OK;
   const SumsWindow w = sums_window(natlig, nposes, cfg, kSumsBytes);
-  const int rc = c.partial.reserve((size_t)w.groups * w.poses * sizeof(float), "group sums");
+  const int rc = c.partial.reserve((size_t)w.atoms * w.poses * sizeof(float), "atom sums");
   if (rc) return rc;
   CullArgs a = cull_args(c, cfg);
   a.ligand = ligand;
@@ -152,38 +148,36 @@ CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vec
     if (chunks.empty()) return;
     w.item0 = (int)plan.items.size();
     w.fold0 = (int)plan.folds.size();
-    for (const Chunk &k : chunks) plan.folds.push_back(make_int4((int)k.pose, k.n, cull_groups(natlig(k.lig)), k.lig));
-    // Longest ligands first; the chunks of one ligand and group next to each other (they read the
-    // same records).
+    for (const Chunk &k : chunks) plan.folds.push_back(make_int4((int)k.pose, k.n, natlig(k.lig), k.lig));
+    // Longest ligands first; the chunks of one ligand and atom next to each other (they read the same
+    // records).
     std::stable_sort(chunks.begin(), chunks.end(),
                      [&](const Chunk &x, const Chunk &y) { return natlig(x.lig) > natlig(y.lig); });
     for (size_t i = 0, j = 0; i < chunks.size(); i = j) {
       while (j < chunks.size() && chunks[j].lig == chunks[i].lig) ++j;
       const int l = chunks[i].lig;
-      for (int g = 0; g < cull_groups(natlig(l)); ++g)
+      for (int r = 0; r < natlig(l); ++r)
         for (size_t k = i; k < j; ++k)
-          plan.items.push_back(make_int4(c.lig_off[l] + g * kGroupAtoms,
-                                         std::min(kGroupAtoms, natlig(l) - g * kGroupAtoms) | g << 8,
-                                         (int)chunks[k].pose, chunks[k].n));
+          plan.items.push_back(make_int4(c.lig_off[l] + r, r, (int)chunks[k].pose, chunks[k].n));
     }
     w.items = (int)plan.items.size() - w.item0;
     w.folds = (int)plan.folds.size() - w.fold0;
-    plan.sums_bytes = std::max(plan.sums_bytes, (size_t)w.n * w.groups * sizeof(float));
+    plan.sums_bytes = std::max(plan.sums_bytes, (size_t)w.n * w.atoms * sizeof(float));
     plan.windows.push_back(w);
     chunks.clear();
     w = CullPlan::Window{};
   };
   for (size_t i = 0; i < lig.size(); ++i) {
-    const int per = even_chunk(count[i], most), groups = cull_groups(natlig(lig[i]));
+    const int per = even_chunk(count[i], most);
     for (long long p = 0; p < count[i]; p += per) {
       const int n = (int)std::min<long long>(per, count[i] - p);
       const long long at = first[i] + p;
       if (!chunks.empty() &&
-          (size_t)(at + n - w.first) * std::max(w.groups, groups) * sizeof(float) > kSumsBytes)
+          (size_t)(at + n - w.first) * std::max(w.atoms, natlig(lig[i])) * sizeof(float) > kSumsBytes)
         close();
       if (chunks.empty()) w.first = at;
       w.n = at + n - w.first;
-      w.groups = std::max(w.groups, groups);
+      w.atoms = std::max(w.atoms, natlig(lig[i]));
       chunks.push_back({lig[i], n, at});
     }
   }
@@ -216,23 +210,24 @@ int enqueue_plan(Context &c, const bude_launch_cfg &shape, const CullPlan &plan,
 }
 
 // A chunk wants to be large (its groups are tighter: 4,096 poses of the 4,096 x 64 deck leave 69 records
-// per group of 64, 2,048 leave 82), but the launch wants several blocks per SM, one per chunk and group
-// of ligand atoms.  The lines lie where one shape overtook the next over 64 to 262,144 poses against 938
-// x 26, 2,672 x 48 and 4,096 x 64 atoms (us, smaller | larger shape): 1 x 256 | 2 x 256 at 120k points
-// (poses x ligand atoms) 104 | 108, at 288k 141 | 125; 2 x 256 | 4 x 512 at 426k 68 | 76, at 1.0M 131 |
-// 123; 4 x 512 | 8 x 512 at 1.9M 417 | 419, at 6.3M 1,061 | 996.  One point per lane below the first line
-// (latency: twice the warps), two above it; four lose to two everywhere.  Ligands of fewer poses than a
-// chunk take the smallest shape that holds them: 1,024 ligands of 410 poses 4 x 128 4.9 ms, 2 x 256 5.0,
-// 4 x 64 6.2; 128 of 205 2 x 128 0.46 ms, 1 x 256 0.50.
+// per group of 64, 2,048 leave 82), but the launch wants several blocks per SM, one per chunk and ligand
+// atom.  The lines lie where one shape overtook the next over 64 to 262,144 poses against 938 x 26,
+// 2,672 x 48 and 4,096 x 64 atoms (us, smaller | larger shape): 1 x 256 | 2 x 512 at 65k points (poses x
+// ligand atoms) 33 | 37, at 120k 94 | 78; 2 x 512 | 4 x 512 at 786k 190 | 200, at 1.05M 119 | 116; 4 x 512
+// | 8 x 512 at 3.1M 480 | 491, at 6.3M 1,023 | 944.  One point per lane below the first line (latency:
+// twice the warps), two above it; four lose to two nearly everywhere.  Ligands of fewer poses than a chunk
+// take the smallest shape that holds them: 1,024 ligands of 410 poses 4 x 128 4.9 ms, 2 x 256 5.1, 4 x 64
+// 6.2; 64 of 1,000 4 x 256 0.66 ms, 2 x 256 0.73; 128 of 205 2 x 128 0.45 ms, 1 x 256 0.49.
 bude_launch_cfg cull_shape(long long n, int natlig, int ligands) {
   const double points = (double)n * natlig * ligands;
   bude_launch_cfg s{1, n <= 64 ? 64 : (n <= 128 ? 128 : 256), 1, 64, 1, 0};
-  if (points < 2e5) return s;
-  const int shapes[][2] = {{8, 512}, {4, 512}, {4, 256}, {2, 256}, {4, 128}, {2, 128}};
-  int k = points < 7e5 ? 3 : (points < 2.2e6 ? 1 : 0);
-  while (k < 5 && (long long)shapes[k + 1][0] * shapes[k + 1][1] >= n) ++k;
-  s.ppwi = shapes[k][0];
-  s.wgsize = shapes[k][1];
+  if (points < 9e4) return s;
+  const int many[][2] = {{8, 512}, {4, 512}, {4, 256}, {4, 128}, {2, 128}}, few[][2] = {{2, 512}, {2, 256}, {2, 128}};
+  const int(*shape)[2] = points < 9e5 ? few : (points < 3.8e6 ? many + 1 : many);
+  const int(*last)[2] = points < 9e5 ? few + 2 : many + 4;
+  while (shape < last && (long long)shape[1][0] * shape[1][1] >= n) ++shape;
+  s.ppwi = (*shape)[0];
+  s.wgsize = (*shape)[1];
   s.unroll = 2;
   return s;
 }

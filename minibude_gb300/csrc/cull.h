@@ -1,5 +1,5 @@
 // cull.h -- host side of the exact kernel (cull_kernel.cuh): launch shapes, the cut of poses into
-// chunks, and the windows that bound the memory of the group sums.
+// chunks, and the windows that bound the memory of the atom sums.
 #pragma once
 #include <vector>
 
@@ -11,12 +11,12 @@ struct CullArgs;
 struct FinishArgs;
 
 // A batch evaluation's work, cut for one launch shape: block items and finish items in windows of
-// consecutive poses, each window's group sums at most kSumsBytes.
+// consecutive poses, each window's atom sums at most kSumsBytes.
 struct CullPlan {
   struct Window {
     int item0, items, fold0, folds;
     long long first, n; // poses
-    int groups;         // the most groups of a ligand in the window
+    int atoms;          // the most of a ligand in the window
   };
   std::vector<int4> items, folds; // CullArgs::items, FinishArgs::folds
   std::vector<Window> windows;
@@ -33,10 +33,10 @@ inline int even_chunk(long long n, int most) {
   return (int)((per + 31) / 32 * 32 < most ? (per + 31) / 32 * 32 : most);
 }
 
-// One ligand's poses, evaluated in windows whose group sums, [groups][poses], take at most `most` bytes
-// (and room for one group of a chunk).
+// One ligand's poses, evaluated in windows whose atom sums, [atoms][poses], take at most `most` bytes (and
+// room for one atom of a chunk).
 struct SumsWindow {
-  int chunk, groups;
+  int chunk, atoms;
   long long poses;
 };
 SumsWindow sums_window(int natlig, long long nposes, const bude_launch_cfg &cfg, size_t most);

@@ -23,29 +23,30 @@
 // Angstroms, so sorting the poses by where they put the atom gives groups of 64 whose positions share
 // a box of 2-3 A, and a box is tested against 32 protein atoms by one warp instruction sequence.
 //
-//   * a block takes a chunk of poses (ppwi * wgsize of them) and a group of kGroupAtoms ligand atoms.
-//     Per ligand atom it transforms every pose's atom, bins the positions over an 8 x 8 x 8 grid of
-//     their bounding box in Hilbert order (a counting sort in shared memory) and hands the sorted
-//     points out in groups of 32 * P, P per lane, to its warps;
+//   * a block takes a chunk of poses (ppwi * wgsize of them) and one ligand atom: it transforms the atom
+//     for every pose, bins the positions over an 8 x 8 x 8 grid of their bounding box in Hilbert order
+//     (a counting sort in shared memory) and hands the sorted points out in groups of 32 * P, P per
+//     lane, to its warps;
 //   * a warp reduces its group to a box and walks the protein, which lies in clusters of 32 atoms near
 //     each other (k-d order, ensure_slab): 32 clusters at a time are tested against the box with one
 //     cluster per lane, then the 32 atoms of each cluster that is in reach with one atom per lane and
 //     its own reach for this ligand type; the atoms left are evaluated for the group's points with the
 //     48-byte records brought into shared memory, eight at a time, ahead of their use;
-//   * a point's terms add up in protein order per ligand atom, the atoms of a group in ligand order, and
-//     the groups in order (cull_finish_kernel).  Nothing in that order depends on the other poses, so a
-//     pose's energy is the same bits for every launch shape, chunk, batch or position.
+//   * a point's terms add up in protein order, and a pose's atoms in ligand order (cull_finish_kernel).
+//     Nothing in that order depends on the other poses, so a pose's energy is the same bits for every
+//     launch shape, chunk, batch or position.
 //
-// What bounds it: instruction issue (76% of the slots on the 4,096 x 64 deck).  Of 935 M warp
-// instructions for 262,144 poses, 630 M are the record loop (35 per record and 64 points, 23 of them the
-// pair arithmetic), 70 M the groups' share of the candidate lists and 230 M the sort, the boxes and the
-// candidates.  Measured, all pairs evaluated (records broadcast to 16 poses per thread, TMA-staged) | this
-// kernel, end to end from pinned host memory: 4,096 x 64 x 1,048,576 101.7 | 4.5 ms, 938 x 26 x 65,536
-// 0.753 | 0.193 ms, 2,672 x 48 x 400,003 streamed 21.2 | 3.5 ms; 64 ligands of 12-96 atoms x 1,024-16,384
-// poses against 2,672 atoms 67.0 | 3.3 ms.  What went into it, on 4,096 x 64 x 262,144: records read
-// through L1 one by one 1,140 us (and 64 poses took 105 us for 35); 64-byte records with the packed
-// instructions' operands twice, 1,250; 48 bytes 1,100 (the loads' register writes bound two points per
-// lane); lists of 64 records 1,095, of 128 in stages of 10 1,067; no shared candidate lists 1,218.
+// What bounds it: instruction issue (76% of the slots on the 4,096 x 64 deck), two thirds of it the record
+// loop (35 instructions per record and 64 points, 23 of them the pair arithmetic), the rest the sort, the
+// boxes and the candidate lists.  Measured, all pairs evaluated (records broadcast to 16 poses per thread,
+// TMA-staged) | this kernel, end to end from pinned host memory: 4,096 x 64 x 1,048,576 101.6 | 3.30 ms,
+// 938 x 26 x 65,536 0.750 | 0.147 ms, 938 x 26 x 64 201 | 53 us, 2,672 x 48 x 400,003 streamed 21.2 | 2.69
+// ms; 64 ligands of 12-96 atoms x 1,024-16,384 poses against 2,672 atoms 67.0 | 2.40 ms.  What went into
+// it, on 4,096 x 64 x 262,144: records read through L1 one by one 1,140 us (and 64 poses took 105 us for
+// 41); 64-byte records with the packed instructions' operands twice, 1,250; 48 bytes 1,100 (the loads'
+// register writes bound two points per lane); lists of 64 records 1,095, of 128 in stages of 10 1,067; no
+// shared candidate lists 1,218.  One ligand atom per block instead of two, binned over the box of its own
+// positions (no registers spill any more): the 4,096 x 64 x 1,048,576 deck 4.52 -> 3.30 ms.
 #pragma once
 #include <cstdint>
 #include <type_traits>
@@ -66,15 +67,14 @@ struct CullArgs {
   const float4 *box;     // [clusters][2]: lower and upper corner of the cluster's atoms
   const float *box_reach; // [type][clusters]: the largest squared reach in the cluster
   const float *xform;    // 12 floats per pose
-  const int4 *items;     // {first atom, atoms | group << 8, first pose, poses} per block, or nullptr:
-                         // block b = group b / chunks, chunk b % chunks of one ligand
-  float *sums;           // [group][stride] group sums, from pose `first` on
+  const int4 *items;     // {atom, row, first pose, poses} per block, or nullptr: block b = row b / chunks,
+                         // chunk b % chunks of one ligand
+  float *sums;           // [row][stride]: a ligand atom's sum over the protein, from pose `first` on
   long long stride, first;
   long long nposes;      // without items: poses of the ligand
   float3 lo, hi;         // protein atoms' bounding box, widened by the longest reach
   const unsigned *words; // optional: a deck checked on the device (edge_pose.cuh); nothing runs on a bad one
-  int natlig;            // without items: the ligand's atoms
-  int group0;            // without items: the first group (row 0 of sums)
+  int atom0;             // without items: the atom of row 0
   int chunk, chunks;     // without items: poses of a chunk (at most K * blockDim.x) and chunks of the ligand
   int natpro_pad;        // records per type
   int clusters;          // of kClusterAtoms; the last may be short
@@ -342,189 +342,170 @@ template <int K, int P> __global__ void __launch_bounds__(kMaxThreads, 2) cull_k
   Candidates *cand = reinterpret_cast<Candidates *>(reinterpret_cast<WarpList *>(pts + K * T) + warps);
   __shared__ int bins[kBins];
   __shared__ int warp_total[kMaxThreads / 32];
-  __shared__ float red[6][kMaxThreads / 32], range[6];
+  __shared__ float red[6][kMaxThreads / 32];
   __shared__ int next_group;
 
-  int atom0, natoms, group;
+  int atom, row, n;
   long long pose0;
-  int n;
   if (a.items) {
     const int4 it = __ldg(&a.items[blockIdx.x]);
-    atom0 = it.x, natoms = it.y & 255, group = it.y >> 8, pose0 = it.z, n = it.w;
+    atom = it.x, row = it.y, pose0 = it.z, n = it.w;
   } else {
-    group = (int)(blockIdx.x / (unsigned)a.chunks) + a.group0;
+    row = (int)(blockIdx.x / (unsigned)a.chunks);
+    atom = row + a.atom0;
     pose0 = (long long)(blockIdx.x % (unsigned)a.chunks) * a.chunk;
-    atom0 = group * kGroupAtoms;
-    natoms = min(kGroupAtoms, a.natlig - atom0);
     n = (int)min((long long)a.chunk, a.nposes - pose0);
   }
   if (a.words && deck_bad_type(a.words)) return;
   const float4 *xf = reinterpret_cast<const float4 *>(a.xform) + pose0 * 3;
 
-  // Range of the chunk's translations (regular poses, edge_pose.cuh).
+  // 1. positions, their box (of regular positions, edge_pose.cuh, where the protein is in reach) and cells
+  const float4 la = __ldg(&a.ligand[atom]);
+  float x[K], y[K], z[K];
+  float3 lo = make_float3(INFINITY, INFINITY, INFINITY), hi = make_float3(-INFINITY, -INFINITY, -INFINITY);
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int i = tid + k * T;
+    if (i >= n) continue;
+    const float4 r0 = __ldg(xf + i * 3), r1 = __ldg(xf + i * 3 + 1), r2 = __ldg(xf + i * 3 + 2);
+    // serial/fasten.hpp:66-73
+    x[k] = r0.w + la.x * r0.x + la.y * r0.y + la.z * r0.z;
+    y[k] = r1.w + la.x * r1.x + la.y * r1.y + la.z * r1.z;
+    z[k] = r2.w + la.x * r2.x + la.y * r2.y + la.z * r2.z;
+    if (fabsf(x[k]) + fabsf(y[k]) + fabsf(z[k]) < kPoseReach) {
+      lo = make_float3(fminf(lo.x, x[k]), fminf(lo.y, y[k]), fminf(lo.z, z[k]));
+      hi = make_float3(fmaxf(hi.x, x[k]), fmaxf(hi.y, y[k]), fmaxf(hi.z, z[k]));
+    }
+  }
   {
-    float tlo[3] = {INFINITY, INFINITY, INFINITY}, thi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    const float v[6] = {warp_min(lo.x), warp_min(lo.y), warp_min(lo.z), warp_max(hi.x), warp_max(hi.y), warp_max(hi.z)};
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int i = tid + k * T;
-      if (i >= n) continue;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const float t = __ldg(reinterpret_cast<const float *>(xf + i * 3 + d) + 3);
-        if (fabsf(t) < kPoseReach) {
-          tlo[d] = fminf(tlo[d], t);
-          thi[d] = fmaxf(thi[d], t);
-        }
-      }
-    }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      tlo[d] = warp_min(tlo[d]);
-      thi[d] = warp_max(thi[d]);
-      if (lane == 0) red[d][warp] = tlo[d], red[3 + d][warp] = thi[d];
-    }
+    for (int d = 0; d < 6; ++d)
+      if (lane == 0) red[d][warp] = v[d];
     for (int b = tid; b < kBins; b += T) bins[b] = 0;
     __syncthreads();
-    for (int d = warp; d < 6; d += warps) {
-      const float v = red[d][lane < warps ? lane : 0];
-      const float r = d < 3 ? warp_min(v) : warp_max(v);
-      if (lane == 0) range[d] = r;
+    const int w = lane < warps ? lane : 0;
+    lo = make_float3(fmaxf(warp_min(red[0][w]), a.lo.x), fmaxf(warp_min(red[1][w]), a.lo.y),
+                     fmaxf(warp_min(red[2][w]), a.lo.z));
+    hi = make_float3(fminf(warp_max(red[3][w]), a.hi.x), fminf(warp_max(red[4][w]), a.hi.y),
+                     fminf(warp_max(red[5][w]), a.hi.z));
+  }
+  const float ix = hi.x > lo.x ? 8.f / (hi.x - lo.x) : 0.f, iy = hi.y > lo.y ? 8.f / (hi.y - lo.y) : 0.f,
+              iz = hi.z > lo.z ? 8.f / (hi.z - lo.z) : 0.f;
+  int slot[K]; // cell << 16 | rank in the cell
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    slot[k] = -1;
+    if (tid + k * T >= n) continue;
+    const int qx = min(max((int)((x[k] - lo.x) * ix), 0), 7), qy = min(max((int)((y[k] - lo.y) * iy), 0), 7),
+              qz = min(max((int)((z[k] - lo.z) * iz), 0), 7);
+    const int cell = kHilbert.at[qz * 64 + qy * 8 + qx];
+    slot[k] = cell << 16 | atomicAdd(&bins[cell], 1);
+  }
+  __syncthreads();
+  // 2. first point of every cell: exclusive scan of the counts.  Scanning warp w owns `per` cells.
+  const int scanners = 1 << (31 - __clz(min(warps, kBins / 32))), per = kBins / scanners;
+  if (warp < scanners) {
+    int run = 0;
+    for (int b = warp * per; b < (warp + 1) * per; b += 32) {
+      const int v = bins[b + lane];
+      int s = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= o) s += u;
+      }
+      bins[b + lane] = run + s - v;
+      run += __shfl_sync(0xffffffffu, s, 31);
+    }
+    if (lane == 0) warp_total[warp] = run;
+  }
+  if (tid == 0) next_group = 0;
+  __syncthreads();
+  if (warp > 0 && warp < scanners) {
+    const int before = __reduce_add_sync(0xffffffffu, lane < warp ? warp_total[lane] : 0);
+    for (int b = warp * per; b < (warp + 1) * per; b += 32) bins[b + lane] += before;
+  }
+  __syncthreads();
+  // 3. scatter into sorted order
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (slot[k] >= 0)
+      pts[bins[slot[k] >> 16] + (slot[k] & 0xffff)] = make_float4(x[k], y[k], z[k], __int_as_float(tid + k * T));
+  __syncthreads();
+  // 4. candidates of every super group
+  const int lt = __float_as_int(la.w);
+  if (a.supers) {
+    constexpr int kPoints = 32 * P * kSuperGroups;
+    for (int sg = warp; sg * kPoints < n; sg += warps) {
+      float3 lo, hi;
+      points_box(pts, sg * kPoints, min(kPoints, n - sg * kPoints), lo, hi);
+      const float4 *reach = a.reach + (size_t)lt * a.natpro_pad;
+      int count = 0;
+      for (int c0 = 0; c0 < a.clusters && count <= kCandidates; c0 += 32) {
+        unsigned todo = near_clusters(lo, hi, c0, a.clusters, a.box_reach + (size_t)lt * a.clusters, a.box);
+        while (todo && count <= kCandidates) {
+          int at[4];
+          float4 t[4];
+          next_clusters(todo, c0, 0, reach, at, a.natpro_pad, t);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) push_hits(cand[sg].at, count, lo, hi, t[i], at[i]);
+        }
+      }
+      if (lane == 0) cand[sg].n = count <= kCandidates ? count : -1;
     }
     __syncthreads();
   }
-
-  for (int il = 0; il < natoms; ++il) {
-    const float4 la = __ldg(&a.ligand[atom0 + il]);
-    // 1. positions and cells
-    const float rl = sqrtf(la.x * la.x + la.y * la.y + la.z * la.z);
-    const float lox = fmaxf(range[0] - rl, a.lo.x), loy = fmaxf(range[1] - rl, a.lo.y),
-                loz = fmaxf(range[2] - rl, a.lo.z);
-    const float wx = fminf(range[3] + rl, a.hi.x) - lox, wy = fminf(range[4] + rl, a.hi.y) - loy,
-                wz = fminf(range[5] + rl, a.hi.z) - loz;
-    const float ix = wx > 0.f ? 8.f / wx : 0.f, iy = wy > 0.f ? 8.f / wy : 0.f, iz = wz > 0.f ? 8.f / wz : 0.f;
-    float x[K], y[K], z[K];
-    int slot[K]; // cell << 16 | rank in the cell
+  // 5. groups of 32 * P sorted points
+  for (;;) {
+    int g = 0;
+    if (lane == 0) g = atomicAdd(&next_group, 1);
+    g = __shfl_sync(0xffffffffu, g, 0);
+    const int first = g * 32 * P;
+    if (first >= n) break;
+    Points<P> pt;
+    float3 lo, hi;
+    points_box(pts, first, min(32 * P, n - first), lo, hi);
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int i = tid + k * T;
-      slot[k] = -1;
-      if (i >= n) continue;
-      const float4 r0 = __ldg(xf + i * 3), r1 = __ldg(xf + i * 3 + 1), r2 = __ldg(xf + i * 3 + 2);
-      // serial/fasten.hpp:66-73
-      x[k] = r0.w + la.x * r0.x + la.y * r0.y + la.z * r0.z;
-      y[k] = r1.w + la.x * r1.x + la.y * r1.y + la.z * r1.z;
-      z[k] = r2.w + la.x * r2.x + la.y * r2.y + la.z * r2.z;
-      const int qx = min(max((int)((x[k] - lox) * ix), 0), 7), qy = min(max((int)((y[k] - loy) * iy), 0), 7),
-                qz = min(max((int)((z[k] - loz) * iz), 0), 7);
-      const int cell = kHilbert.at[qz * 64 + qy * 8 + qx];
-      slot[k] = cell << 16 | atomicAdd(&bins[cell], 1);
-    }
-    __syncthreads();
-    // 2. first point of every cell: exclusive scan of the counts.  Scanning warp w owns `per` cells.
-    const int scanners = 1 << (31 - __clz(min(warps, kBins / 32))), per = kBins / scanners;
-    if (warp < scanners) {
-      int run = 0;
-      for (int b = warp * per; b < (warp + 1) * per; b += 32) {
-        const int v = bins[b + lane];
-        int s = v;
+    for (int i = 0; i < P; ++i) pt.set(i, pts[min(first + i * 32 + lane, n - 1)]);
+    pt.clear();
+    const int k = a.supers ? cand[g / kSuperGroups].n : -1;
+    cull_eval<P>(pt, lo, hi, lt, k >= 0 ? cand[g / kSuperGroups].at : nullptr, k, list, a);
+    __syncwarp(); // every lane has read its points
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int u = __shfl_up_sync(0xffffffffu, s, o);
-          if (lane >= o) s += u;
-        }
-        bins[b + lane] = run + s - v;
-        run += __shfl_sync(0xffffffffu, s, 31);
-      }
-      if (lane == 0) warp_total[warp] = run;
-    }
-    if (tid == 0) next_group = 0;
-    __syncthreads();
-    if (warp > 0 && warp < scanners) {
-      const int before = __reduce_add_sync(0xffffffffu, lane < warp ? warp_total[lane] : 0);
-      for (int b = warp * per; b < (warp + 1) * per; b += 32) bins[b + lane] += before;
-    }
-    __syncthreads();
-    // 3. scatter into sorted order
+    for (int i = 0; i < P; ++i)
+      if (first + i * 32 + lane < n) pts[first + i * 32 + lane].x = pt.energy(i); // in place of the point
+  }
+  __syncthreads();
+  // 6. the energies in pose order
+  float *out = a.sums + (long long)row * a.stride + (pose0 - a.first);
+  float *flat = reinterpret_cast<float *>(pts);
+  float e[K];
+  int at[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k)
-      if (slot[k] >= 0)
-        pts[bins[slot[k] >> 16] + (slot[k] & 0xffff)] = make_float4(x[k], y[k], z[k], __int_as_float(tid + k * T));
-    __syncthreads();
-    for (int b = tid; b < kBins; b += T) bins[b] = 0;
-    // 4. candidates of every super group
-    const int lt = __float_as_int(la.w);
-    if (a.supers) {
-      constexpr int kPoints = 32 * P * kSuperGroups;
-      for (int sg = warp; sg * kPoints < n; sg += warps) {
-        float3 lo, hi;
-        points_box(pts, sg * kPoints, min(kPoints, n - sg * kPoints), lo, hi);
-        const float4 *reach = a.reach + (size_t)lt * a.natpro_pad;
-        int count = 0;
-        for (int c0 = 0; c0 < a.clusters && count <= kCandidates; c0 += 32) {
-          unsigned todo = near_clusters(lo, hi, c0, a.clusters, a.box_reach + (size_t)lt * a.clusters, a.box);
-          while (todo && count <= kCandidates) {
-            int at[4];
-            float4 t[4];
-            next_clusters(todo, c0, 0, reach, at, a.natpro_pad, t);
+  for (int k = 0; k < K; ++k)
+    if (tid + k * T < n) e[k] = pts[tid + k * T].x, at[k] = __float_as_int(pts[tid + k * T].w);
+  __syncthreads();
 #pragma unroll
-            for (int i = 0; i < 4; ++i) push_hits(cand[sg].at, count, lo, hi, t[i], at[i]);
-          }
-        }
-        if (lane == 0) cand[sg].n = count <= kCandidates ? count : -1;
-      }
-      __syncthreads();
-    }
-    // 5. groups of 32 * P sorted points
-    for (;;) {
-      int g = 0;
-      if (lane == 0) g = atomicAdd(&next_group, 1);
-      g = __shfl_sync(0xffffffffu, g, 0);
-      const int first = g * 32 * P;
-      if (first >= n) break;
-      Points<P> pt;
-      float3 lo, hi;
-      points_box(pts, first, min(32 * P, n - first), lo, hi);
+  for (int k = 0; k < K; ++k)
+    if (tid + k * T < n) flat[at[k]] = e[k];
+  __syncthreads();
 #pragma unroll
-      for (int i = 0; i < P; ++i) pt.set(i, pts[min(first + i * 32 + lane, n - 1)]);
-      pt.clear();
-      const int k = a.supers ? cand[g / kSuperGroups].n : -1;
-      cull_eval<P>(pt, lo, hi, lt, k >= 0 ? cand[g / kSuperGroups].at : nullptr, k, list, a);
-      __syncwarp(); // every lane has read its points
-#pragma unroll
-      for (int i = 0; i < P; ++i)
-        if (first + i * 32 + lane < n) pts[first + i * 32 + lane].x = pt.energy(i); // in place of the point
-    }
-    __syncthreads();
-    // 6. the atom's energies in pose order, added to the group's
-    float *out = a.sums + (long long)(group - a.group0) * a.stride + (pose0 - a.first);
-    float *flat = reinterpret_cast<float *>(pts);
-    float e[K];
-    int at[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-      if (tid + k * T < n) e[k] = pts[tid + k * T].x, at[k] = __float_as_int(pts[tid + k * T].w);
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-      if (tid + k * T < n) flat[at[k]] = e[k];
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int i = tid + k * T;
-      if (i < n) out[i] = il == 0 ? flat[i] : __fadd_rn(out[i], flat[i]);
-    }
+  for (int k = 0; k < K; ++k) {
+    const int i = tid + k * T;
+    if (i < n) out[i] = flat[i];
   }
 }
 
-// energies[p] = 0.5 * the sum of pose p's group sums in group order (0 groups: 0), for the poses
-// [first, first + n) of one ligand, or, with folds, for {first pose, poses, groups, ligand} per block.
+// energies[p] = 0.5 * the sum over pose p's ligand atoms in order (no atoms: 0), for the poses
+// [first, first + n) of one ligand, or, with folds, for {first pose, poses, rows, ligand} per block.
 // With `edges` the irregular poses among them (every pose of an irregular deck or ligand) then get the
 // reference's arithmetic: edge_energy of edge_pose.cuh, one pose per warp at a time.
 struct FinishArgs {
-  const float *sums; // [group][stride], from pose `first` on
+  const float *sums; // [row][stride], from pose `first` on
   long long stride, first, n;
-  int groups;
-  int more, last; // the sums add to what energies hold; these are the last groups
+  int rows;
+  int more, last; // the sums add to what energies hold; these are the last rows
   const int4 *folds;
   float *energies;
   const unsigned *words; // as CullArgs::words; its deck decides whether every pose is irregular
@@ -534,7 +515,7 @@ struct FinishArgs {
 
 static __global__ void __launch_bounds__(256) cull_finish_kernel(const FinishArgs a) {
   long long p0 = a.first + (long long)blockIdx.x * blockDim.x, p1 = min(p0 + blockDim.x, a.first + a.n);
-  int groups = a.groups;
+  int rows = a.rows;
   bool all = a.e.all != 0;
   if (a.words) {
     if (deck_bad_type(a.words)) return;
@@ -542,7 +523,7 @@ static __global__ void __launch_bounds__(256) cull_finish_kernel(const FinishArg
   }
   if (a.folds) {
     const int4 f = __ldg(&a.folds[blockIdx.x]);
-    p0 = f.x, p1 = (long long)f.x + f.y, groups = f.z;
+    p0 = f.x, p1 = (long long)f.x + f.y, rows = f.z;
     if (a.edges && *a.e.lig_any > 0) all = a.e.lig_all[f.w] != 0;
   }
   for (long long w = p0 + (threadIdx.x & ~31u); w < p1; w += blockDim.x) {
@@ -551,15 +532,15 @@ static __global__ void __launch_bounds__(256) cull_finish_kernel(const FinishArg
     if (p < p1) {
       const float *s = a.sums + (p - a.first);
       float acc = a.more ? a.energies[p] : 0.f;
-      int g = 0;
-      for (; g + 8 <= groups; g += 8) {
+      int r = 0;
+      for (; r + 8 <= rows; r += 8) {
         float v[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = s[(long long)(g + j) * a.stride];
+        for (int j = 0; j < 8; ++j) v[j] = s[(long long)(r + j) * a.stride];
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc = __fadd_rn(acc, v[j]);
       }
-      for (; g < groups; ++g) acc = __fadd_rn(acc, s[(long long)g * a.stride]);
+      for (; r < rows; ++r) acc = __fadd_rn(acc, s[(long long)r * a.stride]);
       a.energies[p] = a.last ? 0.5f * acc : acc;
       irregular = a.edges && a.last && (all || ((a.e.mask[p >> 5] >> (p & 31)) & 1u));
     }

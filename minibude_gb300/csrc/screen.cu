@@ -312,7 +312,7 @@ __global__ void fallback_copy_kernel(const long long *pose_off, const int *fallb
 
 struct ScreenState {
   DevBuf pose_off, flag, counts, comp_off, comp_pose, comp_xform, comp_exact, err, final_e, rescored, items, folds, fb;
-  DevBuf sums;                // group sums of the exact evaluations
+  DevBuf sums;                // atom sums of the exact evaluations
   cudaStream_t side = nullptr; // the exact rescoring beside the surrogate
   long long result_for = -1;   // Context::batch_uploads of the batch the stored result belongs to
 };
@@ -332,7 +332,7 @@ void release_screen(Context &c) {
 static int upload_plan(Context &c, ScreenState &s, const CullPlan &plan) {
   int rc = s.items.reserve(std::max<size_t>(plan.items.size(), 1) * sizeof(int4), "screen items");
   if (!rc) rc = s.folds.reserve(std::max<size_t>(plan.folds.size(), 1) * sizeof(int4), "screen items");
-  if (!rc) rc = s.sums.reserve(std::max<size_t>(plan.sums_bytes, 16), "screen group sums");
+  if (!rc) rc = s.sums.reserve(std::max<size_t>(plan.sums_bytes, 16), "screen atom sums");
   if (rc) return rc;
   cudaError_t e = cudaSuccess; // pageable sources: staged before the calls return
   if (!plan.items.empty())

@@ -12,7 +12,6 @@
 
 #include <algorithm>
 
-#include "exact_shape.h"
 #include "internal.h"
 #include "pose_xform.cuh"
 
@@ -80,9 +79,9 @@ static int score_stream(Context &c, const bude_launch_cfg &cfg, const float *pos
   int rc = check_cfg(c, cfg);
   if (rc) return rc;
   // Whole blocks of poses, and enough of them that a chunk's launch fills the GPU: four blocks per SM
-  // (one block per group of ligand atoms and ppwi * wgsize poses).
+  // (one block per ligand atom and ppwi * wgsize poses).
   const long long ppb = (long long)cfg.ppwi * cfg.wgsize;
-  const long long fill = 4LL * std::max(c.num_sms, 1) * kGroupAtoms / std::max(c.natlig, 1) + 1;
+  const long long fill = 4LL * std::max(c.num_sms, 1) / std::max(c.natlig, 1) + 1;
   chunk = std::max((chunk + ppb - 1) / ppb, fill) * ppb;
   chunk = std::min(chunk, std::max(nposes, 1LL));
   StreamState *sp = nullptr;

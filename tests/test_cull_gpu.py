@@ -1,7 +1,7 @@
 """The exact kernel evaluates only the pairs that can interact (csrc/cull_kernel.cuh).  Its energies are
 checked where finding those pairs can go wrong: clusters of 32 protein atoms and blocks of 32 clusters
 that are just full, pose chunks and groups at their edges, a protein so dense that a list of candidates
-overflows, proteins past the 16-bit list indices, poses far from the protein, and group sums that take
+overflows, proteins past the 16-bit list indices, poses far from the protein, and atom sums that take
 several windows.  The oracle evaluates every pair; against FP64 the bound is the one of
 test_forcefield_and_deck_sizes (4x the FP32 oracle's own error, at least 2e-4).  The order of a pose's sum
 depends on nothing else, so every launch shape has to give the same bits."""
@@ -92,9 +92,9 @@ def test_poses_far_from_the_protein(ctx):
     assert np.all(got[5::13] == 0.0)
 
 
-def test_group_sums_in_several_windows(ctx):
-    # 1,000 groups of two ligand atoms x 300,000 poses: 1.2 GB of group sums, two windows; the batch
-    # path cuts its windows between chunks of poses.
+def test_atom_sums_in_several_windows(ctx):
+    # 2,000 ligand atoms x 300,000 poses: 2.4 GB of atom sums, three windows; the batch path cuts its
+    # windows between chunks of poses.
     rng = np.random.default_rng(8)
     base = deck_of(40, 5.0, 4, 8, seed=8)
     ligand = synthetic_ligand(rng, 2000, 5.0, base.ntypes)
