@@ -148,7 +148,10 @@ CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vec
     if (chunks.empty()) return;
     w.item0 = (int)plan.items.size();
     w.fold0 = (int)plan.folds.size();
-    for (const Chunk &k : chunks) plan.folds.push_back(make_int4((int)k.pose, k.n, natlig(k.lig), k.lig));
+    for (const Chunk &k : chunks)
+      for_each_item(k.n, 1, kFoldPoses, [&](long long p, int n) {
+        plan.folds.push_back(make_int4((int)(k.pose + p), n, natlig(k.lig), k.lig));
+      });
     // Longest ligands first; the chunks of one ligand and atom next to each other (they read the same
     // records).
     std::stable_sort(chunks.begin(), chunks.end(),

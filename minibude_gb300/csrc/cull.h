@@ -24,6 +24,8 @@ struct CullPlan {
 };
 
 constexpr size_t kSumsBytes = (size_t)1 << 30;
+// Poses of a finish block: with a chunk of 4,096 per block 64 ligands gave 108 blocks (89 us, so 17.5).
+constexpr int kFoldPoses = 256;
 
 // Poses of a chunk for n poses at `most` per block: as many chunks as that takes, evenly filled (a
 // short last chunk would sort few poses into loose groups).
