@@ -57,7 +57,7 @@ struct Surrogate {
   DevBuf labels, pose_lig_first, pose_lig_n, epoch_pose, epoch_rowoff, epoch_pose2, epoch_rowoff2, epoch_loss;
   long long rows_cap = 0;
   // scoring
-  DevBuf items, scores, next;
+  DevBuf items, scores, next;    // items: ligand by ligand, then all of them longest ligand first
   std::vector<int> item_lig_off; // nligands + 1: first scoring item of each ligand
   long long items_for = -1; // Context::batch_gen the items were built for
   int n_items = 0;
@@ -806,11 +806,13 @@ int surrogate_prepare(Context &c, bool xform_ready) {
       });
       s.item_lig_off.push_back((int)items.size());
     }
+    s.n_items = (int)items.size();
+    items.insert(items.end(), items.begin(), items.begin() + s.n_items);
+    std::stable_sort(items.begin() + s.n_items, items.end(), [](const int4 &x, const int4 &y) { return x.y > y.y; });
     rc = s.items.reserve(std::max<size_t>(items.size(), 1) * sizeof(int4), "surrogate items");
     if (rc) return rc;
     const cudaError_t e = copy_sync(c, s.items.ptr, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_error(e, "surrogate items");
-    s.n_items = (int)items.size();
     s.items_for = c.batch_gen;
   }
   if (!xform_ready) {
@@ -831,7 +833,8 @@ int surrogate_score_range(Context &c, int lig0, int lig1, int groups, cudaStream
   a.g = s.fg;
   a.ligands = c.b_ligands.as<float4>();
   a.xform = c.b_xform.as<float4>();
-  a.items = s.items.as<int4>() + i0;
+  // Every ligand at once: the items longest first, so that the groups finish together.
+  a.items = s.items.as<int4>() + (n_items == s.n_items ? s.n_items : i0);
   a.scores = s.scores.as<float>();
   a.n_items = n_items;
   int per_sm = 0;
@@ -848,6 +851,11 @@ int surrogate_score_range(Context &c, int lig0, int lig1, int groups, cudaStream
     std::memcpy(t.w4, s.w4_host, sizeof t.w4);
     t.w = TcWeights{s.emb_h.ptr, s.w1_h.ptr, s.w2_h.ptr, s.w3_h.ptr, a.W.b1, a.W.b2, a.W.b3, a.W.w4, a.W.b4};
     t.err = c.err.as<unsigned int>();
+    int rc = s.next.reserve(256, "work counters");
+    if (rc) return rc;
+    t.next = s.next.as<unsigned int>() + 2; // the first two are the training step's
+    e = cudaMemsetAsync(t.next, 0, sizeof(unsigned int), st);
+    if (e != cudaSuccess) return cuda_error(e, "work counter");
     // One block per SM: a block holds all of its SM's TMEM it allocates.
     const int g = groups == 3 ? 3 : 4;
     const int grid = std::min((n_items + g - 1) / g, std::max(c.num_sms, 1));
