@@ -554,8 +554,9 @@ __global__ void __launch_bounds__(kBwdGroups * kTcGroupThreads, 1) train_backwar
   for (;;) {
     if (lt == 0) s.item[g] = (int)atomicAdd(A.next, 1u);
     named_sync(bar_id, kTcGroupThreads);
-    const int tile = s.item[g]; // rewritten only after the group's end-of-tile barrier below
-    if (tile >= tiles) break;
+    // From the last tile back: the forward pass stored those last, and L2 still holds them.
+    const int tile = tiles - 1 - s.item[g]; // rewritten only after the group's end-of-tile barrier below
+    if (tile < 0) break;
     const long long row = (long long)tile * kTcGroupThreads + lt;
     const bool valid = row < A.rows;
     uint4 z[16];
