@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <numeric>
 
+#include "chain.h"
 #include "cull.h"
 #include "cull_kernel.cuh"
 
@@ -33,8 +34,8 @@ template <int K, int P>
 static cudaError_t launch_kp(const CullArgs *a, unsigned grid, int threads, cudaStream_t st) {
   if (!a)
     return cudaFuncSetAttribute(cull_kernel<K, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCullMaxSmem);
-  cull_kernel<K, P><<<grid, threads, cull_smem_bytes(K * threads, threads, P, a->supers), st>>>(*a);
-  return cudaGetLastError();
+  return launch_chained(cull_kernel<K, P>, grid, (unsigned)threads, cull_smem_bytes(K * threads, threads, P, a->supers),
+                        st, *a);
 }
 
 template <int K>
@@ -73,8 +74,7 @@ static int launch(const CullArgs &a, long long grid, const bude_launch_cfg &s, c
 }
 
 static int finish(const FinishArgs &f, long long grid, cudaStream_t st, long long &launches) {
-  cull_finish_kernel<<<(unsigned)grid, 256, 0, st>>>(f);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_chained(cull_finish_kernel, (unsigned)grid, 256u, 0, st, f);
   if (e != cudaSuccess) return cuda_error(e, "cull_finish_kernel launch");
   launches++;
   return BUDE_OK;

@@ -345,6 +345,7 @@ template <int K, int P> __global__ void __launch_bounds__(kMaxThreads, 2) cull_k
   __shared__ float red[6][kMaxThreads / 32];
   __shared__ int next_group;
 
+  grid_dep_wait();
   int atom, row, n;
   long long pose0;
   if (a.items) {
@@ -517,6 +518,7 @@ static __global__ void __launch_bounds__(256) cull_finish_kernel(const FinishArg
   long long p0 = a.first + (long long)blockIdx.x * blockDim.x, p1 = min(p0 + blockDim.x, a.first + a.n);
   int rows = a.rows;
   bool all = a.e.all != 0;
+  grid_dep_wait();
   if (a.words) {
     if (deck_bad_type(a.words)) return;
     all = deck_irregular(a.words, a.e.natpro, a.e.natlig);

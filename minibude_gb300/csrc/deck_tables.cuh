@@ -11,6 +11,7 @@
 #include "../../include/minibude_gb300.h"
 #include "exact_shape.h"
 #include "pair_record.h"
+#include "ptx.cuh"
 #include "warp.cuh"
 
 namespace bude {
@@ -35,6 +36,7 @@ static __global__ void __launch_bounds__(256) deck_table_kernel(const bude_atom 
                                                                 float4 *__restrict__ reach, float4 *__restrict__ box,
                                                                 float *__restrict__ box_reach) {
   const int lane = threadIdx.x & 31;
+  grid_dep_wait();
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
   for (long long w = warp; w < (long long)ntypes * clusters; w += warps) {

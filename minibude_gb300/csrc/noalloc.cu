@@ -29,6 +29,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "chain.h"
 #include "cull.h"
 #include "cull_kernel.cuh"
 #include "deck_tables.cuh"
@@ -243,13 +244,15 @@ extern "C" int bude_gpu_fasten_noalloc(const bude_atom *protein, int32_t natpro,
   if (e != cudaSuccess) return cuda_error(e, "no-alloc deck kernel");
   auto *sorted = reinterpret_cast<bude_atom *>(rest);
   na_deck_kernel<<<1, 1024, keys, st>>>(protein, natpro, ligand, natlig, forcefield, ntypes, sort, words, sorted);
-  deck_table_kernel<<<deck_table_grid(ntypes, clusters), 256, 0, st>>>(sort ? sorted : protein, natpro, forcefield,
-                                                                       ntypes, natpro_pad, clusters, slab, reach, box,
-                                                                       box_reach);
+  e = launch_chained(deck_table_kernel, deck_table_grid(ntypes, clusters), 256u, 0, st,
+                     sort ? (const bude_atom *)sorted : protein, natpro, forcefield, ntypes, natpro_pad, clusters, slab,
+                     reach, box, box_reach);
   // 2. pose transforms and the exact kernel; irregular poses (or every pose of an irregular deck) by the
   //    reference's arithmetic.
-  pose_xform_kernel<<<(unsigned)((nposes + 255) / 256), 256, 0, st>>>(poses, pose_stride, nposes, xform, mask);
-  e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = launch_chained(pose_xform_kernel, (unsigned)((nposes + 255) / 256), 256u, 0, st, poses, (long long)pose_stride,
+                       (long long)nposes, xform, mask);
+  if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_error(e, "no-alloc deck launch");
   const bude_launch_cfg cfg = cull_shape(nposes, natlig, 1);
   CullArgs a{};

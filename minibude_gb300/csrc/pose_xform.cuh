@@ -1,6 +1,7 @@
 // pose_xform.cuh -- the 3x4 transforms of the poses.
 #pragma once
 #include "edge_pose.cuh"
+#include "ptx.cuh"
 
 namespace bude {
 
@@ -14,6 +15,7 @@ static __global__ void __launch_bounds__(256) pose_xform_kernel(const float *__r
                                                          unsigned *__restrict__ edge_mask) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   bool irregular = false;
+  grid_dep_wait();
   if (i < nposes) {
     float sx, cx, sy, cy, sz, cz;
     sincosf(poses[i], &sx, &cx);

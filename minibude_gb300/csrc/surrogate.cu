@@ -17,6 +17,7 @@
 #include <utility>
 #include <vector>
 
+#include "chain.h"
 #include "cull.h"
 #include "pose_xform.cuh"
 #include "score_tc.cuh"
@@ -352,27 +353,6 @@ static int ensure_train_scratch(Surrogate &s, long long rows, int batch, int wg_
   if (!rc) rc = s.part_w.reserve((size_t)std::max(wg_blocks, 1) * kWgPart * 4, "gradient parts");
   if (!rc) rc = s.S_sum.reserve((size_t)kHid * kMaxTypes * 4, "per-type dz1 sums");
   return rc;
-}
-
-// Launch one kernel of a training step with programmatic stream serialisation: its blocks are
-// scheduled as the kernel before it finishes, and run their setup (barriers, TMEM allocation) until
-// grid_dep_wait (ptx.cuh) while that kernel's completion is processed.  Every kernel launched this
-// way waits before it touches the step's buffers.  80 epochs of 512 ligands x 4096 poses: 6.03 s
-// this way, 6.48 s in plain stream order.
-template <class... KArgs, class... Args>
-static cudaError_t launch_chained(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem,
-                                  cudaStream_t st, Args &&...args) {
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
 // One optimisation step on `nb` poses whose indices/row offsets are at dpose/drowoff; the poses'
