@@ -37,7 +37,6 @@ static int time_cfg(Context &c, const bude_launch_cfg &cfg, int reps, float *ms)
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  if (!rc) rc = check_device_error(c);
   return rc;
 }
 

@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <numeric>
 #include <vector>
 
@@ -20,7 +21,6 @@ namespace bude {
 void release_batch(Context &c) {
   if (c.graph) cudaGraphExecDestroy(c.graph);
   c.graph = nullptr;
-  c.b_ligands.release();
   c.b_poses.release();
   c.b_xform.release();
   c.b_energies.release();
@@ -28,11 +28,7 @@ void release_batch(Context &c) {
   c.b_folds.release();
   c.b_sums.release();
   c.b_edge_mask.release();
-  c.b_pose_off.release();
-  c.b_lig_off.release();
-  c.b_lig_all.release();
-  c.b_lig_any.release();
-  c.b_irregular_ligands = 0;
+  c.b_meta.release();
   c.b_lig_all_host.clear();
   c.have_batch = false;
   delete c.plan;
@@ -83,38 +79,42 @@ int upload_batch(Context &c, const bude_atom *protein, int natpro, const bude_ff
   const bool keep = same_shape && !rebuilt;
   if (!keep) drop_graph(c);
   const long long np = std::max(total_poses, 1LL);
-  rc = c.b_ligands.reserve((size_t)std::max(total_atoms, 1) * 16, "batch ligands");
-  if (!rc) rc = c.b_poses.reserve((size_t)6 * np * sizeof(float), "batch poses");
-  if (!rc) rc = c.b_xform.reserve((size_t)12 * np * sizeof(float), "batch transforms");
-  if (!rc) rc = c.b_energies.reserve((size_t)np * sizeof(float), "batch energies");
-  if (!rc) rc = c.b_edge_mask.reserve((size_t)(np + 31) / 32 * sizeof(unsigned), "batch irregular-pose bits");
-  if (!rc) rc = c.b_pose_off.reserve((size_t)(nligands + 1) * sizeof(long long), "batch pose offsets");
-  if (!rc) rc = c.b_lig_off.reserve((size_t)(nligands + 1) * sizeof(int), "batch atom offsets");
-  if (!rc) rc = c.b_lig_all.reserve((size_t)std::max(nligands, 1), "batch irregular ligands");
-  if (!rc) rc = c.b_lig_any.reserve(sizeof(int), "batch irregular ligand count");
+  const size_t at_any = (size_t)(nligands + 1) * sizeof(long long), at_lig = at_any + 2 * sizeof(int),
+               at_atoms = (at_lig + (size_t)(nligands + 1) * sizeof(int) + 15) / 16 * 16,
+               at_all = at_atoms + (size_t)total_atoms * sizeof(bude_atom), meta_bytes = at_all + (size_t)nligands;
+  rc = reserve_together({{&c.b_poses, (size_t)6 * np * sizeof(float)},
+                         {&c.b_xform, (size_t)12 * np * sizeof(float)},
+                         {&c.b_energies, (size_t)np * sizeof(float)},
+                         {&c.b_edge_mask, (size_t)(np + 31) / 32 * sizeof(unsigned)},
+                         {&c.b_meta, meta_bytes}},
+                        "batch");
   if (rc) return rc;
-  // Ligands outside the regular-deck bounds (edge_pose.cuh): all their poses go to edge_pose_kernel.
-  std::vector<unsigned char> lig_all((size_t)std::max(nligands, 1), 0);
+  std::vector<unsigned char> meta(meta_bytes);
+  std::memcpy(meta.data(), pose_off, at_any);
+  std::memcpy(meta.data() + at_lig, lig_off, (size_t)(nligands + 1) * sizeof(int));
+  if (total_atoms > 0) std::memcpy(meta.data() + at_atoms, atoms, (size_t)total_atoms * sizeof(bude_atom));
+  // Ligands outside the regular-deck bounds (edge_pose.cuh): all their poses go to edge_energy.
+  unsigned char *lig_all = meta.data() + at_all;
   int n_irregular = 0;
   for (int l = 0; l < nligands; ++l) {
-    lig_all[(size_t)l] = !ligand_regular(c, atoms + lig_off[l], lig_off[l + 1] - lig_off[l], ff);
-    n_irregular += lig_all[(size_t)l];
+    lig_all[l] = !ligand_regular(c, atoms + lig_off[l], lig_off[l + 1] - lig_off[l], ff);
+    n_irregular += lig_all[l];
   }
-  cudaError_t e = cudaSuccess;
-  if (total_atoms > 0) e = copy_sync(c, c.b_ligands.ptr, atoms, (size_t)total_atoms * 16, cudaMemcpyHostToDevice);
+  std::memcpy(meta.data() + at_any, &n_irregular, sizeof n_irregular);
+  cudaError_t e = cudaMemcpyAsync(c.b_meta.ptr, meta.data(), meta_bytes, cudaMemcpyHostToDevice, c.stream);
   if (e == cudaSuccess && total_poses > 0)
     e = copy2d_sync(c, c.b_poses.ptr, (size_t)total_poses * sizeof(float), poses, (size_t)pose_stride * sizeof(float),
                     (size_t)total_poses * sizeof(float), 6, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess)
-    e = copy_sync(c, c.b_pose_off.ptr, pose_off, (size_t)(nligands + 1) * sizeof(long long), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess)
-    e = copy_sync(c, c.b_lig_off.ptr, lig_off, (size_t)(nligands + 1) * sizeof(int), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && nligands > 0)
-    e = copy_sync(c, c.b_lig_all.ptr, lig_all.data(), (size_t)nligands, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = copy_sync(c, c.b_lig_any.ptr, &n_irregular, sizeof(int), cudaMemcpyHostToDevice);
+  else if (e == cudaSuccess)
+    e = cudaStreamSynchronize(c.stream);
   if (e != cudaSuccess) return cuda_error(e, "batch upload");
-  c.b_irregular_ligands = n_irregular;
-  c.b_lig_all_host.assign(lig_all.begin(), lig_all.begin() + nligands);
+  const unsigned char *dev = c.b_meta.as<unsigned char>();
+  c.b_pose_off = reinterpret_cast<const long long *>(dev);
+  c.b_lig_any = reinterpret_cast<const int *>(dev + at_any);
+  c.b_lig_off = reinterpret_cast<const int *>(dev + at_lig);
+  c.b_ligands = reinterpret_cast<const float4 *>(dev + at_atoms);
+  c.b_lig_all = dev + at_all;
+  c.b_lig_all_host.assign(lig_all, lig_all + nligands);
   c.have_batch = true;
   ++c.batch_uploads;
   if (keep) return BUDE_OK;
@@ -218,7 +218,7 @@ int enqueue_batch(Context &c, const bude_launch_cfg &cfg, int per_ligand) {
   // One plain launch per ligand after one transform pass over all poses.
   rc = enqueue_transforms(c);
   for (int l = 0; l < c.nligands && !rc; ++l)
-    rc = launch_exact_range(c, cfg, c.b_ligands.as<float4>() + c.lig_off[l], c.lig_off[l + 1] - c.lig_off[l], false,
+    rc = launch_exact_range(c, cfg, c.b_ligands + c.lig_off[l], c.lig_off[l + 1] - c.lig_off[l], false,
                             nullptr, c.b_xform.as<float>() + c.pose_off[l] * 12,
                             c.b_energies.as<float>() + c.pose_off[l], c.pose_off[l + 1] - c.pose_off[l]);
   return rc ? rc : enqueue_edge_batch(c, c.b_xform.as<float>(), c.b_energies.as<float>(), nullptr, c.stream);
@@ -263,7 +263,6 @@ int autotune_batch(Context &c, int max_ms, bude_launch_cfg &best, float *best_ms
     }
     if (spent > (float)std::max(max_ms, 1)) break;
   }
-  if (!rc) rc = check_device_error(c);
   if (rc) return rc;
   if (best_t >= 1e30f) return set_error(BUDE_ERR_ARG, "no batch launch shape fits this device");
   c.batch_tuned = best;
@@ -313,7 +312,7 @@ int bude_gpu_run_batch(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, int32_t pe
   cudaError_t e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) return cuda_error(e, "batch evaluation");
   if (ms) cudaEventElapsedTime(ms, ctx->ev0, ctx->ev1);
-  return check_device_error(*ctx);
+  return BUDE_OK;
 }
 
 int bude_gpu_download_batch(bude_gpu_ctx *ctx, float *energies, int64_t total_poses) {

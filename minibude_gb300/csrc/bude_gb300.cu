@@ -114,22 +114,26 @@ int ensure_slab(Context &c, const bude_atom *protein, int natpro, const bude_ffp
   const int clusters = c.natpro_pad / kClusterAtoms;
   const size_t records = (size_t)ntypes * c.natpro_pad;
   const size_t nb = (size_t)natpro * sizeof(bude_atom), nf = (size_t)ntypes * sizeof(bude_ffparams);
-  int rc = c.slab.reserve(records * kPairF4 * sizeof(float4), "deck tables");
-  if (!rc) rc = c.reach.reserve(records * sizeof(float4), "deck tables");
-  if (!rc) rc = c.box.reserve((size_t)clusters * 2 * sizeof(float4), "deck tables");
-  if (!rc) rc = c.box_reach.reserve((size_t)ntypes * clusters * sizeof(float), "deck tables");
-  if (!rc) rc = c.raw.reserve(2 * nb + nf, "deck records");
+  const int rc = reserve_together({{&c.slab, records * kPairF4 * sizeof(float4)},
+                                   {&c.reach, records * sizeof(float4)},
+                                   {&c.box, (size_t)clusters * 2 * sizeof(float4)},
+                                   {&c.box_reach, (size_t)ntypes * clusters * sizeof(float)},
+                                   {&c.raw, 2 * nb + nf}},
+                                  "deck tables");
   if (rc) return rc;
   // One copy: the protein in cluster order, the protein as given, the forcefield.
   std::vector<int> order((size_t)natpro);
   for (int i = 0; i < natpro; ++i) order[(size_t)i] = i;
   cluster_order(protein, order.data(), natpro);
-  std::vector<unsigned char> raw(2 * nb + nf);
+  cudaStreamSynchronize(c.stream); // an earlier copy from `staging` has finished
+  std::vector<unsigned char> &raw = c.staging;
+  raw.resize(2 * nb + nf);
   auto *sorted = reinterpret_cast<bude_atom *>(raw.data());
   for (int i = 0; i < natpro; ++i) sorted[i] = protein[order[(size_t)i]];
   if (nb) std::memcpy(raw.data() + nb, protein, nb);
   std::memcpy(raw.data() + 2 * nb, ff, nf);
-  cudaError_t e = copy_sync(c, c.raw.ptr, raw.data(), raw.size(), cudaMemcpyHostToDevice);
+  // Waited for by the caller's last copy.
+  cudaError_t e = cudaMemcpyAsync(c.raw.ptr, raw.data(), raw.size(), cudaMemcpyHostToDevice, c.stream);
   if (e != cudaSuccess) return cuda_error(e, "deck upload");
   c.raw_protein = c.raw.as<bude_atom>() + natpro;
   c.raw_ff = reinterpret_cast<const bude_ffparams *>(c.raw.as<bude_atom>() + 2 * (size_t)natpro);
@@ -195,12 +199,12 @@ EdgeArgs edge_args_single(const Context &c, const float4 *ligand, int natlig, bo
 }
 
 EdgeArgs edge_args_batch(const Context &c, const float *xform) {
-  EdgeArgs a = edge_args_single(c, c.b_ligands.as<float4>(), 0, false, c.b_edge_mask.as<unsigned>(), xform);
+  EdgeArgs a = edge_args_single(c, c.b_ligands, 0, false, c.b_edge_mask.as<unsigned>(), xform);
   a.nposes = c.batch_poses;
-  a.pose_off = c.b_pose_off.as<long long>();
-  a.lig_off = c.b_lig_off.as<int>();
-  a.lig_any = c.b_lig_any.as<int>();
-  a.lig_all = c.b_lig_all.as<unsigned char>();
+  a.pose_off = c.b_pose_off;
+  a.lig_off = c.b_lig_off;
+  a.lig_any = c.b_lig_any;
+  a.lig_all = c.b_lig_all;
   a.nlig = c.nligands;
   return a;
 }
@@ -219,21 +223,53 @@ int enqueue_edge_batch(Context &c, const float *xform, float *energies, unsigned
 
 // ---------------------------------------------------------------------------------------------
 // Device buffers
+static int allocate(std::shared_ptr<void> &block, size_t nbytes, const char *what) {
+  void *p = nullptr;
+  const cudaError_t e = cudaMalloc(&p, std::max<size_t>(nbytes, 256));
+  if (e != cudaSuccess) return cuda_error(e, what);
+  block = std::shared_ptr<void>(p, [](void *q) { cudaFree(q); });
+  return BUDE_OK;
+}
+
 int DevBuf::reserve(size_t nbytes, const char *what) {
   if (nbytes <= cap) return BUDE_OK;
-  if (ptr) cudaFree(ptr);
-  ptr = nullptr;
-  cap = 0;
-  cudaError_t e = cudaMalloc(&ptr, std::max<size_t>(nbytes, 256));
-  if (e != cudaSuccess) return cuda_error(e, what);
+  release();
+  const int rc = allocate(block, nbytes, what);
+  if (rc) return rc;
+  ptr = block.get();
   cap = nbytes;
   return BUDE_OK;
 }
 
 void DevBuf::release() {
-  if (ptr) cudaFree(ptr);
+  block.reset();
   ptr = nullptr;
   cap = 0;
+}
+
+int reserve_together(std::initializer_list<DevWant> wants, const char *what) {
+  auto room = [](size_t bytes) { return (bytes + 511) / 512 * 512; };
+  size_t total = 0;
+  for (const DevWant &w : wants)
+    if (!w.buf->ptr) total += room(w.bytes);
+  std::shared_ptr<void> block;
+  if (total > 0) {
+    const int rc = allocate(block, total, what);
+    if (rc) return rc;
+  }
+  size_t at = 0;
+  for (const DevWant &w : wants) {
+    if (w.buf->ptr) {
+      const int rc = w.buf->reserve(w.bytes, what);
+      if (rc) return rc;
+      continue;
+    }
+    w.buf->block = block;
+    w.buf->ptr = static_cast<unsigned char *>(block.get()) + at;
+    w.buf->cap = w.bytes;
+    at += room(w.bytes);
+  }
+  return BUDE_OK;
 }
 
 } // namespace bude
@@ -301,9 +337,25 @@ static __global__ void wait_selftest_kernel(unsigned int *err, unsigned long lon
   }
 }
 
+int ensure_error_word(Context &c) {
+  if (c.err.ptr) return BUDE_OK;
+  const int rc = c.err.reserve(sizeof(unsigned int) * 4, "error word");
+  if (rc) return rc;
+  cudaError_t e = cudaMemsetAsync(c.err.ptr, 0, sizeof(unsigned int) * 4, c.stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream); // its first user may be on another stream
+  if (e != cudaSuccess) c.err.release();
+  return e == cudaSuccess ? BUDE_OK : cuda_error(e, "error word");
+}
+
+int sync_stream(Context &c, const char *what) {
+  const cudaError_t e = cudaStreamSynchronize(c.stream);
+  return e == cudaSuccess ? BUDE_OK : cuda_error(e, what);
+}
+
 // Read (and clear) the device error word after the stream has drained.
 int check_device_error(Context &c) {
   unsigned int h = 0;
+  if (!c.err.ptr) return sync_stream(c, "device error word");
   cudaError_t e = cudaMemcpyAsync(&h, c.err.ptr, sizeof h, cudaMemcpyDeviceToHost, c.stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
   if (e != cudaSuccess) return cuda_error(e, "device error word");
@@ -336,10 +388,14 @@ static int upload_poses(Context &c, const float *poses, long long stride, long l
   if (nposes < 0 || (nposes > 0 && (!poses || stride < nposes)))
     return set_error(BUDE_ERR_ARG, "bad pose block (nposes %lld, stride %lld)", nposes, stride);
   const long long n = std::max(nposes, 1LL);
-  int rc = c.poses.reserve((size_t)6 * n * sizeof(float), "poses");
-  if (!rc) rc = c.xform.reserve((size_t)12 * n * sizeof(float), "transforms");
-  if (!rc) rc = c.energies.reserve((size_t)n * sizeof(float), "energies");
-  if (!rc) rc = c.edge_mask.reserve((size_t)(n + 31) / 32 * sizeof(unsigned), "irregular-pose bits");
+  // With the sums that an evaluation of the deck needs, unless they are large.
+  const size_t sums = (size_t)c.natlig * (size_t)n * sizeof(float);
+  const int rc = reserve_together({{&c.poses, (size_t)6 * n * sizeof(float)},
+                                   {&c.xform, (size_t)12 * n * sizeof(float)},
+                                   {&c.energies, (size_t)n * sizeof(float)},
+                                   {&c.edge_mask, (size_t)(n + 31) / 32 * sizeof(unsigned)},
+                                   {&c.partial, c.partial.ptr || sums > ((size_t)64 << 20) ? 0 : sums}},
+                                  "poses and energies");
   if (rc) return rc;
   if (nposes > 0) {
     cudaError_t e = cudaMemcpy2DAsync(c.poses.ptr, (size_t)nposes * sizeof(float), poses, (size_t)stride * sizeof(float),
@@ -398,15 +454,6 @@ int make_context(int device, Context **out) {
   if (e != cudaSuccess) {
     destroy_context(c);
     return cuda_error(e, "stream/event creation");
-  }
-  int rc = c->err.reserve(sizeof(unsigned int) * 4, "error word");
-  if (!rc) {
-    e = cudaMemsetAsync(c->err.ptr, 0, sizeof(unsigned int) * 4, c->stream);
-    if (e != cudaSuccess) rc = cuda_error(e, "error word");
-  }
-  if (rc) {
-    destroy_context(c);
-    return rc;
   }
   *out = c;
   return BUDE_OK;
@@ -549,7 +596,7 @@ int bude_gpu_run(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, float *kernel_ms
     e = cudaEventElapsedTime(kernel_ms, ctx->ev0, ctx->ev1);
     if (e != cudaSuccess) return cuda_error(e, "event timing");
   }
-  return bude::check_device_error(*ctx);
+  return BUDE_OK;
 }
 
 int bude_gpu_run_many(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, int32_t iterations, int32_t flush_l2,
@@ -579,8 +626,7 @@ int bude_gpu_run_many(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, int32_t ite
   }
   for (auto &x : ev)
     if (x) cudaEventDestroy(x);
-  if (rc) return rc;
-  return bude::check_device_error(*ctx);
+  return rc;
 }
 
 int bude_gpu_download(bude_gpu_ctx *ctx, float *energies, int64_t nposes) {
@@ -609,7 +655,7 @@ int bude_gpu_score_host(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, const bud
                                     cudaMemcpyDeviceToHost, ctx->stream);
     if (e != cudaSuccess) return cuda_error(e, "energy download");
   }
-  return bude::check_device_error(*ctx); // synchronises the stream
+  return bude::sync_stream(*ctx, "evaluation");
 }
 
 int bude_gpu_fasten(int device, int32_t ppwi, int32_t wgsize, const bude_atom *protein, int32_t natpro,
@@ -638,6 +684,8 @@ int bude_gpu_selftest_wait(bude_gpu_ctx *ctx, int32_t limit_us, float *elapsed_m
   if (!ctx) return set_error(BUDE_ERR_ARG, "NULL context");
   if (limit_us < 1 || limit_us > 1000000) return set_error(BUDE_ERR_ARG, "limit_us must be in [1, 1000000]");
   bude::Context &c = *ctx;
+  const int rc = bude::ensure_error_word(c);
+  if (rc) return rc;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);

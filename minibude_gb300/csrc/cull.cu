@@ -191,7 +191,7 @@ CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vec
 int enqueue_plan(Context &c, const bude_launch_cfg &shape, const CullPlan &plan, const int4 *items, const int4 *folds,
                  const float *xform, float *energies, float *sums, bool edges, cudaStream_t st) {
   CullArgs a = cull_args(c, shape);
-  a.ligand = c.b_ligands.as<float4>();
+  a.ligand = c.b_ligands;
   a.xform = xform;
   a.sums = sums;
   FinishArgs f{};

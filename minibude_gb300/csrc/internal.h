@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <initializer_list>
+#include <memory>
 #include <vector>
 
 #include "../../include/minibude_gb300.h"
@@ -38,14 +40,23 @@ struct EventSet {
   }
 };
 
-// A growable device allocation.
+// A growable device allocation, or its part of one that several buffers share (reserve_together).
 struct DevBuf {
   void *ptr = nullptr;
   size_t cap = 0;
+  std::shared_ptr<void> block; // freed with its last buffer
   int reserve(size_t nbytes, const char *what);
   void release();
   template <class T> T *as() const { return static_cast<T *>(ptr); }
 };
+
+// Reserve several buffers, those that have none yet as parts of one allocation: an upload into a new
+// context makes one cudaMalloc instead of a dozen.
+struct DevWant {
+  DevBuf *buf;
+  size_t bytes;
+};
+int reserve_together(std::initializer_list<DevWant> wants, const char *what);
 
 // State behind a bude_gpu_ctx handle.
 struct Context {
@@ -65,6 +76,7 @@ struct Context {
   // Irregular poses and decks (edge_pose.cuh): the raw protein and forcefield records, the
   // transform pass's irregular-pose bits of the deck's poses, and whether the deck is irregular.
   DevBuf raw, edge_mask; // raw: the protein in cluster order, as given, the forcefield
+  std::vector<unsigned char> staging; // host side of raw, until the stream has drained
   const bude_atom *raw_protein = nullptr; // as given
   const bude_ffparams *raw_ff = nullptr;
   std::vector<bude_ffparams> host_ff; // the forcefield the slab was built from
@@ -79,12 +91,15 @@ struct Context {
   std::vector<int> lig_off;        // nligands + 1 atom offsets
   std::vector<long long> pose_off; // nligands + 1 pose offsets
   long long batch_poses = 0;
-  DevBuf b_ligands, b_poses, b_xform, b_energies;
+  DevBuf b_poses, b_xform, b_energies;
   DevBuf b_items, b_folds, b_sums; // the device half of `plan` and its atom sums (graph-owned)
   // Irregular poses of the batch: transform-pass bits, device pose/atom offsets, and the ligands
   // whose every pose goes to edge_pose_kernel (lig_all flags and their count, both on the device).
-  DevBuf b_edge_mask, b_pose_off, b_lig_off, b_lig_all, b_lig_any;
-  int b_irregular_ligands = 0;
+  DevBuf b_edge_mask, b_meta; // b_meta: [pose_off | lig_any | lig_off | atoms | lig_all], one copy per upload
+  const long long *b_pose_off = nullptr;
+  const int *b_lig_any = nullptr, *b_lig_off = nullptr;
+  const float4 *b_ligands = nullptr;
+  const unsigned char *b_lig_all = nullptr;
   std::vector<unsigned char> b_lig_all_host; // host copy of the lig_all flags
   CullPlan *plan = nullptr;  // the batch cut for graph_cfg
   cudaGraphExec_t graph = nullptr;
@@ -171,7 +186,11 @@ EdgeArgs edge_args_single(const Context &c, const float4 *ligand, int natlig, bo
 EdgeArgs edge_args_batch(const Context &c, const float *xform);
 // Enqueue edge_pose_kernel over the uploaded batch's poses (flag: optional per-pose marks).
 int enqueue_edge_batch(Context &c, const float *xform, float *energies, unsigned char *flag, cudaStream_t st);
+// The device error word, allocated by the first kernel that has waits to bound (the exact kernels have
+// none), and its check, which waits for the stream.
+int ensure_error_word(Context &c);
 int check_device_error(Context &c);
+int sync_stream(Context &c, const char *what);
 int flush_l2(Context &c);
 int probe_kernel_arch(int device, int *cc);
 

@@ -334,7 +334,7 @@ static int upload_plan(Context &c, ScreenState &s, const CullPlan &plan) {
   if (!rc) rc = s.folds.reserve(std::max<size_t>(plan.folds.size(), 1) * sizeof(int4), "screen items");
   if (!rc) rc = s.sums.reserve(std::max<size_t>(plan.sums_bytes, 16), "screen atom sums");
   if (rc) return rc;
-  cudaError_t e = cudaSuccess; // pageable sources: staged before the calls return
+  cudaError_t e = cudaSuccess; // the plan outlives the copies: every way out of screen_run drains the stream
   if (!plan.items.empty())
     e = cudaMemcpyAsync(s.items.ptr, plan.items.data(), plan.items.size() * sizeof(int4), cudaMemcpyHostToDevice, c.stream);
   if (e == cudaSuccess && !plan.folds.empty())
@@ -430,9 +430,11 @@ int screen_run(Context &c, const bude_screen_cfg &sc, bude_screen_stats *stats) 
   cudaMemcpyAsync(s.pose_off.ptr, c.pose_off.data(), (size_t)(nl + 1) * 8, cudaMemcpyHostToDevice, c.stream);
   cudaMemcpyAsync(s.comp_off.ptr, comp_off.data(), comp_off.size() * 8, cudaMemcpyHostToDevice, c.stream);
   rc = upload_plan(c, s, plan);
-  if (rc) return rc;
-  rc = surrogate_prepare(c, false); // pose transforms of every pose
-  if (rc) return rc;
+  if (!rc) rc = surrogate_prepare(c, false); // pose transforms of every pose
+  if (rc) {
+    cudaStreamSynchronize(c.stream);
+    return rc;
+  }
   const float *scores = surrogate_scores(c);
   cudaStream_t rs = overlap ? s.side : c.stream;
   // 1-3. per chunk: surrogate, picks and audit sample, compaction; exact rescoring on `rs`
@@ -519,9 +521,7 @@ int screen_run(Context &c, const bude_screen_cfg &sc, bude_screen_stats *stats) 
   rc = enqueue_edge_batch(c, c.b_xform.as<float>(), s.final_e.as<float>(), s.rescored.as<unsigned char>(), c.stream);
   if (rc) return rc;
   cudaEventRecord(ev[4], c.stream);
-  e = cudaStreamSynchronize(c.stream);
-  if (e != cudaSuccess) return cuda_error(e, "screen");
-  rc = check_device_error(c);
+  rc = check_device_error(c); // waits for the stream
   if (rc) return rc;
   if (stats) {
     cudaEventElapsedTime(&stats->total_ms, ev[0], ev[4]);

@@ -141,7 +141,7 @@ static int score_stream(Context &c, const bude_launch_cfg &cfg, const float *pos
   if (e != cudaSuccess) return cuda_error(e, "streamed evaluation");
   if (es != cudaSuccess) return cuda_error(es, "streamed evaluation");
   if (ms) cudaEventElapsedTime(ms, c.ev0, c.ev1);
-  return check_device_error(c);
+  return BUDE_OK;
 }
 
 } // namespace bude

@@ -55,6 +55,14 @@ struct Surrogate {
   long long step = 0;
   // training scratch
   DevBuf X, row_type, Z1, Z2, Z3, dZ1, dZ2, dZ3, y, dy, pred, loss, dsum, part_w, S_sum;
+  // pose -> ligand (first atom, atoms) of the batch shape pose_lig_for, on the device and (atoms) here
+  std::vector<int> lig_n;
+  long long pose_lig_for = -1;
+  // training pipeline: copy stream, events and pinned epoch buffers, kept between calls
+  cudaStream_t copy_stream = nullptr;
+  cudaEvent_t copied[2] = {}, used[2] = {}, e0 = nullptr, e1 = nullptr;
+  int *host_epoch[2] = {}; // pinned: an epoch's pose order, then its row offsets
+  size_t host_epoch_ints = 0;
   DevBuf labels, pose_lig_first, pose_lig_n, epoch_pose, epoch_rowoff, epoch_pose2, epoch_rowoff2, epoch_loss;
   long long rows_cap = 0;
   // scoring
@@ -90,6 +98,11 @@ void release_surrogate(Context &c) {
                    &s.epoch_pose, &s.epoch_rowoff, &s.epoch_pose2, &s.epoch_rowoff2, &s.epoch_loss, &s.items,
                    &s.scores, &s.next};
   for (DevBuf *b : all) b->release();
+  if (s.copy_stream) cudaStreamDestroy(s.copy_stream);
+  for (cudaEvent_t ev : {s.copied[0], s.copied[1], s.used[0], s.used[1], s.e0, s.e1})
+    if (ev) cudaEventDestroy(ev);
+  for (int *h : s.host_epoch)
+    if (h) cudaFreeHost(h);
   delete c.surrogate;
   c.surrogate = nullptr;
 }
@@ -372,12 +385,13 @@ static int train_step(Context &c, Surrogate &s, const int *dpose, const int *dro
   const int wg_grid = (int)std::min<long long>((rows + kWgTile - 1) / kWgTile, std::max(c.num_sms, 1));
   int rc = ensure_train_scratch(s, rows, nb, wg_grid);
   if (!rc) rc = s.next.reserve(256, "work counters");
+  if (!rc) rc = ensure_error_word(c);
   if (rc) return rc;
   // The step's kernels run as one chain of programmatic dependent launches (launch_chained); the
   // features kernel zeroes the forward (next[0]) and backward (next[1]) tile counters.
   unsigned int *counters = s.next.as<unsigned int>();
   cudaError_t le = launch_chained(train_features_kernel, (unsigned)((nb * 32 + 255) / 256), 256u, 0, c.stream, W,
-                                  s.fg, c.b_ligands.as<float4>(), c.b_xform.as<float4>(), m,
+                                  s.fg, c.b_ligands, c.b_xform.as<float4>(), m,
                                   s.X.as<__nv_bfloat16>(), s.row_type.as<int>(), counters);
   {
     // Forward on the tensor cores (score_tc.cuh): z1, z2, z3 as BF16 and y per row.
@@ -488,25 +502,56 @@ static int train_step(Context &c, Surrogate &s, const int *dpose, const int *dro
   return BUDE_OK;
 }
 
-// Pose -> (first ligand atom, natlig) for every pose of the uploaded batch.
-static int upload_pose_ligands(Context &c, Surrogate &s, std::vector<int> &lig_n) {
+// Pose -> (first ligand atom, natlig) for every pose of the uploaded batch, kept for its shape: on the
+// device, and the atom counts on the host.
+__global__ void __launch_bounds__(256) pose_ligand_kernel(const long long *pose_off, const int *lig_off, int nlig,
+                                                          long long np, int *first, int *n) {
+  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= np) return;
+  const int l = edge_ligand_of(pose_off, nlig, p);
+  first[p] = lig_off[l];
+  n[p] = lig_off[l + 1] - lig_off[l];
+}
+
+static int ensure_pose_ligands(Context &c, Surrogate &s) {
+  if (s.pose_lig_for == c.batch_gen) return BUDE_OK;
+  s.pose_lig_for = -1;
   const long long np = c.batch_poses;
-  std::vector<int> first((size_t)np);
-  lig_n.assign((size_t)np, 0);
+  s.lig_n.resize((size_t)np);
   for (int l = 0; l < c.nligands; ++l)
-    for (long long p = c.pose_off[l]; p < c.pose_off[l + 1]; ++p) {
-      first[(size_t)p] = c.lig_off[l];
-      lig_n[(size_t)p] = c.lig_off[l + 1] - c.lig_off[l];
-    }
+    std::fill(s.lig_n.begin() + c.pose_off[l], s.lig_n.begin() + c.pose_off[l + 1], c.lig_off[l + 1] - c.lig_off[l]);
   int rc = s.pose_lig_first.reserve((size_t)std::max(np, 1LL) * 4, "pose ligands");
   if (!rc) rc = s.pose_lig_n.reserve((size_t)std::max(np, 1LL) * 4, "pose ligands");
   if (rc) return rc;
   if (np > 0) {
-    cudaError_t e = copy_sync(c, s.pose_lig_first.ptr, first.data(), (size_t)np * 4, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = copy_sync(c, s.pose_lig_n.ptr, lig_n.data(), (size_t)np * 4, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return cuda_error(e, "pose ligands");
+    pose_ligand_kernel<<<(unsigned)((np + 255) / 256), 256, 0, c.stream>>>(c.b_pose_off, c.b_lig_off, c.nligands, np,
+                                                                           s.pose_lig_first.as<int>(),
+                                                                           s.pose_lig_n.as<int>());
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_error(e, "pose_ligand_kernel launch");
   }
+  s.pose_lig_for = c.batch_gen;
   return BUDE_OK;
+}
+
+// The training pipeline with pinned room for `ints` values per epoch buffer.
+static int ensure_pipeline(Surrogate &s, size_t ints) {
+  cudaError_t e = cudaSuccess;
+  if (!s.copy_stream) e = cudaStreamCreateWithFlags(&s.copy_stream, cudaStreamNonBlocking);
+  for (cudaEvent_t *ev : {&s.copied[0], &s.copied[1], &s.used[0], &s.used[1]})
+    if (e == cudaSuccess && !*ev) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+  for (cudaEvent_t *ev : {&s.e0, &s.e1})
+    if (e == cudaSuccess && !*ev) e = cudaEventCreate(ev);
+  if (ints > s.host_epoch_ints) {
+    s.host_epoch_ints = 0;
+    for (int *&h : s.host_epoch) {
+      if (h) cudaFreeHost(h);
+      h = nullptr;
+      if (e == cudaSuccess) e = cudaMallocHost((void **)&h, ints * sizeof(int));
+    }
+    if (e == cudaSuccess) s.host_epoch_ints = ints;
+  }
+  return e == cudaSuccess ? BUDE_OK : cuda_error(e, "training pipeline (stream, events, pinned buffers)");
 }
 
 static int batch_transforms(Context &c) {
@@ -539,26 +584,33 @@ int surrogate_train(Context &c, int epochs, int batch, float lr, const float *la
   int rc = s.labels.reserve((size_t)np * 4, "labels");
   if (rc) return rc;
   if (labels) {
-    const cudaError_t e = copy_sync(c, s.labels.ptr, labels, (size_t)np * 4, cudaMemcpyHostToDevice);
+    const cudaError_t e = cudaMemcpyAsync(s.labels.ptr, labels, (size_t)np * 4, cudaMemcpyHostToDevice, c.stream);
     if (e != cudaSuccess) return cuda_error(e, "labels");
   } else {
     // Labels: exact energies of every pose from the batched exact kernel.
     rc = enqueue_batch(c, batch_shape(c), 0);
-    if (!rc) rc = check_device_error(c);
     if (rc) return rc;
     cudaMemcpyAsync(s.labels.ptr, c.b_energies.ptr, (size_t)np * 4, cudaMemcpyDeviceToDevice, c.stream);
   }
-  std::vector<int> lig_n;
-  rc = upload_pose_ligands(c, s, lig_n);
+  rc = ensure_pose_ligands(c, s);
   if (!rc) rc = batch_transforms(c);
-  if (rc) return rc;
   // The poses learnt from: regular ones (edge_pose.cuh: finite transforms, translations and atoms
   // within bounds) with finite labels.  Every pose of an ordinary batch qualifies.
-  std::vector<float> hl((size_t)np);
+  std::vector<float> computed;
   std::vector<unsigned> edge((size_t)(np + 31) / 32);
-  cudaError_t e = copy_sync(c, hl.data(), s.labels.ptr, (size_t)np * 4, cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = copy_sync(c, edge.data(), c.b_edge_mask.ptr, edge.size() * 4, cudaMemcpyDeviceToHost);
+  cudaError_t e = cudaSuccess;
+  if (!rc && !labels) {
+    computed.resize((size_t)np);
+    e = cudaMemcpyAsync(computed.data(), s.labels.ptr, (size_t)np * 4, cudaMemcpyDeviceToHost, c.stream);
+  }
+  const float *hl = labels ? labels : computed.data();
+  if (!rc && e == cudaSuccess)
+    e = cudaMemcpyAsync(edge.data(), c.b_edge_mask.ptr, edge.size() * 4, cudaMemcpyDeviceToHost, c.stream);
+  const cudaError_t es = cudaStreamSynchronize(c.stream); // also before an error returns: the copies' host ends
+  if (rc) return rc;
+  if (e == cudaSuccess) e = es;
   if (e != cudaSuccess) return cuda_error(e, "labels read-back");
+  const std::vector<int> &lig_n = s.lig_n;
   std::vector<int> order;
   order.reserve((size_t)np);
   for (int l = 0; l < c.nligands; ++l) {
@@ -595,16 +647,13 @@ int surrogate_train(Context &c, int epochs, int batch, float lr, const float *la
   }
   if (!rc) rc = s.epoch_loss.reserve((size_t)n_used * 4, "last-epoch losses");
   if (rc) return rc;
-  int *hpose[2] = {}, *hrow[2] = {};
-  cudaStream_t cs = nullptr;
-  cudaEvent_t copied[2] = {}, used[2] = {}, e0 = nullptr, e1 = nullptr;
-  bool setup_ok = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) == cudaSuccess;
-  for (int k = 0; k < 2 && setup_ok; ++k)
-    setup_ok = cudaMallocHost((void **)&hpose[k], (size_t)n_used * 4) == cudaSuccess &&
-               cudaMallocHost((void **)&hrow[k], nrow_off * 4) == cudaSuccess &&
-               cudaEventCreateWithFlags(&copied[k], cudaEventDisableTiming) == cudaSuccess &&
-               cudaEventCreateWithFlags(&used[k], cudaEventDisableTiming) == cudaSuccess;
-  setup_ok = setup_ok && cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess;
+  rc = ensure_pipeline(s, (size_t)n_used + nrow_off);
+  if (rc) return rc;
+  const cudaStream_t cs = s.copy_stream;
+  cudaEvent_t *const copied = s.copied, *const used = s.used;
+  const cudaEvent_t e0 = s.e0, e1 = s.e1;
+  int *const hpose[2] = {s.host_epoch[0], s.host_epoch[1]};
+  int *const hrow[2] = {hpose[0] + n_used, hpose[1] + n_used};
   std::vector<long long> rows_of[2] = {std::vector<long long>(steps_per_epoch),
                                        std::vector<long long>(steps_per_epoch)};
   // Shuffle epoch `ep` into host buffer k and queue its copy into device pair k.
@@ -629,8 +678,7 @@ int surrogate_train(Context &c, int epochs, int batch, float lr, const float *la
     if (ce == cudaSuccess) ce = cudaEventRecord(copied[k], cs);
     return ce == cudaSuccess ? BUDE_OK : cuda_error(ce, "epoch order copy");
   };
-  if (!setup_ok) rc = set_error(BUDE_ERR_CUDA, "training pipeline setup (stream, events, pinned buffers)");
-  if (!rc) cudaEventRecord(e0, c.stream);
+  cudaEventRecord(e0, c.stream);
   if (!rc && epochs > 0) rc = prepare(0, 0);
   long long done = 0;
   for (int ep = 0; ep < epochs && !rc; ++ep) {
@@ -659,9 +707,9 @@ int surrogate_train(Context &c, int epochs, int batch, float lr, const float *la
       rc = ce == cudaSuccess ? prepare(ep + 1, k ^ 1) : cuda_error(ce, "epoch order copy");
     }
   }
-  if (e1) cudaEventRecord(e1, c.stream);
-  e = cudaStreamSynchronize(c.stream);
-  if (!rc && e != cudaSuccess) rc = cuda_error(e, "surrogate training");
+  cudaEventRecord(e1, c.stream);
+  const int waits = check_device_error(c); // waits for the stream; a wait of the training kernels that ran out
+  if (!rc) rc = waits;
   double last_loss = 0;
   if (!rc && epochs > 0) {
     // The last epoch's losses in pose order, summed in that order.
@@ -672,19 +720,8 @@ int surrogate_train(Context &c, int epochs, int batch, float lr, const float *la
     for (float v : lh) loss_sum += v;
     last_loss = loss_sum / (double)n_used;
   }
-  if (cs) {
-    cudaStreamSynchronize(cs);
-    cudaStreamDestroy(cs);
-  }
-  for (int k = 0; k < 2; ++k) {
-    if (hpose[k]) cudaFreeHost(hpose[k]);
-    if (hrow[k]) cudaFreeHost(hrow[k]);
-    if (copied[k]) cudaEventDestroy(copied[k]);
-    if (used[k]) cudaEventDestroy(used[k]);
-  }
+  cudaStreamSynchronize(cs);
   if (!rc && train_ms) cudaEventElapsedTime(train_ms, e0, e1);
-  if (e0) cudaEventDestroy(e0);
-  if (e1) cudaEventDestroy(e1);
   if (!rc && final_loss) *final_loss = (float)last_loss;
   return rc;
 }
@@ -695,26 +732,28 @@ int surrogate_gradient(Context &c, const int *poses, int n, const float *labels,
   if (!s.ready || !c.have_batch) return set_error(BUDE_ERR_STATE, "surrogate or batch missing");
   if (check_batch_types(c)) return BUDE_ERR_ARG;
   const long long np = c.batch_poses;
-  std::vector<int> lig_n;
-  int rc = upload_pose_ligands(c, s, lig_n);
-  if (!rc) rc = batch_transforms(c);
-  if (!rc) rc = s.labels.reserve((size_t)np * 4, "labels");
+  for (int i = 0; i < n; ++i)
+    if (poses[i] < 0 || poses[i] >= np) return set_error(BUDE_ERR_ARG, "pose index out of range");
+  int rc = s.labels.reserve((size_t)np * 4, "labels");
   if (!rc) rc = s.epoch_pose.reserve((size_t)n * 4, "poses");
   if (!rc) rc = s.epoch_rowoff.reserve((size_t)(n + 1) * 4, "row offsets");
+  if (!rc) rc = ensure_pose_ligands(c, s);
+  if (!rc) rc = batch_transforms(c);
   if (rc) return rc;
-  cudaError_t e = copy_sync(c, s.labels.ptr, labels, (size_t)np * 4, cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) return cuda_error(e, "labels");
   std::vector<int> ro(n + 1, 0);
-  for (int i = 0; i < n; ++i) {
-    if (poses[i] < 0 || poses[i] >= np) return set_error(BUDE_ERR_ARG, "pose index out of range");
-    ro[i + 1] = ro[i] + lig_n[(size_t)poses[i]];
+  for (int i = 0; i < n; ++i) ro[i + 1] = ro[i] + s.lig_n[(size_t)poses[i]];
+  cudaError_t e = cudaMemcpyAsync(s.labels.ptr, labels, (size_t)np * 4, cudaMemcpyHostToDevice, c.stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(s.epoch_pose.ptr, poses, (size_t)n * 4, cudaMemcpyHostToDevice, c.stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(s.epoch_rowoff.ptr, ro.data(), ro.size() * 4, cudaMemcpyHostToDevice, c.stream);
+  if (e != cudaSuccess) {
+    cudaStreamSynchronize(c.stream);
+    return cuda_error(e, "gradient inputs");
   }
-  e = copy_sync(c, s.epoch_pose.ptr, poses, (size_t)n * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = copy_sync(c, s.epoch_rowoff.ptr, ro.data(), ro.size() * 4, cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) return cuda_error(e, "gradient rows");
   rc = train_step(c, s, s.epoch_pose.as<int>(), s.epoch_rowoff.as<int>(), n, ro[n], 0.f, nullptr);
-  e = cudaStreamSynchronize(c.stream);
-  if (!rc && e != cudaSuccess) rc = cuda_error(e, "surrogate gradient");
+  const int waits = check_device_error(c); // waits for the stream
+  if (!rc) rc = waits;
   if (rc) return rc;
   if (grad_out) e = copy_sync(c, grad_out, s.grads.ptr, kNParams * 4, cudaMemcpyDeviceToHost);
   if (e == cudaSuccess && pred_out) e = copy_sync(c, pred_out, s.pred.ptr, (size_t)n * 4, cudaMemcpyDeviceToHost);
@@ -726,10 +765,10 @@ int surrogate_features(Context &c, const int *poses, int n, float *X, int *types
   Surrogate &s = sur(c);
   if (!s.ready || !c.have_batch) return set_error(BUDE_ERR_STATE, "surrogate or batch missing");
   if (check_batch_types(c)) return BUDE_ERR_ARG;
-  std::vector<int> lig_n;
-  int rc = upload_pose_ligands(c, s, lig_n);
+  int rc = ensure_pose_ligands(c, s);
   if (!rc) rc = batch_transforms(c);
   if (rc) return rc;
+  const std::vector<int> &lig_n = s.lig_n;
   std::vector<int> ro(n + 1, 0);
   for (int i = 0; i < n; ++i) {
     if (poses[i] < 0 || poses[i] >= c.batch_poses) return set_error(BUDE_ERR_ARG, "pose index out of range");
@@ -749,7 +788,7 @@ int surrogate_features(Context &c, const int *poses, int n, float *X, int *types
   m.lig_first = s.pose_lig_first.as<int>();
   m.lig_n = s.pose_lig_n.as<int>();
   m.nposes = n;
-  train_features_kernel<<<(n * 32 + 255) / 256, 256, 0, c.stream>>>(weights(s), s.fg, c.b_ligands.as<float4>(),
+  train_features_kernel<<<(n * 32 + 255) / 256, 256, 0, c.stream>>>(weights(s), s.fg, c.b_ligands,
                                                                       c.b_xform.as<float4>(), m,
                                                                       s.X.as<__nv_bfloat16>(), s.row_type.as<int>(),
                                                                       nullptr);
@@ -811,7 +850,7 @@ int surrogate_score_range(Context &c, int lig0, int lig1, int groups, cudaStream
   ScoreArgs a;
   a.W = weights(s);
   a.g = s.fg;
-  a.ligands = c.b_ligands.as<float4>();
+  a.ligands = c.b_ligands;
   a.xform = c.b_xform.as<float4>();
   // Every ligand at once: the items longest first, so that the groups finish together.
   a.items = s.items.as<int4>() + (n_items == s.n_items ? s.n_items : i0);
@@ -830,9 +869,10 @@ int surrogate_score_range(Context &c, int lig0, int lig1, int groups, cudaStream
     t.s = a;
     std::memcpy(t.w4, s.w4_host, sizeof t.w4);
     t.w = TcWeights{s.emb_h.ptr, s.w1_h.ptr, s.w2_h.ptr, s.w3_h.ptr, a.W.b1, a.W.b2, a.W.b3, a.W.w4, a.W.b4};
-    t.err = c.err.as<unsigned int>();
     int rc = s.next.reserve(256, "work counters");
+    if (!rc) rc = ensure_error_word(c);
     if (rc) return rc;
+    t.err = c.err.as<unsigned int>();
     t.next = s.next.as<unsigned int>() + 2; // the first two are the training step's
     e = cudaMemsetAsync(t.next, 0, sizeof(unsigned int), st);
     if (e != cudaSuccess) return cuda_error(e, "work counter");
@@ -943,10 +983,9 @@ int bude_surrogate_score(bude_gpu_ctx *ctx, float *ms) {
   int rc = surrogate_score_enqueue(*ctx, nullptr);
   if (rc) return rc;
   cudaEventRecord(ctx->ev1, ctx->stream);
-  cudaError_t e = cudaStreamSynchronize(ctx->stream);
-  if (e != cudaSuccess) return cuda_error(e, "surrogate scoring");
-  if (ms) cudaEventElapsedTime(ms, ctx->ev0, ctx->ev1);
-  return check_device_error(*ctx);
+  rc = check_device_error(*ctx); // waits for the stream
+  if (!rc && ms) cudaEventElapsedTime(ms, ctx->ev0, ctx->ev1);
+  return rc;
 }
 
 int bude_surrogate_set_scorer(bude_gpu_ctx *ctx, int32_t scorer) {
