@@ -21,7 +21,6 @@
 #include "exact_shape.h"
 #include "internal.h"
 #include "pair_record.h"
-#include "pose_xform.cuh"
 #include "ptx.cuh"
 
 namespace bude {
@@ -310,18 +309,13 @@ int enqueue_eval(Context &c, const bude_launch_cfg &cfg, cudaEvent_t mid) {
     if (mid) cudaEventRecord(mid, c.stream);
     return BUDE_OK;
   }
-  {
-    const int tb = 256;
-    const long long nb = (c.nposes + tb - 1) / tb;
-    pose_xform_kernel<<<(unsigned)nb, tb, 0, c.stream>>>(c.poses.as<float>(), c.pose_stride, c.nposes,
-                                                         c.xform.as<float4>(), c.edge_mask.as<unsigned>());
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_error(e, "pose_xform_kernel launch");
-    c.launches++;
-  }
+  const int *perm = nullptr;
+  rc = enqueue_poses(c, c.poses.as<float>(), c.pose_stride, c.nposes, c.xform.as<float>(), c.edge_mask.as<unsigned>(),
+                     &perm);
+  if (rc) return rc;
   if (mid) cudaEventRecord(mid, c.stream);
   return launch_exact_range(c, cfg, c.ligand.as<float4>(), c.natlig, c.deck_irregular, c.edge_mask.as<unsigned>(),
-                            c.xform.as<float>(), c.energies.as<float>(), c.nposes);
+                            c.xform.as<float>(), c.energies.as<float>(), c.nposes, perm);
 }
 
 // Self-test of the bounded wait: one thread waits on an mbarrier that nothing arrives on, with a
@@ -394,6 +388,7 @@ static int upload_poses(Context &c, const float *poses, long long stride, long l
                                    {&c.xform, (size_t)12 * n * sizeof(float)},
                                    {&c.energies, (size_t)n * sizeof(float)},
                                    {&c.edge_mask, (size_t)(n + 31) / 32 * sizeof(unsigned)},
+                                   {&c.order, sort_poses(c.natlig, n) ? pose_order_bytes(c, n) : 0},
                                    {&c.partial, c.partial.ptr || sums > ((size_t)64 << 20) ? 0 : sums}},
                                   "poses and energies");
   if (rc) return rc;
@@ -470,6 +465,7 @@ void destroy_context(Context *c) {
   c->box_reach.release();
   c->poses.release();
   c->xform.release();
+  c->order.release();
   c->energies.release();
   c->err.release();
   c->flush.release();

@@ -36,6 +36,9 @@
 //     Nothing in that order depends on the other poses, so a pose's energy is the same bits for every
 //     launch shape, chunk, batch or position.
 //
+//   * a large pose set comes in the order of its translations (pose_order.cuh), so that a chunk's poses
+//     are near each other and the groups tighter still.
+//
 // What bounds it: instruction issue (76% of the slots on the 4,096 x 64 deck), two thirds of it the record
 // loop (35 instructions per record and 64 points, 23 of them the pair arithmetic), the rest the sort, the
 // boxes and the candidate lists.  Measured, all pairs evaluated (records broadcast to 16 poses per thread,
@@ -509,6 +512,7 @@ struct FinishArgs {
   int more, last; // the sums add to what energies hold; these are the last rows
   const int4 *folds;
   float *energies;
+  const int *perm;       // optional: the pose at each place of the sums and transforms (pose_order.cuh)
   const unsigned *words; // as CullArgs::words; its deck decides whether every pose is irregular
   int edges;
   EdgeArgs e;
@@ -530,10 +534,12 @@ static __global__ void __launch_bounds__(256) cull_finish_kernel(const FinishArg
   }
   for (long long w = p0 + (threadIdx.x & ~31u); w < p1; w += blockDim.x) {
     const long long p = w + (threadIdx.x & 31);
+    long long q = p;
     bool irregular = false;
     if (p < p1) {
       const float *s = a.sums + (p - a.first);
-      float acc = a.more ? a.energies[p] : 0.f;
+      if (a.perm) q = __ldg(&a.perm[p]);
+      float acc = a.more ? a.energies[q] : 0.f;
       int r = 0;
       for (; r + 8 <= rows; r += 8) {
         float v[8];
@@ -543,15 +549,15 @@ static __global__ void __launch_bounds__(256) cull_finish_kernel(const FinishArg
         for (int j = 0; j < 8; ++j) acc = __fadd_rn(acc, v[j]);
       }
       for (; r < rows; ++r) acc = __fadd_rn(acc, s[(long long)r * a.stride]);
-      a.energies[p] = a.last ? 0.5f * acc : acc;
-      irregular = a.edges && a.last && (all || ((a.e.mask[p >> 5] >> (p & 31)) & 1u));
+      a.energies[q] = a.last ? 0.5f * acc : acc;
+      irregular = a.edges && a.last && (all || ((a.e.mask[q >> 5] >> (q & 31)) & 1u));
     }
     unsigned bits = __ballot_sync(0xffffffffu, irregular);
     while (bits) {
       const int b = __ffs(bits) - 1;
       bits &= bits - 1u;
       const float e = __shfl_sync(0xffffffffu, edge_energy(a.e, w + b), 0);
-      if ((threadIdx.x & 31) == b) a.energies[p] = e;
+      if ((threadIdx.x & 31) == b) a.energies[q] = e;
     }
   }
 }

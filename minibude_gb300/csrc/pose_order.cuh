@@ -1,0 +1,144 @@
+// pose_order.cuh -- poses sorted by where they put the ligand, for the exact kernel's chunks.
+//
+// A block of cull_kernel groups the positions of one ligand atom over one chunk of poses; the closer the
+// chunk's poses are to each other, the smaller the boxes of its groups and the fewer protein atoms pass
+// their tests.  So a large pose set is first put in the order of an 8 x 8 x 8 grid over the box of its
+// translations (Hilbert order of the cells): a group of 64 of 4,096 poses meets 157 of 2,672 atoms at
+// real density, 125 when the 4,096 are a 16th of 65,536 poses and 109 when they are a 256th of 1,048,576
+// (58 interact with a pose).  Cells of the orientation as well as the translation gave 106 to 126.  An
+// energy does not depend on the order (cull_kernel.cuh), and a ligand that turns about a far origin only
+// loses the gain.
+//
+// Three kernels: the box, the cells (a counting sort: every block counts its tile in shared memory and
+// takes its places in each cell by one atomic per cell), the transforms in sorted order.  Latency-bound
+// at 65,536 poses (3, 6 and 7 us, pose_xform_kernel 5), by the scattered 48-byte rows at 1,048,576 (6, 11
+// and 44 us).  Evaluations before | with them, end to end from the host: 4,096 x 64 x 1,048,576 3.64 |
+// 3.01 ms, 2,672 x 48 x 400,003 streamed 2.77 | 2.39 ms, 938 x 26 x 65,536 155 | 147 us.
+#pragma once
+#include "cull_kernel.cuh"
+#include "pose_xform.cuh"
+#include "warp.cuh"
+
+namespace bude {
+
+constexpr int kOrderThreads = 512;
+constexpr int kOrderBoxes = 128; // blocks of the box kernel, at most
+
+// Scratch of a sort of n poses in `tiles` tiles.
+struct PoseOrder {
+  int *perm;     // [n] pose of each place
+  unsigned *key; // [n] cell << 16 | rank among the tile's poses of the cell
+  float *boxes;  // [kOrderBoxes][6]
+  int *count;    // [cells] poses of each cell
+  int *base;     // [tiles][cells] the tile's first place in each cell
+  int tile;      // poses of a tile, a multiple of kOrderThreads, at most 65,536
+  int coarse;    // 0: kBins cells; 1: 8 of them at a time
+  __host__ __device__ int cells() const { return coarse ? kBins / 8 : kBins; }
+};
+
+// The box of the regular translations, one per block; the counts set to zero.
+static __global__ void __launch_bounds__(kOrderThreads) pose_box_kernel(const float *__restrict__ poses,
+                                                                        long long pstride, long long n, PoseOrder o) {
+  __shared__ float red[6][kOrderThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (blockIdx.x == 0)
+    for (int b = tid; b < o.cells(); b += kOrderThreads) o.count[b] = 0;
+  float v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  for (long long i = (long long)blockIdx.x * kOrderThreads + tid; i < n; i += (long long)gridDim.x * kOrderThreads) {
+    const float x = poses[3 * pstride + i], y = poses[4 * pstride + i], z = poses[5 * pstride + i];
+    if (!(fabsf(x) + fabsf(y) + fabsf(z) < kPoseReach)) continue;
+    v[0] = fminf(v[0], x), v[1] = fminf(v[1], y), v[2] = fminf(v[2], z);
+    v[3] = fmaxf(v[3], x), v[4] = fmaxf(v[4], y), v[5] = fmaxf(v[5], z);
+  }
+#pragma unroll
+  for (int d = 0; d < 6; ++d) {
+    const float m = d < 3 ? warp_min(v[d]) : warp_max(v[d]);
+    if (lane == 0) red[d][warp] = m;
+  }
+  __syncthreads();
+  if (warp < 6) {
+    const float m = red[warp][lane % (kOrderThreads / 32)];
+    const float r = warp < 3 ? warp_min(m) : warp_max(m);
+    if (lane == 0) o.boxes[blockIdx.x * 6 + warp] = r;
+  }
+}
+
+static __global__ void __launch_bounds__(kOrderThreads) pose_cell_kernel(const float *__restrict__ poses,
+                                                                         long long pstride, long long n, int boxes,
+                                                                         PoseOrder o) {
+  __shared__ int bins[kBins];
+  __shared__ float box[6];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int cells = o.cells(), shift = o.coarse ? 3 : 0;
+  for (int b = tid; b < cells; b += kOrderThreads) bins[b] = 0;
+  grid_dep_wait();
+  if (warp < 6) {
+    float m = warp < 3 ? INFINITY : -INFINITY;
+    for (int b = lane; b < boxes; b += 32)
+      m = warp < 3 ? fminf(m, o.boxes[b * 6 + warp]) : fmaxf(m, o.boxes[b * 6 + warp]);
+    m = warp < 3 ? warp_min(m) : warp_max(m);
+    if (lane == 0) box[warp] = m;
+  }
+  __syncthreads();
+  float s[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) s[d] = box[3 + d] > box[d] ? 8.f / (box[3 + d] - box[d]) : 0.f;
+  const long long first = (long long)blockIdx.x * o.tile, last = min(first + o.tile, n);
+  for (long long i = first + tid; i < last; i += kOrderThreads) {
+    int q[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) q[d] = min(max((int)((poses[(3 + d) * pstride + i] - box[d]) * s[d]), 0), 7);
+    const int cell = kHilbert.at[q[2] * 64 + q[1] * 8 + q[0]] >> shift;
+    o.key[i] = (unsigned)cell << 16 | (unsigned)atomicAdd(&bins[cell], 1);
+  }
+  __syncthreads();
+  for (int b = tid; b < cells; b += kOrderThreads)
+    o.base[(size_t)blockIdx.x * cells + b] = bins[b] ? atomicAdd(&o.count[b], bins[b]) : 0;
+}
+
+// The tile's transforms at their places; the irregular-pose bits in pose order (pose_xform_kernel).
+static __global__ void __launch_bounds__(kOrderThreads) pose_place_kernel(const float *__restrict__ poses,
+                                                                          long long pstride, long long n, PoseOrder o,
+                                                                          float4 *__restrict__ xform,
+                                                                          unsigned *__restrict__ edge_mask) {
+  static_assert(kBins == kOrderThreads, "one cell per thread");
+  __shared__ int start[kBins];
+  __shared__ int warp_total[kOrderThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int cells = o.cells();
+  grid_dep_wait();
+  {
+    const int v = tid < cells ? o.count[tid] : 0;
+    int sum = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, sum, d);
+      if (lane >= d) sum += u;
+    }
+    if (lane == 31) warp_total[warp] = sum;
+    __syncthreads();
+    const int before = __reduce_add_sync(0xffffffffu, lane < warp ? warp_total[lane] : 0);
+    if (tid < cells) start[tid] = before + sum - v + o.base[(size_t)blockIdx.x * cells + tid];
+  }
+  __syncthreads();
+  const long long first = (long long)blockIdx.x * o.tile, last = min(first + o.tile, n);
+  for (long long w = first + (tid & ~31); w < last; w += kOrderThreads) {
+    const long long i = w + lane;
+    bool irregular = false;
+    if (i < last) {
+      float4 r0, r1, r2;
+      pose_rows(poses, pstride, i, r0, r1, r2);
+      const unsigned k = o.key[i];
+      const int at = start[k >> 16] + (int)(k & 0xffffu);
+      xform[3ll * at + 0] = r0;
+      xform[3ll * at + 1] = r1;
+      xform[3ll * at + 2] = r2;
+      o.perm[at] = (int)i;
+      irregular = !pose_regular(r0, r1, r2);
+    }
+    const unsigned bits = __ballot_sync(0xffffffffu, irregular);
+    if (lane == 0) edge_mask[w >> 5] = bits;
+  }
+}
+
+} // namespace bude

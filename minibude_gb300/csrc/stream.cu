@@ -13,7 +13,6 @@
 #include <algorithm>
 
 #include "internal.h"
-#include "pose_xform.cuh"
 
 namespace bude {
 
@@ -109,15 +108,13 @@ static int score_stream(Context &c, const bude_launch_cfg &cfg, const float *pos
     if (e != cudaSuccess) break;
     cudaStreamWaitEvent(c.stream, s.copied[b], 0);
     if (i >= 2) cudaStreamWaitEvent(c.stream, s.returned[b], 0); // energies slot copied back
-    const int tb = 256;
-    pose_xform_kernel<<<(unsigned)((n + tb - 1) / tb), tb, 0, c.stream>>>(s.poses[b].as<float>(), n, n,
-                                                                          s.xform.as<float4>(),
-                                                                          s.edge_mask.as<unsigned>());
-    c.launches++;
+    const int *perm = nullptr;
+    rc = enqueue_poses(c, s.poses[b].as<float>(), n, n, s.xform.as<float>(), s.edge_mask.as<unsigned>(), &perm);
+    if (rc) break;
     e = cudaEventRecord(s.consumed[b], c.stream);
     if (e != cudaSuccess) break;
     rc = launch_exact_range(c, cfg, c.ligand.as<float4>(), c.natlig, c.deck_irregular, s.edge_mask.as<unsigned>(),
-                            s.xform.as<float>(), s.energies[b].as<float>(), n);
+                            s.xform.as<float>(), s.energies[b].as<float>(), n, perm);
     if (rc) break;
     e = cudaEventRecord(s.computed[b], c.stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s.d2h, s.computed[b], 0);

@@ -117,3 +117,49 @@ def test_atom_sums_in_several_windows(ctx):
     at = got[[0, 1, 150000, 262143, 262144, 268287, 268288, 299999]]
     scale = np.maximum(np.abs(e64), 1.0)
     assert (np.abs(at - e64) / scale).max() < max(2e-4, 4 * (np.abs(e32 - e64) / scale).max())
+
+
+def evaluated(ctx, deck):
+    """The deck's energies from the single-deck path, streamed in chunks, and as a batch of one ligand,
+    which takes the poses as they come."""
+    cfg = launch_cfg(4, 512, 1, 64, 2)
+    ctx.upload(deck)
+    ctx.run(cfg)
+    got = ctx.download()
+    streamed = np.full(deck.nposes, 7.0, np.float32)
+    ctx.score_stream(cfg, deck.poses, streamed, 32768)
+    ctx.upload_batch(BatchDeck(deck.protein, deck.forcefield, [deck.ligand], [deck.poses]))
+    ctx.run_batch(cfg)
+    return got, streamed, ctx.download_batch()
+
+
+# On both sides of the line from which poses are sorted, of the line between 64 and 512 cells, and of a tile.
+@pytest.mark.parametrize("natlig,nposes", [(100, 8191), (100, 8192), (91, 8193), (11, 68180), (11, 68182), (7, 131071),
+                                           (3, 262144), (3, 262145), (2, 500001)])
+def test_sorted_poses(ctx, natlig, nposes):
+    deck = deck_of(300, 9.0, natlig, nposes, seed=nposes)
+    got, streamed, plain = evaluated(ctx, deck)
+    assert np.array_equal(got, plain)
+    assert np.array_equal(streamed, plain)
+
+
+@pytest.mark.parametrize("kind", ["one place", "a line", "two places", "far", "irregular"])
+def test_sorted_poses_of_every_spread(ctx, kind):
+    deck = deck_of(300, 9.0, 20, 40000, seed=9)
+    t = deck.poses[3:]
+    if kind == "one place":
+        t[:] = 1.25
+    elif kind == "a line":
+        t[1:] = 0.0
+    elif kind == "two places":
+        t[:] = np.where(np.arange(40000) % 2, 4.0, -2.0)
+    elif kind == "far":
+        t[:, ::3] *= 1e30
+        t[0, 1::3] -= 1e9
+    else:
+        t[0, 5::701] = np.nan
+        t[2, 7::503] = np.inf
+        deck.poses[1, 9::997] = np.inf
+    got, streamed, plain = evaluated(ctx, deck)
+    assert np.array_equal(got, plain, equal_nan=True)
+    assert np.array_equal(streamed, plain, equal_nan=True)
