@@ -44,8 +44,8 @@ struct SumsWindow {
 SumsWindow sums_window(int natlig, long long nposes, const bude_launch_cfg &cfg, size_t most);
 int cull_range(CullArgs a, FinishArgs f, const bude_launch_cfg &cfg, const SumsWindow &w, int natlig, long long nposes,
                cudaStream_t st, long long &launches);
-// Whether the groups of a launch share candidate lists (CullArgs::supers).
-int cull_supers(int natpro_pad, const bude_launch_cfg &shape);
+// Which groups of a launch share candidate lists (CullArgs::supers).
+int cull_supers(int natpro_pad, const bude_launch_cfg &shape, bool sorted);
 
 // Plan of the poses [first[i], first[i] + count[i]) of ligand lig[i]; first ascending.
 CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vector<long long> &first,

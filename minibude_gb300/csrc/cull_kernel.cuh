@@ -81,7 +81,7 @@ struct CullArgs {
   int chunk, chunks;     // without items: poses of a chunk (at most K * blockDim.x) and chunks of the ligand
   int natpro_pad;        // records per type
   int clusters;          // of kClusterAtoms; the last may be short
-  int supers;            // groups share lists of candidates (protein indices below 65,536)
+  int supers;            // 2^supers groups share a list of candidates (protein indices below 65,536); 0: no lists
 };
 
 // Cell (x, y, z) of an 8 x 8 x 8 grid, at z * 64 + y * 8 + x, to its place on a Hilbert curve (Skilling,
@@ -310,8 +310,7 @@ __device__ __forceinline__ void cull_eval(Points<P> &pt, float3 lo, float3 hi, i
   }
 }
 
-// Four groups that follow each other share a list of candidates, found by one warp for their common box.
-constexpr int kSuperGroups = 4;
+// Groups that follow each other share a list of candidates, found by one warp for their common box.
 constexpr int kCandidates = 512; // of a list; a super group with more leaves its groups to the clusters
 struct Candidates {
   int n; // -1: too many
@@ -333,7 +332,7 @@ __device__ __forceinline__ void points_box(const float4 *pts, int first, int cou
 // Dynamic shared memory: the chunk's points, the warps' lists and the super groups' candidates.
 inline size_t cull_smem_bytes(int chunk, int threads, int P, int supers) {
   return (size_t)chunk * sizeof(float4) + (size_t)(threads / 32) * sizeof(WarpList) +
-         (size_t)(supers ? (chunk + 32 * P * kSuperGroups - 1) / (32 * P * kSuperGroups) : 0) * sizeof(Candidates);
+         (size_t)(supers ? (chunk + (32 * P << supers) - 1) / (32 * P << supers) : 0) * sizeof(Candidates);
 }
 
 // K poses per thread (a chunk of K * blockDim.x poses per block), P points per lane of a group.
@@ -440,10 +439,10 @@ template <int K, int P> __global__ void __launch_bounds__(kMaxThreads, 2) cull_k
   // 4. candidates of every super group
   const int lt = __float_as_int(la.w);
   if (a.supers) {
-    constexpr int kPoints = 32 * P * kSuperGroups;
-    for (int sg = warp; sg * kPoints < n; sg += warps) {
+    const int points = 32 * P << a.supers;
+    for (int sg = warp; sg * points < n; sg += warps) {
       float3 lo, hi;
-      points_box(pts, sg * kPoints, min(kPoints, n - sg * kPoints), lo, hi);
+      points_box(pts, sg * points, min(points, n - sg * points), lo, hi);
       const float4 *reach = a.reach + (size_t)lt * a.natpro_pad;
       int count = 0;
       for (int c0 = 0; c0 < a.clusters && count <= kCandidates; c0 += 32) {
@@ -473,8 +472,8 @@ template <int K, int P> __global__ void __launch_bounds__(kMaxThreads, 2) cull_k
 #pragma unroll
     for (int i = 0; i < P; ++i) pt.set(i, pts[min(first + i * 32 + lane, n - 1)]);
     pt.clear();
-    const int k = a.supers ? cand[g / kSuperGroups].n : -1;
-    cull_eval<P>(pt, lo, hi, lt, k >= 0 ? cand[g / kSuperGroups].at : nullptr, k, list, a);
+    const int k = a.supers ? cand[g >> a.supers].n : -1;
+    cull_eval<P>(pt, lo, hi, lt, k >= 0 ? cand[g >> a.supers].at : nullptr, k, list, a);
     __syncwarp(); // every lane has read its points
 #pragma unroll
     for (int i = 0; i < P; ++i)

@@ -268,7 +268,7 @@ extern "C" int bude_gpu_fasten_noalloc(const bude_atom *protein, int32_t natpro,
   a.words = words;
   a.natpro_pad = natpro_pad;
   a.clusters = clusters;
-  a.supers = cull_supers(natpro_pad, cfg);
+  a.supers = cull_supers(natpro_pad, cfg, false);
   FinishArgs f{};
   f.energies = energies;
   f.words = words;
