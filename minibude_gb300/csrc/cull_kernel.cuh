@@ -329,6 +329,21 @@ __device__ __forceinline__ void points_box(const float4 *pts, int first, int cou
   hi = make_float3(warp_max(hi.x), warp_max(hi.y), warp_max(hi.z));
 }
 
+// The points of the group at `first` (the last point in place of those past n) and their box.
+template <int P>
+__device__ __forceinline__ void group_points(Points<P> &pt, const float4 *pts, int first, int n, float3 &lo, float3 &hi) {
+  lo = make_float3(INFINITY, INFINITY, INFINITY), hi = make_float3(-INFINITY, -INFINITY, -INFINITY);
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    const float4 p = pts[min(first + i * 32 + (int)(threadIdx.x & 31), n - 1)];
+    pt.set(i, p);
+    lo = make_float3(fminf(lo.x, p.x), fminf(lo.y, p.y), fminf(lo.z, p.z));
+    hi = make_float3(fmaxf(hi.x, p.x), fmaxf(hi.y, p.y), fmaxf(hi.z, p.z));
+  }
+  lo = make_float3(warp_min(lo.x), warp_min(lo.y), warp_min(lo.z));
+  hi = make_float3(warp_max(hi.x), warp_max(hi.y), warp_max(hi.z));
+}
+
 // Dynamic shared memory: the chunk's points, the warps' lists and the super groups' candidates.
 inline size_t cull_smem_bytes(int chunk, int threads, int P, int supers) {
   return (size_t)chunk * sizeof(float4) + (size_t)(threads / 32) * sizeof(WarpList) +
@@ -400,8 +415,8 @@ template <int K, int P> __global__ void __launch_bounds__(kMaxThreads, 2) cull_k
   for (int k = 0; k < K; ++k) {
     slot[k] = -1;
     if (tid + k * T >= n) continue;
-    const int qx = min(max((int)((x[k] - lo.x) * ix), 0), 7), qy = min(max((int)((y[k] - lo.y) * iy), 0), 7),
-              qz = min(max((int)((z[k] - lo.z) * iz), 0), 7);
+    const unsigned qx = min(__float2uint_rz((x[k] - lo.x) * ix), 7u), qy = min(__float2uint_rz((y[k] - lo.y) * iy), 7u),
+                   qz = min(__float2uint_rz((z[k] - lo.z) * iz), 7u); // below the box, or not a number: 0
     const int cell = kHilbert.at[qz * 64 + qy * 8 + qx];
     slot[k] = cell << 16 | atomicAdd(&bins[cell], 1);
   }
@@ -460,6 +475,7 @@ template <int K, int P> __global__ void __launch_bounds__(kMaxThreads, 2) cull_k
     __syncthreads();
   }
   // 5. groups of 32 * P sorted points
+  float *out = a.sums + (long long)row * a.stride + (pose0 - a.first);
   for (;;) {
     int g = 0;
     if (lane == 0) g = atomicAdd(&next_group, 1);
@@ -468,35 +484,15 @@ template <int K, int P> __global__ void __launch_bounds__(kMaxThreads, 2) cull_k
     if (first >= n) break;
     Points<P> pt;
     float3 lo, hi;
-    points_box(pts, first, min(32 * P, n - first), lo, hi);
-#pragma unroll
-    for (int i = 0; i < P; ++i) pt.set(i, pts[min(first + i * 32 + lane, n - 1)]);
+    group_points(pt, pts, first, n, lo, hi);
     pt.clear();
     const int k = a.supers ? cand[g >> a.supers].n : -1;
     cull_eval<P>(pt, lo, hi, lt, k >= 0 ? cand[g >> a.supers].at : nullptr, k, list, a);
-    __syncwarp(); // every lane has read its points
+    // The energies to their poses, up to 32 sectors a store; a chunk's row stays in L2 until it is full.  Put
+    // in order in shared memory first, three more barriers: 4,096 x 64 x 1,048,576 2,773 us, so 2,628.
 #pragma unroll
     for (int i = 0; i < P; ++i)
-      if (first + i * 32 + lane < n) pts[first + i * 32 + lane].x = pt.energy(i); // in place of the point
-  }
-  __syncthreads();
-  // 6. the energies in pose order
-  float *out = a.sums + (long long)row * a.stride + (pose0 - a.first);
-  float *flat = reinterpret_cast<float *>(pts);
-  float e[K];
-  int at[K];
-#pragma unroll
-  for (int k = 0; k < K; ++k)
-    if (tid + k * T < n) e[k] = pts[tid + k * T].x, at[k] = __float_as_int(pts[tid + k * T].w);
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < K; ++k)
-    if (tid + k * T < n) flat[at[k]] = e[k];
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const int i = tid + k * T;
-    if (i < n) out[i] = flat[i];
+      if (first + i * 32 + lane < n) out[__float_as_int(pts[first + i * 32 + lane].w)] = pt.energy(i);
   }
 }
 
