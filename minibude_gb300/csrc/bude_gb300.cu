@@ -388,7 +388,7 @@ static int upload_poses(Context &c, const float *poses, long long stride, long l
                                    {&c.xform, (size_t)12 * n * sizeof(float)},
                                    {&c.energies, (size_t)n * sizeof(float)},
                                    {&c.edge_mask, (size_t)(n + 31) / 32 * sizeof(unsigned)},
-                                   {&c.order, sort_poses(c.natlig, n) ? pose_order_bytes(c, n) : 0},
+                                   {&c.order, sort_poses(c, n) ? pose_order_bytes(n) : 0},
                                    {&c.partial, c.partial.ptr || sums > ((size_t)64 << 20) ? 0 : sums}},
                                   "poses and energies");
   if (rc) return rc;

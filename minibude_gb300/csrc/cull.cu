@@ -125,56 +125,68 @@ int cull_range(CullArgs a, FinishArgs f, const bude_launch_cfg &cfg, const SumsW
 }
 
 // Whether an evaluation puts its poses in order first: two launches more, and 8 us more than the plain
-// transforms at 65,536 poses, 20 at 1,048,576, against groups with fewer records.  The line is where it
-// overtook the plain order (us, plain | sorted): 938 x 26 x 16,384 52.9 | 53.2, x 32,768 74.1 | 72.1, x
-// 65,536 118.6 | 107.8; 4,096 x 64 x 8,192 63.0 | 64.6, x 16,384 92.5 | 88.4, x 1,048,576 3,332 | 2,710;
-// 2,672 x 48 x 16,384 193 | 166, x 65,536 482 | 419.  Fewer than 8,192 poses are a chunk or two.
-bool sort_poses(int natlig, long long nposes) {
-  return nposes >= 8192 && (double)nposes * natlig >= 7.5e5 && nposes < (1LL << 31);
+// transforms at 65,536 poses, 20 at 1,048,576, against groups with fewer records.  What that saves goes with
+// the points and with the atoms near one, so the line is points x protein atoms per cubic Angstrom of their
+// box (widened by the reach) = 3,300, where the two were equal or the sorted faster (6 to 96 ligand atoms;
+// us plain, then sorted / plain): 400 atoms at 0.05 per cubic Angstrom 500k points 100, 0.98, 1.2M 167, 0.95;
+// 1,237 300k 90, 0.91, 900k 176, 0.86; 3,500 220k 77, 0.89, 900k 151, 0.84; 3,500 at 0.015 400k 55, 1.00,
+// 740k 82, 0.94.  Fewer than 4,096 poses are a few chunks.
+bool sort_poses(const Context &c, long long nposes) {
+  double volume = 1.0;
+  for (int d = 0; d < 3; ++d) volume *= (double)c.reach_hi[d] - c.reach_lo[d];
+  const double near = (double)nposes * c.natlig * c.natpro / volume;
+  return c.natpro > 0 && nposes >= 4096 && near >= 3300.0 && nposes < (1LL << 31);
 }
 
-static int order_tile(const Context &c, long long n) {
-  const long long per = (n + 4LL * std::max(c.num_sms, 1) - 1) / (4LL * std::max(c.num_sms, 1));
+static int order_tile(long long n) {
+  const long long per = (n + 607) / 608; // four blocks per SM
   return (int)std::min<long long>((per + kOrderThreads - 1) / kOrderThreads * kOrderThreads, 65536);
 }
 
-size_t pose_order_bytes(const Context &c, long long n) {
-  const long long tiles = (n + order_tile(c, n) - 1) / order_tile(c, n);
-  return ((size_t)2 * n + 6 * kOrderBoxes + (size_t)(tiles + 1) * kBins) * sizeof(int);
+static int order_coarse(long long n) { return n <= 262144; } // 64 chunks of 4,096: finer cells made none tighter
+
+size_t pose_order_bytes(long long n) {
+  const long long tiles = (n + order_tile(n) - 1) / order_tile(n), cells = order_coarse(n) ? kBins / 8 : kBins;
+  return ((size_t)2 * n + 6 * kOrderBoxes + (size_t)(tiles + 1) * cells) * sizeof(int);
+}
+
+int enqueue_sorted(void *scratch, const float *poses, long long stride, long long n, float4 *xform, unsigned *mask,
+                   const int **perm, cudaStream_t st) {
+  PoseOrder o;
+  o.perm = static_cast<int *>(scratch);
+  o.key = static_cast<unsigned *>(scratch) + n;
+  o.boxes = static_cast<float *>(scratch) + 2 * n;
+  o.count = static_cast<int *>(scratch) + 2 * n + 6 * kOrderBoxes;
+  o.coarse = order_coarse(n);
+  o.base = o.count + o.cells();
+  o.tile = order_tile(n);
+  const unsigned tiles = (unsigned)((n + o.tile - 1) / o.tile);
+  const int boxes = (int)std::min<long long>(kOrderBoxes, (n + kOrderThreads - 1) / kOrderThreads);
+  pose_box_kernel<<<boxes, kOrderThreads, 0, st>>>(poses, stride, n, o);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = launch_chained(pose_cell_kernel, tiles, (unsigned)kOrderThreads, 0, st, poses, stride, n, boxes, o);
+  if (e == cudaSuccess)
+    e = launch_chained(pose_place_kernel, tiles, (unsigned)kOrderThreads, 0, st, poses, stride, n, o, xform, mask);
+  if (e != cudaSuccess) return cuda_error(e, "pose order launch");
+  *perm = o.perm;
+  return BUDE_OK;
 }
 
 int enqueue_poses(Context &c, const float *poses, long long stride, long long n, float *xform, unsigned *mask,
                   const int **perm) {
   *perm = nullptr;
   float4 *rows = reinterpret_cast<float4 *>(xform);
-  if (!sort_poses(c.natlig, n)) {
-    pose_xform_kernel<<<(unsigned)((n + 255) / 256), 256, 0, c.stream>>>(poses, stride, n, rows, mask);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_error(e, "pose_xform_kernel launch");
-    c.launches++;
-    return BUDE_OK;
+  if (sort_poses(c, n)) {
+    int rc = c.order.reserve(pose_order_bytes(n), "pose order");
+    if (!rc) rc = enqueue_sorted(c.order.ptr, poses, stride, n, rows, mask, perm, c.stream);
+    c.launches += rc ? 0 : 3;
+    return rc;
   }
-  const int rc = c.order.reserve(pose_order_bytes(c, n), "pose order");
-  if (rc) return rc;
-  PoseOrder o;
-  o.perm = c.order.as<int>();
-  o.key = c.order.as<unsigned>() + n;
-  o.boxes = c.order.as<float>() + 2 * n;
-  o.count = c.order.as<int>() + 2 * n + 6 * kOrderBoxes;
-  o.base = o.count + kBins;
-  o.tile = order_tile(c, n);
-  o.coarse = n <= 262144; // 64 chunks of 4,096: finer cells would not make them tighter
-  const unsigned tiles = (unsigned)((n + o.tile - 1) / o.tile);
-  const int boxes = (int)std::min<long long>(kOrderBoxes, (n + kOrderThreads - 1) / kOrderThreads);
-  pose_box_kernel<<<boxes, kOrderThreads, 0, c.stream>>>(poses, stride, n, o);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess)
-    e = launch_chained(pose_cell_kernel, tiles, (unsigned)kOrderThreads, 0, c.stream, poses, stride, n, boxes, o);
-  if (e == cudaSuccess)
-    e = launch_chained(pose_place_kernel, tiles, (unsigned)kOrderThreads, 0, c.stream, poses, stride, n, o, rows, mask);
-  if (e != cudaSuccess) return cuda_error(e, "pose order launch");
-  c.launches += 3;
-  *perm = o.perm;
+  pose_xform_kernel<<<(unsigned)((n + 255) / 256), 256, 0, c.stream>>>(poses, stride, n, rows, mask);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_error(e, "pose_xform_kernel launch");
+  c.launches++;
   return BUDE_OK;
 }
 

@@ -44,6 +44,10 @@ struct SumsWindow {
 SumsWindow sums_window(int natlig, long long nposes, const bude_launch_cfg &cfg, size_t most);
 int cull_range(CullArgs a, FinishArgs f, const bude_launch_cfg &cfg, const SumsWindow &w, int natlig, long long nposes,
                cudaStream_t st, long long &launches);
+// The transforms of n poses in the order of their translations, and that order, with pose_order_bytes(n) of
+// scratch (internal.h; pose_order.cuh).
+int enqueue_sorted(void *scratch, const float *poses, long long stride, long long n, float4 *xform, unsigned *mask,
+                   const int **perm, cudaStream_t st);
 // Which groups of a launch share candidate lists (CullArgs::supers).
 int cull_supers(int natpro_pad, const bude_launch_cfg &shape, bool sorted);
 

@@ -178,8 +178,8 @@ int enqueue_eval(Context &c, const bude_launch_cfg &cfg, cudaEvent_t mid = nullp
 // uploaded deck, and `perm` then says which pose each transform belongs to (otherwise nullptr).
 int enqueue_poses(Context &c, const float *poses, long long stride, long long n, float *xform, unsigned *mask,
                   const int **perm);
-bool sort_poses(int natlig, long long nposes);
-size_t pose_order_bytes(const Context &c, long long n);
+bool sort_poses(const Context &c, long long nposes);
+size_t pose_order_bytes(long long n);
 // The energies of `nposes` poses (transforms at `xform`) of the ligand at `ligand`; with `mask` the
 // irregular ones of them, or all of an irregular deck, by the reference's arithmetic.
 int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *ligand, int natlig, bool all_irregular,

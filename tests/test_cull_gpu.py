@@ -133,8 +133,8 @@ def evaluated(ctx, deck):
     return got, streamed, ctx.download_batch()
 
 
-# On both sides of the line from which poses are sorted, of the line between 64 and 512 cells, and of a tile.
-@pytest.mark.parametrize("natlig,nposes", [(100, 8191), (100, 8192), (91, 8193), (11, 68180), (11, 68182), (7, 131071),
+# On both sides of 4,096 poses, from which sets are sorted, of the line between 64 and 512 cells, and of a tile.
+@pytest.mark.parametrize("natlig,nposes", [(200, 4095), (200, 4096), (91, 8193), (11, 68180), (11, 68182), (7, 131071),
                                            (3, 262144), (3, 262145), (2, 500001)])
 def test_sorted_poses(ctx, natlig, nposes):
     deck = deck_of(300, 9.0, natlig, nposes, seed=nposes)

@@ -1,5 +1,5 @@
 """bude_gpu_fasten_noalloc over the decks that its tables lay out differently: below one cluster, at the
-edges of the sort and of the record array, and with more atom sums than the working memory holds."""
+edges of the sort and of the record array, with sorted poses, and with more atom sums than the working memory holds."""
 import numpy as np
 import pytest
 
@@ -15,7 +15,10 @@ DECKS = [(1, 2.0, 3, 5, 100), (31, 5.0, 3, 5, 100), (32, 5.0, 3, 5, 100), (33, 5
          (1023, 14.0, 9, 26, 1000), (1025, 14.0, 9, 26, 1000),
          (16384, 34.0, 8, 9, 300), (16385, 34.0, 7, 9, 300),
          (131072, 68.0, 1, 4, 64), (8, 3.0, 16384, 4, 200),
-         (300, 9.0, 5, 70, 65535)]
+         (300, 9.0, 5, 70, 65535),
+         # poses sorted from 400,000 points on
+         (500, 10.0, 5, 50, 7999), (500, 10.0, 5, 50, 8000), (500, 10.0, 5, 100, 4095), (500, 10.0, 5, 100, 4097),
+         (500, 10.0, 5, 9, 65536)]
 
 
 @pytest.mark.parametrize("natpro,half_box,ntypes,natlig,nposes", DECKS)
