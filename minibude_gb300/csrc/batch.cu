@@ -27,6 +27,7 @@ void release_batch(Context &c) {
   c.b_items.release();
   c.b_folds.release();
   c.b_sums.release();
+  c.b_order.release();
   c.b_edge_mask.release();
   c.b_meta.release();
   c.b_lig_all_host.clear();
@@ -142,6 +143,8 @@ static int build_plan(Context &c, const bude_launch_cfg &cfg, CullPlan *out) {
   *out = plan_cull(c, lig, c.pose_off, count, cfg);
   int rc = c.b_items.reserve(std::max<size_t>(out->items.size(), 1) * sizeof(int4), "batch items");
   if (!rc) rc = c.b_folds.reserve(std::max<size_t>(out->folds.size(), 1) * sizeof(int4), "batch items");
+  out->sorted = sort_batch(c, cfg.ppwi * cfg.wgsize);
+  if (!rc && out->sorted) rc = c.b_order.reserve(batch_order_bytes(c, out->folds.size()), "batch pose order");
   if (!rc) rc = c.b_sums.reserve(std::max<size_t>(out->sums_bytes, 16), "batch atom sums");
   if (rc) return rc;
   cudaError_t e = copy_sync(c, c.b_items.ptr, out->items.data(), out->items.size() * sizeof(int4), cudaMemcpyHostToDevice);
@@ -160,12 +163,16 @@ static int enqueue_transforms(Context &c) {
   return e == cudaSuccess ? BUDE_OK : cuda_error(e, "pose transforms");
 }
 
-// Enqueue one evaluation of the whole batch: transforms, then the plan's windows.
+// Enqueue one evaluation of the whole batch: transforms, their order, then the plan's windows.
 static int enqueue_whole(Context &c, const bude_launch_cfg &cfg, const CullPlan &plan) {
-  const int rc = enqueue_transforms(c);
+  int rc = enqueue_transforms(c);
+  const float *xform = c.b_xform.as<float>();
+  const int *perm = nullptr;
+  if (!rc && plan.sorted)
+    rc = enqueue_batch_order(c, plan, c.b_folds.as<int4>(), xform, c.b_order.ptr, &xform, &perm);
   if (rc) return rc;
-  return enqueue_plan(c, cfg, plan, c.b_items.as<int4>(), c.b_folds.as<int4>(), c.b_xform.as<float>(),
-                      c.b_energies.as<float>(), c.b_sums.as<float>(), true, c.stream);
+  return enqueue_plan(c, cfg, plan, c.b_items.as<int4>(), c.b_folds.as<int4>(), xform, c.b_energies.as<float>(),
+                      c.b_sums.as<float>(), true, c.stream, perm);
 }
 
 // The evaluation as a CUDA graph, captured once per launch shape.

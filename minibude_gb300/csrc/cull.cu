@@ -131,10 +131,14 @@ int cull_range(CullArgs a, FinishArgs f, const bude_launch_cfg &cfg, const SumsW
 // us plain, then sorted / plain): 400 atoms at 0.05 per cubic Angstrom 500k points 100, 0.98, 1.2M 167, 0.95;
 // 1,237 300k 90, 0.91, 900k 176, 0.86; 3,500 220k 77, 0.89, 900k 151, 0.84; 3,500 at 0.015 400k 55, 1.00,
 // 740k 82, 0.94.  Fewer than 4,096 poses are a few chunks.
-bool sort_poses(const Context &c, long long nposes) {
+static double density(const Context &c) {
   double volume = 1.0;
   for (int d = 0; d < 3; ++d) volume *= (double)c.reach_hi[d] - c.reach_lo[d];
-  const double near = (double)nposes * c.natlig * c.natpro / volume;
+  return c.natpro / volume;
+}
+
+bool sort_poses(const Context &c, long long nposes) {
+  const double near = (double)nposes * c.natlig * density(c);
   return c.natpro > 0 && nposes >= 4096 && near >= 3300.0 && nposes < (1LL << 31);
 }
 
@@ -169,6 +173,46 @@ int enqueue_sorted(void *scratch, const float *poses, long long stride, long lon
   if (e == cudaSuccess)
     e = launch_chained(pose_place_kernel, tiles, (unsigned)kOrderThreads, 0, st, poses, stride, n, o, xform, mask);
   if (e != cudaSuccess) return cuda_error(e, "pose order launch");
+  *perm = o.perm;
+  return BUDE_OK;
+}
+
+// As sort_poses, for the ligands of more than a chunk, with four launches instead of one: 64 ligands of 12
+// to 96 atoms x 1,024 to 16,384 poses 2,217 us plain, 2,167 sorted, 256 x 4,096 to 65,536 16.83 and 15.02 ms.
+// Ligands of a chunk or less gain nothing (24 of 20 to 40 atoms x 256 to 1,024 stay plain, 177 us).
+bool sort_batch(const Context &c, int chunk) {
+  double points = 0;
+  for (int l = 0; l < c.nligands; ++l) {
+    const long long n = c.pose_off[l + 1] - c.pose_off[l];
+    if (n > chunk) points += (double)n * (c.lig_off[l + 1] - c.lig_off[l]);
+  }
+  return c.natpro > 0 && points * density(c) >= 10000.0;
+}
+
+size_t batch_order_bytes(const Context &c, size_t tiles) {
+  return (size_t)c.batch_poses * (3 * sizeof(float4) + 2 * sizeof(int)) +
+         ((size_t)c.nligands * (6 + kBatchCells) + tiles * kBatchCells) * sizeof(int);
+}
+
+int enqueue_batch_order(Context &c, const CullPlan &plan, const int4 *tiles, const float *xform, void *scratch,
+                        const float **sorted, const int **perm) {
+  BatchOrder o;
+  o.pose_off = c.b_pose_off;
+  o.tiles = tiles;
+  o.xform = reinterpret_cast<const float4 *>(xform);
+  o.sorted = static_cast<float4 *>(scratch);
+  o.perm = reinterpret_cast<int *>(o.sorted + 3 * c.batch_poses);
+  o.key = reinterpret_cast<unsigned *>(o.perm + c.batch_poses);
+  o.boxes = reinterpret_cast<float *>(o.key + c.batch_poses);
+  o.count = reinterpret_cast<int *>(o.boxes + 6 * (size_t)c.nligands);
+  o.base = o.count + kBatchCells * (size_t)c.nligands;
+  const unsigned n = (unsigned)plan.folds.size();
+  cudaError_t e = launch_chained(batch_box_kernel, (unsigned)c.nligands, (unsigned)kOrderThreads, 0, c.stream, o);
+  if (e == cudaSuccess) e = launch_chained(batch_cell_kernel, n, 256u, 0, c.stream, o);
+  if (e == cudaSuccess) e = launch_chained(batch_place_kernel, n, 256u, 0, c.stream, o);
+  if (e != cudaSuccess) return cuda_error(e, "batch pose order launch");
+  c.launches += 3;
+  *sorted = reinterpret_cast<const float *>(o.sorted);
   *perm = o.perm;
   return BUDE_OK;
 }
@@ -264,14 +308,15 @@ CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vec
 }
 
 int enqueue_plan(Context &c, const bude_launch_cfg &shape, const CullPlan &plan, const int4 *items, const int4 *folds,
-                 const float *xform, float *energies, float *sums, bool edges, cudaStream_t st) {
-  CullArgs a = cull_args(c, shape, false);
+                 const float *xform, float *energies, float *sums, bool edges, cudaStream_t st, const int *perm) {
+  CullArgs a = cull_args(c, shape, perm != nullptr);
   a.ligand = c.b_ligands;
   a.xform = xform;
   a.sums = sums;
   FinishArgs f{};
   f.sums = sums;
   f.energies = energies;
+  f.perm = perm;
   f.edges = edges;
   f.last = 1;
   f.e = edge_args_batch(c, xform);

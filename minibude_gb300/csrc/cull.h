@@ -20,6 +20,7 @@ struct CullPlan {
   };
   std::vector<int4> items, folds; // CullArgs::items, FinishArgs::folds
   std::vector<Window> windows;
+  bool sorted = false; // the batch's poses are put in order first (sort_batch)
   size_t sums_bytes = 0; // the largest window's
 };
 
@@ -54,11 +55,19 @@ int cull_supers(int natpro_pad, const bude_launch_cfg &shape, bool sorted);
 // Plan of the poses [first[i], first[i] + count[i]) of ligand lig[i]; first ascending.
 CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vector<long long> &first,
                    const std::vector<long long> &count, const bude_launch_cfg &shape);
+// Whether evaluating the uploaded batch in chunks of `chunk` poses puts each ligand's poses in order first.
+bool sort_batch(const Context &c, int chunk);
+// Memory of that order for a batch of `poses` poses, and its kernels: the transforms at `xform` and their
+// order in `scratch`.
+size_t batch_order_bytes(const Context &c, size_t tiles);
+int enqueue_batch_order(Context &c, const CullPlan &plan, const int4 *tiles, const float *xform, void *scratch,
+                        const float **sorted, const int **perm);
 // Enqueue the windows of a plan whose items and folds are on the device: energies of its poses from the
 // transforms at `xform`; `sums` holds plan.sums_bytes.  edges: irregular poses of the uploaded batch
 // get the reference's arithmetic.
 int enqueue_plan(Context &c, const bude_launch_cfg &shape, const CullPlan &plan, const int4 *items, const int4 *folds,
-                 const float *xform, float *energies, float *sums, bool edges, cudaStream_t st);
+                 const float *xform, float *energies, float *sums, bool edges, cudaStream_t st,
+                 const int *perm = nullptr);
 // Shared-memory limit of the shape's kernel (before a stream capture).
 int prepare_shape(const bude_launch_cfg &shape);
 // The launch shape for n poses of a ligand of natlig atoms, `ligands` such ligands at once.

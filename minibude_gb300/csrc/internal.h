@@ -92,7 +92,7 @@ struct Context {
   std::vector<long long> pose_off; // nligands + 1 pose offsets
   long long batch_poses = 0;
   DevBuf b_poses, b_xform, b_energies;
-  DevBuf b_items, b_folds, b_sums; // the device half of `plan` and its atom sums (graph-owned)
+  DevBuf b_items, b_folds, b_sums, b_order; // the device half of `plan` and its atom sums (graph-owned)
   // Irregular poses of the batch: transform-pass bits, device pose/atom offsets, and the ligands
   // whose every pose goes to edge_pose_kernel (lig_all flags and their count, both on the device).
   DevBuf b_edge_mask, b_meta; // b_meta: [pose_off | lig_any | lig_off | atoms | lig_all], one copy per upload

@@ -141,4 +141,101 @@ static __global__ void __launch_bounds__(kOrderThreads) pose_place_kernel(const 
   }
 }
 
+// The same for a batch: every ligand's poses in the order of 64 cells over the box of their translations,
+// within the ligand's own range of places.  The transforms and irregular-pose bits are there already
+// (pose_xform_kernel); a tile is a finish item of the batch's plan, {first pose, poses, rows, ligand} of at
+// most 256 poses.
+constexpr int kBatchCells = kBins / 8;
+struct BatchOrder {
+  const long long *pose_off; // [ligands + 1]
+  const int4 *tiles;
+  const float4 *xform; // in pose order
+  float4 *sorted;      // in the new order
+  int *perm;           // [poses] pose of each place
+  unsigned *key;       // [poses] cell << 16 | rank among the tile's poses of the cell
+  float *boxes;        // [ligands][6]
+  int *count;          // [ligands][kBatchCells]
+  int *base;           // [tiles][kBatchCells]
+};
+
+// One ligand per block.
+static __global__ void __launch_bounds__(kOrderThreads) batch_box_kernel(const BatchOrder o) {
+  __shared__ float red[6][kOrderThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, l = blockIdx.x;
+  grid_dep_wait();
+  if (tid < kBatchCells) o.count[l * kBatchCells + tid] = 0;
+  float v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  for (long long i = o.pose_off[l] + tid; i < o.pose_off[l + 1]; i += kOrderThreads) {
+    const float x = o.xform[3 * i].w, y = o.xform[3 * i + 1].w, z = o.xform[3 * i + 2].w;
+    if (!(fabsf(x) + fabsf(y) + fabsf(z) < kPoseReach)) continue;
+    v[0] = fminf(v[0], x), v[1] = fminf(v[1], y), v[2] = fminf(v[2], z);
+    v[3] = fmaxf(v[3], x), v[4] = fmaxf(v[4], y), v[5] = fmaxf(v[5], z);
+  }
+#pragma unroll
+  for (int d = 0; d < 6; ++d) {
+    const float m = d < 3 ? warp_min(v[d]) : warp_max(v[d]);
+    if (lane == 0) red[d][warp] = m;
+  }
+  __syncthreads();
+  if (warp < 6) {
+    const float m = red[warp][lane % (kOrderThreads / 32)];
+    const float r = warp < 3 ? warp_min(m) : warp_max(m);
+    if (lane == 0) o.boxes[l * 6 + warp] = r;
+  }
+}
+
+// One tile per block, one pose per thread.
+static __global__ void __launch_bounds__(256) batch_cell_kernel(const BatchOrder o) {
+  __shared__ int bins[kBatchCells];
+  const int tid = threadIdx.x;
+  if (tid < kBatchCells) bins[tid] = 0;
+  grid_dep_wait();
+  const int4 t = __ldg(&o.tiles[blockIdx.x]);
+  __syncthreads();
+  if (tid < t.y) {
+    const long long i = (long long)t.x + tid;
+    int q[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const float lo = o.boxes[t.w * 6 + d], hi = o.boxes[t.w * 6 + 3 + d];
+      q[d] = min(max((int)((o.xform[3 * i + d].w - lo) * (hi > lo ? 8.f / (hi - lo) : 0.f)), 0), 7);
+    }
+    const int cell = kHilbert.at[q[2] * 64 + q[1] * 8 + q[0]] >> 3;
+    o.key[i] = (unsigned)cell << 16 | (unsigned)atomicAdd(&bins[cell], 1);
+  }
+  __syncthreads();
+  if (tid < kBatchCells)
+    o.base[(size_t)blockIdx.x * kBatchCells + tid] =
+        bins[tid] ? atomicAdd(&o.count[t.w * kBatchCells + tid], bins[tid]) : 0;
+}
+
+static __global__ void __launch_bounds__(256) batch_place_kernel(const BatchOrder o) {
+  __shared__ int start[kBatchCells], half;
+  const int tid = threadIdx.x, lane = tid & 31;
+  grid_dep_wait();
+  const int4 t = __ldg(&o.tiles[blockIdx.x]);
+  int v = 0, sum = 0;
+  if (tid < kBatchCells) {
+    v = sum = o.count[t.w * kBatchCells + tid];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, sum, d);
+      if (lane >= d) sum += u;
+    }
+    if (tid == 31) half = sum;
+  }
+  __syncthreads();
+  if (tid < kBatchCells)
+    start[tid] = sum - v + (tid >= 32 ? half : 0) + o.base[(size_t)blockIdx.x * kBatchCells + tid];
+  __syncthreads();
+  if (tid >= t.y) return;
+  const long long i = (long long)t.x + tid;
+  const unsigned k = o.key[i];
+  const long long at = o.pose_off[t.w] + start[k >> 16] + (int)(k & 0xffffu);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) o.sorted[3 * at + d] = o.xform[3 * i + d];
+  o.perm[at] = (int)i;
+}
+static_assert(kBatchCells == 64, "two warps scan a ligand's cells");
+
 } // namespace bude

@@ -163,3 +163,32 @@ def test_sorted_poses_of_every_spread(ctx, kind):
     got, streamed, plain = evaluated(ctx, deck)
     assert np.array_equal(got, plain, equal_nan=True)
     assert np.array_equal(streamed, plain, equal_nan=True)
+
+
+@pytest.mark.parametrize("irregular", [False, True])
+@pytest.mark.parametrize("ppwi,wgsize", [(2, 512), (4, 512), (1, 64)])
+def test_batch_with_sorted_poses(ctx, ppwi, wgsize, irregular):
+    # A dense protein, so that the batch's poses are sorted; one launch per ligand takes them as they come.
+    rng = np.random.default_rng(11)
+    base = deck_of(700, 6.0, 4, 8, seed=11)
+    sizes = [(60, 1), (50, 5000), (20, 300), (64, 9001), (33, 257), (45, 4097)]
+    ligands = [synthetic_ligand(rng, a, 5.0, base.ntypes) for a, _ in sizes]
+    poses = [synthetic_poses(rng, n) for _, n in sizes]
+    if irregular:
+        ligands[4]["x"][3] = np.float32(1e30)
+        poses[1][3, ::777] = np.nan
+        poses[3][1, 5::901] = np.inf
+        poses[5][4] = 0.5
+    ctx.upload_batch(BatchDeck(base.protein, base.forcefield, ligands, poses))
+    cfg = launch_cfg(ppwi, wgsize, 1, 64, 2)
+    ctx.run_batch(cfg, per_ligand=True)
+    want = ctx.download_batch()
+    ctx.run_batch(cfg)
+    assert np.array_equal(ctx.download_batch(), want, equal_nan=True)
+    if not irregular:
+        for l in (1, 3):
+            deck = base.head(8)
+            pick = np.arange(0, poses[l].shape[1], 97)
+            deck.ligand, deck.poses = ligands[l], np.ascontiguousarray(poses[l][:, pick])
+            first = sum(n for _, n in sizes[:l])
+            assert_parity(want[first + pick], deck)
