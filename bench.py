@@ -180,7 +180,7 @@ def measured_peaks():
     return {}
 
 
-def traffic_per_launch(nposes: int, kernel: str = "exact_kernel"):
+def traffic_per_launch(nposes: int, kernel: str):
     """DRAM bytes per launch of `kernel` from its committed ncu summary (scaled to nposes)."""
     path = os.path.join(ROOT, "profiles", f"{kernel}_traffic.txt")
     if not os.path.exists(path):

@@ -10,7 +10,7 @@ namespace bude {
 // it in the stream finishes, and run their setup (barriers, TMEM allocation) until grid_dep_wait (ptx.cuh)
 // while that kernel's completion is processed.  Every kernel launched this way waits before it touches
 // memory that an earlier one writes or reads.  A training epoch of 512 ligands x 4,096 poses ran 7% faster
-// this way than in plain stream order; an evaluation of 64 poses (three kernels) takes 22.0 us instead
+// this way than in plain stream order; an evaluation of 64 poses (three kernels) took 22.0 us instead
 // of 26.5, of 65,536 116.6 instead of 122.4.
 template <class... KArgs, class... Args>
 inline cudaError_t launch_chained(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem,
