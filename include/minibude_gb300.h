@@ -135,7 +135,8 @@ int bude_gpu_score_host(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, const bud
  * host.  poses: six fields at poses + k*pose_stride (poses.in layout); energies: nposes floats.
  * Pinned host buffers (bude_host_alloc) let the copies overlap.  The energies equal those of
  * bude_gpu_run over all poses, bit for bit, for any chunk.  The chunk is rounded up to whole blocks,
- * and to enough of them that a chunk's launch fills the GPU.
+ * and to enough of them that a chunk's launch fills the GPU many times over, within 2^19 poses (or
+ * four blocks per SM, if those are more).
  * *ms (optional): CUDA-event time of the whole call.  No counterpart in the reference. */
 int bude_gpu_score_stream(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, const float *poses, int64_t pose_stride,
                           int64_t nposes, int64_t chunk, float *energies, float *ms);

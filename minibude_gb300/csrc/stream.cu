@@ -77,10 +77,12 @@ static int score_stream(Context &c, const bude_launch_cfg &cfg, const float *pos
   if (chunk <= 0) return set_error(BUDE_ERR_ARG, "chunk must be positive (got %lld)", chunk);
   int rc = check_cfg(c, cfg);
   if (rc) return rc;
-  // Whole blocks of poses, and enough of them that a chunk's launch fills the GPU: four blocks per SM
-  // (one block per ligand atom and ppwi * wgsize poses).
-  const long long ppb = (long long)cfg.ppwi * cfg.wgsize;
-  const long long fill = 4LL * std::max(c.num_sms, 1) / std::max(c.natlig, 1) + 1;
+  // Whole blocks of poses (one per ligand atom and ppwi * wgsize poses), and enough of them that the tail of
+  // a chunk's launch is short beside it: sixteen per SM where 2^19 poses hold as many, at least four.  Four |
+  // eight | sixteen, us: 2,672 x 48 x 400,003 in chunks of 65,536 2,538 | 2,229 | 1,980, of 16,384 2,847 |
+  // 2,303 | 2,080; 1,200 x 20 x 300,000 890 | 814 | 726; 3,500 x 14 x 250,000 624 | 506 | 506.
+  const long long ppb = (long long)cfg.ppwi * cfg.wgsize, sms = std::max(c.num_sms, 1), atoms = std::max(c.natlig, 1);
+  const long long fill = std::max(4 * sms / atoms + 1, std::min(16 * sms / atoms + 1, (1LL << 19) / ppb));
   chunk = std::max((chunk + ppb - 1) / ppb, fill) * ppb;
   chunk = std::min(chunk, std::max(nposes, 1LL));
   StreamState *sp = nullptr;

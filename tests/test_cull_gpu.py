@@ -192,3 +192,15 @@ def test_batch_with_sorted_poses(ctx, ppwi, wgsize, irregular):
             deck.ligand, deck.poses = ligands[l], np.ascontiguousarray(poses[l][:, pick])
             first = sum(n for _, n in sizes[:l])
             assert_parity(want[first + pick], deck)
+
+
+# Whole chunks and a remainder, of one and of many blocks of poses.
+@pytest.mark.parametrize("natlig,nposes,ppwi", [(200, 60001, 2), (200, 120001, 8), (2432, 3000, 1), (40, 300007, 4)])
+def test_streamed_chunks(ctx, natlig, nposes, ppwi):
+    deck = deck_of(150, 7.0, natlig, nposes, seed=natlig)
+    cfg = launch_cfg(ppwi, 512, 1, 64, 2)
+    ctx.upload(deck)
+    ctx.run(cfg)
+    got = np.full(nposes, 7.0, np.float32)
+    ctx.score_stream(cfg, deck.poses, got, 1)
+    assert np.array_equal(got, ctx.download())
