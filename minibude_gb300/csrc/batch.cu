@@ -157,7 +157,8 @@ static int enqueue_transforms(Context &c) {
   if (c.batch_poses == 0) return BUDE_OK;
   const int tb = 256;
   pose_xform_kernel<<<(unsigned)((c.batch_poses + tb - 1) / tb), tb, 0, c.stream>>>(
-      c.b_poses.as<float>(), c.batch_poses, c.batch_poses, c.b_xform.as<float4>(), c.b_edge_mask.as<unsigned>());
+      c.b_poses.as<float>(), c.batch_poses, c.batch_poses, c.b_xform.as<float4>(), c.b_edge_mask.as<unsigned>(),
+      RowOrder{});
   c.launches++;
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? BUDE_OK : cuda_error(e, "pose transforms");

@@ -315,7 +315,7 @@ int enqueue_eval(Context &c, const bude_launch_cfg &cfg, cudaEvent_t mid) {
   if (rc) return rc;
   if (mid) cudaEventRecord(mid, c.stream);
   return launch_exact_range(c, cfg, c.ligand.as<float4>(), c.natlig, c.deck_irregular, c.edge_mask.as<unsigned>(),
-                            c.xform.as<float>(), c.energies.as<float>(), c.nposes, perm);
+                            c.xform.as<float>(), c.energies.as<float>(), c.nposes, true, perm);
 }
 
 // Self-test of the bounded wait: one thread waits on an mbarrier that nothing arrives on, with a
@@ -389,6 +389,7 @@ static int upload_poses(Context &c, const float *poses, long long stride, long l
                                    {&c.energies, (size_t)n * sizeof(float)},
                                    {&c.edge_mask, (size_t)(n + 31) / 32 * sizeof(unsigned)},
                                    {&c.order, sort_poses(c, n) ? pose_order_bytes(n) : 0},
+                                   {&c.rows, 4096},
                                    {&c.partial, c.partial.ptr || sums > ((size_t)64 << 20) ? 0 : sums}},
                                   "poses and energies");
   if (rc) return rc;
@@ -466,6 +467,7 @@ void destroy_context(Context *c) {
   c->poses.release();
   c->xform.release();
   c->order.release();
+  c->rows.release();
   c->energies.release();
   c->err.release();
   c->flush.release();

@@ -101,6 +101,7 @@ int cull_range(CullArgs a, FinishArgs f, const bude_launch_cfg &cfg, const SumsW
                cudaStream_t st, long long &launches) {
   const float *xform = a.xform;
   a.chunk = w.chunk;
+  if (w.atoms < natlig) a.rows = nullptr;
   f.sums = a.sums;
   for (long long w0 = 0; w0 < nposes; w0 += w.poses) {
     const long long n = std::min(w.poses, nposes - w0);
@@ -142,6 +143,12 @@ bool sort_poses(const Context &c, long long nposes) {
   return c.natpro > 0 && nposes >= 4096 && near >= 3300.0 && nposes < (1LL << 31);
 }
 
+// Blocks that all run at once have no last ones: below 100,000 points (one point per thread) there are fewer
+// than a wave of them, and 938 x 26 x 64 takes 48 us with or without.
+bool row_order_pays(long long n, int natlig) {
+  return (double)n * natlig >= 1e5 && natlig > 1 && natlig <= kRowOrderMax;
+}
+
 static int order_tile(long long n) {
   const long long per = (n + 607) / 608; // four blocks per SM
   return (int)std::min<long long>((per + kOrderThreads - 1) / kOrderThreads * kOrderThreads, 65536);
@@ -155,7 +162,7 @@ size_t pose_order_bytes(long long n) {
 }
 
 int enqueue_sorted(void *scratch, const float *poses, long long stride, long long n, float4 *xform, unsigned *mask,
-                   const int **perm, cudaStream_t st) {
+                   const RowOrder &ro, const int **perm, cudaStream_t st) {
   PoseOrder o;
   o.perm = static_cast<int *>(scratch);
   o.key = static_cast<unsigned *>(scratch) + n;
@@ -169,7 +176,8 @@ int enqueue_sorted(void *scratch, const float *poses, long long stride, long lon
   pose_box_kernel<<<boxes, kOrderThreads, 0, st>>>(poses, stride, n, o);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess)
-    e = launch_chained(pose_cell_kernel, tiles, (unsigned)kOrderThreads, 0, st, poses, stride, n, boxes, o);
+    e = launch_chained(pose_cell_kernel, tiles + (ro.rows ? 1u : 0u), (unsigned)kOrderThreads, 0, st, poses, stride, n,
+                       boxes, o, ro);
   if (e == cudaSuccess)
     e = launch_chained(pose_place_kernel, tiles, (unsigned)kOrderThreads, 0, st, poses, stride, n, o, xform, mask);
   if (e != cudaSuccess) return cuda_error(e, "pose order launch");
@@ -221,13 +229,19 @@ int enqueue_poses(Context &c, const float *poses, long long stride, long long n,
                   const int **perm) {
   *perm = nullptr;
   float4 *rows = reinterpret_cast<float4 *>(xform);
+  int rc = c.rows.reserve(kRowOrderMax * sizeof(int), "row order");
+  if (rc) return rc;
+  const RowOrder ro{c.ligand.as<float4>(), c.reach.as<float4>(), c.natlig,
+                    c.natpro,              c.natpro_pad,         row_order_pays(n, c.natlig) ? c.rows.as<int>() : nullptr,
+                    nullptr};
   if (sort_poses(c, n)) {
-    int rc = c.order.reserve(pose_order_bytes(n), "pose order");
-    if (!rc) rc = enqueue_sorted(c.order.ptr, poses, stride, n, rows, mask, perm, c.stream);
+    rc = c.order.reserve(pose_order_bytes(n), "pose order");
+    if (!rc) rc = enqueue_sorted(c.order.ptr, poses, stride, n, rows, mask, ro, perm, c.stream);
     c.launches += rc ? 0 : 3;
     return rc;
   }
-  pose_xform_kernel<<<(unsigned)((n + 255) / 256), 256, 0, c.stream>>>(poses, stride, n, rows, mask);
+  pose_xform_kernel<<<(unsigned)((n + 255) / 256 + (ro.rows ? 1 : 0)), 256, 0, c.stream>>>(poses, stride, n, rows, mask,
+                                                                                         ro);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_error(e, "pose_xform_kernel launch");
   c.launches++;
@@ -235,7 +249,8 @@ int enqueue_poses(Context &c, const float *poses, long long stride, long long n,
 }
 
 int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *ligand, int natlig, bool all_irregular,
-                       const unsigned *mask, const float *xform, float *energies, long long nposes, const int *perm) {
+                       const unsigned *mask, const float *xform, float *energies, long long nposes, bool ordered,
+                       const int *perm) {
   if (nposes == 0) return BUDE_OK;
   const SumsWindow w = sums_window(natlig, nposes, cfg, kSumsBytes);
   const int rc = c.partial.reserve((size_t)w.atoms * w.poses * sizeof(float), "atom sums");
@@ -244,6 +259,7 @@ int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *lig
   a.ligand = ligand;
   a.xform = xform;
   a.sums = c.partial.as<float>();
+  if (ordered && row_order_pays(nposes, natlig)) a.rows = c.rows.as<int>();
   FinishArgs f{};
   f.energies = energies;
   f.perm = perm;

@@ -9,6 +9,7 @@ namespace bude {
 
 struct CullArgs;
 struct FinishArgs;
+struct RowOrder;
 
 // A batch evaluation's work, cut for one launch shape: block items and finish items in windows of
 // consecutive poses, each window's atom sums at most kSumsBytes.
@@ -48,7 +49,9 @@ int cull_range(CullArgs a, FinishArgs f, const bude_launch_cfg &cfg, const SumsW
 // The transforms of n poses in the order of their translations, and that order, with pose_order_bytes(n) of
 // scratch (internal.h; pose_order.cuh).
 int enqueue_sorted(void *scratch, const float *poses, long long stride, long long n, float4 *xform, unsigned *mask,
-                   const int **perm, cudaStream_t st);
+                   const RowOrder &ro, const int **perm, cudaStream_t st);
+// Whether the blocks of an evaluation take the ligand's atoms longest first (RowOrder).
+bool row_order_pays(long long n, int natlig);
 // Which groups of a launch share candidate lists (CullArgs::supers).
 int cull_supers(int natpro_pad, const bude_launch_cfg &shape, bool sorted);
 

@@ -43,8 +43,8 @@
 // record loop (35 instructions per record and 64 points, 23 of them the pair arithmetic), the rest the
 // sort, the boxes and the candidate lists.  Measured, all pairs evaluated (records broadcast to 16 poses
 // per thread, TMA-staged) | this kernel, end to end from pinned host memory: 4,096 x 64 x 1,048,576 101.5 |
-// 2.46 ms, 938 x 26 x 65,536 0.750 | 0.133 ms, 938 x 26 x 64 201 | 47 us, 2,672 x 48 x 400,003 streamed
-// 21.2 | 1.68 ms; 64 ligands of 12-96 atoms x 1,024-16,384 poses against 2,672 atoms 67.0 | 2.17 ms.  What
+// 2.46 ms, 938 x 26 x 65,536 0.750 | 0.128 ms, 938 x 26 x 64 201 | 47 us, 2,672 x 48 x 400,003 streamed
+// 21.2 | 1.63 ms; 64 ligands of 12-96 atoms x 1,024-16,384 poses against 2,672 atoms 67.0 | 2.17 ms.  What
 // went into it, on 4,096 x 64 x 262,144 unsorted poses: records read through L1 one by one 1,140 us (and 64
 // poses took 105 us for 41); 64-byte records with the packed instructions' operands twice, 1,250; 48 bytes
 // 1,100 (the loads' register writes bound two points per lane); lists of 64 records 1,095, of 128 in stages
@@ -78,6 +78,7 @@ struct CullArgs {
   long long nposes;      // without items: poses of the ligand
   float3 lo, hi;         // protein atoms' bounding box, widened by the longest reach
   const unsigned *words; // optional: a deck checked on the device (edge_pose.cuh); nothing runs on a bad one
+  const int *rows;       // optional, without items: the rows in the order in which the blocks take them (RowOrder)
   int atom0;             // without items: the atom of row 0
   int chunk, chunks;     // without items: poses of a chunk (at most K * blockDim.x) and chunks of the ligand
   int natpro_pad;        // records per type
@@ -371,6 +372,7 @@ template <int K, int P> __global__ void __launch_bounds__(kMaxThreads, 2) cull_k
     atom = it.x, row = it.y, pose0 = it.z, n = it.w;
   } else {
     row = (int)(blockIdx.x / (unsigned)a.chunks);
+    if (a.rows) row = __ldg(&a.rows[row]);
     atom = row + a.atom0;
     pose0 = (long long)(blockIdx.x % (unsigned)a.chunks) * a.chunk;
     n = (int)min((long long)a.chunk, a.nposes - pose0);

@@ -68,7 +68,7 @@ struct Context {
   bool have_deck = false;
   int natpro = 0, natpro_pad = 0, natlig = 0, ntypes = 0;
   long long nposes = 0, pose_stride = 0;
-  DevBuf ligand, slab, poses, xform, energies, err, flush, partial, order;
+  DevBuf ligand, slab, poses, xform, energies, err, flush, partial, order, rows;
   // What the exact kernel finds the interacting pairs by (cull_kernel.cuh): per pair its reach, the
   // clusters' boxes and reaches, and the box outside which no ligand atom interacts.
   DevBuf reach, box, box_reach;
@@ -180,11 +180,12 @@ int enqueue_poses(Context &c, const float *poses, long long stride, long long n,
                   const int **perm);
 bool sort_poses(const Context &c, long long nposes);
 size_t pose_order_bytes(long long n);
-// The energies of `nposes` poses (transforms at `xform`) of the ligand at `ligand`; with `mask` the
+// The energies of `nposes` poses (transforms at `xform`) of the ligand at `ligand` (ordered: the uploaded
+// one, whose row order enqueue_poses has written); with `mask` the
 // irregular ones of them, or all of an irregular deck, by the reference's arithmetic.
 int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *ligand, int natlig, bool all_irregular,
                        const unsigned *mask, const float *xform, float *energies, long long nposes,
-                       const int *perm = nullptr);
+                       bool ordered = false, const int *perm = nullptr);
 // Whether a ligand of natlig atoms keeps the uploaded protein's deck regular (edge_pose.cuh).
 bool ligand_regular(const Context &c, const bude_atom *ligand, int natlig, const bude_ffparams *ff);
 // Arguments of edge_energy for one ligand of natlig atoms, and for the uploaded batch.

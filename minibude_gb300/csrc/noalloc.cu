@@ -57,11 +57,11 @@ constexpr int kNaSortMax = 16384; // atoms one block sorts; a larger protein kee
 constexpr size_t kNaSumsBytes = 512 * 1024;
 static_assert(kNaSumsBytes >= kNaSortMax * sizeof(bude_atom), "the protein in cluster order fits the sums");
 constexpr size_t kNaScratchBytes =
-    kNaWordBytes + kNaOrderBytes + kNaXformBytes + kNaMaskBytes + kNaBoxBytes + kNaBoxReachBytes + kNaTableBytes +
+    kNaWordBytes + kRowOrderMax * sizeof(int) + kNaOrderBytes + kNaXformBytes + kNaMaskBytes + kNaBoxBytes + kNaBoxReachBytes + kNaTableBytes +
     kNaSumsBytes;
 
-// The working memory of bude_gpu_fasten_noalloc: [check words | pose order | pose transforms | irregular-pose bits |
-// cluster boxes | cluster reaches | tables | sums].
+// The working memory of bude_gpu_fasten_noalloc: [check words | row order | pose order | pose transforms |
+// irregular-pose bits | cluster boxes | cluster reaches | tables | sums].
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNaScratchBytes];
 
 constexpr int kNaMaxDevices = 64;
@@ -226,6 +226,7 @@ extern "C" int bude_gpu_fasten_noalloc(const bude_atom *protein, int32_t natpro,
     return p;
   };
   unsigned *words = reinterpret_cast<unsigned *>(take(kNaWordBytes));
+  int *rows = reinterpret_cast<int *>(take(kRowOrderMax * sizeof(int)));
   void *order = take(kNaOrderBytes);
   float4 *xform = reinterpret_cast<float4 *>(take(kNaXformBytes));
   unsigned *mask = reinterpret_cast<unsigned *>(take(kNaMaskBytes));
@@ -257,13 +258,15 @@ extern "C" int bude_gpu_fasten_noalloc(const bude_atom *protein, int32_t natpro,
   // The protein's box is not known here: sorted from a number of points on that pays at the density of real
   // proteins (sort_poses; 1,237 x 37 x 12,345 190 us plain, 182 sorted).
   const int *perm = nullptr;
+  const RowOrder ro{reinterpret_cast<const float4 *>(ligand), reach, natlig, natpro, natpro_pad,
+                    row_order_pays(nposes, natlig) ? rows : nullptr, words};
   const bool order_poses = nposes >= 4096 && (double)nposes * natlig >= 4e5 && pose_order_bytes(nposes) <= kNaOrderBytes;
   if (e == cudaSuccess && order_poses) {
-    rc = enqueue_sorted(order, poses, pose_stride, nposes, xform, mask, &perm, st);
+    rc = enqueue_sorted(order, poses, pose_stride, nposes, xform, mask, ro, &perm, st);
     if (rc) return rc;
   } else if (e == cudaSuccess)
-    e = launch_chained(pose_xform_kernel, (unsigned)((nposes + 255) / 256), 256u, 0, st, poses, (long long)pose_stride,
-                       (long long)nposes, xform, mask);
+    e = launch_chained(pose_xform_kernel, (unsigned)((nposes + 255) / 256 + (ro.rows ? 1 : 0)), 256u, 0, st, poses,
+                       (long long)pose_stride, (long long)nposes, xform, mask, ro);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_error(e, "no-alloc deck launch");
   const bude_launch_cfg cfg = cull_shape(nposes, natlig, 1);
@@ -278,6 +281,7 @@ extern "C" int bude_gpu_fasten_noalloc(const bude_atom *protein, int32_t natpro,
   a.lo = make_float3(-INFINITY, -INFINITY, -INFINITY); // the poses' own range bins them
   a.hi = make_float3(INFINITY, INFINITY, INFINITY);
   a.words = words;
+  a.rows = ro.rows;
   a.natpro_pad = natpro_pad;
   a.clusters = clusters;
   a.supers = cull_supers(natpro_pad, cfg, order_poses);

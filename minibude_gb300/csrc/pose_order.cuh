@@ -65,13 +65,17 @@ static __global__ void __launch_bounds__(kOrderThreads) pose_box_kernel(const fl
 
 static __global__ void __launch_bounds__(kOrderThreads) pose_cell_kernel(const float *__restrict__ poses,
                                                                          long long pstride, long long n, int boxes,
-                                                                         PoseOrder o) {
+                                                                         PoseOrder o, const RowOrder ro) {
   __shared__ int bins[kBins];
   __shared__ float box[6];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cells = o.cells(), shift = o.coarse ? 3 : 0;
   for (int b = tid; b < cells; b += kOrderThreads) bins[b] = 0;
   grid_dep_wait();
+  if (ro.rows && blockIdx.x == gridDim.x - 1) {
+    row_order(ro);
+    return;
+  }
   if (warp < 6) {
     float m = warp < 3 ? INFINITY : -INFINITY;
     for (int b = lane; b < boxes; b += 32)

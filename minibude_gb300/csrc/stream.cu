@@ -116,7 +116,7 @@ static int score_stream(Context &c, const bude_launch_cfg &cfg, const float *pos
     e = cudaEventRecord(s.consumed[b], c.stream);
     if (e != cudaSuccess) break;
     rc = launch_exact_range(c, cfg, c.ligand.as<float4>(), c.natlig, c.deck_irregular, s.edge_mask.as<unsigned>(),
-                            s.xform.as<float>(), s.energies[b].as<float>(), n, perm);
+                            s.xform.as<float>(), s.energies[b].as<float>(), n, true, perm);
     if (rc) break;
     e = cudaEventRecord(s.computed[b], c.stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s.d2h, s.computed[b], 0);

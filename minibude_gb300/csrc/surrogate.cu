@@ -558,7 +558,7 @@ static int batch_transforms(Context &c) {
   if (c.batch_poses == 0) return BUDE_OK;
   const int tb = 256;
   pose_xform_kernel<<<(unsigned)((c.batch_poses + tb - 1) / tb), tb, 0, c.stream>>>(
-      c.b_poses.as<float>(), c.batch_poses, c.batch_poses, c.b_xform.as<float4>(), c.b_edge_mask.as<unsigned>());
+      c.b_poses.as<float>(), c.batch_poses, c.batch_poses, c.b_xform.as<float4>(), c.b_edge_mask.as<unsigned>(), RowOrder{});
   c.launches++;
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? BUDE_OK : cuda_error(e, "pose transforms");

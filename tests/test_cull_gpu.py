@@ -204,3 +204,22 @@ def test_streamed_chunks(ctx, natlig, nposes, ppwi):
     got = np.full(nposes, 7.0, np.float32)
     ctx.score_stream(cfg, deck.poses, got, 1)
     assert np.array_equal(got, ctx.download())
+
+
+# One atom, about as many as are put in order, and more; an empty protein; atoms that are not numbers.
+@pytest.mark.parametrize("natlig,nposes,odd", [(1, 100001, ""), (2, 50001, ""), (1023, 101, ""), (1024, 98, ""),
+                                               (1025, 98, ""), (50, 2001, "nan"), (50, 2001, "empty")])
+def test_atoms_longest_first(ctx, natlig, nposes, odd):
+    deck = deck_of(200, 7.0, natlig, nposes, seed=natlig + nposes)
+    if odd == "nan":
+        deck.ligand["x"][[3, 40]] = np.nan
+        deck.ligand["z"][7] = np.inf
+    if odd == "empty":
+        deck.protein = deck.protein[:0].copy()
+    cfg = launch_cfg(4, 512, 1, 64, 2)
+    ctx.upload(deck)
+    ctx.run(cfg)
+    got = ctx.download()
+    ctx.upload_batch(BatchDeck(deck.protein, deck.forcefield, [deck.ligand], [deck.poses]))
+    ctx.run_batch(cfg)
+    assert np.array_equal(got, ctx.download_batch(), equal_nan=True)
