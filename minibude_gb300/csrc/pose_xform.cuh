@@ -33,25 +33,29 @@ struct RowOrder {
   const unsigned *words; // as CullArgs::words
 };
 
+// The weight of ligand atom a, the whole warp's work; 0 where it is not a number.
+__device__ __forceinline__ float atom_weight(const float4 a, const float4 *all_reach, int natpro, int natpro_pad) {
+  constexpr int kPerLane = 8; // 256 protein atoms, evenly spread
+  const float4 *reach = all_reach + (size_t)__float_as_int(a.w) * natpro_pad;
+  const float wide = 0.5f * sqrtf(a.x * a.x + a.y * a.y + a.z * a.z) + 0.5f;
+  float w = 0.f;
+#pragma unroll
+  for (int k = 0; k < kPerLane; ++k) {
+    const int at = (int)((long long)(k * 32 + (int)(threadIdx.x & 31)) * natpro / (32 * kPerLane));
+    const float x = (natpro > 0 ? sqrtf(reach[at].w) : 0.f) + wide;
+    w += x * x * x;
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) w += __shfl_xor_sync(0xffffffffu, w, d);
+  return w >= 0.f ? w : 0.f;
+}
+
 __device__ __forceinline__ void row_order(const RowOrder &o) {
   __shared__ float weight[kRowOrderMax];
-  constexpr int kPerLane = 8; // 256 protein atoms, evenly spread
-  const int lane = threadIdx.x & 31;
   if (o.words && deck_bad_type(o.words)) return;
   for (int i = threadIdx.x >> 5; i < o.natlig; i += blockDim.x >> 5) {
-    const float4 a = o.ligand[i];
-    const float4 *reach = o.reach + (size_t)__float_as_int(a.w) * o.natpro_pad;
-    const float wide = 0.5f * sqrtf(a.x * a.x + a.y * a.y + a.z * a.z) + 0.5f;
-    float w = 0.f;
-#pragma unroll
-    for (int k = 0; k < kPerLane; ++k) {
-      const int at = (int)((long long)(k * 32 + lane) * o.natpro / (32 * kPerLane));
-      const float x = (o.natpro > 0 ? sqrtf(reach[at].w) : 0.f) + wide;
-      w += x * x * x;
-    }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) w += __shfl_xor_sync(0xffffffffu, w, d);
-    if (lane == 0) weight[i] = w >= 0.f ? w : 0.f; // not a number: last
+    const float w = atom_weight(o.ligand[i], o.reach, o.natpro, o.natpro_pad);
+    if ((threadIdx.x & 31) == 0) weight[i] = w;
   }
   __syncthreads();
   for (int i = threadIdx.x; i < o.natlig; i += blockDim.x) {

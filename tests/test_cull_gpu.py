@@ -223,3 +223,19 @@ def test_atoms_longest_first(ctx, natlig, nposes, odd):
     ctx.upload_batch(BatchDeck(deck.protein, deck.forcefield, [deck.ligand], [deck.poses]))
     ctx.run_batch(cfg)
     assert np.array_equal(got, ctx.download_batch(), equal_nan=True)
+
+
+# Plans of one block, of the most that are put in order, and of one more; a protein shorter than the sample.
+@pytest.mark.parametrize("atoms", [(1,), (1, 1), (500, 524), (500, 525)])
+def test_batch_items_longest_first(ctx, atoms):
+    rng = np.random.default_rng(len(atoms) + sum(atoms))
+    base = deck_of(90, 6.0, 4, 8, seed=5)
+    ligands = [synthetic_ligand(rng, a, 5.0, base.ntypes) for a in atoms]
+    ligands[-1]["y"][0] = np.nan
+    poses = [synthetic_poses(rng, 40 + 7 * l) for l in range(len(atoms))]
+    ctx.upload_batch(BatchDeck(base.protein, base.forcefield, ligands, poses))
+    cfg = launch_cfg(1, 64, 1, 64, 1)
+    ctx.run_batch(cfg, per_ligand=True)
+    want = ctx.download_batch()
+    ctx.run_batch(cfg)
+    assert np.array_equal(ctx.download_batch(), want, equal_nan=True)
