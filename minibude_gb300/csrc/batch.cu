@@ -133,11 +133,11 @@ bude_launch_cfg batch_shape(const Context &c) {
   return cull_shape(std::max(c.batch_poses / nl, 1LL), std::max(c.lig_off[c.nligands] / nl, 1), nl);
 }
 
-// A plan of few blocks in the order of their work, longest first (RowOrder): the weights, one warp per item
+// A plan's blocks in the order of their work, longest first (RowOrder): the weights, one warp per item
 // {atom, row, first pose, poses}, and the ranks, one thread per item; once per plan, 8 us.  24 ligands of 20 to
-// 40 atoms x 256 to 1,024 poses (736 blocks) 179 -> 163 us an evaluation; a plan of many waves has no tail
-// worth it (64 ligands of 12 to 96 atoms, 6,253 blocks, as before).
-constexpr int kPlanOrderMax = 1024;
+// 40 atoms x 256 to 1,024 poses (736 blocks) 179 -> 163 us an evaluation, 64 of 12 to 96 atoms x 1,024 to
+// 16,384 (6,253 blocks) 2,197 -> 2,100.  Every item is compared with every other, so up to 16,384.
+constexpr int kPlanOrderMax = 16384;
 static __global__ void __launch_bounds__(256) item_weight_kernel(const int4 *items, int n, const float4 *ligands,
                                                                  const float4 *reach, int natpro, int natpro_pad,
                                                                  float *weight) {
@@ -147,16 +147,20 @@ static __global__ void __launch_bounds__(256) item_weight_kernel(const int4 *ite
   if ((threadIdx.x & 31) == 0) weight[i] = w;
 }
 
-static __global__ void __launch_bounds__(kPlanOrderMax) item_rank_kernel(const int4 *items, int n, const float *weight,
-                                                                         int4 *ranked) {
-  __shared__ float w[kPlanOrderMax];
-  const int i = threadIdx.x;
-  if (i < n) w[i] = weight[i];
-  __syncthreads();
-  if (i >= n) return;
+static __global__ void __launch_bounds__(256) item_rank_kernel(const int4 *items, int n, const float *weight,
+                                                               int4 *ranked) {
+  __shared__ float tile[256];
+  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  const float w = i < n ? weight[i] : 0.f;
   int rank = 0;
-  for (int j = 0; j < n; ++j) rank += w[j] > w[i] || (w[j] == w[i] && j < i);
-  ranked[rank] = items[i];
+  for (int t = 0; t < n; t += 256) {
+    const int j = t + (int)threadIdx.x;
+    __syncthreads();
+    tile[threadIdx.x] = j < n ? weight[j] : -1.f; // weights are at least 0
+    __syncthreads();
+    for (int k = 0; k < 256; ++k) rank += tile[k] > w || (tile[k] == w && t + k < i);
+  }
+  if (i < n) ranked[rank] = items[i];
 }
 
 // Plan of the whole batch for a launch shape, on the device (b_items, b_folds, b_sums).
@@ -167,7 +171,7 @@ static int build_plan(Context &c, const bude_launch_cfg &cfg, CullPlan *out) {
   std::vector<long long> count((size_t)c.nligands);
   for (int l = 0; l < c.nligands; ++l) count[(size_t)l] = c.pose_off[l + 1] - c.pose_off[l];
   *out = plan_cull(c, lig, c.pose_off, count, cfg);
-  // Few blocks: uploaded behind the ranked ones, with the weights behind both.
+  // Not too many blocks: uploaded behind the ranked ones, with the weights behind both.
   const int n = (int)out->items.size();
   const bool rank = n > 1 && n <= kPlanOrderMax && out->windows.size() == 1;
   int rc = c.b_items.reserve((size_t)std::max(n, 1) * (2 * sizeof(int4) + sizeof(float)), "batch items");
@@ -182,7 +186,7 @@ static int build_plan(Context &c, const bude_launch_cfg &cfg, CullPlan *out) {
     float *weight = reinterpret_cast<float *>(items + 2 * n);
     item_weight_kernel<<<(unsigned)(n + 7) / 8, 256, 0, c.stream>>>(given, n, c.b_ligands, c.reach.as<float4>(), c.natpro,
                                                                     c.natpro_pad, weight);
-    item_rank_kernel<<<1, kPlanOrderMax, 0, c.stream>>>(given, n, weight, items);
+    item_rank_kernel<<<(unsigned)(n + 255) / 256, 256, 0, c.stream>>>(given, n, weight, items);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess)

@@ -44,7 +44,7 @@
 // sort, the boxes and the candidate lists.  Measured, all pairs evaluated (records broadcast to 16 poses
 // per thread, TMA-staged) | this kernel, end to end from pinned host memory: 4,096 x 64 x 1,048,576 101.5 |
 // 2.46 ms, 938 x 26 x 65,536 0.750 | 0.128 ms, 938 x 26 x 64 201 | 47 us, 2,672 x 48 x 400,003 streamed
-// 21.2 | 1.63 ms; 64 ligands of 12-96 atoms x 1,024-16,384 poses against 2,672 atoms 67.0 | 2.17 ms.  What
+// 21.2 | 1.63 ms; 64 ligands of 12-96 atoms x 1,024-16,384 poses against 2,672 atoms 67.0 | 2.10 ms.  What
 // went into it, on 4,096 x 64 x 262,144 unsorted poses: records read through L1 one by one 1,140 us (and 64
 // poses took 105 us for 41); 64-byte records with the packed instructions' operands twice, 1,250; 48 bytes
 // 1,100 (the loads' register writes bound two points per lane); lists of 64 records 1,095, of 128 in stages

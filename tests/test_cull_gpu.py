@@ -225,8 +225,9 @@ def test_atoms_longest_first(ctx, natlig, nposes, odd):
     assert np.array_equal(got, ctx.download_batch(), equal_nan=True)
 
 
-# Plans of one block, of the most that are put in order, and of one more; a protein shorter than the sample.
-@pytest.mark.parametrize("atoms", [(1,), (1, 1), (500, 524), (500, 525)])
+# Plans of one block, around the ranking's tiles, of the most that are put in order and of one more; a protein
+# shorter than the sample.
+@pytest.mark.parametrize("atoms", [(1,), (1, 1), (100, 156), (100, 157), (8000, 8384), (8000, 8385)])
 def test_batch_items_longest_first(ctx, atoms):
     rng = np.random.default_rng(len(atoms) + sum(atoms))
     base = deck_of(90, 6.0, 4, 8, seed=5)
