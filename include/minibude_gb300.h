@@ -94,9 +94,11 @@ int bude_gpu_upload(bude_gpu_ctx *ctx, const bude_atom *protein, int32_t natpro,
 int bude_gpu_set_poses(bude_gpu_ctx *ctx, const bude_atom *ligand, int32_t natlig, const float *poses,
                        int64_t pose_stride, int64_t nposes);
 
-/* The launch shape for the uploaded deck's size, whatever the reference's (PPWI, wgsize) pair: the
- * pair is how the reference spreads poses over threads, which the library does by the number of poses
- * and ligand atoms.  Results do not depend on the shape. */
+/* The launch shape for the reference's (PPWI, wgsize) pair: PPWI poses per thread (the largest of 1, 2,
+ * 4, 8 and 16 that it holds: 32/64/128 use 16) and wgsize threads per block (rounded up to a multiple of
+ * 32, at most 512).  A ppwi below 1 or a wgsize below 32 leaves that half to the library, which chooses
+ * by the uploaded deck's poses and ligand atoms; (0, 0) is its own shape, the fastest here without
+ * measuring.  Results do not depend on the shape. */
 int bude_gpu_default_cfg(const bude_gpu_ctx *ctx, int32_t ppwi, int32_t wgsize, bude_launch_cfg *cfg);
 
 /* Choose a launch shape for the uploaded deck by measurement; replaces the reference driver's

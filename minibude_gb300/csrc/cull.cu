@@ -17,16 +17,16 @@ constexpr size_t kCullMaxSmem = 200 * 1024; // 16 poses per thread x 512 threads
 // Lists of candidates serve four groups, or the eight tighter ones of sorted poses (4,096 x 64 x 1,048,576
 // 2,603 us with four, 2,519 with eight; 64 unsorted ligands 2,664 and 2,703).  A chunk of 256 poses has too
 // few groups for them: 64 poses of 938 x 26 27.0 us with, 25.0 without, 205 of 2,672 x 48 45.9 and 41.5.
-int cull_supers(int natpro_pad, const bude_launch_cfg &s, bool sorted) {
-  const int chunk = s.ppwi * s.wgsize, shift = sorted ? 3 : 2;
-  return natpro_pad <= 65536 && chunk > 256 && cull_smem_bytes(chunk, s.wgsize, s.unroll, shift) <= kCullMaxSmem
+int cull_supers(int natpro_pad, const bude_launch_cfg &s, int chunk, bool sorted) {
+  const int most = s.ppwi * s.wgsize, shift = sorted ? 3 : 2;
+  return natpro_pad <= 65536 && chunk > 256 && cull_smem_bytes(most, s.wgsize, s.unroll, shift) <= kCullMaxSmem
              ? shift
              : 0;
 }
 
-static CullArgs cull_args(const Context &c, const bude_launch_cfg &s, bool sorted) {
+static CullArgs cull_args(const Context &c, const bude_launch_cfg &s, int chunk, bool sorted) {
   CullArgs a{};
-  a.supers = cull_supers(c.natpro_pad, s, sorted);
+  a.supers = cull_supers(c.natpro_pad, s, chunk, sorted);
   a.slab = c.slab.as<float4>();
   a.reach = c.reach.as<float4>();
   a.box = c.box.as<float4>();
@@ -255,7 +255,7 @@ int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *lig
   const SumsWindow w = sums_window(natlig, nposes, cfg, kSumsBytes);
   const int rc = c.partial.reserve((size_t)w.atoms * w.poses * sizeof(float), "atom sums");
   if (rc) return rc;
-  CullArgs a = cull_args(c, cfg, perm != nullptr);
+  CullArgs a = cull_args(c, cfg, w.chunk, perm != nullptr);
   a.ligand = ligand;
   a.xform = xform;
   a.sums = c.partial.as<float>();
@@ -325,7 +325,7 @@ CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vec
 
 int enqueue_plan(Context &c, const bude_launch_cfg &shape, const CullPlan &plan, const int4 *items, const int4 *folds,
                  const float *xform, float *energies, float *sums, bool edges, cudaStream_t st, const int *perm) {
-  CullArgs a = cull_args(c, shape, perm != nullptr);
+  CullArgs a = cull_args(c, shape, shape.ppwi * shape.wgsize, perm != nullptr);
   a.ligand = c.b_ligands;
   a.xform = xform;
   a.sums = sums;

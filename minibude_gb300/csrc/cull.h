@@ -52,8 +52,8 @@ int enqueue_sorted(void *scratch, const float *poses, long long stride, long lon
                    const RowOrder &ro, const int **perm, cudaStream_t st);
 // Whether the blocks of an evaluation take the ligand's atoms longest first (RowOrder).
 bool row_order_pays(long long n, int natlig);
-// Which groups of a launch share candidate lists (CullArgs::supers).
-int cull_supers(int natpro_pad, const bude_launch_cfg &shape, bool sorted);
+// Which groups of a launch in chunks of `chunk` poses share candidate lists (CullArgs::supers).
+int cull_supers(int natpro_pad, const bude_launch_cfg &shape, int chunk, bool sorted);
 
 // Plan of the poses [first[i], first[i] + count[i]) of ligand lig[i]; first ascending.
 CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vector<long long> &first,

@@ -284,7 +284,8 @@ extern "C" int bude_gpu_fasten_noalloc(const bude_atom *protein, int32_t natpro,
   a.rows = ro.rows;
   a.natpro_pad = natpro_pad;
   a.clusters = clusters;
-  a.supers = cull_supers(natpro_pad, cfg, order_poses);
+  const SumsWindow window = sums_window(natlig, nposes, cfg, rest_bytes);
+  a.supers = cull_supers(natpro_pad, cfg, window.chunk, order_poses);
   FinishArgs f{};
   f.energies = energies;
   f.perm = perm;
@@ -299,7 +300,7 @@ extern "C" int bude_gpu_fasten_noalloc(const bude_atom *protein, int32_t natpro,
   f.e.ff = forcefield;
   f.e.xform = a.xform;
   long long launches = 0;
-  rc = cull_range(a, f, cfg, sums_window(natlig, nposes, cfg, rest_bytes), natlig, nposes, st, launches);
+  rc = cull_range(a, f, cfg, window, natlig, nposes, st, launches);
   if (rc) return rc;
   unsigned h = 0;
   rc = na_read_words(words, 1, st, &h);

@@ -15,8 +15,8 @@
 //             giga_interactions/s/gflop/s/gfinst/s/energies/best and the CSV columns
 //             (src/main.cpp:431-476, 550-559); exit status = all results valid
 // Additions: `max_diff_abs_%` (the validator with |ref| in the denominator), `fp32_peak_%` (the
-// reference's per-interaction operation count over the device's FP32 peak) and `-w 0` for the
-// library's automatic launch shape.  Pose counts that are not a multiple of ppwi*wgsize run
+// reference's per-interaction operation count over the device's FP32 peak) and `-w 0` for a
+// block size chosen by the library (any wgsize below 32, the default 1 included).  Pose counts that are not a multiple of ppwi*wgsize run
 // (the kernel handles ragged tails) instead of being skipped.
 #include "bude.h"
 #include "gb300/fasten.hpp"
@@ -131,7 +131,7 @@ void usage() {
             << "  -n --poses   N       Compute energies for only N poses, 0 for the whole deck [default 0]\n"
             << "  -p --ppwi    PPWI    CSV list of poses per work-item, or `all` [default 1; available "
             << joined(kPPWIs) << "]\n"
-            << "  -w --wgsize  WGSIZE  CSV list of work-group sizes, 0 = automatic launch shape [default 1]\n"
+            << "  -w --wgsize  WGSIZE  CSV list of work-group sizes, below 32 = chosen by the library [default 1]\n"
             << "     --deck    DIR     Input deck directory [default `" << DATA_DIR << "`]\n"
             << "  -o --out     PATH    Save energies of the first result to PATH\n"
             << "  -r --rows    N       Show the first N energies of each result [default " << DEFAULT_ENERGY_ENTRIES

@@ -163,7 +163,7 @@ int main(int argc, char **argv) {
       if (!rc) rc = bude_gpu_upload(ctx, protein.atoms.data(), (int32_t)protein.atoms.size(), ligand.atoms.data(),
                                     (int32_t)ligand.atoms.size(), table.data(), (int32_t)table.size(), soa.data(),
                                     (int64_t)nposes, (int64_t)nposes);
-      if (!rc) rc = bude_gpu_default_cfg(ctx, 16, 256, &cfg);
+      if (!rc) rc = bude_gpu_default_cfg(ctx, 0, 0, &cfg);
       if (!rc) rc = bude_gpu_run(ctx, &cfg, nullptr);
       if (!rc) rc = bude_gpu_download(ctx, e.data(), (int64_t)nposes);
       if (ctx) bude_gpu_destroy(ctx);

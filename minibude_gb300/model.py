@@ -284,7 +284,7 @@ class GpuContext:
         """Upload, evaluate once and download: the energies of every pose of `deck`."""
         self.upload(deck)
         if cfg is None:
-            cfg = self.default_cfg(8, 128)
+            cfg = self.default_cfg(0, 0)
         self.run(cfg)
         return self.download()
 

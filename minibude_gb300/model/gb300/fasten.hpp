@@ -9,8 +9,8 @@
 //     energies in pose order;
 //   * errors become std::runtime_error carrying the library's message (as `checkError` does,
 //     src/cuda/fasten.hpp:168-172); `compatible` only reports.
-// PPWI keeps its meaning (poses per thread, register-blocked; 32/64/128 use 16) and wgsize is
-// the block size (values below 32 become the library's default of 128).  Any pose count is
+// PPWI keeps its meaning (poses per thread; 32/64/128 use 16) and wgsize is the block size
+// (multiples of 32 up to 512; values below 32 leave it to the library).  Any pose count is
 // accepted: ragged tails are handled by the kernel.
 #pragma once
 
