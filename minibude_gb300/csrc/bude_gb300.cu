@@ -418,8 +418,8 @@ int upload_deck(Context &c, const bude_atom *protein, int natpro, const bude_ato
   if (rc) return rc;
   rc = upload_ligand(c, ligand, natlig);
   if (!rc) rc = upload_poses(c, poses, stride, nposes);
+  const cudaError_t e = cudaStreamSynchronize(c.stream); // also before an error returns: the copies' host ends
   if (rc) return rc;
-  cudaError_t e = cudaStreamSynchronize(c.stream);
   if (e != cudaSuccess) return cuda_error(e, "deck upload");
   c.have_deck = true;
   return BUDE_OK;
@@ -569,9 +569,9 @@ int bude_gpu_set_poses(bude_gpu_ctx *ctx, const bude_atom *ligand, int32_t natli
                        int64_t pose_stride, int64_t nposes) {
   if (!ctx) return set_error(BUDE_ERR_ARG, "ctx is NULL");
   cudaSetDevice(ctx->device);
-  int rc = bude::set_poses(*ctx, ligand, natlig, poses, pose_stride, nposes);
+  const int rc = bude::set_poses(*ctx, ligand, natlig, poses, pose_stride, nposes);
+  const cudaError_t e = cudaStreamSynchronize(ctx->stream); // also before an error returns: the copies' host ends
   if (rc) return rc;
-  cudaError_t e = cudaStreamSynchronize(ctx->stream);
   return e == cudaSuccess ? BUDE_OK : cuda_error(e, "pose upload");
 }
 
@@ -647,11 +647,14 @@ int bude_gpu_score_host(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, const bud
   cudaSetDevice(ctx->device);
   int rc = bude::set_poses(*ctx, ligand, natlig, poses, pose_stride, nposes);
   if (!rc) rc = bude::enqueue_eval(*ctx, *cfg);
-  if (rc) return rc;
-  if (nposes > 0) {
-    cudaError_t e = cudaMemcpyAsync(energies, ctx->energies.ptr, (size_t)nposes * sizeof(float),
-                                    cudaMemcpyDeviceToHost, ctx->stream);
-    if (e != cudaSuccess) return cuda_error(e, "energy download");
+  if (!rc && nposes > 0) {
+    const cudaError_t e = cudaMemcpyAsync(energies, ctx->energies.ptr, (size_t)nposes * sizeof(float),
+                                          cudaMemcpyDeviceToHost, ctx->stream);
+    if (e != cudaSuccess) rc = cuda_error(e, "energy download");
+  }
+  if (rc) {
+    cudaStreamSynchronize(ctx->stream); // the caller's buffers are its own again
+    return rc;
   }
   return bude::sync_stream(*ctx, "evaluation");
 }
