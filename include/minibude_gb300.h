@@ -104,8 +104,8 @@ int bude_gpu_default_cfg(const bude_gpu_ctx *ctx, int32_t ppwi, int32_t wgsize, 
 /* Choose a launch shape for the uploaded deck by measurement; replaces the reference driver's
  * brute-force PPWI x wgsize sweep (src/main.cpp:517-541).  The shape of bude_gpu_default_cfg and its
  * neighbours are timed with CUDA events (on a ligand prefix where the deck is large), within about
- * max_ms of GPU time.  The pick is cached per deck shape in the context.  best_ms (optional) receives
- * the predicted time of one full evaluation. */
+ * max_ms of GPU time.  The pick is cached in the context until the protein, the forcefield, the ligand or
+ * the number of poses changes.  best_ms (optional) receives the predicted time of one full evaluation. */
 int bude_gpu_autotune(bude_gpu_ctx *ctx, int32_t max_ms, bude_launch_cfg *best, float *best_ms);
 
 /* One evaluation of all uploaded poses (one iteration of the reference's hot loop,

@@ -2,7 +2,8 @@
 //
 // Replaces the reference driver's brute-force PPWI x wgsize sweep (src/main.cpp:517-541) with a rule
 // on the deck's size (cull_shape) and a short measured search around its pick, timed with CUDA events.
-// The pick is cached per deck shape in the context.  A sweep that is asked for runs: default_cfg takes
+// The pick is cached in the context for the protein, forcefield, ligand and pose count that it was timed
+// on: what an evaluation takes goes with the geometry, not with the sizes alone.  A sweep that is asked for runs: default_cfg takes
 // the pair that it is given.
 #include <cuda_runtime.h>
 

@@ -107,6 +107,7 @@ int ensure_slab(Context &c, const bude_atom *protein, int natpro, const bude_ffp
   if (rebuilt) *rebuilt = false;
   if (c.slab.ptr && key == c.slab_key) return BUDE_OK;
   c.slab_key.clear();
+  c.tuned_key[0] = -1;
   c.ntypes = ntypes;
   c.natpro = natpro;
   c.natpro_pad = std::max(round_up(natpro, kClusterAtoms), kClusterAtoms);
@@ -369,6 +370,11 @@ static int upload_ligand(Context &c, const bude_atom *ligand, int natlig) {
   int rc = c.ligand.reserve((size_t)std::max(natlig, 1) * 16, "ligand");
   if (rc) return rc;
   c.deck_irregular = !ligand_regular(c, ligand, natlig, c.host_ff.data());
+  const size_t bytes = (size_t)natlig * sizeof(bude_atom);
+  if (c.host_ligand.size() != (size_t)natlig || (bytes && std::memcmp(c.host_ligand.data(), ligand, bytes))) {
+    c.host_ligand.assign(ligand, ligand + natlig);
+    c.tuned_key[0] = -1;
+  }
   if (natlig > 0) {
     // bude_atom is {x, y, z, int32 type}: the same 16 bytes as the kernel's float4 view.
     cudaError_t e = cudaMemcpyAsync(c.ligand.ptr, ligand, (size_t)natlig * 16, cudaMemcpyHostToDevice, c.stream);

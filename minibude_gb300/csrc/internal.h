@@ -80,6 +80,7 @@ struct Context {
   const bude_atom *raw_protein = nullptr; // as given
   const bude_ffparams *raw_ff = nullptr;
   std::vector<bude_ffparams> host_ff; // the forcefield the slab was built from
+  std::vector<bude_atom> host_ligand; // the uploaded ligand
   bool protein_regular = true;      // every protein atom and its forcefield record within bounds
   float protein_min_radius = 0.f;   // smallest radius of the protein's atom types
   bool deck_irregular = false;      // the uploaded deck (protein + ligand) is scored by edge_pose_kernel
@@ -113,7 +114,8 @@ struct Context {
   Surrogate *surrogate = nullptr; // learned pre-screen (surrogate.cu)
   ScreenState *screen = nullptr;  // last screening run (screen.cu)
   StreamState *streamer = nullptr; // chunked evaluation of host-resident poses (stream.cu)
-  // autotuner cache: the deck shape it was tuned for and the pick
+  // autotuner cache: the sizes it was tuned for and the pick, dropped with the protein, forcefield or ligand
+  // that was timed (ensure_slab, upload_ligand)
   long long tuned_key[3] = {-1, -1, -1};
   bude_launch_cfg tuned{};
   float tuned_ms = 0.f;
