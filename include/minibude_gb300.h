@@ -165,7 +165,8 @@ int bude_gpu_upload_batch(bude_gpu_ctx *ctx, const bude_atom *protein, int32_t n
                           int64_t pose_stride, const int64_t *pose_offsets);
 
 /* Launch shape for the batch (ppwi, wgsize, unroll): a few shapes around the one the batch's size
- * calls for, each timed on the whole batch, within about max_ms.  Cached per batch. */
+ * calls for, each timed on the whole batch, within about max_ms.  Cached until other ligands, pose
+ * counts or another protein are uploaded. */
 int bude_gpu_autotune_batch(bude_gpu_ctx *ctx, int32_t max_ms, bude_launch_cfg *best, float *best_ms);
 
 /* One evaluation of the whole batch, then a stream synchronise.  per_ligand = 0: one launch over all

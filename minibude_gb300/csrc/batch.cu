@@ -31,6 +31,7 @@ void release_batch(Context &c) {
   c.b_edge_mask.release();
   c.b_meta.release();
   c.b_lig_all_host.clear();
+  c.b_atoms_host.clear();
   c.have_batch = false;
   delete c.plan;
   c.plan = nullptr;
@@ -41,12 +42,55 @@ static void drop_graph(Context &c) {
   c.graph = nullptr;
 }
 
+// A plan's blocks in the order of their work, longest first (RowOrder): the weights, one warp per item
+// {atom, row, first pose, poses}, and the ranks, one thread per item; once per plan and set of ligands, 8 us.  24 ligands of 20 to
+// 40 atoms x 256 to 1,024 poses (736 blocks) 179 -> 163 us an evaluation, 64 of 12 to 96 atoms x 1,024 to
+// 16,384 (6,253 blocks) 2,197 -> 2,100.  Every item is compared with every other, so up to 16,384.
+constexpr int kPlanOrderMax = 16384;
+static __global__ void __launch_bounds__(256) item_weight_kernel(const int4 *items, int n, const float4 *ligands,
+                                                                 const float4 *reach, int natpro, int natpro_pad,
+                                                                 float *weight) {
+  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (i >= n) return;
+  const float w = (float)items[i].w * atom_weight(ligands[items[i].x], reach, natpro, natpro_pad);
+  if ((threadIdx.x & 31) == 0) weight[i] = w;
+}
+
+static __global__ void __launch_bounds__(256) item_rank_kernel(const int4 *items, int n, const float *weight,
+                                                               int4 *ranked) {
+  __shared__ float tile[256];
+  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  const float w = i < n ? weight[i] : 0.f;
+  int rank = 0;
+  for (int t = 0; t < n; t += 256) {
+    const int j = t + (int)threadIdx.x;
+    __syncthreads();
+    tile[threadIdx.x] = j < n ? weight[j] : -1.f; // weights are at least 0
+    __syncthreads();
+    for (int k = 0; k < 256; ++k) rank += tile[k] > w || (tile[k] == w && t + k < i);
+  }
+  if (i < n) ranked[rank] = items[i];
+}
+
+// b_items: a ranked plan's items as they are run, as they were cut, their weights.
+static int rank_items(Context &c, int n) {
+  int4 *items = c.b_items.as<int4>(), *given = items + n;
+  float *weight = reinterpret_cast<float *>(items + 2 * n);
+  item_weight_kernel<<<(unsigned)(n + 7) / 8, 256, 0, c.stream>>>(given, n, c.b_ligands, c.reach.as<float4>(), c.natpro,
+                                                                  c.natpro_pad, weight);
+  item_rank_kernel<<<(unsigned)(n + 255) / 256, 256, 0, c.stream>>>(given, n, weight, items);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_error(e, "batch item ranking");
+  c.launches += 2;
+  return BUDE_OK;
+}
+
 int upload_batch(Context &c, const bude_atom *protein, int natpro, const bude_ffparams *ff, int ntypes, int nligands,
                  const bude_atom *atoms, const int32_t *lig_off, const float *poses, long long pose_stride,
                  const int64_t *pose_off) {
   // A batch of the same shape as the uploaded one (same ligand sizes and pose counts, same protein
-  // and forcefield) keeps its work items, captured graph and tuned launch shape: only the atoms and
-  // poses are copied.
+  // and forcefield) keeps its work items and captured graph: only the atoms and poses are copied.  Other
+  // atoms rank the items anew and end the tuned launch shape.
   const bool same_shape = c.have_batch && nligands == c.nligands && lig_off && pose_off &&
                           std::equal(lig_off, lig_off + nligands + 1, c.lig_off.begin()) &&
                           std::equal(pose_off, pose_off + nligands + 1, c.pose_off.begin());
@@ -116,6 +160,15 @@ int upload_batch(Context &c, const bude_atom *protein, int natpro, const bude_ff
   c.b_ligands = reinterpret_cast<const float4 *>(dev + at_atoms);
   c.b_lig_all = dev + at_all;
   c.b_lig_all_host.assign(lig_all, lig_all + nligands);
+  const size_t atom_bytes = (size_t)total_atoms * sizeof(bude_atom);
+  const bool same_atoms = c.b_atoms_host.size() == (size_t)total_atoms &&
+                          (atom_bytes == 0 || std::memcmp(c.b_atoms_host.data(), atoms, atom_bytes) == 0);
+  if (!same_atoms) {
+    c.b_atoms_host.assign(atoms, atoms + total_atoms);
+    c.batch_tuned_key = -1;
+    if (keep && c.graph && c.plan->ranked) rc = rank_items(c, (int)c.plan->items.size());
+    if (rc) return rc;
+  }
   c.have_batch = true;
   ++c.batch_uploads;
   if (keep) return BUDE_OK;
@@ -133,36 +186,6 @@ bude_launch_cfg batch_shape(const Context &c) {
   return cull_shape(std::max(c.batch_poses / nl, 1LL), std::max(c.lig_off[c.nligands] / nl, 1), nl);
 }
 
-// A plan's blocks in the order of their work, longest first (RowOrder): the weights, one warp per item
-// {atom, row, first pose, poses}, and the ranks, one thread per item; once per plan, 8 us.  24 ligands of 20 to
-// 40 atoms x 256 to 1,024 poses (736 blocks) 179 -> 163 us an evaluation, 64 of 12 to 96 atoms x 1,024 to
-// 16,384 (6,253 blocks) 2,197 -> 2,100.  Every item is compared with every other, so up to 16,384.
-constexpr int kPlanOrderMax = 16384;
-static __global__ void __launch_bounds__(256) item_weight_kernel(const int4 *items, int n, const float4 *ligands,
-                                                                 const float4 *reach, int natpro, int natpro_pad,
-                                                                 float *weight) {
-  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (i >= n) return;
-  const float w = (float)items[i].w * atom_weight(ligands[items[i].x], reach, natpro, natpro_pad);
-  if ((threadIdx.x & 31) == 0) weight[i] = w;
-}
-
-static __global__ void __launch_bounds__(256) item_rank_kernel(const int4 *items, int n, const float *weight,
-                                                               int4 *ranked) {
-  __shared__ float tile[256];
-  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const float w = i < n ? weight[i] : 0.f;
-  int rank = 0;
-  for (int t = 0; t < n; t += 256) {
-    const int j = t + (int)threadIdx.x;
-    __syncthreads();
-    tile[threadIdx.x] = j < n ? weight[j] : -1.f; // weights are at least 0
-    __syncthreads();
-    for (int k = 0; k < 256; ++k) rank += tile[k] > w || (tile[k] == w && t + k < i);
-  }
-  if (i < n) ranked[rank] = items[i];
-}
-
 // Plan of the whole batch for a launch shape, on the device (b_items, b_folds, b_sums).
 static int build_plan(Context &c, const bude_launch_cfg &cfg, CullPlan *out) {
   if (c.batch_poses > 0x7fffffffLL) return set_error(BUDE_ERR_ARG, "batch too large for 32-bit pose indices");
@@ -171,24 +194,19 @@ static int build_plan(Context &c, const bude_launch_cfg &cfg, CullPlan *out) {
   std::vector<long long> count((size_t)c.nligands);
   for (int l = 0; l < c.nligands; ++l) count[(size_t)l] = c.pose_off[l + 1] - c.pose_off[l];
   *out = plan_cull(c, lig, c.pose_off, count, cfg);
-  // Not too many blocks: uploaded behind the ranked ones, with the weights behind both.
   const int n = (int)out->items.size();
-  const bool rank = n > 1 && n <= kPlanOrderMax && out->windows.size() == 1;
+  out->ranked = n > 1 && n <= kPlanOrderMax && out->windows.size() == 1;
   int rc = c.b_items.reserve((size_t)std::max(n, 1) * (2 * sizeof(int4) + sizeof(float)), "batch items");
   if (!rc) rc = c.b_folds.reserve(std::max<size_t>(out->folds.size(), 1) * sizeof(int4), "batch items");
   out->sorted = sort_batch(c, cfg.ppwi * cfg.wgsize);
   if (!rc && out->sorted) rc = c.b_order.reserve(batch_order_bytes(c, out->folds.size()), "batch pose order");
   if (!rc) rc = c.b_sums.reserve(std::max<size_t>(out->sums_bytes, 16), "batch atom sums");
   if (rc) return rc;
-  int4 *items = c.b_items.as<int4>(), *given = rank ? items + n : items;
-  cudaError_t e = copy_sync(c, given, out->items.data(), out->items.size() * sizeof(int4), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && rank) {
-    float *weight = reinterpret_cast<float *>(items + 2 * n);
-    item_weight_kernel<<<(unsigned)(n + 7) / 8, 256, 0, c.stream>>>(given, n, c.b_ligands, c.reach.as<float4>(), c.natpro,
-                                                                    c.natpro_pad, weight);
-    item_rank_kernel<<<(unsigned)(n + 255) / 256, 256, 0, c.stream>>>(given, n, weight, items);
-    e = cudaGetLastError();
-  }
+  int4 *items = c.b_items.as<int4>();
+  cudaError_t e = copy_sync(c, out->ranked ? items + n : items, out->items.data(), out->items.size() * sizeof(int4),
+                            cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && out->ranked) rc = rank_items(c, n);
+  if (rc) return rc;
   if (e == cudaSuccess)
     e = copy_sync(c, c.b_folds.ptr, out->folds.data(), out->folds.size() * sizeof(int4), cudaMemcpyHostToDevice);
   return e == cudaSuccess ? BUDE_OK : cuda_error(e, "batch item upload");

@@ -22,6 +22,7 @@ struct CullPlan {
   std::vector<int4> items, folds; // CullArgs::items, FinishArgs::folds
   std::vector<Window> windows;
   bool sorted = false; // the batch's poses are put in order first (sort_batch)
+  bool ranked = false; // the items are in the order of their work, which goes with the batch's atoms
   size_t sums_bytes = 0; // the largest window's
 };
 

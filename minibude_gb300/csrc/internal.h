@@ -102,6 +102,7 @@ struct Context {
   const float4 *b_ligands = nullptr;
   const unsigned char *b_lig_all = nullptr;
   std::vector<unsigned char> b_lig_all_host; // host copy of the lig_all flags
+  std::vector<bude_atom> b_atoms_host;       // and of the ligands' atoms
   CullPlan *plan = nullptr;  // the batch cut for graph_cfg
   cudaGraphExec_t graph = nullptr;
   long long graph_launches = 0; // kernels of one replay

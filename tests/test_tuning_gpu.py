@@ -2,7 +2,7 @@
 protein, ligand or pose count."""
 import pytest
 
-from minibude_gb300.deck import DeckSpec, synthetic_deck
+from minibude_gb300.deck import BatchSpec, DeckSpec, synthetic_batch, synthetic_deck
 from minibude_gb300.model import GpuContext
 
 pytestmark = pytest.mark.gpu
@@ -37,3 +37,31 @@ def test_pick_follows_the_deck(built_library):
         c.set_poses(sparse.poses[:, :4000])
         assert timed(c)[0]
         assert not timed(c)[0]
+
+
+def batch(seed):
+    """Batches of one shape; the seed gives the ligands' atoms."""
+    d = deck(12.0)
+    return synthetic_batch(BatchSpec("tune", 6, 20, 20, 200, 200), d.protein, d.forcefield, seed=seed)
+
+
+def test_kept_batch_plan_follows_the_ligands(built_library):
+    with GpuContext(0) as c, GpuContext(0) as alone:
+        c.upload_batch(batch(1))
+        cfg, ms = c.autotune_batch(200)
+        c.run_batch(cfg)
+        before = c.launch_count()
+        c.upload_batch(batch(1))
+        assert c.launch_count() == before  # nothing to rank anew
+        assert c.autotune_batch(200)[1] == ms and c.launch_count() == before
+        c.run_batch(cfg)
+        before = c.launch_count()
+        c.upload_batch(batch(2))  # the same shape, other atoms
+        assert c.launch_count() == before + 2
+        c.run_batch(cfg)
+        alone.upload_batch(batch(2))
+        alone.run_batch(cfg)
+        assert (c.download_batch() == alone.download_batch()).all()
+        before = c.launch_count()
+        c.autotune_batch(200)
+        assert c.launch_count() > before
