@@ -221,61 +221,9 @@ int enqueue_edge_batch(Context &c, const float *xform, float *energies, unsigned
   return BUDE_OK;
 }
 
-// ---------------------------------------------------------------------------------------------
-// Device buffers
-static int allocate(std::shared_ptr<void> &block, size_t nbytes, const char *what) {
-  void *p = nullptr;
-  const cudaError_t e = cudaMalloc(&p, std::max<size_t>(nbytes, 256));
-  if (e != cudaSuccess) return cuda_error(e, what);
-  block = std::shared_ptr<void>(p, [](void *q) { cudaFree(q); });
-  return BUDE_OK;
-}
-
-int DevBuf::reserve(size_t nbytes, const char *what) {
-  if (nbytes <= cap) return BUDE_OK;
-  release();
-  const int rc = allocate(block, nbytes, what);
-  if (rc) return rc;
-  ptr = block.get();
-  cap = nbytes;
-  return BUDE_OK;
-}
-
-void DevBuf::release() {
-  block.reset();
-  ptr = nullptr;
-  cap = 0;
-}
-
-int reserve_together(std::initializer_list<DevWant> wants, const char *what) {
-  auto room = [](size_t bytes) { return (bytes + 511) / 512 * 512; };
-  size_t total = 0;
-  for (const DevWant &w : wants)
-    if (!w.buf->ptr) total += room(w.bytes);
-  std::shared_ptr<void> block;
-  if (total > 0) {
-    const int rc = allocate(block, total, what);
-    if (rc) return rc;
-  }
-  size_t at = 0;
-  for (const DevWant &w : wants) {
-    if (w.buf->ptr) {
-      const int rc = w.buf->reserve(w.bytes, what);
-      if (rc) return rc;
-      continue;
-    }
-    w.buf->block = block;
-    w.buf->ptr = static_cast<unsigned char *>(block.get()) + at;
-    w.buf->cap = w.bytes;
-    at += room(w.bytes);
-  }
-  return BUDE_OK;
-}
-
 } // namespace bude
 
 using namespace bude;
-
 
 // ---------------------------------------------------------------------------------------------
 // Launch helpers
@@ -396,7 +344,7 @@ static int upload_poses(Context &c, const float *poses, long long stride, long l
                                    {&c.edge_mask, (size_t)(n + 31) / 32 * sizeof(unsigned)},
                                    {&c.order, sort_poses(c, n) ? pose_order_bytes(n) : 0},
                                    {&c.rows, 4096},
-                                   {&c.partial, c.partial.ptr || sums > ((size_t)64 << 20) ? 0 : sums}},
+                                   {&c.partial, sums > ((size_t)64 << 20) ? 0 : sums}},
                                   "poses and energies");
   if (rc) return rc;
   if (nposes > 0) {

@@ -50,8 +50,8 @@ struct DevBuf {
   template <class T> T *as() const { return static_cast<T *>(ptr); }
 };
 
-// Reserve several buffers, those that have none yet as parts of one allocation: an upload into a new
-// context makes one cudaMalloc instead of a dozen.
+// Reserve several buffers as parts of one allocation, all of them anew where one is too small (their
+// contents are lost): an upload into a new context makes one cudaMalloc instead of a dozen.
 struct DevWant {
   DevBuf *buf;
   size_t bytes;

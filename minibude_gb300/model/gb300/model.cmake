@@ -21,7 +21,7 @@ register_flag_optional(GB300_NVCC
         "nvcc")
 
 # The translation units of libbude_gb300.so (minibude_gb300/build.py builds the same list).
-set(GB300_CU_SOURCES bude_gb300 cull autotune batch surrogate screen noalloc stream arch_probe)
+set(GB300_CU_SOURCES bude_gb300 devbuf cull autotune batch surrogate screen noalloc stream arch_probe)
 
 macro(setup)
     set(CMAKE_CXX_STANDARD 17)
