@@ -193,15 +193,20 @@ static int build_plan(Context &c, const bude_launch_cfg &cfg, CullPlan *out) {
   std::iota(lig.begin(), lig.end(), 0);
   std::vector<long long> count((size_t)c.nligands);
   for (int l = 0; l < c.nligands; ++l) count[(size_t)l] = c.pose_off[l + 1] - c.pose_off[l];
-  *out = plan_cull(c, lig, c.pose_off, count, cfg);
+  int rc = reserve_sums(c.b_sums, [&](size_t most) {
+    *out = plan_cull(c, lig, c.pose_off, count, cfg, most);
+    return out->sums_bytes;
+  });
+  if (rc) return rc;
   const int n = (int)out->items.size();
   out->ranked = n > 1 && n <= kPlanOrderMax && out->windows.size() == 1;
-  int rc = c.b_items.reserve((size_t)std::max(n, 1) * (2 * sizeof(int4) + sizeof(float)), "batch items");
+  rc = c.b_items.reserve((size_t)std::max(n, 1) * (out->ranked ? 2 * sizeof(int4) + sizeof(float) : sizeof(int4)),
+                         "batch items");
   if (!rc) rc = c.b_folds.reserve(std::max<size_t>(out->folds.size(), 1) * sizeof(int4), "batch items");
-  out->sorted = sort_batch(c, cfg.ppwi * cfg.wgsize);
-  if (!rc && out->sorted) rc = c.b_order.reserve(batch_order_bytes(c, out->folds.size()), "batch pose order");
-  if (!rc) rc = c.b_sums.reserve(std::max<size_t>(out->sums_bytes, 16), "batch atom sums");
   if (rc) return rc;
+  // In the order given where there is no memory for another: the same energies.
+  out->sorted = sort_batch(c, cfg.ppwi * cfg.wgsize) &&
+                c.b_order.reserve(batch_order_bytes(c, out->folds.size()), "batch pose order") == BUDE_OK;
   int4 *items = c.b_items.as<int4>();
   cudaError_t e = copy_sync(c, out->ranked ? items + n : items, out->items.data(), out->items.size() * sizeof(int4),
                             cudaMemcpyHostToDevice);

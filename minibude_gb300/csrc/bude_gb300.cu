@@ -336,16 +336,22 @@ static int upload_poses(Context &c, const float *poses, long long stride, long l
   if (nposes < 0 || (nposes > 0 && (!poses || stride < nposes)))
     return set_error(BUDE_ERR_ARG, "bad pose block (nposes %lld, stride %lld)", nposes, stride);
   const long long n = std::max(nposes, 1LL);
-  // With the sums that an evaluation of the deck needs, unless they are large.
-  const size_t sums = (size_t)c.natlig * (size_t)n * sizeof(float);
-  const int rc = reserve_together({{&c.poses, (size_t)6 * n * sizeof(float)},
-                                   {&c.xform, (size_t)12 * n * sizeof(float)},
-                                   {&c.energies, (size_t)n * sizeof(float)},
-                                   {&c.edge_mask, (size_t)(n + 31) / 32 * sizeof(unsigned)},
-                                   {&c.order, sort_poses(c, n) ? pose_order_bytes(n) : 0},
-                                   {&c.rows, 4096},
-                                   {&c.partial, sums > ((size_t)64 << 20) ? 0 : sums}},
-                                  "poses and energies");
+  // With the order and the sums that an evaluation of the deck takes, unless those are large; without them
+  // where there is no room (enqueue_poses and launch_exact_range do with less).
+  const size_t all_sums = (size_t)c.natlig * (size_t)n * sizeof(float);
+  const size_t sums = all_sums > ((size_t)64 << 20) ? 0 : all_sums, order = sort_poses(c, n) ? pose_order_bytes(n) : 0;
+  auto reserve = [&](size_t order_bytes, size_t sums_bytes) {
+    return reserve_together({{&c.poses, (size_t)6 * n * sizeof(float)},
+                             {&c.xform, (size_t)12 * n * sizeof(float)},
+                             {&c.energies, (size_t)n * sizeof(float)},
+                             {&c.edge_mask, (size_t)(n + 31) / 32 * sizeof(unsigned)},
+                             {&c.order, order_bytes},
+                             {&c.rows, 4096},
+                             {&c.partial, sums_bytes}},
+                            "poses and energies");
+  };
+  int rc = reserve(order, sums);
+  if (rc) rc = reserve(0, 0);
   if (rc) return rc;
   if (nposes > 0) {
     cudaError_t e = cudaMemcpy2DAsync(c.poses.ptr, (size_t)nposes * sizeof(float), poses, (size_t)stride * sizeof(float),

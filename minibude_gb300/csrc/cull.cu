@@ -234,9 +234,9 @@ int enqueue_poses(Context &c, const float *poses, long long stride, long long n,
   const RowOrder ro{c.ligand.as<float4>(), c.reach.as<float4>(), c.natlig,
                     c.natpro,              c.natpro_pad,         row_order_pays(n, c.natlig) ? c.rows.as<int>() : nullptr,
                     nullptr};
-  if (sort_poses(c, n)) {
-    rc = c.order.reserve(pose_order_bytes(n), "pose order");
-    if (!rc) rc = enqueue_sorted(c.order.ptr, poses, stride, n, rows, mask, ro, perm, c.stream);
+  // In the order given where there is no memory for another: the same energies.
+  if (sort_poses(c, n) && c.order.reserve(pose_order_bytes(n), "pose order") == BUDE_OK) {
+    rc = enqueue_sorted(c.order.ptr, poses, stride, n, rows, mask, ro, perm, c.stream);
     c.launches += rc ? 0 : 3;
     return rc;
   }
@@ -252,8 +252,11 @@ int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *lig
                        const unsigned *mask, const float *xform, float *energies, long long nposes, bool ordered,
                        const int *perm) {
   if (nposes == 0) return BUDE_OK;
-  const SumsWindow w = sums_window(natlig, nposes, cfg, kSumsBytes);
-  const int rc = c.partial.reserve((size_t)w.atoms * w.poses * sizeof(float), "atom sums");
+  SumsWindow w{};
+  const int rc = reserve_sums(c.partial, [&](size_t most) {
+    w = sums_window(natlig, nposes, cfg, most);
+    return (size_t)w.atoms * w.poses * sizeof(float);
+  });
   if (rc) return rc;
   CullArgs a = cull_args(c, cfg, w.chunk, perm != nullptr);
   a.ligand = ligand;
@@ -269,9 +272,9 @@ int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *lig
 }
 
 CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vector<long long> &first,
-                   const std::vector<long long> &count, const bude_launch_cfg &shape) {
+                   const std::vector<long long> &count, const bude_launch_cfg &shape, size_t most) {
   CullPlan plan;
-  const int most = shape.ppwi * shape.wgsize;
+  const int block = shape.ppwi * shape.wgsize;
   struct Chunk {
     int lig, n;
     long long pose;
@@ -306,12 +309,12 @@ CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vec
     w = CullPlan::Window{};
   };
   for (size_t i = 0; i < lig.size(); ++i) {
-    const int per = even_chunk(count[i], most);
+    const int per = even_chunk(count[i], block);
     for (long long p = 0; p < count[i]; p += per) {
       const int n = (int)std::min<long long>(per, count[i] - p);
       const long long at = first[i] + p;
       if (!chunks.empty() &&
-          (size_t)(at + n - w.first) * std::max(w.atoms, natlig(lig[i])) * sizeof(float) > kSumsBytes)
+          (size_t)(at + n - w.first) * std::max(w.atoms, natlig(lig[i])) * sizeof(float) > most)
         close();
       if (chunks.empty()) w.first = at;
       w.n = at + n - w.first;

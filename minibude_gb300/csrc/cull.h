@@ -1,6 +1,7 @@
 // cull.h -- host side of the exact kernel (cull_kernel.cuh): launch shapes, the cut of poses into
 // chunks, and the windows that bound the memory of the atom sums.
 #pragma once
+#include <algorithm>
 #include <vector>
 
 #include "internal.h"
@@ -12,7 +13,7 @@ struct FinishArgs;
 struct RowOrder;
 
 // A batch evaluation's work, cut for one launch shape: block items and finish items in windows of
-// consecutive poses, each window's atom sums at most kSumsBytes.
+// consecutive poses, with a bound on each window's atom sums.
 struct CullPlan {
   struct Window {
     int item0, items, fold0, folds;
@@ -26,7 +27,17 @@ struct CullPlan {
   size_t sums_bytes = 0; // the largest window's
 };
 
-constexpr size_t kSumsBytes = (size_t)1 << 30;
+constexpr size_t kSumsBytes = (size_t)1 << 30, kSumsLeast = (size_t)1 << 20;
+
+// Memory for atom sums: bytes_for(most) cuts the work into windows of at most `most` bytes and returns what
+// the largest takes.  Where the device has no room for it, the windows get smaller; no energy changes.
+template <class F> int reserve_sums(DevBuf &sums, F &&bytes_for) {
+  for (size_t most = kSumsBytes;; most /= 4) {
+    const int rc = sums.reserve(std::max<size_t>(bytes_for(most), 16), "atom sums");
+    if (!rc || most <= kSumsLeast) return rc;
+  }
+}
+
 // Poses of a finish block: with a chunk of 4,096 per block 64 ligands gave 108 blocks (89 us, so 17.5).
 constexpr int kFoldPoses = 256;
 
@@ -56,9 +67,10 @@ bool row_order_pays(long long n, int natlig);
 // Which groups of a launch in chunks of `chunk` poses share candidate lists (CullArgs::supers).
 int cull_supers(int natpro_pad, const bude_launch_cfg &shape, int chunk, bool sorted);
 
-// Plan of the poses [first[i], first[i] + count[i]) of ligand lig[i]; first ascending.
+// Plan of the poses [first[i], first[i] + count[i]) of ligand lig[i]; first ascending.  A window's sums take
+// at most `most` bytes (and room for one chunk of a ligand).
 CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vector<long long> &first,
-                   const std::vector<long long> &count, const bude_launch_cfg &shape);
+                   const std::vector<long long> &count, const bude_launch_cfg &shape, size_t most);
 // Whether evaluating the uploaded batch in chunks of `chunk` poses puts each ligand's poses in order first.
 bool sort_batch(const Context &c, int chunk);
 // Memory of that order for a batch of `poses` poses, and its kernels: the transforms at `xform` and their

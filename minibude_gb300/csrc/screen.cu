@@ -328,11 +328,10 @@ void release_screen(Context &c) {
   c.screen = nullptr;
 }
 
-// Device copies of a plan's items and folds, and room for its group sums.
+// Device copies of a plan's items and folds.
 static int upload_plan(Context &c, ScreenState &s, const CullPlan &plan) {
   int rc = s.items.reserve(std::max<size_t>(plan.items.size(), 1) * sizeof(int4), "screen items");
   if (!rc) rc = s.folds.reserve(std::max<size_t>(plan.folds.size(), 1) * sizeof(int4), "screen items");
-  if (!rc) rc = s.sums.reserve(std::max<size_t>(plan.sums_bytes, 16), "screen atom sums");
   if (rc) return rc;
   cudaError_t e = cudaSuccess; // the plan outlives the copies: every way out of screen_run drains the stream
   if (!plan.items.empty())
@@ -396,29 +395,36 @@ int screen_run(Context &c, const bude_screen_cfg &sc, bude_screen_stats *stats) 
   }
   // One plan for all picks; chunk j's share of it is a plan of its own over the same device arrays.
   std::vector<int> chunk_lig(nchunks + 1, nl);
-  std::vector<CullPlan> chunk_plan((size_t)nchunks);
+  std::vector<CullPlan> chunk_plan;
   CullPlan plan;
-  for (int j = 0; j < nchunks; ++j) {
-    chunk_lig[j] = (int)((long long)nl * j / nchunks);
-    std::vector<int> lig;
-    std::vector<long long> first, cnt;
-    for (int l = chunk_lig[j]; l < (int)((long long)nl * (j + 1) / nchunks); ++l) {
-      const int k = counts[2 * l] + counts[2 * l + 1];
-      if (k == 0) continue;
-      lig.push_back(l);
-      first.push_back(comp_off[l]);
-      cnt.push_back(k);
+  auto cut = [&](size_t most) {
+    plan = CullPlan{};
+    chunk_plan.assign((size_t)nchunks, CullPlan{});
+    for (int j = 0; j < nchunks; ++j) {
+      chunk_lig[j] = (int)((long long)nl * j / nchunks);
+      std::vector<int> lig;
+      std::vector<long long> first, cnt;
+      for (int l = chunk_lig[j]; l < (int)((long long)nl * (j + 1) / nchunks); ++l) {
+        const int k = counts[2 * l] + counts[2 * l + 1];
+        if (k == 0) continue;
+        lig.push_back(l);
+        first.push_back(comp_off[l]);
+        cnt.push_back(k);
+      }
+      CullPlan p = plan_cull(c, lig, first, cnt, small, most);
+      for (CullPlan::Window w : p.windows) {
+        w.item0 += (int)plan.items.size();
+        w.fold0 += (int)plan.folds.size();
+        chunk_plan[j].windows.push_back(w);
+      }
+      plan.items.insert(plan.items.end(), p.items.begin(), p.items.end());
+      plan.folds.insert(plan.folds.end(), p.folds.begin(), p.folds.end());
+      plan.sums_bytes = std::max(plan.sums_bytes, p.sums_bytes);
     }
-    CullPlan p = plan_cull(c, lig, first, cnt, small);
-    for (CullPlan::Window w : p.windows) {
-      w.item0 += (int)plan.items.size();
-      w.fold0 += (int)plan.folds.size();
-      chunk_plan[j].windows.push_back(w);
-    }
-    plan.items.insert(plan.items.end(), p.items.begin(), p.items.end());
-    plan.folds.insert(plan.folds.end(), p.folds.begin(), p.folds.end());
-    plan.sums_bytes = std::max(plan.sums_bytes, p.sums_bytes);
-  }
+    return plan.sums_bytes;
+  };
+  rc = reserve_sums(s.sums, cut);
+  if (rc) return rc;
   if (overlap && !s.side) {
     cudaError_t es = cudaStreamCreateWithFlags(&s.side, cudaStreamNonBlocking);
     if (es != cudaSuccess) return cuda_error(es, "screen rescoring stream");
@@ -488,8 +494,12 @@ int screen_run(Context &c, const bude_screen_cfg &sc, bude_screen_stats *stats) 
       fb_cnt.push_back(c.pose_off[l + 1] - c.pose_off[l]);
     }
   if (!fb_lig.empty()) {
-    const CullPlan fb_plan = plan_cull(c, fb_lig, fb_first, fb_cnt, cfg);
-    rc = upload_plan(c, s, fb_plan);
+    CullPlan fb_plan;
+    rc = reserve_sums(s.sums, [&](size_t most) {
+      fb_plan = plan_cull(c, fb_lig, fb_first, fb_cnt, cfg, most);
+      return fb_plan.sums_bytes;
+    });
+    if (!rc) rc = upload_plan(c, s, fb_plan);
     if (!rc)
       rc = enqueue_plan(c, cfg, fb_plan, s.items.as<int4>(), s.folds.as<int4>(), c.b_xform.as<float>(),
                         c.b_energies.as<float>(), s.sums.as<float>(), false, c.stream);

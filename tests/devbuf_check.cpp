@@ -65,8 +65,11 @@ int main() {
     CHECK(!energies.reserve(64 * last, "alone"));
     CHECK(!bude::reserve_together({{&poses, 25 * last}, {&energies, 4 * last}, {&rows, kOnce}}, "group"));
     CHECK(g_blocks.size() == 1 && energies.cap >= 64 * last);
+    // Where there is no room for that, with what is asked for.
+    g_limit = 50 * last;
+    CHECK(!bude::reserve_together({{&poses, 30 * last}, {&energies, 4 * last}, {&rows, kOnce}}, "group"));
+    CHECK(poses.cap == 30 * last && energies.cap == 4 * last && g_blocks.size() == 1);
     // One that cannot be had leaves no buffer that looks reserved.
-    g_limit = g_held;
     CHECK(bude::reserve_together({{&poses, 50 * last}, {&energies, 4 * last}, {&rows, kOnce}}, "group"));
     CHECK(!poses.ptr && !energies.ptr && !rows.ptr && poses.cap + energies.cap + rows.cap == 0 && g_held == 0);
     g_limit = 1 << 30;
