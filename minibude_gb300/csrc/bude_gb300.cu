@@ -316,7 +316,10 @@ static int upload_ligand(Context &c, const bude_atom *ligand, int natlig) {
       return set_error(BUDE_ERR_TYPE, "ligand atom %d has type %d outside the forcefield (%d types)", i,
                        ligand[i].type, c.ntypes);
   int rc = c.ligand.reserve((size_t)std::max(natlig, 1) * 16, "ligand");
-  if (rc) return rc;
+  if (rc) {
+    c.have_deck = false; // the buffer of the old ligand is gone
+    return rc;
+  }
   c.deck_irregular = !ligand_regular(c, ligand, natlig, c.host_ff.data());
   const size_t bytes = (size_t)natlig * sizeof(bude_atom);
   if (c.host_ligand.size() != (size_t)natlig || (bytes && std::memcmp(c.host_ligand.data(), ligand, bytes))) {
@@ -352,7 +355,10 @@ static int upload_poses(Context &c, const float *poses, long long stride, long l
   };
   int rc = reserve(order, sums);
   if (rc) rc = reserve(0, 0);
-  if (rc) return rc;
+  if (rc) {
+    c.have_deck = false; // the buffers of the old poses are gone
+    return rc;
+  }
   if (nposes > 0) {
     cudaError_t e = cudaMemcpy2DAsync(c.poses.ptr, (size_t)nposes * sizeof(float), poses, (size_t)stride * sizeof(float),
                                       (size_t)nposes * sizeof(float), 6, cudaMemcpyHostToDevice, c.stream);

@@ -4,6 +4,7 @@ a buffer that nothing writes."""
 import numpy as np
 import pytest
 
+from minibude_gb300.capi import BudeError
 from minibude_gb300.deck import BatchDeck, DeckSpec, synthetic_deck, synthetic_ligand, synthetic_poses
 from minibude_gb300.model import GpuContext
 
@@ -72,3 +73,22 @@ def test_deck(built_library):
         finally:
             give_back(held)
     assert np.array_equal(got, want)
+
+
+def test_poses_that_do_not_fit_leave_no_deck(built_library):
+    deck = synthetic_deck(DECK, seed=1)
+    many = np.zeros((6, 4_000_000), np.float32)
+    with GpuContext(0) as c:
+        want = c.energies(deck)
+        cfg = c.default_cfg(0, 0)
+        held = [leave(64 * MB)]  # 76 bytes a pose are asked for
+        try:
+            with pytest.raises(BudeError, match="out of memory"):
+                c.set_poses(many)
+            for call in (lambda: c.run(cfg), lambda: c.set_poses(deck.poses), c.download):
+                with pytest.raises(BudeError, match="no deck"):
+                    call()
+            assert np.array_equal(c.energies(deck), want)
+        finally:
+            give_back(held)
+        assert np.array_equal(c.energies(deck), want)
