@@ -47,7 +47,8 @@ typedef struct bude_ffparams {
  * src/cuda/fasten.hpp:272-275).  Here a block takes ppwi * wgsize poses and one ligand atom, and
  * evaluates the pairs in reach for 32 * unroll poses at a time.  No field changes an energy's bits. */
 typedef struct bude_launch_cfg {
-  int32_t ppwi;    /* poses per thread: 1, 2, 4, 8 or 16 */
+  int32_t ppwi;    /* poses per thread: 1, 2, 4, 8 or 16 (at most 4 of many poses against a protein of up to
+                      64 atoms, all of whose pairs are evaluated) */
   int32_t wgsize;  /* threads per block: a multiple of 32 in [32, 512] */
   int32_t split;   /* 1..8 with cluster = 1, 1..64 with cluster = 0; checked, without effect: the ligand's
                       atoms are what spreads over the GPU, and their sums are added up in order */
@@ -97,7 +98,7 @@ int bude_gpu_set_poses(bude_gpu_ctx *ctx, const bude_atom *ligand, int32_t natli
 /* The launch shape for the reference's (PPWI, wgsize) pair: PPWI poses per thread (the largest of 1, 2,
  * 4, 8 and 16 that it holds: 32/64/128 use 16) and wgsize threads per block (rounded up to a multiple of
  * 32, at most 512).  A ppwi below 1 or a wgsize below 32 leaves that half to the library, which chooses
- * by the uploaded deck's poses and ligand atoms; (0, 0) is its own shape, the fastest here without
+ * by the uploaded deck's atoms and poses; (0, 0) is its own shape, the fastest here without
  * measuring.  Results do not depend on the shape. */
 int bude_gpu_default_cfg(const bude_gpu_ctx *ctx, int32_t ppwi, int32_t wgsize, bude_launch_cfg *cfg);
 
@@ -138,7 +139,7 @@ int bude_gpu_score_host(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, const bud
  * Pinned host buffers (bude_host_alloc) let the copies overlap.  The energies equal those of
  * bude_gpu_run over all poses, bit for bit, for any chunk.  The chunk is rounded up to whole blocks,
  * and to enough of them that a chunk's launch fills the GPU many times over, within 2^19 poses (or
- * four blocks per SM, if those are more).
+ * four blocks per SM, if those are more); against a protein of up to 64 atoms it is at least 2^18 poses.
  * *ms (optional): CUDA-event time of the whole call.  No counterpart in the reference. */
 int bude_gpu_score_stream(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, const float *poses, int64_t pose_stride,
                           int64_t nposes, int64_t chunk, float *energies, float *ms);

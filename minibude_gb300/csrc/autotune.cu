@@ -21,7 +21,7 @@ namespace bude {
 // follows the rule's chunk; both open is the rule.  A small pair is slow (small chunks, loose groups):
 // 938 x 26 x 65,536 86 us an evaluation at 8 x 512, 96 at 8 x 128, 109 at 8 x 64, 235 at 1 x 32.
 int default_cfg(const Context &c, int ppwi, int wgsize, bude_launch_cfg &cfg) {
-  cfg = cull_shape(c.have_deck ? c.nposes : 1LL << 20, c.have_deck ? c.natlig : 32, 1);
+  cfg = c.have_deck ? exact_shape(c, c.nposes, c.natlig, 1) : cull_shape(1LL << 20, 32, 1);
   const int chunk = cfg.ppwi * cfg.wgsize;
   const bool ask_p = ppwi >= 1, ask_w = wgsize >= 32;
   if (!ask_p && !ask_w) return BUDE_OK;

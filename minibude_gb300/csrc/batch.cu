@@ -183,7 +183,7 @@ int upload_batch(Context &c, const bude_atom *protein, int natpro, const bude_ff
 
 bude_launch_cfg batch_shape(const Context &c) {
   const int nl = std::max(c.nligands, 1);
-  return cull_shape(std::max(c.batch_poses / nl, 1LL), std::max(c.lig_off[c.nligands] / nl, 1), nl);
+  return exact_shape(c, std::max(c.batch_poses / nl, 1LL), std::max(c.lig_off[c.nligands] / nl, 1), nl);
 }
 
 // Plan of the whole batch for a launch shape, on the device (b_items, b_folds, b_sums).
@@ -205,7 +205,7 @@ static int build_plan(Context &c, const bude_launch_cfg &cfg, CullPlan *out) {
   if (!rc) rc = c.b_folds.reserve(std::max<size_t>(out->folds.size(), 1) * sizeof(int4), "batch items");
   if (rc) return rc;
   // In the order given where there is no memory for another: the same energies.
-  out->sorted = sort_batch(c, cfg.ppwi * cfg.wgsize) &&
+  out->sorted = !out->direct && sort_batch(c, cfg.ppwi * cfg.wgsize) &&
                 c.b_order.reserve(batch_order_bytes(c, out->folds.size()), "batch pose order") == BUDE_OK;
   int4 *items = c.b_items.as<int4>();
   cudaError_t e = copy_sync(c, out->ranked ? items + n : items, out->items.data(), out->items.size() * sizeof(int4),
@@ -308,7 +308,8 @@ int autotune_batch(Context &c, int max_ms, bude_launch_cfg &best, float *best_ms
   std::vector<bude_launch_cfg> cands{batch_shape(c)};
   for (const bude_launch_cfg &s : {bude_launch_cfg{8, 512, 1, 64, 2, 0}, bude_launch_cfg{4, 512, 1, 64, 2, 0},
                                    bude_launch_cfg{4, 256, 1, 64, 2, 0}, bude_launch_cfg{2, 256, 1, 64, 2, 0},
-                                   bude_launch_cfg{4, 128, 1, 64, 2, 0}, bude_launch_cfg{1, 256, 1, 64, 1, 0}})
+                                   bude_launch_cfg{4, 128, 1, 64, 2, 0}, bude_launch_cfg{2, 128, 1, 64, 2, 0},
+                                   bude_launch_cfg{1, 256, 1, 64, 1, 0}, bude_launch_cfg{1, 128, 1, 64, 1, 0}})
     if (s.ppwi != cands[0].ppwi || s.wgsize != cands[0].wgsize || s.unroll != cands[0].unroll) cands.push_back(s);
   float best_t = 1e30f;
   float spent = 0.f;

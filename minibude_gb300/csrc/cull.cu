@@ -7,6 +7,7 @@
 #include "chain.h"
 #include "cull.h"
 #include "cull_kernel.cuh"
+#include "direct_kernel.cuh"
 #include "pose_order.cuh"
 #include "pose_xform.cuh"
 
@@ -88,6 +89,40 @@ static int finish(const FinishArgs &f, long long grid, cudaStream_t st, long lon
   return BUDE_OK;
 }
 
+// Against a protein of a few dozen atoms nearly every pair is in reach, and many poses leave no SM idle
+// without the ligand's atoms spread over the blocks: then sorting positions, boxes, lists and atom sums cost
+// more than the pairs they leave out.  The line is 64 natpro^2 poses (at least 16,384), where the two were
+// equal or direct_kernel the faster for 1 to 64 ligand atoms, protein at the density of a real one (us culled
+// | direct, 1 and 64 ligand atoms): 8 atoms x 16,384 poses 17 | 12 and 44 | 44, x 524,288 36 | 25 and 565 |
+// 154; 32 atoms x 65,536 21 | 15 and 132 | 141, x 524,288 41 | 30 and 830 | 496; 64 atoms x 131,072 27 | 21
+// and 290 | 361, x 262,144 33 | 27 and 540 | 547, x 524,288 48 | 37 and 1,048 | 953; 96 atoms x 524,288 56 |
+// 44 and 1,288 | 1,408, so not above 64.
+bool direct_pays(const Context &c, long long poses) {
+  return c.natpro > 0 && c.natpro <= 64 && poses >= std::max(16384LL, 64LL * c.natpro * c.natpro);
+}
+
+// As above; ragged ligands leave a tail, so twice the poses: 64 ligands of 12 to 96 atoms, 321,818 poses, 8 |
+// 32 | 64 atoms 292 | 472 | 606 us culled, 112 | 355 | 677 direct; 1,048,576 poses 964 | 1,401 | 1,793 and 253 |
+// 865 | 1,636; 256 of 8 to 32, 36,368 poses, 8 | 32 atoms 32 | 42 and 24 | 59.
+static bool direct_batch_pays(const Context &c, long long poses) { return direct_pays(c, poses / 2); }
+
+static int launch_direct(const Context &c, const FinishArgs &f, const float4 *ligand, long long grid,
+                         const bude_launch_cfg &s, cudaStream_t st, long long &launches) {
+  DirectArgs a{ligand, c.slab.as<float4>(), c.natpro, c.natpro_pad, f};
+  cudaError_t e;
+  switch (s.ppwi) {
+  case 1: e = launch_chained(direct_kernel<1>, (unsigned)grid, (unsigned)s.wgsize, 0, st, a); break;
+  case 2: e = launch_chained(direct_kernel<2>, (unsigned)grid, (unsigned)s.wgsize, 0, st, a); break;
+  default: e = launch_chained(direct_kernel<4>, (unsigned)grid, (unsigned)s.wgsize, 0, st, a); break;
+  }
+  if (e != cudaSuccess) return cuda_error(e, "direct_kernel launch");
+  launches++;
+  return BUDE_OK;
+}
+
+// Poses of a direct_kernel block.
+static int direct_chunk(const bude_launch_cfg &s) { return std::min(s.ppwi, kDirectPoses) * s.wgsize; }
+
 SumsWindow sums_window(int natlig, long long nposes, const bude_launch_cfg &cfg, size_t most) {
   SumsWindow w;
   w.chunk = even_chunk(nposes, cfg.ppwi * cfg.wgsize);
@@ -140,7 +175,7 @@ static double density(const Context &c) {
 
 bool sort_poses(const Context &c, long long nposes) {
   const double near = (double)nposes * c.natlig * density(c);
-  return c.natpro > 0 && nposes >= 4096 && near >= 3300.0 && nposes < (1LL << 31);
+  return c.natpro > 0 && nposes >= 4096 && near >= 3300.0 && nposes < (1LL << 31) && !direct_pays(c, nposes);
 }
 
 // Blocks that all run at once have no last ones: below 100,000 points (one point per thread) there are fewer
@@ -231,8 +266,12 @@ int enqueue_poses(Context &c, const float *poses, long long stride, long long n,
   float4 *rows = reinterpret_cast<float4 *>(xform);
   int rc = c.rows.reserve(kRowOrderMax * sizeof(int), "row order");
   if (rc) return rc;
-  const RowOrder ro{c.ligand.as<float4>(), c.reach.as<float4>(), c.natlig,
-                    c.natpro,              c.natpro_pad,         row_order_pays(n, c.natlig) ? c.rows.as<int>() : nullptr,
+  const RowOrder ro{c.ligand.as<float4>(),
+                    c.reach.as<float4>(),
+                    c.natlig,
+                    c.natpro,
+                    c.natpro_pad,
+                    row_order_pays(n, c.natlig) && !direct_pays(c, n) ? c.rows.as<int>() : nullptr,
                     nullptr};
   // In the order given where there is no memory for another: the same energies.
   if (sort_poses(c, n) && c.order.reserve(pose_order_bytes(n), "pose order") == BUDE_OK) {
@@ -252,6 +291,16 @@ int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *lig
                        const unsigned *mask, const float *xform, float *energies, long long nposes, bool ordered,
                        const int *perm) {
   if (nposes == 0) return BUDE_OK;
+  FinishArgs f{};
+  f.energies = energies;
+  f.perm = perm;
+  f.edges = mask != nullptr;
+  f.e = edge_args_single(c, ligand, natlig, all_irregular, mask, xform);
+  if (!perm && direct_pays(c, nposes)) {
+    f.n = nposes;
+    f.rows = natlig;
+    return launch_direct(c, f, ligand, (nposes + direct_chunk(cfg) - 1) / direct_chunk(cfg), cfg, c.stream, c.launches);
+  }
   SumsWindow w{};
   const int rc = reserve_sums(c.partial, [&](size_t most) {
     w = sums_window(natlig, nposes, cfg, most);
@@ -263,17 +312,23 @@ int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *lig
   a.xform = xform;
   a.sums = c.partial.as<float>();
   if (ordered && row_order_pays(nposes, natlig)) a.rows = c.rows.as<int>();
-  FinishArgs f{};
-  f.energies = energies;
-  f.perm = perm;
-  f.edges = mask != nullptr;
-  f.e = edge_args_single(c, ligand, natlig, all_irregular, mask, xform);
   return cull_range(a, f, cfg, w, natlig, nposes, c.stream, c.launches);
 }
 
 CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vector<long long> &first,
                    const std::vector<long long> &count, const bude_launch_cfg &shape, size_t most) {
   CullPlan plan;
+  plan.direct = direct_batch_pays(c, std::accumulate(count.begin(), count.end(), 0LL));
+  if (plan.direct) {
+    for (size_t i = 0; i < lig.size(); ++i)
+      for_each_item(count[i], 1, direct_chunk(shape), [&](long long p, int n) {
+        plan.folds.push_back(make_int4((int)(first[i] + p), n, c.lig_off[lig[i] + 1] - c.lig_off[lig[i]], lig[i]));
+      });
+    CullPlan::Window w{};
+    w.folds = (int)plan.folds.size();
+    plan.windows.push_back(w);
+    return plan;
+  }
   const int block = shape.ppwi * shape.wgsize;
   struct Chunk {
     int lig, n;
@@ -339,6 +394,14 @@ int enqueue_plan(Context &c, const bude_launch_cfg &shape, const CullPlan &plan,
   f.edges = edges;
   f.last = 1;
   f.e = edge_args_batch(c, xform);
+  if (plan.direct) {
+    int rc = BUDE_OK;
+    for (const CullPlan::Window &w : plan.windows) {
+      f.folds = folds + w.fold0;
+      if (!rc && w.folds > 0) rc = launch_direct(c, f, c.b_ligands, w.folds, shape, st, c.launches);
+    }
+    return rc;
+  }
   for (const CullPlan::Window &w : plan.windows) {
     a.items = items + w.item0;
     a.stride = f.stride = w.n;
@@ -371,6 +434,18 @@ bude_launch_cfg cull_shape(long long n, int natlig, int ligands) {
   s.ppwi = (*shape)[0];
   s.wgsize = (*shape)[1];
   s.unroll = 2;
+  return s;
+}
+
+// Of direct_kernel, one pose per thread where there are few, to have warps enough, four where there are many:
+// 8 | 32 protein atoms x 26 ligand atoms x 32,768 poses 29 | 65 us with one, 29 | 64 with two, 35 | 88 with
+// four; x 131,072 64 | 184, 37 | 94, 40 | 98; x 262,144 80 | 253, 63 | 180, 50 | 132.
+bude_launch_cfg exact_shape(const Context &c, long long n, int natlig, int ligands) {
+  const long long all = n * ligands;
+  if (ligands > 1 ? !direct_batch_pays(c, all) : !direct_pays(c, all)) return cull_shape(n, natlig, ligands);
+  bude_launch_cfg s{all >= 200000 ? 4 : (all >= 32768 ? 2 : 1), 128, 1, 64, 1, 0};
+  while (s.wgsize > 32 && (long long)s.ppwi * s.wgsize > n) s.wgsize /= 2;
+  while (s.ppwi > 1 && (long long)s.ppwi * s.wgsize > n) s.ppwi /= 2;
   return s;
 }
 

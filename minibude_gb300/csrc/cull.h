@@ -22,6 +22,7 @@ struct CullPlan {
   };
   std::vector<int4> items, folds; // CullArgs::items, FinishArgs::folds
   std::vector<Window> windows;
+  bool direct = false; // every pair, finish items of at most ppwi * wgsize poses alone (direct_kernel.cuh)
   bool sorted = false; // the batch's poses are put in order first (sort_batch)
   bool ranked = false; // the items are in the order of their work, which goes with the batch's atoms
   size_t sums_bytes = 0; // the largest window's
@@ -86,8 +87,12 @@ int enqueue_plan(Context &c, const bude_launch_cfg &shape, const CullPlan &plan,
                  const int *perm = nullptr);
 // Shared-memory limit of the shape's kernel (before a stream capture).
 int prepare_shape(const bude_launch_cfg &shape);
-// The launch shape for n poses of a ligand of natlig atoms, `ligands` such ligands at once.
+// Whether an evaluation of `poses` poses in all evaluates every pair (direct_kernel.cuh).
+bool direct_pays(const Context &c, long long poses);
+// The launch shape for n poses of a ligand of natlig atoms, `ligands` such ligands at once; and that for the
+// uploaded protein.
 bude_launch_cfg cull_shape(long long n, int natlig, int ligands);
+bude_launch_cfg exact_shape(const Context &c, long long n, int natlig, int ligands);
 // The same for the uploaded batch (its mean ligand).
 bude_launch_cfg batch_shape(const Context &c);
 

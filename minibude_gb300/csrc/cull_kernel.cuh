@@ -36,6 +36,7 @@
 //     Nothing in that order depends on the other poses, so a pose's energy is the same bits for every
 //     launch shape, chunk, batch or position.
 //
+//   * many poses against a protein of a few dozen atoms go to direct_kernel (direct_kernel.cuh) instead;
 //   * a large pose set comes in the order of its translations (pose_order.cuh), so that a chunk's poses
 //     are near each other and the groups tighter still.
 //
@@ -516,6 +517,17 @@ struct FinishArgs {
   EdgeArgs e;
 };
 
+// The irregular ones of a warp's 32 poses, at the places from w on; this lane's is at energies[q].
+__device__ __forceinline__ void rescore_irregular(const FinishArgs &a, bool irregular, long long w, long long q) {
+  unsigned bits = __ballot_sync(0xffffffffu, irregular);
+  while (bits) {
+    const int b = __ffs(bits) - 1;
+    bits &= bits - 1u;
+    const float e = __shfl_sync(0xffffffffu, edge_energy(a.e, w + b), 0);
+    if ((threadIdx.x & 31) == b) a.energies[q] = e;
+  }
+}
+
 static __global__ void __launch_bounds__(256) cull_finish_kernel(const FinishArgs a) {
   long long p0 = a.first + (long long)blockIdx.x * blockDim.x, p1 = min(p0 + blockDim.x, a.first + a.n);
   int rows = a.rows;
@@ -550,13 +562,7 @@ static __global__ void __launch_bounds__(256) cull_finish_kernel(const FinishArg
       a.energies[q] = a.last ? 0.5f * acc : acc;
       irregular = a.edges && a.last && (all || ((a.e.mask[q >> 5] >> (q & 31)) & 1u));
     }
-    unsigned bits = __ballot_sync(0xffffffffu, irregular);
-    while (bits) {
-      const int b = __ffs(bits) - 1;
-      bits &= bits - 1u;
-      const float e = __shfl_sync(0xffffffffu, edge_energy(a.e, w + b), 0);
-      if ((threadIdx.x & 31) == b) a.energies[q] = e;
-    }
+    rescore_irregular(a, irregular, w, q);
   }
 }
 

@@ -383,7 +383,7 @@ int screen_run(Context &c, const bude_screen_cfg &sc, bude_screen_stats *stats) 
   const bool overlap = nchunks > 1;
   int with_picks = 0;
   for (int l = 0; l < nl; ++l) with_picks += counts[2 * l] + counts[2 * l + 1] > 0;
-  bude_launch_cfg small = cull_shape(with_picks ? ncomp / with_picks : 1,
+  bude_launch_cfg small = exact_shape(c, with_picks ? ncomp / with_picks : 1,
                                      nl ? std::max(c.lig_off[nl] / nl, 1) : 1, std::max(with_picks, 1));
   if (sc.rescore.ppwi != 0) {
     small = bude_launch_cfg{sc.rescore.ppwi, sc.rescore.wgsize, cfg.split, sc.rescore.tile > 0 ? sc.rescore.tile : cfg.tile,
@@ -412,6 +412,7 @@ int screen_run(Context &c, const bude_screen_cfg &sc, bude_screen_stats *stats) 
         cnt.push_back(k);
       }
       CullPlan p = plan_cull(c, lig, first, cnt, small, most);
+      chunk_plan[j].direct = p.direct;
       for (CullPlan::Window w : p.windows) {
         w.item0 += (int)plan.items.size();
         w.fold0 += (int)plan.folds.size();
