@@ -44,8 +44,9 @@ typedef struct bude_ffparams {
 
 /* Kernel launch shape of the exact kernel.  The reference exposes two knobs, PPWI (poses per work
  * item, a template parameter, src/main.cpp:48-53) and wgsize (threads per block,
- * src/cuda/fasten.hpp:272-275).  Here a block takes ppwi * wgsize poses and one ligand atom, and
- * evaluates the pairs in reach for 32 * unroll poses at a time.  No field changes an energy's bits. */
+ * src/cuda/fasten.hpp:272-275).  Here a block takes up to ppwi * wgsize poses and one ligand atom,
+ * and evaluates the pairs in reach for 32 * unroll poses at a time; of a few thousand poses x ligand atoms
+ * or fewer every one gets a warp, in blocks of wgsize threads.  No field changes an energy's bits. */
 typedef struct bude_launch_cfg {
   int32_t ppwi;    /* poses per thread: 1, 2, 4, 8 or 16 (at most 4 of many poses against a protein of up to
                       64 atoms, all of whose pairs are evaluated) */

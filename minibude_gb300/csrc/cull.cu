@@ -72,8 +72,16 @@ int prepare_shape(const bude_launch_cfg &shape) {
   return e == cudaSuccess ? BUDE_OK : cuda_error(e, "launch shape");
 }
 
-static int launch(const CullArgs &a, long long grid, const bude_launch_cfg &s, cudaStream_t st, long long &launches) {
+static int launch(const CullArgs &a, long long grid, const bude_launch_cfg &s, bool points, cudaStream_t st,
+                  long long &launches) {
   if (grid > 0x7fffffffLL) return set_error(BUDE_ERR_ARG, "too many poses for one launch");
+  if (points) {
+    const cudaError_t e =
+        launch_chained(point_kernel, (unsigned)grid, (unsigned)s.wgsize, point_smem_bytes(s.wgsize), st, a);
+    if (e != cudaSuccess) return cuda_error(e, "point_kernel launch");
+    launches++;
+    return BUDE_OK;
+  }
   int rc = prepare_shape(s);
   if (rc) return rc;
   const cudaError_t e = launch_shape(&a, (unsigned)grid, s, st);
@@ -123,9 +131,24 @@ static int launch_direct(const Context &c, const FinishArgs &f, const float4 *li
 // Poses of a direct_kernel block.
 static int direct_chunk(const bude_launch_cfg &s) { return std::min(s.ppwi, kDirectPoses) * s.wgsize; }
 
-SumsWindow sums_window(int natlig, long long nposes, const bude_launch_cfg &cfg, size_t most) {
+constexpr double kFewPoints = 9e4; // cull_shape's first line
+
+// Few points (poses x ligand atoms) get a warp each, point_kernel: the GPU has room for 4,864 warps at once,
+// and groups of 32 would leave most of it idle and, of poses far apart, span the whole protein.  us culled |
+// point_kernel, translations within 3 | 20 A: 4,096 atoms x 26 x 64 46 | 23 and 136 | 22, x 8 x 1,024 38 | 38 and
+// 86 | 35; 938 x 26 x 64 38 | 22 and 44 | 21, x 26 x 256 36 | 34 and 40 | 25; 10,000 x 64 x 64 50 | 33 and 257 |
+// 32.  Past the line the shared boxes of poses near each other win: 4,096 x 8 x 2,048 37 | 57; small proteins
+// reach it sooner: 300 x 26 x 64 26 | 20, x 26 x 256 26 | 30; 100 x 64 x 64 20 | 21, x 26 x 256 20 | 25.
+static bool points_pay(int natpro, long long points) { return points <= std::min(8192LL, 4096LL + 4LL * natpro); }
+
+SumsWindow sums_window(int natpro, int natlig, long long nposes, const bude_launch_cfg &cfg, size_t most) {
   SumsWindow w;
-  w.chunk = even_chunk(nposes, cfg.ppwi * cfg.wgsize);
+  w.points = points_pay(natpro, nposes * natlig);
+  // Of fewer points than cull_shape's first line a block takes at most 256 poses, whatever its shape could take:
+  // more leave SMs idle (8 x 128 938 x 26 x 1,024 94 us with 1,024, 46 with 256).
+  const int block = cfg.ppwi * cfg.wgsize;
+  w.chunk = w.points ? cfg.wgsize / 32
+                     : even_chunk(nposes, (double)nposes * natlig < kFewPoints ? std::min(block, 256) : block);
   const long long floats = std::max((long long)(most / sizeof(float)), (long long)w.chunk);
   w.atoms = (int)std::min<long long>(natlig, floats / w.chunk);
   w.poses = std::min(nposes, floats / std::max(w.atoms, 1) / w.chunk * w.chunk);
@@ -152,7 +175,7 @@ int cull_range(CullArgs a, FinishArgs f, const bude_launch_cfg &cfg, const SumsW
       f.more = l > 0;
       l += f.rows;
       f.last = l >= natlig;
-      int rc = f.rows > 0 ? launch(a, (long long)f.rows * a.chunks, cfg, st, launches) : BUDE_OK;
+      int rc = f.rows > 0 ? launch(a, (long long)f.rows * a.chunks, cfg, w.points, st, launches) : BUDE_OK;
       if (!rc) rc = finish(f, (n + 255) / 256, st, launches);
       if (rc) return rc;
     } while (l < natlig);
@@ -303,7 +326,7 @@ int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *lig
   }
   SumsWindow w{};
   const int rc = reserve_sums(c.partial, [&](size_t most) {
-    w = sums_window(natlig, nposes, cfg, most);
+    w = sums_window(c.natpro, natlig, nposes, cfg, most);
     return (size_t)w.atoms * w.poses * sizeof(float);
   });
   if (rc) return rc;
@@ -329,7 +352,10 @@ CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vec
     plan.windows.push_back(w);
     return plan;
   }
-  const int block = shape.ppwi * shape.wgsize;
+  long long points = 0;
+  for (size_t i = 0; i < lig.size(); ++i) points += count[i] * (c.lig_off[lig[i] + 1] - c.lig_off[lig[i]]);
+  plan.points = points_pay(c.natpro, points);
+  const int block = plan.points ? shape.wgsize / 32 : shape.ppwi * shape.wgsize;
   struct Chunk {
     int lig, n;
     long long pose;
@@ -364,7 +390,7 @@ CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vec
     w = CullPlan::Window{};
   };
   for (size_t i = 0; i < lig.size(); ++i) {
-    const int per = even_chunk(count[i], block);
+    const int per = plan.points ? block : even_chunk(count[i], block);
     for (long long p = 0; p < count[i]; p += per) {
       const int n = (int)std::min<long long>(per, count[i] - p);
       const long long at = first[i] + p;
@@ -406,7 +432,7 @@ int enqueue_plan(Context &c, const bude_launch_cfg &shape, const CullPlan &plan,
     a.items = items + w.item0;
     a.stride = f.stride = w.n;
     a.first = f.first = w.first;
-    int rc = w.items > 0 ? launch(a, w.items, shape, st, c.launches) : BUDE_OK;
+    int rc = w.items > 0 ? launch(a, w.items, shape, plan.points, st, c.launches) : BUDE_OK;
     f.folds = folds + w.fold0;
     if (!rc && w.folds > 0) rc = finish(f, w.folds, st, c.launches);
     if (rc) return rc;
@@ -426,7 +452,7 @@ int enqueue_plan(Context &c, const bude_launch_cfg &shape, const CullPlan &plan,
 bude_launch_cfg cull_shape(long long n, int natlig, int ligands) {
   const double points = (double)n * natlig * ligands;
   bude_launch_cfg s{1, n <= 64 ? 64 : (n <= 128 ? 128 : 256), 1, 64, 1, 0};
-  if (points < 9e4) return s;
+  if (points < kFewPoints) return s;
   const int many[][2] = {{8, 512}, {4, 512}, {4, 256}, {4, 128}, {2, 128}}, few[][2] = {{2, 512}, {2, 256}, {2, 128}};
   const int(*shape)[2] = points < 9e5 ? few : (points < 3.8e6 ? many + 1 : many);
   const int(*last)[2] = points < 9e5 ? few + 2 : many + 4;

@@ -23,6 +23,7 @@ struct CullPlan {
   std::vector<int4> items, folds; // CullArgs::items, FinishArgs::folds
   std::vector<Window> windows;
   bool direct = false; // every pair, finish items of at most ppwi * wgsize poses alone (direct_kernel.cuh)
+  bool points = false; // items of at most one pose per warp (point_kernel)
   bool sorted = false; // the batch's poses are put in order first (sort_batch)
   bool ranked = false; // the items are in the order of their work, which goes with the batch's atoms
   size_t sums_bytes = 0; // the largest window's
@@ -55,8 +56,9 @@ inline int even_chunk(long long n, int most) {
 struct SumsWindow {
   int chunk, atoms;
   long long poses;
+  bool points; // of point_kernel
 };
-SumsWindow sums_window(int natlig, long long nposes, const bude_launch_cfg &cfg, size_t most);
+SumsWindow sums_window(int natpro, int natlig, long long nposes, const bude_launch_cfg &cfg, size_t most);
 int cull_range(CullArgs a, FinishArgs f, const bude_launch_cfg &cfg, const SumsWindow &w, int natlig, long long nposes,
                cudaStream_t st, long long &launches);
 // The transforms of n poses in the order of their translations, and that order, with pose_order_bytes(n) of

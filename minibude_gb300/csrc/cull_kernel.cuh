@@ -500,6 +500,44 @@ template <int K, int P> __global__ void __launch_bounds__(kMaxThreads, 2) cull_k
   }
 }
 
+// A warp for every point, all of whose lanes hold it: its own box, as tight as any.  For so few points that each
+// has a warp of its own (points_pay, cull.cu), where latency is all: 64 poses of 938 x 26 16 -> 8 us of kernel.
+inline size_t point_smem_bytes(int threads) { return (size_t)(threads / 32) * sizeof(WarpList); }
+
+static __global__ void __launch_bounds__(kMaxThreads, 2) point_kernel(const CullArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  WarpList &list = reinterpret_cast<WarpList *>(smem)[warp];
+  grid_dep_wait();
+  int atom, row, n;
+  long long pose0;
+  if (a.items) {
+    const int4 it = __ldg(&a.items[blockIdx.x]);
+    atom = it.x, row = it.y, pose0 = it.z, n = it.w;
+  } else {
+    row = (int)(blockIdx.x / (unsigned)a.chunks);
+    atom = row + a.atom0;
+    pose0 = (long long)(blockIdx.x % (unsigned)a.chunks) * a.chunk;
+    n = (int)min((long long)a.chunk, a.nposes - pose0);
+  }
+  if (a.words && deck_bad_type(a.words)) return;
+  const float4 la = __ldg(&a.ligand[atom]);
+  const float4 *xf = reinterpret_cast<const float4 *>(a.xform) + pose0 * 3;
+  float *out = a.sums + (long long)row * a.stride + (pose0 - a.first);
+  for (int i = warp; i < n; i += warps) {
+    const float4 r0 = __ldg(xf + i * 3), r1 = __ldg(xf + i * 3 + 1), r2 = __ldg(xf + i * 3 + 2);
+    const float4 p = make_float4(r0.w + la.x * r0.x + la.y * r0.y + la.z * r0.z,
+                                 r1.w + la.x * r1.x + la.y * r1.y + la.z * r1.z,
+                                 r2.w + la.x * r2.x + la.y * r2.y + la.z * r2.z, 0.f); // as in cull_kernel
+    Points<1> pt;
+    pt.set(0, p);
+    pt.clear();
+    const float3 at = make_float3(p.x, p.y, p.z);
+    cull_eval<1>(pt, at, at, __float_as_int(la.w), nullptr, -1, list, a);
+    if ((threadIdx.x & 31) == 0) out[i] = pt.energy(0);
+  }
+}
+
 // energies[p] = 0.5 * the sum over pose p's ligand atoms in order (no atoms: 0), for the poses
 // [first, first + n) of one ligand, or, with folds, for {first pose, poses, rows, ligand} per block.
 // With `edges` the irregular poses among them (every pose of an irregular deck or ligand) then get the

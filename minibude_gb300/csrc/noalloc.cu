@@ -284,7 +284,7 @@ extern "C" int bude_gpu_fasten_noalloc(const bude_atom *protein, int32_t natpro,
   a.rows = ro.rows;
   a.natpro_pad = natpro_pad;
   a.clusters = clusters;
-  const SumsWindow window = sums_window(natlig, nposes, cfg, rest_bytes);
+  const SumsWindow window = sums_window(natpro, natlig, nposes, cfg, rest_bytes);
   a.supers = cull_supers(natpro_pad, cfg, window.chunk, order_poses);
   FinishArgs f{};
   f.energies = energies;

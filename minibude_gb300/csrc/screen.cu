@@ -413,6 +413,7 @@ int screen_run(Context &c, const bude_screen_cfg &sc, bude_screen_stats *stats) 
       }
       CullPlan p = plan_cull(c, lig, first, cnt, small, most);
       chunk_plan[j].direct = p.direct;
+      chunk_plan[j].points = p.points;
       for (CullPlan::Window w : p.windows) {
         w.item0 += (int)plan.items.size();
         w.fold0 += (int)plan.folds.size();
