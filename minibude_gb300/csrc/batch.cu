@@ -308,8 +308,7 @@ int autotune_batch(Context &c, int max_ms, bude_launch_cfg &best, float *best_ms
   std::vector<bude_launch_cfg> cands{batch_shape(c)};
   for (const bude_launch_cfg &s : {bude_launch_cfg{8, 512, 1, 64, 2, 0}, bude_launch_cfg{4, 512, 1, 64, 2, 0},
                                    bude_launch_cfg{4, 256, 1, 64, 2, 0}, bude_launch_cfg{2, 256, 1, 64, 2, 0},
-                                   bude_launch_cfg{4, 128, 1, 64, 2, 0}, bude_launch_cfg{2, 128, 1, 64, 2, 0},
-                                   bude_launch_cfg{1, 256, 1, 64, 1, 0}, bude_launch_cfg{1, 128, 1, 64, 1, 0}})
+                                   bude_launch_cfg{4, 128, 1, 64, 2, 0}, bude_launch_cfg{1, 256, 1, 64, 1, 0}})
     if (s.ppwi != cands[0].ppwi || s.wgsize != cands[0].wgsize || s.unroll != cands[0].unroll) cands.push_back(s);
   float best_t = 1e30f;
   float spent = 0.f;
