@@ -826,7 +826,8 @@ int surrogate_prepare(Context &c, bool xform_ready) {
       s.item_lig_off.push_back((int)items.size());
     }
     s.n_items = (int)items.size();
-    items.insert(items.end(), items.begin(), items.begin() + s.n_items);
+    items.resize(2 * (size_t)s.n_items);
+    std::copy_n(items.begin(), s.n_items, items.begin() + s.n_items);
     std::stable_sort(items.begin() + s.n_items, items.end(), [](const int4 &x, const int4 &y) { return x.y > y.y; });
     rc = s.items.reserve(std::max<size_t>(items.size(), 1) * sizeof(int4), "surrogate items");
     if (rc) return rc;
