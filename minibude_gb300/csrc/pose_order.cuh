@@ -24,6 +24,19 @@ namespace bude {
 constexpr int kOrderThreads = 512;
 constexpr int kOrderBoxes = 128; // blocks of the box kernel, at most
 
+// Cell of a translation in the 8 x 8 x 8 grid over the box from `lo` on with `s` cells per Angstrom, in Hilbert
+// order.  Translations that are not regular go to a cell by the pose's index: their poses are irregular and
+// are scored one after the other by the warp that finds them (cull_finish_kernel), so they have to stay as
+// spread as they came.  One in ten of 65,536 poses against 938 x 26 not a number: 5.3 ms with all in one cell,
+// 1.9 so.
+__device__ __forceinline__ int order_cell(float3 t, float3 lo, float3 s, long long pose) {
+  if (!(fabsf(t.x) + fabsf(t.y) + fabsf(t.z) < kPoseReach)) return (int)(pose % kBins);
+  const int x = min(max((int)((t.x - lo.x) * s.x), 0), 7), y = min(max((int)((t.y - lo.y) * s.y), 0), 7),
+            z = min(max((int)((t.z - lo.z) * s.z), 0), 7);
+  return kHilbert.at[z * 64 + y * 8 + x];
+}
+__device__ __forceinline__ float order_scale(float lo, float hi) { return hi > lo ? 8.f / (hi - lo) : 0.f; }
+
 // Scratch of a sort of n poses in `tiles` tiles.
 struct PoseOrder {
   int *perm;     // [n] pose of each place
@@ -84,15 +97,12 @@ static __global__ void __launch_bounds__(kOrderThreads) pose_cell_kernel(const f
     if (lane == 0) box[warp] = m;
   }
   __syncthreads();
-  float s[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) s[d] = box[3 + d] > box[d] ? 8.f / (box[3 + d] - box[d]) : 0.f;
+  const float3 lo = make_float3(box[0], box[1], box[2]);
+  const float3 s = make_float3(order_scale(box[0], box[3]), order_scale(box[1], box[4]), order_scale(box[2], box[5]));
   const long long first = (long long)blockIdx.x * o.tile, last = min(first + o.tile, n);
   for (long long i = first + tid; i < last; i += kOrderThreads) {
-    int q[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) q[d] = min(max((int)((poses[(3 + d) * pstride + i] - box[d]) * s[d]), 0), 7);
-    const int cell = kHilbert.at[q[2] * 64 + q[1] * 8 + q[0]] >> shift;
+    const float3 t = make_float3(poses[3 * pstride + i], poses[4 * pstride + i], poses[5 * pstride + i]);
+    const int cell = order_cell(t, lo, s, i) >> shift;
     o.key[i] = (unsigned)cell << 16 | (unsigned)atomicAdd(&bins[cell], 1);
   }
   __syncthreads();
@@ -199,13 +209,10 @@ static __global__ void __launch_bounds__(256) batch_cell_kernel(const BatchOrder
   __syncthreads();
   if (tid < t.y) {
     const long long i = (long long)t.x + tid;
-    int q[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const float lo = o.boxes[t.w * 6 + d], hi = o.boxes[t.w * 6 + 3 + d];
-      q[d] = min(max((int)((o.xform[3 * i + d].w - lo) * (hi > lo ? 8.f / (hi - lo) : 0.f)), 0), 7);
-    }
-    const int cell = kHilbert.at[q[2] * 64 + q[1] * 8 + q[0]] >> 3;
+    const float *b = o.boxes + t.w * 6;
+    const float3 at = make_float3(o.xform[3 * i].w, o.xform[3 * i + 1].w, o.xform[3 * i + 2].w);
+    const float3 s = make_float3(order_scale(b[0], b[3]), order_scale(b[1], b[4]), order_scale(b[2], b[5]));
+    const int cell = order_cell(at, make_float3(b[0], b[1], b[2]), s, i) >> 3;
     o.key[i] = (unsigned)cell << 16 | (unsigned)atomicAdd(&bins[cell], 1);
   }
   __syncthreads();
