@@ -269,11 +269,15 @@ int enqueue_batch_order(Context &c, const CullPlan &plan, const int4 *tiles, con
   o.sorted = static_cast<float4 *>(scratch);
   o.perm = reinterpret_cast<int *>(o.sorted + 3 * c.batch_poses);
   o.key = reinterpret_cast<unsigned *>(o.perm + c.batch_poses);
-  o.boxes = reinterpret_cast<float *>(o.key + c.batch_poses);
+  o.boxes = o.key + c.batch_poses;
   o.count = reinterpret_cast<int *>(o.boxes + 6 * (size_t)c.nligands);
   o.base = o.count + kBatchCells * (size_t)c.nligands;
   const unsigned n = (unsigned)plan.folds.size();
-  cudaError_t e = launch_chained(batch_box_kernel, (unsigned)c.nligands, (unsigned)kOrderThreads, 0, c.stream, o);
+  cudaError_t e = cudaMemsetAsync(o.boxes, 0, (6 + kBatchCells) * sizeof(int) * (size_t)c.nligands, c.stream);
+  if (e == cudaSuccess) {
+    batch_box_kernel<<<n, 256, 0, c.stream>>>(o);
+    e = cudaGetLastError();
+  }
   if (e == cudaSuccess) e = launch_chained(batch_cell_kernel, n, 256u, 0, c.stream, o);
   if (e == cudaSuccess) e = launch_chained(batch_place_kernel, n, 256u, 0, c.stream, o);
   if (e != cudaSuccess) return cuda_error(e, "batch pose order launch");
