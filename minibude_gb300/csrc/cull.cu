@@ -189,7 +189,10 @@ int cull_range(CullArgs a, FinishArgs f, const bude_launch_cfg &cfg, const SumsW
 // box (widened by the reach) = 3,300, where the two were equal or the sorted faster (6 to 96 ligand atoms;
 // us plain, then sorted / plain): 400 atoms at 0.05 per cubic Angstrom 500k points 100, 0.98, 1.2M 167, 0.95;
 // 1,237 300k 90, 0.91, 900k 176, 0.86; 3,500 220k 77, 0.89, 900k 151, 0.84; 3,500 at 0.015 400k 55, 1.00,
-// 740k 82, 0.94.  Fewer than 4,096 poses are a few chunks.
+// 740k 82, 0.94.  Fewer than 4,096 poses are a few chunks.  And per pose the sort takes what it takes, so a
+// ligand of few atoms does not pay for it, however many the poses: the second line is ligand atoms x density
+// = 0.011 (2,000,000 poses, us plain | sorted: 65 x 1 atoms 0.002 134 | 199, 65 x 4 0.008 339 | 386, 100 x 4 0.0106
+// 432 | 467, 400 x 2 0.0116 437 | 421, 100 x 8 0.021 762 | 757, 938 x 2 0.017 543 | 475).
 static double density(const Context &c) {
   double volume = 1.0;
   for (int d = 0; d < 3; ++d) volume *= (double)c.reach_hi[d] - c.reach_lo[d];
@@ -197,8 +200,9 @@ static double density(const Context &c) {
 }
 
 bool sort_poses(const Context &c, long long nposes) {
-  const double near = (double)nposes * c.natlig * density(c);
-  return c.natpro > 0 && nposes >= 4096 && near >= 3300.0 && nposes < (1LL << 31) && !direct_pays(c, nposes);
+  const double near = c.natlig * density(c); // of a pose
+  return c.natpro > 0 && nposes >= 4096 && nposes * near >= 3300.0 && near >= 0.011 && nposes < (1LL << 31) &&
+         !direct_pays(c, nposes);
 }
 
 // Blocks that all run at once have no last ones: below 100,000 points (one point per thread) there are fewer
@@ -246,13 +250,18 @@ int enqueue_sorted(void *scratch, const float *poses, long long stride, long lon
 // As sort_poses, for the ligands of more than a chunk, with four launches instead of one: 64 ligands of 12
 // to 96 atoms x 1,024 to 16,384 poses 2,217 us plain, 2,167 sorted, 256 x 4,096 to 65,536 16.83 and 15.02 ms.
 // Ligands of a chunk or less gain nothing (24 of 20 to 40 atoms x 256 to 1,024 stay plain, 177 us).
+// Its second line is 0.03 for the mean ligand of them (2,000,000 poses of one ligand, plain | sorted: 2,672 x 2
+// atoms 0.026 441 | 525, 200 x 8 0.032 1,022 | 1,064, 938 x 4 0.035 696 | 720, 400 x 8 0.046 1,273 | 1,224; 524,288
+// poses, 938 x 4 220 | 208).
 bool sort_batch(const Context &c, int chunk) {
-  double points = 0;
+  double points = 0, poses = 0;
   for (int l = 0; l < c.nligands; ++l) {
     const long long n = c.pose_off[l + 1] - c.pose_off[l];
-    if (n > chunk) points += (double)n * (c.lig_off[l + 1] - c.lig_off[l]);
+    if (n <= chunk) continue;
+    points += (double)n * (c.lig_off[l + 1] - c.lig_off[l]);
+    poses += (double)n;
   }
-  return c.natpro > 0 && points * density(c) >= 10000.0;
+  return c.natpro > 0 && points * density(c) >= 10000.0 && points * density(c) >= 0.03 * poses;
 }
 
 size_t batch_order_bytes(const Context &c, size_t tiles) {
