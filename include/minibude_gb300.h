@@ -48,8 +48,8 @@ typedef struct bude_ffparams {
  * and evaluates the pairs in reach for 32 * unroll poses at a time; of a few thousand poses x ligand atoms
  * or fewer every one gets a warp, in blocks of wgsize threads.  No field changes an energy's bits. */
 typedef struct bude_launch_cfg {
-  int32_t ppwi;    /* poses per thread: 1, 2, 4, 8 or 16 (at most 4 of many poses against a protein of up to
-                      64 atoms, all of whose pairs are evaluated) */
+  int32_t ppwi;    /* poses per thread: 1, 2, 4, 8 or 16 (at most 4 of many poses against a protein of a few
+                      dozen atoms, all of whose pairs are evaluated) */
   int32_t wgsize;  /* threads per block: a multiple of 32 in [32, 512] */
   int32_t split;   /* 1..8 with cluster = 1, 1..64 with cluster = 0; checked, without effect: the ligand's
                       atoms are what spreads over the GPU, and their sums are added up in order */
@@ -140,7 +140,7 @@ int bude_gpu_score_host(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, const bud
  * Pinned host buffers (bude_host_alloc) let the copies overlap.  The energies equal those of
  * bude_gpu_run over all poses, bit for bit, for any chunk.  The chunk is rounded up to whole blocks,
  * and to enough of them that a chunk's launch fills the GPU many times over, within 2^19 poses (or
- * four blocks per SM, if those are more); against a protein of up to 64 atoms it is at least 2^18 poses.
+ * four blocks per SM, if those are more); against a protein of a few dozen atoms it is at least 2^18 poses.
  * *ms (optional): CUDA-event time of the whole call.  No counterpart in the reference. */
 int bude_gpu_score_stream(bude_gpu_ctx *ctx, const bude_launch_cfg *cfg, const float *poses, int64_t pose_stride,
                           int64_t nposes, int64_t chunk, float *energies, float *ms);

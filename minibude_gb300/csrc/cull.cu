@@ -103,16 +103,20 @@ static int finish(const FinishArgs &f, long long grid, cudaStream_t st, long lon
 // equal or direct_kernel the faster for 1 to 64 ligand atoms, protein at the density of a real one (us culled
 // | direct, 1 and 64 ligand atoms): 8 atoms x 16,384 poses 17 | 12 and 44 | 44, x 524,288 36 | 25 and 565 |
 // 154; 32 atoms x 65,536 21 | 15 and 132 | 141, x 524,288 41 | 30 and 830 | 496; 64 atoms x 131,072 27 | 21
-// and 290 | 361, x 262,144 33 | 27 and 540 | 547, x 524,288 48 | 37 and 1,048 | 953; 96 atoms x 524,288 56 |
-// 44 and 1,288 | 1,408, so not above 64.
-bool direct_pays(const Context &c, long long poses) {
-  return c.natpro > 0 && c.natpro <= 64 && poses >= std::max(16384LL, 64LL * c.natpro * c.natpro);
+// and 290 | 361, x 262,144 33 | 27 and 540 | 547, x 524,288 48 | 37 and 1,048 | 953.  Above 64 atoms it takes
+// ligands of few atoms, for which the culled path's launches weigh more (x 524,288, 1, 8 and 64 ligand atoms:
+// 96 atoms 56 | 44, 208 | 198 and 1,288 | 1,408; 128 atoms 65 | 52, 229 | 255 and 1,415 | 1,864).
+bool direct_pays(const Context &c, long long natlig, long long poses) {
+  const long long most = 64 + std::min(64LL, 256 / std::max(natlig, 1LL));
+  return c.natpro > 0 && c.natpro <= most && poses >= std::max(16384LL, 64LL * c.natpro * c.natpro);
 }
 
 // As above; ragged ligands leave a tail, so twice the poses: 64 ligands of 12 to 96 atoms, 321,818 poses, 8 |
 // 32 | 64 atoms 292 | 472 | 606 us culled, 112 | 355 | 677 direct; 1,048,576 poses 964 | 1,401 | 1,793 and 253 |
 // 865 | 1,636; 256 of 8 to 32, 36,368 poses, 8 | 32 atoms 32 | 42 and 24 | 59.
-static bool direct_batch_pays(const Context &c, long long poses) { return direct_pays(c, poses / 2); }
+static bool direct_batch_pays(const Context &c, long long mean_natlig, long long poses) {
+  return direct_pays(c, mean_natlig, poses / 2);
+}
 
 static int launch_direct(const Context &c, const FinishArgs &f, const float4 *ligand, long long grid,
                          const bude_launch_cfg &s, cudaStream_t st, long long &launches) {
@@ -202,7 +206,7 @@ static double density(const Context &c) {
 bool sort_poses(const Context &c, long long nposes) {
   const double near = c.natlig * density(c); // of a pose
   return c.natpro > 0 && nposes >= 4096 && nposes * near >= 3300.0 && near >= 0.011 && nposes < (1LL << 31) &&
-         !direct_pays(c, nposes);
+         !direct_pays(c, c.natlig, nposes);
 }
 
 // Blocks that all run at once have no last ones: below 100,000 points (one point per thread) there are fewer
@@ -307,7 +311,7 @@ int enqueue_poses(Context &c, const float *poses, long long stride, long long n,
                     c.natlig,
                     c.natpro,
                     c.natpro_pad,
-                    row_order_pays(n, c.natlig) && !direct_pays(c, n) ? c.rows.as<int>() : nullptr,
+                    row_order_pays(n, c.natlig) && !direct_pays(c, c.natlig, n) ? c.rows.as<int>() : nullptr,
                     nullptr};
   // In the order given where there is no memory for another: the same energies.
   if (sort_poses(c, n) && c.order.reserve(pose_order_bytes(n), "pose order") == BUDE_OK) {
@@ -332,7 +336,7 @@ int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *lig
   f.perm = perm;
   f.edges = mask != nullptr;
   f.e = edge_args_single(c, ligand, natlig, all_irregular, mask, xform);
-  if (!perm && direct_pays(c, nposes)) {
+  if (!perm && direct_pays(c, natlig, nposes)) {
     f.n = nposes;
     f.rows = natlig;
     return launch_direct(c, f, ligand, (nposes + direct_chunk(cfg) - 1) / direct_chunk(cfg), cfg, c.stream, c.launches);
@@ -354,7 +358,12 @@ int launch_exact_range(Context &c, const bude_launch_cfg &cfg, const float4 *lig
 CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vector<long long> &first,
                    const std::vector<long long> &count, const bude_launch_cfg &shape, size_t most) {
   CullPlan plan;
-  plan.direct = direct_batch_pays(c, std::accumulate(count.begin(), count.end(), 0LL));
+  long long points = 0, poses = 0;
+  for (size_t i = 0; i < lig.size(); ++i) {
+    points += count[i] * (c.lig_off[lig[i] + 1] - c.lig_off[lig[i]]);
+    poses += count[i];
+  }
+  plan.direct = direct_batch_pays(c, points / std::max(poses, 1LL), poses);
   if (plan.direct) {
     for (size_t i = 0; i < lig.size(); ++i)
       for_each_item(count[i], 1, direct_chunk(shape), [&](long long p, int n) {
@@ -365,8 +374,6 @@ CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vec
     plan.windows.push_back(w);
     return plan;
   }
-  long long points = 0;
-  for (size_t i = 0; i < lig.size(); ++i) points += count[i] * (c.lig_off[lig[i] + 1] - c.lig_off[lig[i]]);
   plan.points = points_pay(c.natpro, points);
   const int block = plan.points ? shape.wgsize / 32 : shape.ppwi * shape.wgsize;
   struct Chunk {
@@ -481,7 +488,8 @@ bude_launch_cfg cull_shape(long long n, int natlig, int ligands) {
 // four; x 131,072 64 | 184, 37 | 94, 40 | 98; x 262,144 80 | 253, 63 | 180, 50 | 132.
 bude_launch_cfg exact_shape(const Context &c, long long n, int natlig, int ligands) {
   const long long all = n * ligands;
-  if (ligands > 1 ? !direct_batch_pays(c, all) : !direct_pays(c, all)) return cull_shape(n, natlig, ligands);
+  if (ligands > 1 ? !direct_batch_pays(c, natlig, all) : !direct_pays(c, natlig, all))
+    return cull_shape(n, natlig, ligands);
   bude_launch_cfg s{all >= 200000 ? 4 : (all >= 32768 ? 2 : 1), 128, 1, 64, 1, 0};
   while (s.wgsize > 32 && (long long)s.ppwi * s.wgsize > n) s.wgsize /= 2;
   while (s.ppwi > 1 && (long long)s.ppwi * s.wgsize > n) s.ppwi /= 2;

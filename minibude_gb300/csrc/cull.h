@@ -89,8 +89,8 @@ int enqueue_plan(Context &c, const bude_launch_cfg &shape, const CullPlan &plan,
                  const int *perm = nullptr);
 // Shared-memory limit of the shape's kernel (before a stream capture).
 int prepare_shape(const bude_launch_cfg &shape);
-// Whether an evaluation of `poses` poses in all evaluates every pair (direct_kernel.cuh).
-bool direct_pays(const Context &c, long long poses);
+// Whether an evaluation of `poses` poses of a ligand of natlig atoms evaluates every pair (direct_kernel.cuh).
+bool direct_pays(const Context &c, long long natlig, long long poses);
 // The launch shape for n poses of a ligand of natlig atoms, `ligands` such ligands at once; and that for the
 // uploaded protein.
 bude_launch_cfg cull_shape(long long n, int natlig, int ligands);

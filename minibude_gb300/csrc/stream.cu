@@ -87,7 +87,7 @@ static int score_stream(Context &c, const bude_launch_cfg &cfg, const float *pos
   // A set whose every pair is evaluated: in even chunks of at least 2^18, as direct_kernel has its blocks over
   // poses alone.  32 x 48 x 1,500,000 in chunks of 65,536 | 133,335 | 200,002 | 400,003 2,953 | 1,697 | 1,281 |
   // 1,217 us; 8 x 8 282 | 282 | 270 | 256.
-  if (direct_pays(c, nposes)) {
+  if (direct_pays(c, c.natlig, nposes)) {
     const long long n = std::max(1LL, nposes / std::max(chunk, 1LL << 18));
     chunk = (nposes + n - 1) / n;
   }

@@ -1,6 +1,6 @@
 """Many poses against a protein of a few dozen atoms have every pair evaluated (csrc/direct_kernel.cuh).  The
-energies are the bits of the culled kernel, which takes the same poses in pieces of fewer than 16,384 and
-any protein above 64 atoms; the oracle bounds both.  Sizes lie on both sides of the rule's line."""
+energies are the bits of the culled kernel, which takes the same poses in pieces of fewer than 16,384; the
+oracle bounds both.  Sizes lie on both sides of the rule's line (64 atoms, up to 128 for ligands of few)."""
 import numpy as np
 import pytest
 
@@ -54,7 +54,8 @@ def synthetic_like(deck, n):
 @pytest.mark.parametrize("natpro,natlig,nposes,half_box", [
     (1, 1, 16384, None), (1, 3, 16383, None), (8, 5, 20001, 1.0), (15, 2, 16384, None), (16, 26, 16385, None),
     (31, 4, 64 * 31 * 31, None), (32, 0, 70000, None), (32, 2, 65535, None), (32, 33, 65536, 2.0), (33, 1, 70001, None),
-    (64, 3, 262143, None), (64, 2, 262144, 3.0), (65, 2, 300000, None)])
+    (64, 3, 262143, None), (64, 2, 262144, 3.0), (65, 2, 300000, None), (128, 1, 1 << 20, None), (128, 4, 1 << 20, None),
+    (96, 8, 589823, None), (96, 8, 589824, None), (96, 9, 589824, None)])
 def test_sizes_around_the_line(ctx, natpro, natlig, nposes, half_box):
     deck = deck_of(natpro, natlig, nposes, half_box, seed=natpro)
     ctx.upload(deck)

@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("natpro,natlig,nposes,sorts", [(400, 8, 131072, True), (400, 8, 65536, False),
-                                                        (100, 3, 1_500_000, False), (400, 2, 300_000, True)])
+                                                        (140, 2, 1_500_000, False), (400, 2, 300_000, True)])
 def test_deck_and_batch(built_library, natpro, natlig, nposes, sorts):
     box = 0.5 * (natpro / 0.05) ** (1 / 3)
     deck = synthetic_deck(DeckSpec("order", natpro, box, natlig, 34, 64), seed=1)
