@@ -4,7 +4,7 @@
 //
 // The reference scores one ligand per run of its driver (src/main.cpp); a virtual screen runs it
 // once per ligand.  Here the batch shares the protein's tables and the pose-transform pass, and one
-// launch takes the (ligand, pose chunk, atom group) items of all ligands, longest ligands first.
+// launch takes the (ligand, pose chunk, atom) items of all ligands, longest first.
 #include <cuda_runtime.h>
 
 #include <algorithm>

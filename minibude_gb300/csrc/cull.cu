@@ -13,7 +13,9 @@
 
 namespace bude {
 
-constexpr size_t kCullMaxSmem = 200 * 1024; // 16 poses per thread x 512 threads: 185 KB
+// 16 poses per thread x 512 threads: 161, 171 or 191 KiB with lists; with one pose per lane and lists of four
+// groups it would be 231, so those go without.
+constexpr size_t kCullMaxSmem = 200 * 1024;
 
 // Lists of candidates serve four groups, or the eight tighter ones of sorted poses (4,096 x 64 x 1,048,576
 // 2,603 us with four, 2,519 with eight; 64 unsorted ligands 2,664 and 2,703).  A chunk of 256 poses has too

@@ -36,7 +36,8 @@
 //     Nothing in that order depends on the other poses, so a pose's energy is the same bits for every
 //     launch shape, chunk, batch or position.
 //
-//   * many poses against a protein of a few dozen atoms go to direct_kernel (direct_kernel.cuh) instead;
+//   * few points get a warp each (point_kernel), and many poses against a protein of a few dozen atoms every
+//     pair (direct_kernel.cuh); both give the same bits;
 //   * a large pose set comes in the order of its translations (pose_order.cuh), so that a chunk's poses
 //     are near each other and the groups tighter still.
 //

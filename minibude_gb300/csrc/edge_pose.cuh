@@ -9,7 +9,7 @@
 // these bounds, which are checked once per pose and once per deck:
 //
 //   regular pose   its transform is finite (sin/cos of finite angles) and every translation
-//                  component satisfies |t| < 2^38 A                    (pose_xform_kernel)
+//                  component satisfies |t| < 2^38 A                    (pose_regular)
 //   regular deck   every protein coordinate |p| <= 2^37 A, every ligand atom |x|+|y|+|z| <= 2^36 A,
 //                  every forcefield radius, hphb and elsc in use finite with magnitude <= 2^20,
 //                  and every FP32 radius sum radius_L + radius_P >= 2^-20     (host or device check)
@@ -17,12 +17,13 @@
 // Inside them every ligand-protein distance is below 2^39 A (no overflow, nothing non-finite) and
 // the padding records at 1e15 A stay out of reach, so the saturating form equals the reference's
 // piecewise terms.  Everything else -- the irregular poses (one bit each in a mask written by the
-// transform pass), or every pose of an irregular deck or ligand -- is rescored afterwards by
-// edge_pose_kernel: one warp per pose, the reference's pair set-up and interaction body in FP32
-// over the raw protein and forcefield records, lanes striding over protein atoms, and a fixed-order
-// warp reduction.  It overwrites those poses' energies, so NaN and infinity come out where the
-// reference's serial model gives them.  Regular decks of regular poses (every deck the reference
-// ships) never take this path; it costs one launch that reads the mask.
+// transform pass), or every pose of an irregular deck or ligand -- is rescored afterwards (edge_energy):
+// one warp per pose, the reference's pair set-up and interaction body in FP32 over the raw protein and
+// forcefield records, lanes striding over protein atoms, and a fixed-order warp reduction.  That
+// overwrites those poses' energies, so NaN and infinity come out where the reference's serial model
+// gives them.  The kernel that writes the energies does it (cull_finish_kernel, direct_kernel), a warp's
+// poses one after the other; edge_pose_kernel does it for a screen's final list and for a batch evaluated
+// ligand by ligand.  Regular decks of regular poses (every deck the reference ships) only read the mask.
 #pragma once
 #include <algorithm>
 #include <cmath>
@@ -115,7 +116,7 @@ __device__ __forceinline__ bool deck_irregular(const unsigned *words, int natpro
 }
 
 struct EdgeArgs {
-  const unsigned *mask;         // bit (p & 31) of word p >> 5: pose p is irregular (pose_xform_kernel)
+  const unsigned *mask;         // bit (p & 31) of word p >> 5: pose p is irregular (pose_regular)
   int all;                      // 1: every pose is rescored (the deck is irregular)
   long long nposes;
   // Batches: pose_off / lig_off (nlig + 1 entries, device) give each ligand's poses and atoms;

@@ -83,7 +83,7 @@ struct Context {
   std::vector<bude_atom> host_ligand; // the uploaded ligand
   bool protein_regular = true;      // every protein atom and its forcefield record within bounds
   float protein_min_radius = 0.f;   // smallest radius of the protein's atom types
-  bool deck_irregular = false;      // the uploaded deck (protein + ligand) is scored by edge_pose_kernel
+  bool deck_irregular = false;      // every pose of the uploaded deck (protein + ligand) is rescored by edge_energy
   int flush_gen = 0;
   long long launches = 0;
   // batch of ligands (bude_gpu_upload_batch); shares the protein slab with the deck fields above
@@ -95,7 +95,7 @@ struct Context {
   DevBuf b_poses, b_xform, b_energies;
   DevBuf b_items, b_folds, b_sums, b_order; // the device half of `plan` and its atom sums (graph-owned)
   // Irregular poses of the batch: transform-pass bits, device pose/atom offsets, and the ligands
-  // whose every pose goes to edge_pose_kernel (lig_all flags and their count, both on the device).
+  // whose every pose goes to edge_energy (lig_all flags and their count, both on the device).
   DevBuf b_edge_mask, b_meta; // b_meta: [pose_off | lig_any | lig_off | atoms | lig_all], one copy per upload
   const long long *b_pose_off = nullptr;
   const int *b_lig_any = nullptr, *b_lig_off = nullptr;

@@ -23,7 +23,7 @@ constexpr int kHbtypeE = 69;      // 'E' (src/bude.h:32)
 constexpr float kCnstnt = 45.0f; // src/bude.h:28
 constexpr float kNpNpDist = 5.5f; // src/bude.h:34
 constexpr float kNpPDist = 1.0f;  // src/bude.h:35
-constexpr int kRecFloats = 16;    // floats per record (exact_shape.h: kRecF4 * 4)
+constexpr int kRecFloats = 16;    // floats of a pair_record, of which the kernels' 48-byte records keep ten (deck_tables.cuh)
 
 // rec[0..15] = {px, px, py, py, pz, pz, k_chrg, k_chrg, k_dslv, k_dslv, -1/radij, -1/elcdst,
 //               1 + radij/elcdst, -1/distdslv, 1 + radij/distdslv, 0}

@@ -68,8 +68,8 @@ __device__ __forceinline__ void row_order(const RowOrder &o) {
 
 // Pose transforms: src/cuda/fasten.hpp:45-71 / serial/fasten.hpp:28-53, one thread per pose.
 // Output: three float4 rows per pose (pose_rows).
-// With edge_mask, bit (i & 31) of word i >> 5 is set when pose i is irregular (edge_pose.cuh), so
-// edge_pose_kernel rescores it afterwards; blockDim must be a multiple of 32.  With ro.rows one more block
+// With edge_mask, bit (i & 31) of word i >> 5 is set when pose i is irregular and is rescored afterwards
+// (edge_pose.cuh); blockDim must be a multiple of 32.  With ro.rows one more block
 // than the poses take, for row_order.
 // (Internal linkage, so several translation units may include this file.)
 static __global__ void __launch_bounds__(256) pose_xform_kernel(const float *__restrict__ poses, long long pstride,

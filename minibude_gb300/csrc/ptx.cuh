@@ -132,13 +132,6 @@ __device__ __forceinline__ bool mbar_wait_sleep_bounded(uint64_t *bar, uint32_t 
   return false;
 }
 
-// 16-byte read-only global load that the compiler may not hoist out of a loop.
-__device__ __forceinline__ float4 ldg_stream(const float4 *p) {
-  float4 v;
-  asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-  return v;
-}
-
 // 1-D TMA bulk copy global -> this CTA's shared memory, completing on `bar` by transaction bytes.
 // dst and src must be 16-byte aligned and bytes a multiple of 16.
 __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
