@@ -78,11 +78,14 @@ static int score_stream(Context &c, const bude_launch_cfg &cfg, const float *pos
   int rc = check_cfg(c, cfg);
   if (rc) return rc;
   // Whole blocks of poses (one per ligand atom and ppwi * wgsize poses), and enough of them that the tail of
-  // a chunk's launch is short beside it: sixteen per SM where 2^19 poses hold as many, at least four.  Four |
-  // eight | sixteen, us: 2,672 x 48 x 400,003 in chunks of 65,536 2,538 | 2,229 | 1,980, of 16,384 2,847 |
-  // 2,303 | 2,080; 1,200 x 20 x 300,000 890 | 814 | 726; 3,500 x 14 x 250,000 624 | 506 | 506.
+  // a chunk's launch is short beside it: as many poses as sixteen blocks of 4,096 per SM take, within 2^19,
+  // and at least four blocks per SM.  Four | eight | sixteen, us: 2,672 x 48 x 400,003 in chunks of 65,536
+  // 2,538 | 2,229 | 1,980, of 16,384 2,847 | 2,303 | 2,080; 1,200 x 20 x 300,000 890 | 814 | 726; 3,500 x 14
+  // x 250,000 624 | 506 | 506.  Blocks of fewer poses take as many poses, for the sort: 2,672 x 48 x 400,003
+  // at 8 x 128 in sixteen blocks per SM (65,536 poses) 2,298, in 208,896 poses 2,055.
   const long long ppb = (long long)cfg.ppwi * cfg.wgsize, sms = std::max(c.num_sms, 1), atoms = std::max(c.natlig, 1);
-  const long long fill = std::max(4 * sms / atoms + 1, std::min(16 * sms / atoms + 1, (1LL << 19) / ppb));
+  const long long poses16 = std::min((16 * sms / atoms + 1) * 4096, 1LL << 19);
+  const long long fill = std::max(4 * sms / atoms + 1, poses16 / ppb);
   chunk = std::max((chunk + ppb - 1) / ppb, fill) * ppb;
   // A set whose every pair is evaluated: in even chunks of at least 2^18, as direct_kernel has its blocks over
   // poses alone.  32 x 48 x 1,500,000 in chunks of 65,536 | 133,335 | 200,002 | 400,003 2,953 | 1,697 | 1,281 |
