@@ -44,14 +44,15 @@
 // What bounds it: instruction issue (75% of the slots on the 4,096 x 64 deck), 60 to 75% of the time the
 // record loop (35 instructions per record and 64 points, 23 of them the pair arithmetic), the rest the
 // sort, the boxes and the candidate lists.  Measured, all pairs evaluated (records broadcast to 16 poses
-// per thread, TMA-staged) | this kernel, end to end from pinned host memory: 4,096 x 64 x 1,048,576 101.5 |
-// 2.46 ms, 938 x 26 x 65,536 0.750 | 0.128 ms, 938 x 26 x 64 201 | 47 us, 2,672 x 48 x 400,003 streamed
-// 21.2 | 1.63 ms; 64 ligands of 12-96 atoms x 1,024-16,384 poses against 2,672 atoms 67.0 | 2.10 ms.  What
+// per thread, TMA-staged) | this kernel, end to end from pinned host memory, over several GPUs: 4,096 x 64 x
+// 1,048,576 101.5 | 2.5-2.8 ms, 938 x 26 x 65,536 0.750 | 0.124-0.133 ms, 2,672 x 48 x 400,003 streamed 21.2 |
+// 1.5-1.8 ms; 64 ligands of 12-96 atoms x 1,024-16,384 poses against 2,672 atoms 67.0 | 2.1-2.3 ms.  What
 // went into it, on 4,096 x 64 x 262,144 unsorted poses: records read through L1 one by one 1,140 us (and 64
 // poses took 105 us for 41); 64-byte records with the packed instructions' operands twice, 1,250; 48 bytes
 // 1,100 (the loads' register writes bound two points per lane); lists of 64 records 1,095, of 128 in stages
 // of 10 1,067; no shared candidate lists 1,218.  One ligand atom per block instead of two, binned over the
-// box of its own positions (no registers spill any more): the 4,096 x 64 x 1,048,576 deck 4.52 -> 3.30 ms;
+// box of its own positions (no registers spill any more but 112 to 176 bytes with 16 poses per thread and 16
+// with four per lane): the 4,096 x 64 x 1,048,576 deck 4.52 -> 3.30 ms;
 // poses sorted 3.64 -> 3.01.
 #pragma once
 #include <cstdint>

@@ -5,9 +5,10 @@
 // pose's sums (protein in cluster order, then the ligand's atoms) and so the bits of its energy are those of
 // cull_kernel and cull_finish_kernel: a pair out of reach adds +0.
 //
-// What bounds it: the FMA pipe (12 cycles per warp and pair, Points::add), of whose rate it reaches 0.7 at
-// four poses per thread, 64 x 64 atoms and 524,288 poses (2.3e12 pairs/s); at one pose per thread issue, half
-// of it.  8 | 32 | 64 protein atoms x 64 ligand atoms x 524,288 poses 153 | 496 | 953 us, culled 565 | 830 | 1,048.
+// What bounds it: the FMA pipe (12 cycles per warp and pair, Points::add), 67% busy at four poses per thread,
+// 64 x 64 atoms and 524,288 poses (2.3e12 pairs/s); one pose per thread takes up to 2.4 times as long, for the
+// records' loads.  8 | 32 | 64 protein atoms x 64 ligand atoms x 524,288 poses 153 | 496 | 953 us, culled 565 | 830 |
+// 1,048.
 #pragma once
 #include "cull_kernel.cuh"
 

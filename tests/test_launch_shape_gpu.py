@@ -4,8 +4,9 @@ library's choice.  No shape changes an energy."""
 import numpy as np
 import pytest
 
+from minibude_gb300.capi import BudeError
 from minibude_gb300.deck import DeckSpec, synthetic_deck
-from minibude_gb300.model import Gb300Bude, GpuContext
+from minibude_gb300.model import Gb300Bude, GpuContext, launch_cfg
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +53,17 @@ def test_model_without_a_deck_and_with_few_poses(built_library):
     want = Gb300Bude(1).fasten(few, 1, 0, 1, 0).energies
     for ppwi, wgsize in ((1, 32), (16, 512), (8, 64), (64, 0)):
         assert np.array_equal(Gb300Bude(ppwi).fasten(few, wgsize, 0, 1, 0).energies, want)
+
+
+@pytest.mark.parametrize("split,tile,cluster", [(1, 8, 0), (64, 512, 0), (1, 64, 1), (8, 128, 1), (5, 24, 1)])
+def test_split_tile_and_cluster_are_checked_and_change_no_bit(ctx, split, tile, cluster):
+    own = ctx.energies(DECK)
+    before = ctx.launch_count()
+    ctx.run(launch_cfg(4, 128, 1, 64, 2, 0))
+    launches = ctx.launch_count() - before
+    ctx.run(launch_cfg(4, 128, split, tile, 2, cluster))
+    assert ctx.launch_count() - before == 2 * launches
+    assert np.array_equal(ctx.download(), own)
+    for bad in ((65, 64, 0), (9, 64, 1), (0, 64, 0), (1, 4, 0), (1, 520, 0), (1, 12, 0), (1, 64, 2)):
+        with pytest.raises(BudeError):
+            ctx.run(launch_cfg(4, 128, bad[0], bad[1], 2, bad[2]))
