@@ -377,7 +377,7 @@ CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vec
     return plan;
   }
   plan.points = points_pay(c.natpro, points);
-  const int block = plan.points ? shape.wgsize / 32 : shape.ppwi * shape.wgsize;
+  const int block = shape.wgsize / 32; // of point_kernel
   struct Chunk {
     int lig, n;
     long long pose;
@@ -389,10 +389,14 @@ CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vec
     if (chunks.empty()) return;
     w.item0 = (int)plan.items.size();
     w.fold0 = (int)plan.folds.size();
-    for (const Chunk &k : chunks)
-      for_each_item(k.n, 1, kFoldPoses, [&](long long p, int n) {
-        plan.folds.push_back(make_int4((int)(k.pose + p), n, natlig(k.lig), k.lig));
+    for (size_t i = 0, j = 0; i < chunks.size(); i = j) {
+      long long n = 0; // of the chunks that one cut into folds takes: a ligand's small ones together
+      do n += chunks[j++].n;
+      while (plan.points && j < chunks.size() && chunks[j].lig == chunks[i].lig);
+      for_each_item(n, 1, kFoldPoses, [&](long long p, int m) {
+        plan.folds.push_back(make_int4((int)(chunks[i].pose + p), m, natlig(chunks[i].lig), chunks[i].lig));
       });
+    }
     // Longest ligands first; the chunks of one ligand and atom next to each other (they read the same
     // records).
     std::stable_sort(chunks.begin(), chunks.end(),
@@ -412,7 +416,7 @@ CullPlan plan_cull(const Context &c, const std::vector<int> &lig, const std::vec
     w = CullPlan::Window{};
   };
   for (size_t i = 0; i < lig.size(); ++i) {
-    const int per = plan.points ? block : even_chunk(count[i], block);
+    const int per = plan.points && natlig(lig[i]) > 0 ? block : even_chunk(count[i], shape.ppwi * shape.wgsize);
     for (long long p = 0; p < count[i]; p += per) {
       const int n = (int)std::min<long long>(per, count[i] - p);
       const long long at = first[i] + p;

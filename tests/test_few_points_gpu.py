@@ -111,3 +111,21 @@ def test_batches(ctx):
     for l in (0, 3, 5):
         d = dataclasses.replace(deck, ligand=ligands[l], poses=poses[l])
         assert np.array_equal(run(ctx, d, 2, 64), got[0][off[l]:off[l + 1]], equal_nan=True), l
+
+
+def test_many_poses_without_atoms_beside_few_points(ctx):
+    rng = np.random.default_rng(4)
+    deck = deck_of(700, 1, 64)
+    ligands = [synthetic_ligand(rng, n, 5.0, 12) for n in (0, 6, 0, 2)]
+    poses = [synthetic_poses(rng, n) for n in (400000, 300, 1, 513)]
+    batch = BatchDeck(deck.protein, deck.forcefield, ligands, poses, "none")
+    off = batch.pose_offsets()
+    ctx.upload_batch(batch)
+    for p, w in ((1, 32), (4, 128)):
+        ctx.run_batch(launch_cfg(p, w, 1, 64, 1))
+        got = ctx.download_batch()
+        assert not got[:off[1]].any() and not got[off[2]:off[3]].any()
+        for l in (1, 3):
+            d = dataclasses.replace(deck, ligand=ligands[l], poses=poses[l])
+            assert np.array_equal(run(ctx, d, 2, 64), got[off[l]:off[l + 1]]), (p, w, l)
+        ctx.upload_batch(batch)
